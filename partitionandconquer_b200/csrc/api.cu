@@ -381,6 +381,89 @@ pc_status ensure_dplus(pc_pgraph* pg) {
     return PC_OK;
 }
 
+// ooff[u] = vectors of row u in the oriented copy, for the exclusive sum.
+__global__ void k_oriented_count(const uint32_t* __restrict__ dplus, uint64_t n, uint32_t* __restrict__ ooff) {
+    const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (u <= n) ooff[u] = u < n ? (dplus[u] + 3) / 4 : 0u;
+}
+
+// Fills the oriented copy, a vector per thread; the work is split by vectors,
+// so a long row is spread over many warps: each warp takes 256 consecutive
+// vectors and its lanes search their rows between those of the first and the
+// last.  One read of the oriented half of the adjacency and one write; built
+// once per view (0.3 ms at RMAT-24, against 43 ms for one count).
+__global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                                const uint32_t* __restrict__ dplus, uint64_t n, const uint32_t* __restrict__ ooff,
+                                int4* __restrict__ ids) {
+    constexpr uint64_t kRun = 256;
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t nvec = ooff[n];
+    const int4 none = make_int4(INT32_MAX, INT32_MAX, INT32_MAX, INT32_MAX);
+    if (warp == 0) ids[nvec + lane] = none;
+    auto row = [&](uint64_t lo, uint64_t hi, uint64_t j) {  // largest r in [lo, hi] with ooff[r] <= j
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi + 1) >> 1;
+            if (ooff[mid] <= j) lo = mid; else hi = mid - 1;
+        }
+        return lo;
+    };
+    for (uint64_t c0 = warp * kRun; c0 < nvec; c0 += nwarps * kRun) {
+        const uint64_t c1 = min(c0 + kRun, nvec);
+        uint64_t r = 0;
+        if (lane < 2) r = row(0, n - 1, lane == 0 ? c0 : c1 - 1);
+        const uint64_t r0 = __shfl_sync(0xffffffffu, r, 0), r1 = __shfl_sync(0xffffffffu, r, 1);
+        for (uint64_t j = c0 + lane; j < c1; j += 32) {
+            const uint64_t u = row(r0, r1, j);
+            const uint32_t k = 4 * (uint32_t)(j - ooff[u]), left = dplus[u] - k;
+            const int32_t* src = adj + off[u] + k;
+            int4 v = none;
+            v.x = src[0];
+            if (left > 1) v.y = src[1];
+            if (left > 2) v.z = src[2];
+            if (left > 3) v.w = src[3];
+            ids[j] = v;
+        }
+    }
+}
+
+pc_status ensure_oriented(pc_pgraph* pg) {
+    PC_TRY(ensure_dplus(pg));
+    if (pg->oriented_tried) return PC_OK;
+    const uint64_t n = pg->g->n;
+    pg->oriented_tried = true;
+    if (n == 0 || (pg->g->m + 3 * n) / 4 + 32 >= (1ull << 32)) return PC_OK;
+    if (pg->ooff.alloc((n + 1) * 4, "oriented offsets") != PC_OK) {
+        clear_error();
+        return PC_OK;
+    }
+    cudaStream_t s = pg->g->stream;
+    uint32_t* ooff = pg->ooff.as<uint32_t>();
+    size_t tb = 0;
+    PC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, ooff, ooff, (int64_t)(n + 1), s));
+    PC_TRY(scratch_reserve(pg, tb + 256));
+    void* tmp = pg->scratch.take<char>(std::max<size_t>(tb, 1));
+    k_oriented_count<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(pg->dplus.as<uint32_t>(), n, ooff);
+    PC_LAUNCHED();
+    PC_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, ooff, ooff, (int64_t)(n + 1), s));
+    count_launch();
+    uint32_t nvec = 0;
+    PC_CUDA(cudaMemcpyAsync(&nvec, ooff + n, 4, cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaStreamSynchronize(s));
+    if (pg->oids.alloc(((uint64_t)nvec + 32) * 16, "oriented ids") != PC_OK) {
+        pg->ooff.release();
+        clear_error();
+        return PC_OK;
+    }
+    pg->ovecs = nvec;
+    const uint64_t grid = std::min<uint64_t>((uint64_t)sm_count(pg->g->device) * 16, ceil_div(nvec, 8 * 256));
+    k_oriented_fill<<<(unsigned)std::max<uint64_t>(1, grid), 256, 0, s>>>(pg->off, pg->adj, pg->dplus.as<uint32_t>(), n,
+                                                                          ooff, pg->oids.as<int4>());
+    PC_LAUNCHED();
+    return PC_OK;
+}
+
 }  // namespace pc
 
 using namespace pc;

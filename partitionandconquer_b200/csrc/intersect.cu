@@ -15,6 +15,7 @@
 
 #include "pc_internal.cuh"
 #include "selector.cuh"
+#include "tc_kernels.cuh"
 
 namespace pc {
 namespace ix {
@@ -31,11 +32,10 @@ __device__ __forceinline__ uint32_t lb(const int32_t* __restrict__ p, uint32_t n
 
 // Count of the undirected edge behind CSR entry (u, v) at position e.
 __device__ __forceinline__ uint32_t edge_count(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                                               const uint32_t* __restrict__ dplus, const uint32_t* __restrict__ ecnt,
-                                               uint64_t u, int32_t v, uint64_t e) {
-    if ((uint64_t)v < u) return ecnt[e];
-    const uint64_t rv = off[v];
-    return ecnt[rv + lb(adj + rv, dplus[v], (int32_t)u)];
+                                               const uint32_t* __restrict__ dplus, const uint32_t* __restrict__ ooff,
+                                               const uint32_t* __restrict__ ecnt, uint64_t u, int32_t v, uint64_t e) {
+    if ((uint64_t)v < u) return ecnt[tc::slot_base(ooff, off, (int64_t)u) + (e - off[u])];
+    return ecnt[tc::slot_base(ooff, off, v) + lb(adj + off[v], dplus[v], (int32_t)u)];
 }
 
 // Largest row r in [lo, hi] with off[r] <= j (off[lo] <= j < off[hi + 1]):
@@ -55,8 +55,8 @@ __device__ __forceinline__ uint64_t row_of(const uint64_t* __restrict__ off, uin
 // of serialising one.
 constexpr uint64_t kJacChunk = 256;
 __global__ void k_jaccard_entries(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                                  const uint32_t* __restrict__ dplus, const uint32_t* __restrict__ ecnt, uint64_t n,
-                                  uint64_t m, float* __restrict__ jac) {
+                                  const uint32_t* __restrict__ dplus, const uint32_t* __restrict__ ooff,
+                                  const uint32_t* __restrict__ ecnt, uint64_t n, uint64_t m, float* __restrict__ jac) {
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -68,7 +68,7 @@ __global__ void k_jaccard_entries(const uint64_t* __restrict__ off, const int32_
         for (uint64_t j = c0 + lane; j < c1; j += 32) {
             const uint64_t u = row_of(off, r0, r1, j);
             const int32_t v = adj[j];
-            const uint32_t c = edge_count(off, adj, dplus, ecnt, u, v, j);
+            const uint32_t c = edge_count(off, adj, dplus, ooff, ecnt, u, v, j);
             const uint64_t du = off[u + 1] - off[u], dv = off[v + 1] - off[v];
             // src/Graph.cpp:808-809: c / (deg_u + deg_v - c), in double
             jac[j] = (float)((double)c / ((double)(du + dv) - (double)c));
@@ -208,14 +208,17 @@ pc_status pc_jaccard_edges(pc_pgraph* pg, float* out) {
     // per-edge triangle counts with the triangle-count plan (its variants,
     // the learned or heuristic choice per unit) in per-edge mode
     DevBuf ecnt;
-    PC_TRY(ecnt.alloc(m * 4, "triangles per edge"));
-    PC_CUDA(cudaMemsetAsync(ecnt.p, 0, m * 4, s));
+    uint64_t slots = 0;
+    PC_TRY(tc_edge_slots(pg, &slots));
+    PC_TRY(ecnt.alloc(slots * 4, "triangles per edge"));
+    PC_CUDA(cudaMemsetAsync(ecnt.p, 0, slots * 4, s));
     uint64_t T = 0;
     PC_TRY(tc_edge_triangles(pg, PC_VARIANT_AUTO, ecnt.as<uint32_t>(), &T));
     PC_TRY(scratch_reserve(pg, m * 4 + 1024));
     float* jac = pg->scratch.take<float>(m);
-    k_jaccard_entries<<<sm_count(pg->g->device) * 8, 256, 0, s>>>(pg->off, pg->adj, pg->dplus.as<uint32_t>(),
-                                                                   ecnt.as<uint32_t>(), n, m, jac);
+    k_jaccard_entries<<<sm_count(pg->g->device) * 8, 256, 0, s>>>(
+        pg->off, pg->adj, pg->dplus.as<uint32_t>(), pg->oids.p ? pg->ooff.as<uint32_t>() : nullptr, ecnt.as<uint32_t>(), n,
+        m, jac);
     PC_LAUNCHED();
     // entries are in the graph's own CSR order (internal ids are the graph's ids)
     PC_CUDA(cudaMemcpyAsync(out, jac, m * 4, cudaMemcpyDeviceToHost, s));

@@ -105,6 +105,12 @@ struct pc_pgraph {
     std::vector<int64_t> pstart;  // P+1 partition boundaries (internal ids)
     pc::DevBuf d_pstart;          // int64 [P+1]
     pc::DevBuf dplus;             // uint32 [n]: |N(u) & [0,u)| (internal ids)
+    // oriented copy (ensure_oriented): row u = N(u) & [0,u) in ascending order,
+    // from 16-byte vector ooff[u] of oids, padded with INT_MAX to whole vectors
+    pc::DevBuf ooff;              // uint32 [n+1]
+    pc::DevBuf oids;              // int4 [ovecs + 32]; null when there was no room for it
+    uint64_t ovecs = 0;           // vectors of all rows
+    bool oriented_tried = false;
     pc::DevBuf unit_of;           // int32 [n]: planning unit of each vertex (tc.cu)
     pc::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -155,6 +161,10 @@ int32_t to_internal_id(const pc_pgraph* pg, int32_t api_id);
 
 // Lazily computes pg->dplus.
 pc_status ensure_dplus(pc_pgraph* pg);
+
+// Lazily builds the oriented copy (uses the scratch arena).  Leaves oids null,
+// without an error, when device memory does not hold it.
+pc_status ensure_oriented(pc_pgraph* pg);
 
 // Synchronises the handle's stream and converts a device error to a status.
 pc_status sync(pc_pgraph* pg);

@@ -178,12 +178,11 @@ __global__ void k_item_fill(const uint64_t* __restrict__ off, const uint32_t* __
     if (!c) return;
     const int64_t p = range_pos(ranges, rprefix, nranges, t);
     const int32_t b = pivot_at(plist, p);
-    const uint32_t din = (uint32_t)(off[b + 1] - off[b]) - dplus[b];
+    const uint64_t in0 = off[b] + dplus[b];
+    const uint32_t din = (uint32_t)(off[b + 1] - in0);
     const uint32_t s = start[t];
-    for (uint32_t j = 0; j < c && s + j < cap; ++j) {
-        const uint32_t j0 = j * chunk;
-        items[s + j] = Item{(int32_t)p, (int32_t)j0, (int32_t)min(j0 + chunk, din)};
-    }
+    for (uint32_t j = 0; j < c && s + j < cap; ++j)
+        items[s + j] = Item{in0 + (uint64_t)j * chunk, b, min(chunk, din - j * chunk)};
 }
 
 // H[b - lo][a >> 5] |= bit(a) for a in N+(b), one warp per pivot.
@@ -462,9 +461,10 @@ static bool is_bitmap(int v) {
     return v == PC_VARIANT_BITMAP_WARP || v == PC_VARIANT_BITMAP_GROUP8 || v == PC_VARIANT_BITMAP_LANE;
 }
 
-// Bitmap sets per CTA: K warps share one set; the smallest K whose 16/K sets
-// fit the shared-memory budget (about 100 KB for two CTAs per SM, up to
-// 200 KB for one).
+// Bitmap sets per CTA: K warps share one set, 16 / K sets per CTA.  The
+// smallest K whose CTAs (sets and the per-vertex mode's hub histogram) stay
+// below a third of an SM's shared memory, or a half, or all of it: the scans
+// wait on L2, so resident warps come before sets of fewer warps.
 struct BitmapShape {
     int K;
     uint32_t words;
@@ -472,23 +472,40 @@ struct BitmapShape {
     int ctas_per_sm;
 };
 
-static BitmapShape bitmap_shape(uint32_t max_pivot_plus1) {
+static void fill_shape(BitmapShape* sh, int mode, int kind) {
+    sh->smem = (size_t)(16 / sh->K) * bitmap_set_words(sh->words, mode, kind) * 4 +
+               (mode == kCountVertex ? (size_t)kHubHist * 4 : 0);
+    // 1 KB a CTA is the system's
+    sh->ctas_per_sm = (int)std::min<size_t>(4, 227 * 1024 / (sh->smem + 1280));
+}
+
+static BitmapShape bitmap_shape(uint32_t words, int mode) {
     BitmapShape sh{};
-    sh.words = std::max<uint32_t>(1, (max_pivot_plus1 + 31) / 32);
-    const size_t budget_two = 100 * 1024, budget_one = 200 * 1024;
-    for (int K = 1; K <= 16; K *= 2) {
-        const size_t smem = (size_t)(16 / K) * sh.words * 4;
-        if (smem <= budget_two || (K == 16 && smem <= budget_one)) {
-            sh.K = K;
-            sh.smem = smem;
-            break;
+    sh.words = words;
+    for (int per_sm = 3; per_sm >= 1; --per_sm)
+        for (sh.K = 1; sh.K <= 16; sh.K *= 2) {
+            fill_shape(&sh, mode, kPlainSet);
+            if (sh.ctas_per_sm >= per_sm) return sh;
         }
-    }
-    if (!sh.K) {
-        sh.K = 16;
-        sh.smem = (size_t)sh.words * 4;
-    }
-    sh.ctas_per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (sh.smem + 1024)));
+    sh.K = 16;
+    fill_shape(&sh, mode, kPlainSet);
+    return sh;
+}
+
+// Mixed sets of K warps with `lo` low ids.  kSplitLo: the bitmap units, two
+// warps a set: 7.2 KB sets, so three CTAs and 48 warps stay on an SM (RMAT-24's
+// units of ids 65-196 K: 7.23 ms; 2^16 low ids in 10 KB sets of four warps,
+// whose barriers cost more, 8.27 ms).  kLightLo: the light pivots of the hash
+// variant, a set per warp of 4 KB: 2^13 exact low ids keep most look-ups away
+// (RMAT-24 4.16 ms, RMAT-16 0.16 ms in all, against 4.25 and 0.19 ms with lo = 0;
+// ER-20, whose ids spread evenly, 0.98 against 0.88 ms).
+constexpr uint32_t kSplitLo = 1u << 15, kLightLo = 1u << 13;
+constexpr uint32_t kSplitFrom = 1u << 16;  // bitmap units with pivots past this id have mixed sets
+static BitmapShape mixed_shape(int mode, int K, uint32_t lo) {
+    BitmapShape sh{};
+    sh.K = K;
+    sh.words = lo / 32 + kFilterWords;
+    fill_shape(&sh, mode, kMixedSet);
     return sh;
 }
 
@@ -497,10 +514,8 @@ struct BitmapLaunch {
     unsigned grid;
     size_t smem;
     cudaStream_t s;
-    const uint64_t* off;
+    OrientedView oriented;
     const int32_t* adj;
-    const uint32_t* dp;
-    const int32_t* plist;
     const Item* items;
     const uint32_t* nitems;
     uint32_t* next;
@@ -512,45 +527,39 @@ struct BitmapLaunch {
     uint32_t* ecnt;           // per-edge counts at the oriented slots (Jaccard), or null
 };
 
-template <int K, int G, bool kVC, bool kEC, bool kSplit = false>
-static pc_status launch_bitmap_kgv(const BitmapLaunch& L) {
-    PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, kVC, kEC, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <int K, int G, int kMode, int kKind>
+static pc_status launch_bitmap_kgm(const BitmapLaunch& L) {
+    PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, kMode, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)L.smem));
-    k_tc_bitmap<K, G, kVC, kEC, kSplit><<<L.grid, kCtaThreads, L.smem, L.s>>>(
-        L.off, L.adj, L.dp, L.plist, L.items, L.nitems, L.next, L.total, L.words, L.cost, L.unit_of, L.tri, L.ecnt);
+    k_tc_bitmap<K, G, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.next,
+                                                                        L.total, L.words, L.cost, L.unit_of, L.tri,
+                                                                        L.ecnt);
     return PC_OK;
 }
 
-// Split-set launches: sets of kSplitWords + kHashSlots words (10 KB); K = 2
-// in the count mode (16 sets per SM), K = 4 in the per-vertex mode, whose
-// 32 KB hub histogram per CTA would leave one CTA of 8 sets per SM.
-static pc_status launch_bitmap_split(int K, int G, const BitmapLaunch& L) {
-    if (L.ecnt || (L.tri ? K != 4 : K != 2)) return fail(PC_ERR_UNSUPPORTED, "split pivot sets: unexpected launch shape");
-    if (L.tri) {
-        if (G == 32) return launch_bitmap_kgv<4, 32, true, false, true>(L);
-        if (G == 8) return launch_bitmap_kgv<4, 8, true, false, true>(L);
-        return launch_bitmap_kgv<4, 1, true, false, true>(L);
-    }
-    if (G == 32) return launch_bitmap_kgv<2, 32, false, false, true>(L);
-    if (G == 8) return launch_bitmap_kgv<2, 8, false, false, true>(L);
-    return launch_bitmap_kgv<2, 1, false, false, true>(L);
-}
-
-template <int K, bool kVC, bool kEC>
+template <int K, int kMode, int kKind>
 static pc_status launch_bitmap_kmode(int G, const BitmapLaunch& L) {
-    if (G == 32) return launch_bitmap_kgv<K, 32, kVC, kEC>(L);
-    if (G == 8) return launch_bitmap_kgv<K, 8, kVC, kEC>(L);
-    return launch_bitmap_kgv<K, 1, kVC, kEC>(L);
+    if (G == 32) return launch_bitmap_kgm<K, 32, kMode, kKind>(L);
+    if (G == 8) return launch_bitmap_kgm<K, 8, kMode, kKind>(L);
+    return launch_bitmap_kgm<K, 1, kMode, kKind>(L);
 }
 
 template <int K>
 static pc_status launch_bitmap_k(int G, const BitmapLaunch& L) {
-    if (L.tri) return launch_bitmap_kmode<K, true, false>(G, L);
-    if (L.ecnt) return launch_bitmap_kmode<K, false, true>(G, L);
-    return launch_bitmap_kmode<K, false, false>(G, L);
+    if (L.tri) return launch_bitmap_kmode<K, kCountVertex, kPlainSet>(G, L);
+    if (L.ecnt) return launch_bitmap_kmode<K, kCountEdge, kPlainSet>(G, L);
+    return launch_bitmap_kmode<K, kCountOnly, kPlainSet>(G, L);
 }
 
-static pc_status launch_bitmap(int K, int G, const BitmapLaunch& L) {
+static pc_status launch_bitmap(int K, int G, int kind, const BitmapLaunch& L) {
+    if (kind == kMixedSet) {  // fixed-size sets (mixed_shape)
+        if (K == 1 && L.ecnt) return launch_bitmap_kgm<1, 8, kCountEdge, kMixedSet>(L);
+        if (K == 1 && L.tri) return launch_bitmap_kgm<1, 8, kCountVertex, kMixedSet>(L);
+        if (K == 1) return launch_bitmap_kgm<1, 8, kCountOnly, kMixedSet>(L);
+        if (L.ecnt || K != 2) return fail(PC_ERR_UNSUPPORTED, "mixed pivot sets: unexpected launch shape");
+        if (L.tri) return launch_bitmap_kmode<2, kCountVertex, kMixedSet>(G, L);
+        return launch_bitmap_kmode<2, kCountOnly, kMixedSet>(G, L);
+    }
     switch (K) {
         case 1: return launch_bitmap_k<1>(G, L);
         case 2: return launch_bitmap_k<2>(G, L);
@@ -566,7 +575,7 @@ static pc_status launch_bitmap(int K, int G, const BitmapLaunch& L) {
 using namespace tc;
 
 static pc_status tc_features(pc_pgraph* pg) {
-    PC_TRY(ensure_dplus(pg));
+    PC_TRY(ensure_oriented(pg));
     build_units(pg, &pg->unit_lo, &pg->unit_hi);
     const size_t U = pg->unit_lo.size();
     const uint64_t n = pg->g->n;
@@ -617,7 +626,7 @@ pc_status tc_ensure_features(pc_pgraph* pg) {
 struct LaunchGroup {
     int v = -1;
     uint32_t words = 0;
-    bool split = false;  // bitmap variants: SplitSets (kSplitWords bitmap words + a hash)
+    bool split = false;  // bitmap variants: mixed sets
     std::vector<int64_t> ranges;
     uint64_t npos = 0, item_bound = 0;
     double ein = 0;
@@ -632,7 +641,7 @@ static uint32_t matrix_stride(int64_t hi) { return (uint32_t)((((hi + 31) / 32) 
 // Bytes of the resident pivot bitmap rows of a matrix unit [lo, hi).
 static uint64_t matrix_bytes(int64_t lo, int64_t hi) { return (uint64_t)(hi - lo) * matrix_stride(hi) * 4; }
 
-// Bitmap units whose pivot ids reach kSplitLo or more run with SplitSets in
+// Bitmap units whose pivot ids pass kSplitFrom run with mixed sets in
 // the count and per-vertex modes, unless PC_BITMAP_SPLIT=0 is in the
 // environment (read once; a switch for measurements).
 static bool bitmap_split_enabled() {
@@ -747,12 +756,12 @@ static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
     int64_t* d_pref = nullptr;
     PC_TRY(upload(pg, gr.ranges.data(), gr.ranges.size(), &d_ranges));
     PC_TRY(upload(pg, pref.data(), nr + 1, &d_pref));
-    BitmapShape sh = bitmap_shape((gr.split ? kSplitWords + (uint32_t)kHashSlots : gr.words) * 32u);
-    if (gr.split && d_tri) {
-        sh.K = 4;
-        sh.smem = (size_t)(16 / sh.K) * (kSplitWords + kHashSlots) * 4;
-    }
-    const uint32_t chunk = is_bitmap(v) ? 256u * (uint32_t)sh.K : (uint32_t)kChunkWarp;
+    const int mode = d_tri ? kCountVertex : (d_ecnt ? kCountEdge : kCountOnly);
+    const bool sets = is_bitmap(v) || v == PC_VARIANT_HASH_WARP;  // run by k_tc_bitmap
+    const bool light = v == PC_VARIANT_HASH_WARP;
+    const BitmapShape sh = light ? mixed_shape(mode, 1, mode == kCountEdge ? 0u : kLightLo)
+                                 : (gr.split ? mixed_shape(mode, 2, kSplitLo) : bitmap_shape(gr.words, mode));
+    const uint32_t chunk = sets ? 256u * (uint32_t)sh.K : (uint32_t)kChunkWarp;
     uint32_t* d_cnt = pg->scratch.take<uint32_t>(npos + 1);
     uint32_t* d_start = pg->scratch.take<uint32_t>(npos + 1);
     size_t tmpb = 0;
@@ -774,67 +783,41 @@ static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
     PC_CUDA(cudaMemsetAsync(d_next, 0, 4, s));
     *launches += 3;
     const uint32_t* d_nitems = d_next + 1;
-    if (is_bitmap(v)) {
+    if (sets) {
         BitmapLaunch L;
-        const size_t nsets = (size_t)(kCtaThreads / 32 / sh.K);
-        L.smem = sh.smem + (d_tri ? (size_t)kHubHist * 4 : 0) +
-                 (d_ecnt ? nsets * (((sh.words + 7) / 8) + (size_t)kEcRankCap) * 4 : 0);
-        const int cps = (d_tri || d_ecnt)
-                            ? (int)std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (L.smem + 1024)))
-                            : sh.ctas_per_sm;
-        L.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * cps, gr.item_bound));
+        L.smem = sh.smem;
+        L.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * sh.ctas_per_sm, gr.item_bound));
         L.s = s;
-        L.off = pg->off;
+        L.oriented = OrientedView{pg->ooff.as<uint32_t>(), pg->oids.as<int4>()};
         L.adj = pg->adj;
-        L.dp = dp;
-        L.plist = plist;
         L.items = d_items;
         L.nitems = d_nitems;
         L.next = d_next;
         L.total = d_total;
-        L.words = gr.split ? kSplitWords : sh.words;
+        L.words = sh.words;
         L.cost = d_cost;
         L.unit_of = unit_of;
         L.tri = d_tri;
         L.ecnt = d_ecnt;
         const int Gsel = v == PC_VARIANT_BITMAP_WARP ? 32 : (v == PC_VARIANT_BITMAP_GROUP8 ? 8 : 1);
-        if (gr.split) PC_TRY(launch_bitmap_split(sh.K, Gsel, L));
-        else PC_TRY(launch_bitmap(sh.K, Gsel, L));
+        PC_TRY(launch_bitmap(sh.K, Gsel, light || gr.split ? kMixedSet : kPlainSet, L));
     } else {
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((uint64_t)sms * 8, ceil_div(gr.item_bound, kWarpCtaWarps)));
         const unsigned bs = kWarpCtaWarps * 32;
-        if (d_ecnt) {
-            if (v == PC_VARIANT_HASH_WARP)
-                k_tc_warp<kModeHash, false, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems,
-                                                                      d_next, d_total, d_cost, unit_of, nullptr, d_ecnt);
-            else if (v == PC_VARIANT_MERGE_LANE)
-                k_tc_warp<kModeMerge, false, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems,
-                                                                       d_next, d_total, d_cost, unit_of, nullptr,
-                                                                       d_ecnt);
-            else
-                k_tc_warp<kModeGallop, false, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items,
-                                                                        d_nitems, d_next, d_total, d_cost, unit_of,
-                                                                        nullptr, d_ecnt);
-        } else if (d_tri) {
-            if (v == PC_VARIANT_HASH_WARP)
-                k_tc_warp<kModeHash, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems, d_next,
-                                                               d_total, d_cost, unit_of, d_tri);
-            else if (v == PC_VARIANT_MERGE_LANE)
-                k_tc_warp<kModeMerge, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems, d_next,
-                                                                d_total, d_cost, unit_of, d_tri);
-            else
-                k_tc_warp<kModeGallop, true><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems,
-                                                                 d_next, d_total, d_cost, unit_of, d_tri);
-        } else if (v == PC_VARIANT_HASH_WARP) {
-            k_tc_warp<kModeHash><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems, d_next, d_total,
-                                                     d_cost, unit_of);
-        } else if (v == PC_VARIANT_MERGE_LANE) {
-            k_tc_warp<kModeMerge><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems, d_next, d_total,
-                                                      d_cost, unit_of);
+        const uint32_t* ooff = pg->oids.p ? pg->ooff.as<uint32_t>() : nullptr;
+        auto launch = [&](auto* kernel) {
+            kernel<<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, ooff, d_items, d_nitems, d_next, d_total, d_cost, unit_of,
+                                       d_tri, d_ecnt);
+        };
+        if (v == PC_VARIANT_MERGE_LANE) {
+            if (d_ecnt) launch(k_tc_warp<kModeMerge, false, true>);
+            else if (d_tri) launch(k_tc_warp<kModeMerge, true>);
+            else launch(k_tc_warp<kModeMerge>);
         } else {
-            k_tc_warp<kModeGallop><<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, plist, d_items, d_nitems, d_next, d_total,
-                                                       d_cost, unit_of);
+            if (d_ecnt) launch(k_tc_warp<kModeGallop, false, true>);
+            else if (d_tri) launch(k_tc_warp<kModeGallop, true>);
+            else launch(k_tc_warp<kModeGallop>);
         }
     }
     PC_LAUNCHED();
@@ -858,27 +841,28 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     const size_t U = lo.size();
     // Bitmap units are grouped by their bitmap size rounded up to a power of
     // two, so the hub units (small ids) get small sets and more CTAs per SM;
-    // in the count and per-vertex modes, units with pivot ids past kSplitLo
-    // share one group of fixed-size SplitSets (class kClasses).
+    // in the count and per-vertex modes, units with pivot ids past
+    // kSplitFrom share one group of fixed-size mixed sets (class kClasses).
     constexpr int kClasses = 16;
     const bool split_ok = bitmap_split_enabled() && !d_ecnt;
     std::vector<LaunchGroup> groups(PC_NUM_VARIANTS * (kClasses + 1));
     std::vector<int> group_of(U, -1);
     for (size_t u = 0; u < U; ++u) {
-        const int v = assign[u];
+        int v = assign[u];
         if (v < 0) continue;
+        if ((is_bitmap(v) || v == PC_VARIANT_HASH_WARP) && !pg->oids.p) v = PC_VARIANT_MERGE_LANE;  // no room for the oriented copy
         const uint32_t mid = (uint32_t)feat[u * kNumFeatures + 4];
         int c = 0;
         if (is_bitmap(v)) {
             const uint32_t w = std::max<uint32_t>(1, (mid + 31) / 32);
             while ((1u << c) < w && c < kClasses - 1) ++c;
-            if (split_ok && mid > (uint32_t)kSplitLo) c = kClasses;
+            if (split_ok && mid > kSplitFrom) c = kClasses;
         }
         LaunchGroup& gr = groups[v * (kClasses + 1) + c];
         group_of[u] = v * (kClasses + 1) + c;
         gr.v = v;
         gr.split = c == kClasses;
-        gr.words = gr.split ? kSplitWords : 1u << c;
+        gr.words = gr.split ? 0 : 1u << c;
         if (v == PC_VARIANT_MATRIX) {
             gr.ranges.push_back(lo[u]);
             gr.ranges.push_back(hi[u]);
@@ -1065,10 +1049,18 @@ pc_status tc_vertex_triangles(pc_pgraph* pg, int32_t variant, unsigned long long
     return tc_execute(pg, assign, count, nullptr, nullptr, d_tri);
 }
 
+// Counters tc_edge_triangles needs.
+pc_status tc_edge_slots(pc_pgraph* pg, uint64_t* slots) {
+    PC_TRY(tc_ensure_features(pg));
+    *slots = pg->oids.p ? 4 * pg->ovecs : pg->g->m;
+    return PC_OK;
+}
+
 // Per-edge triangle counts at the oriented slots (the slot of edge {x, y},
-// y < x, is the position of y in row x) into d_ecnt (m zeroed counters,
-// outside the scratch arena), under the plan of `variant`; matrix units run
-// with the 32-lane bitmap kernel.  Returns the triangle count.
+// y < x, is the position of y in row x of the oriented copy, see slot_base)
+// into d_ecnt (tc_edge_slots zeroed counters, outside the scratch arena),
+// under the plan of `variant`; matrix units run with the 32-lane bitmap
+// kernel.  Returns the triangle count.
 pc_status tc_edge_triangles(pc_pgraph* pg, int32_t variant, uint32_t* d_ecnt, uint64_t* count) {
     PC_TRY(tc_ensure_features(pg));
     const size_t U = pg->unit_lo.size();

@@ -17,9 +17,9 @@
 //
 // Pivot sets in shared memory:
 //  * bitmap (CTA-wide): bit a set for a in N+(b), needs b <= capacity;
-//  * split (CTA-wide): a bitmap of the ids below 2^16 and a hash of the rest
-//    (SplitSet), for pivots past 2^16 in the count and per-vertex modes;
-//  * hash (warp-private): open addressing, <= 256 keys in 512 slots;
+//  * mixed: a bitmap of the ids below `lo` and one of the hash values of the
+//    others, whose positives are looked up in an open-addressing table (<= 256
+//    keys in 512 slots); its size does not grow with the pivot's id;
 //  * none: threshold merge (the reference's primitive) or binary search.
 #pragma once
 #include <stdint.h>
@@ -40,13 +40,21 @@ constexpr int kWarpCtaWarps = 8;    // warps per CTA of the warp kernels
 constexpr int kEcRankCap = 512;     // per-edge mode: pivot sets up to this size count by rank in shared memory
 constexpr int kHubHist = 8192;      // per-vertex counting: ids below this count in shared memory
 
-enum WarpMode { kModeHash = 0, kModeMerge = 1, kModeGallop = 2 };
+enum WarpMode { kModeMerge = 1, kModeGallop = 2 };
 
-struct Item {
-    int32_t pos;  // plist position of the pivot
-    int32_t j0;   // in-neighbours [j0, j1) of the pivot (indices into N-(b))
-    int32_t j1;
+// A pivot and a run of its in-neighbours: adj[in0, in0 + n) of the CSR.
+struct __align__(16) Item {
+    uint64_t in0;
+    int32_t b;
+    uint32_t n;
 };
+
+// First slot of row x's counters in the per-edge mode: its place in the
+// oriented copy, or in the CSR when there is none (ooff null).
+__device__ __forceinline__ uint64_t slot_base(const uint32_t* __restrict__ ooff, const uint64_t* __restrict__ off,
+                                              int64_t x) {
+    return ooff ? 4ull * ooff[x] : off[x];
+}
 
 __device__ __forceinline__ int32_t pivot_at(const int32_t* __restrict__ plist, int64_t p) {
     return plist ? plist[p] : (int32_t)p;
@@ -56,44 +64,73 @@ __device__ __forceinline__ uint32_t hash_slot(int32_t a) { return ((uint32_t)a *
 
 // Pivot sets the bitmap kernels test prefix ids against.
 //
-// BitmapSet: bit a of a shared-memory bitmap for every a in N+(b).
+// kPlainSet: for every a in N+(b), bit a of a shared-memory bitmap, the ids of
+// a word from its top bit down, so that a test is one wrapping shift and the
+// word's sign (`bit_of`).
 //
-// SplitSet: ids below kSplitLo in a bitmap of kSplitLo bits (8 KB), ids at or
-// above it in a 512-slot open-addressing hash.  The set's size no longer
-// grows with the pivot's id, so units of pivots up to 2^20 keep 8 sets per
-// CTA.  A pivot with more than kHashCap ids at or above kSplitLo does not fill
-// the hash; its high ids are then found by binary search in N+(b) itself
-// (`ovf`), so the test stays exact for every pivot.
-constexpr int32_t kSplitLo = 1 << 16;
-constexpr uint32_t kSplitWords = (uint32_t)kSplitLo / 32;
+// kMixedSet: bit a for the ids below `lo`; for the others bit lo + h(a), h a
+// hash to kFilterLog bits, and the keys in the 512-slot hash.  The set's size no
+// longer grows with the pivot's id, and nearly every high id is settled by the
+// one bit, because few of them are hits (5-7 % of the prefix ids at RMAT-18
+// past pivot 4096, under 2 % past 16 K); the others are looked up.  The hash
+// holds the last kHashCap entries of N+(b) that are not below lo; when there
+// are more, its keys are found by binary search in N+(b) itself (`ovf`), so the test
+// stays exact for every pivot.  With lo = 0 every id goes through the hash.
+enum SetKind { kPlainSet = 0, kMixedSet = 1 };
+constexpr int kFilterLog = 13;
+constexpr uint32_t kFilterWords = (1u << kFilterLog) / 32;
 
-struct BitmapSet {
-    const uint32_t* bm;
-    __device__ __forceinline__ uint32_t test(int32_t a) const { return (bm[a >> 5] >> (a & 31)) & 1u; }
-};
+__device__ __forceinline__ uint32_t bit_of(const uint32_t* bm, uint32_t a) {
+    return __funnelshift_l(0u, bm[a >> 5], a) >> 31;
+}
+__device__ __forceinline__ uint32_t filter_bit(int32_t a) { return ((uint32_t)a * 0x9E3779B1u) >> (32 - kFilterLog); }
 
-struct SplitSet {
+struct SetView {
     const uint32_t* bm;
-    const int32_t* ht;             // kHashSlots slots, -1 = empty
-    const int32_t* __restrict__ nb;  // N+(b) in the CSR (overflow path)
-    uint32_t dp;
+    int32_t lo;                      // kMixedSet
+    const int32_t* ht;               // kHashSlots slots, -1 = empty
+    const uint16_t* hpos;            // per-edge counts: the rank of each slot's key
+    const int32_t* __restrict__ nb;  // N+(b), padded with INT_MAX to np entries (overflow path)
+    uint32_t np;
     bool ovf;
-    __device__ __forceinline__ uint32_t test(int32_t a) const {
-        if (a < kSplitLo) return (bm[a >> 5] >> (a & 31)) & 1u;
+    // the bit an id is tested at
+    template <int kKind>
+    __device__ __forceinline__ uint32_t place(int32_t a) const {
+        if (kKind == kPlainSet) return (uint32_t)a;
+        return a < lo ? (uint32_t)a : (uint32_t)lo + filter_bit(a);
+    }
+    // whether a is among the hash's keys, and its rank in N+(b) (hpos not null)
+    __device__ __forceinline__ bool find(int32_t a, uint32_t* rank) const {
         if (ovf) {
-            uint32_t lo = 0, hi = dp;
+            uint32_t lo = 0, hi = np;
             while (lo < hi) {
                 const uint32_t mid = (lo + hi) >> 1;
                 if (__ldg(nb + mid) < a) lo = mid + 1; else hi = mid;
             }
-            return (lo < dp && __ldg(nb + lo) == a) ? 1u : 0u;
+            *rank = lo;
+            return lo < np && __ldg(nb + lo) == a;
         }
         uint32_t s = hash_slot(a);
         for (int32_t key; (key = ht[s]) != -1; s = (s + 1) & (kHashSlots - 1))
-            if (key == a) return 1u;
-        return 0u;
+            if (key == a) {
+                if (hpos) *rank = hpos[s];
+                return true;
+            }
+        return false;
     }
 };
+
+// Shared-memory words of one pivot set: the bitmap, then the hash of a mixed
+// set; in the per-edge mode also a plain set's ranks (a 16-bit one per word, a
+// 32-bit one per 64 words) or a mixed set's (one per slot), and the hits by
+// rank.
+constexpr uint32_t kSlotRankWords = (uint32_t)kHashSlots / 2;
+constexpr uint32_t bitmap_set_words(uint32_t bm_words, int mode, int kind) {
+    return bm_words + (kind == kMixedSet ? (uint32_t)kHashSlots : 0u) +
+           (mode != 2 ? 0u
+                      : (kind == kPlainSet ? (bm_words + 63) / 64 + (bm_words + 1) / 2 : kSlotRankWords) +
+                            (uint32_t)kEcRankCap);
+}
 
 // Named barrier over `nthreads` threads of one warp group (ids 1..15; id 0
 // is __syncthreads).
@@ -109,195 +146,188 @@ __device__ __forceinline__ void count_vertex(int32_t a, unsigned long long* __re
     else atomicAdd(&tri[a], 1ull);
 }
 
-// Position of a in the pivot set: bits of the bitmap below a, from the
-// superblock prefix sb (one count per 8 words) and at most 8 word popcounts.
-__device__ __forceinline__ uint32_t rank_in_set(const uint32_t* __restrict__ bm, const uint32_t* __restrict__ sb,
-                                                int32_t a) {
-    const uint32_t w = (uint32_t)a >> 5;
-    uint32_t r = sb[w >> 3];
-    for (uint32_t x = w & ~7u; x < w; ++x) r += __popc(bm[x]);
-    return r + __popc(bm[w] & ((1u << (a & 31)) - 1u));
+// What the pivot-form kernels count: triangles; per-vertex triangle counts
+// (LCC); per-edge counts at the oriented slots (Jaccard), where every
+// triangle a < b < c adds 1 to the slot of a in row c (its scan index), to the
+// slot of a in row b (its rank in the pivot set) and, once per pair, its
+// hits to the slot of b in row c (where the scan stops).  The slot of edge
+// {x, y}, y < x, is the position of y in row x of the oriented copy.
+enum CountMode { kCountOnly = 0, kCountVertex = 1, kCountEdge = 2 };
+
+// The oriented copy of the graph the bitmap kernels scan (Oriented in
+// tc.cu): row x holds N+(x) in ascending order, starts at 16-byte vector
+// off[x] of ids and is padded with INT_MAX to whole vectors; at least 32 vectors of
+// INT_MAX follow the last row.
+struct OrientedView {
+    const uint32_t* __restrict__ off;
+    const int4* __restrict__ ids;
+};
+
+// Ranks in a pivot set (per-edge counts): r16[w] is the rank, modulo 2^16, of
+// the first entry with its bit in word w, and r32[w / 64] that of the first
+// entry of the 64-word block; words without entries hold old values.
+struct SetRanks {
+    const uint16_t* r16;
+    const uint32_t* r32;
+};
+__device__ __forceinline__ uint32_t rank_in_set(const uint32_t* bm, const SetRanks& R, int32_t a) {
+    const uint32_t w = (uint32_t)a >> 5, base = R.r32[w >> 6];
+    return base + (uint16_t)(R.r16[w] - (uint16_t)base) + __popc(__funnelshift_rc(bm[w], 0u, 32u - ((uint32_t)a & 31u)));
 }
 
-// Pipelined group-of-G prefix scan (the 32-lane groups use it): the load of
-// the next G ids is issued before the current ones are tested, so two loads
-// per lane are in flight.  Stops at the first id >= b and never reads past
-// lim = dplus[c].
-// Modes of the pivot-form kernels: count only; kVC per-vertex triangle
-// counts (LCC); kEC per-edge counts at the oriented slots (Jaccard): every
-// triangle a < b < c adds 1 to the slot of a in row c (its scan index), to
-// the slot of a in row b (its rank in the pivot set) and, once per pair,
-// its hits to the slot of b in row c (where the scan stops).
-template <int G, bool kVC = false, bool kEC = false, class Set = BitmapSet>
-__device__ __forceinline__ uint32_t scan_prefix_pipelined(const int32_t* __restrict__ row, uint32_t lim, int32_t b,
-                                                          int gl, unsigned gmask, const Set& S,
-                                                          unsigned long long* __restrict__ tri = nullptr,
-                                                          uint32_t* hist = nullptr,
-                                                          uint32_t* __restrict__ ec_c = nullptr,
-                                                          uint32_t* __restrict__ ec_b = nullptr,
-                                                          const uint32_t* __restrict__ sb = nullptr) {
-    uint32_t hits = 0;
-    uint32_t i = gl;
-    int32_t kb = -1;  // kEC: index of b in the row, seen by one lane of the group
-    int32_t a = i < lim ? __ldg(row + i) : 0x7fffffff;
-    for (;;) {
-        const uint32_t inext = i + G;
-        const int32_t an = inext < lim ? __ldg(row + inext) : 0x7fffffff;
-        if (a < b) {
-            const uint32_t bit = S.test(a);
-            hits += bit;
-            if (kVC && bit) count_vertex(a, tri, hist);
-            if (kEC && bit) {
-                atomicAdd(&ec_c[i], 1u);
-                atomicAdd(&ec_b[rank_in_set(S.bm, sb, a)], 1u);
-            }
-        } else if (kEC && a == b) {
-            kb = (int32_t)i;
+// Where the hits of one warp's scans go besides the count.
+struct HitSink {
+    unsigned long long* __restrict__ tri;  // kCountVertex: per-vertex counts
+    uint32_t* hist;                        // ... of the ids below kHubHist
+    uint32_t* __restrict__ ecnt;           // kCountEdge: per-slot counts
+    uint32_t* by_rank;                     // ... of row b: shared counters, or its slots in ecnt
+    SetRanks ranks;
+};
+
+// Scans the prefixes of up to 32 in-neighbours of pivot b: lane j < nb holds
+// in-neighbour j's id (c) and row start; returns this lane's hits.
+//
+// A group of G lanes takes one in-neighbour at a time, 4 ids per lane and
+// step, and goes on to its next one (NG apart) as soon as its row reaches an
+// id >= b -- b itself is in the row, so a scan ends inside it -- while the
+// other groups go on with theirs: no lane waits for the longest of the 32 / G
+// rows in flight.  All groups step together, so the vote that ends a row is
+// one full-warp ballot, and the load of the next vector is issued between
+// that vote and the tests of the current ids: it is never speculative.
+// Nothing is checked per id: ids past the end of the row (the lanes behind
+// the stop, then a running maximum inside the stopping vector) become >= b,
+// and min(id, b) sends them all to b, whose bit is never set (in a mixed set
+// it may be another key's bit; the look-up settles that).
+//
+// Bound: instruction issue and shared-memory wavefronts (RMAT-20: 74 % issue,
+// 68 % of the wavefronts, 32 of 32 lanes active), then L2 latency.  About 45
+// warp instructions per 128 ids; the earlier scan, which tested each id's
+// position and kept a group waiting for the longest of its warp's rows, took
+// about 130.  Bitmap kernels of RMAT-20: 2.07 -> 0.83 ms; RMAT-24's unit of ids
+// 49-65 K (2.0e9 ids): 3.23 -> 1.92 ms.
+template <int G, int kMode, int kKind>
+__device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, int32_t c, uint32_t start, int nb,
+                                                       int32_t b, const SetView& S, int lane,
+                                                       const HitSink& sink) {
+    constexpr int NG = 32 / G;
+    const int gl = lane % G;
+    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    const unsigned below = gmask & ((1u << lane) - 1u);
+    const int4 none = make_int4(INT32_MAX, INT32_MAX, INT32_MAX, INT32_MAX);
+    int j = lane / G;
+    uint32_t q = __shfl_sync(0xffffffffu, start, j) + gl;
+    bool act = j < nb;
+    int4 v = act ? __ldg(O.ids + q) : none;
+    uint32_t cnt = 0, pair = 0;
+    while (__any_sync(0xffffffffu, act)) {
+        const unsigned stop = __ballot_sync(0xffffffffu, v.w >= b);
+        const bool done = G == 1 ? v.w >= b : (stop & gmask) != 0;
+        const uint32_t qc = q;
+        const int jc = j;
+        int4 a = v;
+        if (G > 1 && (stop & below)) a.x = INT32_MAX;
+        if (done) j += NG;
+        const uint32_t s = __shfl_sync(0xffffffffu, start, j & 31);
+        q = done ? s + gl : q + G;
+        const bool had = act;
+        act = j < nb;
+        v = act ? __ldg(O.ids + q) : none;
+        a.y = max(a.x, a.y);
+        a.z = max(a.y, a.z);
+        a.w = max(a.z, a.w);
+        uint32_t h[4];
+        uint32_t rank[4];  // kMixedSet with lo = 0: of the hits
+        h[0] = bit_of(S.bm, S.place<kKind>(min(a.x, b)));
+        h[1] = bit_of(S.bm, S.place<kKind>(min(a.y, b)));
+        h[2] = bit_of(S.bm, S.place<kKind>(min(a.z, b)));
+        h[3] = bit_of(S.bm, S.place<kKind>(min(a.w, b)));
+        if constexpr (kKind == kMixedSet) {
+            if (h[0] && a.x >= S.lo) h[0] = a.x < b && S.find(a.x, &rank[0]);
+            if (h[1] && a.y >= S.lo) h[1] = a.y < b && S.find(a.y, &rank[1]);
+            if (h[2] && a.z >= S.lo) h[2] = a.z < b && S.find(a.z, &rank[2]);
+            if (h[3] && a.w >= S.lo) h[3] = a.w < b && S.find(a.w, &rank[3]);
         }
-        int32_t last;
-        if constexpr (G == 1) last = a;
-        else last = __shfl_sync(gmask, a, G - 1, G);
-        if (last >= b) break;
-        a = an;
-        i = inext;
-    }
-    if (kEC) {
-        const uint32_t total = G == 1 ? hits : __reduce_add_sync(gmask, hits);
-        if (kb >= 0 && total) atomicAdd(&ec_c[kb], total);
-    }
-    return hits;
-}
-
-// The same scan with 16-byte loads, for groups of G < 32 lanes: each lane
-// takes 4 consecutive ids per step, so a group of 8 reads a whole 128-byte
-// line per dependent round instead of 32 bytes.  The row is read from the
-// 16-byte boundary at or below its start (positions before 0 are masked);
-// a load may run up to 3 ids past lim, which the adjacency array's padding
-// (64 ids after the last row) keeps in bounds.
-template <int G, bool kVC = false, bool kEC = false, class Set = BitmapSet>
-__device__ __forceinline__ uint32_t scan_prefix_vec4(const int32_t* __restrict__ row, uint32_t lim, int32_t b, int gl,
-                                                     unsigned gmask, const Set& S,
-                                                     unsigned long long* __restrict__ tri = nullptr,
-                                                     uint32_t* hist = nullptr, uint32_t* __restrict__ ec_c = nullptr,
-                                                     uint32_t* __restrict__ ec_b = nullptr,
-                                                     const uint32_t* __restrict__ sb = nullptr) {
-    constexpr uint32_t kSpan = 4 * G;  // ids per group step
-    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(row) >> 2) & 3u;
-    const int4* q = reinterpret_cast<const int4*>(row - mis);
-    const uint32_t total = lim + mis;  // ids from q[0] to the end of the bound
-    const int4 none = make_int4(0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff);
-    uint32_t hits = 0;
-    int32_t kb = -1;  // kEC: index of b in the row, seen by one lane of the group
-    uint32_t c0 = 0;
-    int4 v = 4u * gl < total ? __ldg(q + gl) : none;
-    for (;;) {
-        const uint32_t c1 = c0 + kSpan;
-        const int4 vn = c1 + 4u * gl < total ? __ldg(q + c1 / 4 + gl) : none;
-        const int32_t e[4] = {v.x, v.y, v.z, v.w};
-        bool stop = false;
+        const uint32_t hits = h[0] + h[1] + h[2] + h[3];
+        cnt += hits;
+        if constexpr (kMode != kCountOnly) {
+            const int32_t e[4] = {a.x, a.y, a.z, a.w};
+            if (hits) {
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int64_t pos = (int64_t)(c0 + 4u * gl + t) - (int64_t)mis;  // index in row
-            if (pos < 0 || pos >= (int64_t)lim) continue;
-            const int32_t a = e[t];
-            if (a < b) {
-                const uint32_t bit = S.test(a);
-                hits += bit;
-                if (kVC && bit) count_vertex(a, tri, hist);
-                if (kEC && bit) {
-                    atomicAdd(&ec_c[pos], 1u);
-                    atomicAdd(&ec_b[rank_in_set(S.bm, sb, a)], 1u);
+                for (int t = 0; t < 4; ++t) {
+                    if (!h[t]) continue;
+                    if constexpr (kMode == kCountVertex) {
+                        count_vertex(e[t], sink.tri, sink.hist);
+                    } else {
+                        atomicAdd(sink.ecnt + (4ull * qc + t), 1u);
+                        atomicAdd(sink.by_rank + (kKind == kMixedSet ? rank[t] : rank_in_set(S.bm, sink.ranks, e[t])),
+                                  1u);
+                    }
                 }
-            } else {
-                stop = true;
-                if (kEC && a == b) kb = (int32_t)pos;
+            }
+            pair += hits;
+            if (__any_sync(0xffffffffu, done && had)) {
+                uint32_t sum = pair;
+                for (int o = G / 2; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if constexpr (kMode == kCountVertex) {
+                    const int32_t cj = __shfl_sync(0xffffffffu, c, jc & 31);
+                    if (done && had && gl == 0 && sum) atomicAdd(&sink.tri[cj], (unsigned long long)sum);
+                } else {
+                    // the first lane to stop holds b: after the ids below it
+                    if (done && had && sum && ((stop >> lane) & 1u) && !(stop & below))
+                        atomicAdd(sink.ecnt + (4ull * qc + (a.x < b) + (a.y < b) + (a.z < b)), sum);
+                }
+                if (done) pair = 0;
             }
         }
-        bool any_stop;
-        if constexpr (G == 1) any_stop = stop;
-        else any_stop = __any_sync(gmask, stop);
-        if (any_stop || c1 >= total) break;
-        v = vn;
-        c0 = c1;
     }
-    if (kEC) {
-        const uint32_t sum = G == 1 ? hits : __reduce_add_sync(gmask, hits);
-        if (kb >= 0 && sum) atomicAdd(&ec_c[kb], sum);
-    }
-    return hits;
-}
-
-// The prefix scan a group of G lanes runs: 16-byte loads below 32 lanes.
-template <int G, bool kVC = false, bool kEC = false, class Set = BitmapSet>
-__device__ __forceinline__ uint32_t scan_group_prefix(const int32_t* __restrict__ row, uint32_t lim, int32_t b, int gl,
-                                                      unsigned gmask, const Set& S,
-                                                      unsigned long long* __restrict__ tri = nullptr,
-                                                      uint32_t* hist = nullptr, uint32_t* __restrict__ ec_c = nullptr,
-                                                      uint32_t* __restrict__ ec_b = nullptr,
-                                                      const uint32_t* __restrict__ sb = nullptr) {
-    if constexpr (G < 32) return scan_prefix_vec4<G, kVC, kEC>(row, lim, b, gl, gmask, S, tri, hist, ec_c, ec_b, sb);
-    else return scan_prefix_pipelined<G, kVC, kEC>(row, lim, b, gl, gmask, S, tri, hist, ec_c, ec_b, sb);
+    return cnt;
 }
 
 // Bitmap kernel: a CTA of kCtaThreads threads holds 16/K pivot sets in
 // shared memory, one per group of K warps; each group takes its own work
 // items (pivot, a run of its in-neighbours), so a group synchronises only
-// with itself (a named barrier, or nothing when K == 1).  In-neighbour metadata
-// (id, row offset, prefix length) is fetched 32 at a time with one coalesced
-// load and 32 independent gathers, then handed to groups of G lanes by
-// shuffles; each group scans one prefix with scan_group_prefix.
-// With kSplit the sets are SplitSets: bm_words = kSplitWords bitmap words,
-// then kHashSlots hash slots, whatever the pivots' ids (count and per-vertex
-// modes; the per-edge mode needs ranks in a plain bitmap).
-template <int K, int G, bool kVC = false, bool kEC = false, bool kSplit = false>
-__global__ void __launch_bounds__(kCtaThreads) k_tc_bitmap(const uint64_t* __restrict__ off,
-                                                           const int32_t* __restrict__ adj,
-                                                           const uint32_t* __restrict__ dplus,
-                                                           const int32_t* __restrict__ plist,
-                                                           const Item* __restrict__ items,
-                                                           const uint32_t* __restrict__ nitems_p,
-                                                           uint32_t* __restrict__ next_item,
-                                                           unsigned long long* __restrict__ total,
-                                                           uint32_t bm_words,
-                                                           unsigned long long* __restrict__ unit_cost,
-                                                           const int32_t* __restrict__ unit_of,
-                                                           unsigned long long* __restrict__ tri = nullptr,
-                                                           uint32_t* __restrict__ ecnt = nullptr) {
-    static_assert(!(kSplit && kEC), "per-edge counts need the plain bitmap's ranks");
+// with itself (a named barrier, or nothing when K == 1).  A warp fetches 32
+// in-neighbours' ids with one coalesced load and their row starts with 32
+// independent gathers and scans their prefixes (scan_in_neighbours).
+// Mixed sets have (bm_words - kFilterWords) * 32 = lo bits for the low ids,
+// whatever the pivots' ids (0 in the per-edge mode, which needs every hit's
+// rank).
+template <int K, int G, int kMode, int kKind>
+__global__ void __launch_bounds__(kCtaThreads, kMode == kCountOnly ? 3 : 2)
+    k_tc_bitmap(OrientedView O, const int32_t* __restrict__ adj, const Item* __restrict__ items,
+                const uint32_t* __restrict__ nitems_p, uint32_t* __restrict__ next_item,
+                unsigned long long* __restrict__ total, uint32_t bm_words, unsigned long long* __restrict__ unit_cost,
+                const int32_t* __restrict__ unit_of, unsigned long long* __restrict__ tri,
+                uint32_t* __restrict__ ecnt) {
+    constexpr bool kHash = kKind == kMixedSet;
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_item[16];
-    __shared__ uint32_t s_hic[16];  // kSplit: ids >= kSplitLo offered to the set's hash this item
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int set = warp / K, wi = warp % K;
-    const int nsets = (kCtaThreads / 32) / K;
-    const int set_threads = K * 32, tis = wi * 32 + lane;
-    const uint32_t set_words = bm_words + (kSplit ? (uint32_t)kHashSlots : 0u);
+    constexpr int nsets = (kCtaThreads / 32) / K;
+    constexpr int set_threads = K * 32;
+    const int tis = wi * 32 + lane;
+    const uint32_t set_words = bitmap_set_words(bm_words, kMode, kKind);
     uint32_t* bm = smem + (size_t)set * set_words;
-    int32_t* ht = reinterpret_cast<int32_t*>(bm + bm_words);  // kSplit: the set's hash slots
-    uint32_t* hist = smem + (size_t)nsets * set_words;  // kVC: kHubHist counters after the sets
-    // kEC: per set, the rank of the first pivot-set entry of every touched
-    // 256-id superblock (only those are ever read)
-    const uint32_t nsb = (bm_words + 7) / 8;
-    uint32_t* sb = smem + (size_t)nsets * bm_words + (size_t)set * nsb;
-    // kEC: per set, hits by rank in the pivot set (sets up to kEcRankCap),
-    // flushed to the row's slots once per item
-    uint32_t* ecs = smem + (size_t)nsets * (bm_words + nsb) + (size_t)set * kEcRankCap;
-    const uint32_t zero_words = (uint32_t)nsets * set_words + (kVC ? (uint32_t)kHubHist : 0u);
+    int32_t* ht = reinterpret_cast<int32_t*>(bm + bm_words);  // kHash: the set's hash slots
+    // kCountEdge: a plain set's ranks, or the rank of each hash slot's key
+    uint32_t* r32 = bm + bm_words + (kHash ? (uint32_t)kHashSlots : 0u);
+    uint16_t* r16 = reinterpret_cast<uint16_t*>(r32 + (kHash ? 0u : (bm_words + 63) / 64));
+    uint32_t* by_rank = bm + set_words - kEcRankCap;
+    uint32_t* hist = smem + (size_t)nsets * set_words;        // kCountVertex: kHubHist counters after the sets
+    const uint32_t zero_words = (uint32_t)nsets * set_words + (kMode == kCountVertex ? (uint32_t)kHubHist : 0u);
     for (uint32_t i = tid; i < zero_words; i += blockDim.x)
-        smem[i] = (kSplit && i < (uint32_t)nsets * set_words && i % set_words >= bm_words) ? 0xffffffffu : 0u;
-    if (kEC)
-        for (uint32_t i = tid; i < (uint32_t)nsets * kEcRankCap; i += blockDim.x)
-            smem[(size_t)nsets * (bm_words + nsb) + i] = 0;
-    if (tid < 16) s_hic[tid] = 0;
+        smem[i] = (kHash && i < (uint32_t)nsets * set_words && i % set_words >= bm_words &&
+                   i % set_words < bm_words + kHashSlots)
+                      ? 0xffffffffu
+                      : 0u;
     __syncthreads();
     auto set_sync = [&]() {
         if constexpr (K == 1) __syncwarp();
         else group_barrier(1 + set, set_threads);
     };
+    const int32_t lo = kHash ? (int32_t)(bm_words - kFilterWords) * 32 : 0;
     const uint32_t nitems = *nitems_p;
-    constexpr int NG = 32 / G;  // in-neighbours handled at once per warp
-    const int gidx = lane / G, gl = lane % G;
-    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
     unsigned long long cnt = 0;
     for (;;) {
         if (tis == 0) s_item[set] = atomicAdd(next_item, 1u);
@@ -306,87 +336,85 @@ __global__ void __launch_bounds__(kCtaThreads) k_tc_bitmap(const uint64_t* __res
         if (it >= nitems) break;
         const long long t0 = unit_cost ? clock64() : 0;
         const Item I = items[it];
-        const int32_t b = pivot_at(plist, I.pos);
-        const uint64_t rb = off[b], re = off[b + 1];
-        const uint32_t dp = dplus[b];
-        for (uint32_t k = tis; k < dp; k += set_threads) {
-            const int32_t a = adj[rb + k];
-            if (!kSplit || a < kSplitLo) {
-                atomicOr(&bm[a >> 5], 1u << (a & 31));
-            } else if (atomicAdd(&s_hic[set], 1u) < (uint32_t)kHashCap) {
-                // at most kHashCap keys in kHashSlots slots: a free slot exists
-                uint32_t hs = hash_slot(a);
-                while (atomicCAS(&ht[hs], -1, a) != -1) hs = (hs + 1) & (kHashSlots - 1);
-            }
-            if (kEC && (k == 0 || (adj[rb + k - 1] >> 8) != (a >> 8))) sb[a >> 8] = k;
-        }
-        set_sync();
-        const uint32_t hic = kSplit ? s_hic[set] : 0u;
-        std::conditional_t<kSplit, SplitSet, BitmapSet> S;
-        if constexpr (kSplit) S = SplitSet{bm, ht, adj + rb, dp, hic > (uint32_t)kHashCap};
-        else S = BitmapSet{bm};
-        const uint64_t in0 = rb + dp + (uint64_t)I.j0;
-        const uint64_t in1 = min(rb + dp + (uint64_t)I.j1, re);
-        unsigned long long hb = 0;  // kVC: this item's triangles at pivot b
-        for (uint64_t base = in0 + (uint64_t)wi * 32; base < in1; base += (uint64_t)set_threads) {
-            const uint64_t e = base + lane;
-            const bool ok = e < in1;
-            const int32_t c = ok ? adj[e] : 0;
-            const uint64_t rc = ok ? off[c] : 0;
-            const uint32_t lim = ok ? dplus[c] : 0;
-            const uint64_t left = in1 - base;
-            const int nb = left < 32 ? (int)left : 32;
-            for (int j0 = 0; j0 < 32; j0 += NG) {
-                if (j0 >= nb) break;
-                const int j = j0 + gidx;
-                const int src = j < nb ? j : 0;
-                const uint64_t rcj = __shfl_sync(0xffffffffu, rc, src);
-                uint32_t limj = __shfl_sync(0xffffffffu, lim, src);
-                if (j >= nb) limj = 0;
-                if (kEC) {
-                    if (limj) cnt += scan_group_prefix<G, false, true>(adj + rcj, limj, b, gl, gmask, S, nullptr,
-                                                                           nullptr, ecnt + rcj,
-                                                                           dp <= kEcRankCap ? ecs : ecnt + rb, sb);
-                } else if (kVC) {
-                    const int32_t cj = __shfl_sync(0xffffffffu, c, src);
-                    if (limj) {
-                        const uint32_t h = scan_group_prefix<G, true>(adj + rcj, limj, b, gl, gmask, S, tri, hist);
-                        cnt += h;
-                        hb += h;
-                        if (h) atomicAdd(&tri[cj], (unsigned long long)h);
-                    }
-                } else if (limj) {
-                    cnt += scan_group_prefix<G>(adj + rcj, limj, b, gl, gmask, S);
+        const int32_t b = I.b;
+        const uint32_t v0 = O.off[b], v1 = O.off[b + 1];
+        SetView S;
+        S.bm = bm;
+        S.lo = lo;
+        S.ht = ht;
+        S.hpos = kHash && kMode == kCountEdge ? r16 : nullptr;
+        S.nb = reinterpret_cast<const int32_t*>(O.ids + v0);
+        S.np = 4 * (v1 - v0);
+        // the hash takes ranks np - kHashCap and up: all high ids, or it is not used
+        S.ovf = kHash && S.np > (uint32_t)kHashCap && __ldg(S.nb + (S.np - kHashCap - 1)) >= lo;
+        for (uint32_t k = v0 + tis; k < v1; k += set_threads) {
+            const int4 v = __ldg(O.ids + k);
+            const int32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int32_t a = e[t];
+                if (a == INT32_MAX) continue;  // padding
+                const uint32_t rank = 4 * (k - v0) + t;
+                const uint32_t x = S.place<kKind>(a);
+                atomicOr(&bm[x >> 5], 0x80000000u >> (x & 31));
+                if (kHash && !S.ovf && a >= lo) {
+                    // at most kHashCap keys in kHashSlots slots: a free slot exists
+                    uint32_t hs = hash_slot(a);
+                    while (atomicCAS(&ht[hs], -1, a) != -1) hs = (hs + 1) & (kHashSlots - 1);
+                    if (kMode == kCountEdge) r16[hs] = (uint16_t)rank;
+                }
+                if (kMode == kCountEdge && kKind == kPlainSet) {
+                    const int32_t prev = t ? e[t - 1] : (k > v0 ? __ldg(&O.ids[k - 1].w) : -1);
+                    if (prev < 0 || (prev >> 5) != (a >> 5)) r16[a >> 5] = (uint16_t)rank;
+                    if (prev < 0 || (prev >> 11) != (a >> 11)) r32[a >> 11] = rank;
                 }
             }
         }
-        if (kVC) {
+        set_sync();
+        const bool few = S.np <= (uint32_t)kEcRankCap;
+        HitSink sink;
+        sink.tri = tri;
+        sink.hist = hist;
+        sink.ecnt = ecnt;
+        sink.by_rank = few ? by_rank : ecnt + 4ull * v0;
+        sink.ranks = SetRanks{r16, r32};
+        const unsigned long long cnt0 = cnt;
+        for (uint32_t k = wi * 32; k < I.n; k += set_threads) {
+            const int nb = min(32, (int)(I.n - k));
+            const int32_t c = lane < nb ? adj[I.in0 + k + lane] : 0;
+            const uint32_t start = O.off[c];
+            cnt += scan_in_neighbours<G, kMode, kKind>(O, c, start, nb, b, S, lane, sink);
+        }
+        if (kMode == kCountVertex) {
+            unsigned long long hb = cnt - cnt0;  // this item's triangles at pivot b
             for (int o = 16; o; o >>= 1) hb += __shfl_xor_sync(0xffffffffu, hb, o);
             if (lane == 0 && hb) atomicAdd(&tri[b], hb);
         }
         set_sync();
-        for (uint32_t k = tis; k < dp; k += set_threads) {
-            const int32_t a = adj[rb + k];
-            if (!kSplit || a < kSplitLo) bm[a >> 5] = 0;
-            if (kEC && dp <= kEcRankCap) {
-                const uint32_t h = ecs[k];
-                if (h) {
-                    atomicAdd(&ecnt[rb + k], h);
-                    ecs[k] = 0;
+        for (uint32_t k = v0 + tis; k < v1; k += set_threads) {
+            const int4 v = __ldg(O.ids + k);
+            const int32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (kHash || e[t] != INT32_MAX) bm[S.place<kKind>(e[t]) >> 5] = 0;
+                if (kMode == kCountEdge && few) {
+                    const uint32_t h = by_rank[4 * (k - v0) + t];
+                    if (h) {
+                        atomicAdd(ecnt + (4ull * k + t), h);
+                        by_rank[4 * (k - v0) + t] = 0;
+                    }
                 }
             }
         }
-        if (kSplit && hic) {
+        if (kHash && !S.ovf)
             for (uint32_t x = tis; x < (uint32_t)kHashSlots; x += set_threads) ht[x] = -1;
-            if (tis == 0) s_hic[set] = 0;  // every lane read it before the scan barrier
-        }
         set_sync();
         // profiling runs: the set's warp-cycles on this item, charged to its unit
         if (unit_cost && tis == 0) atomicAdd(&unit_cost[unit_of[b]], (unsigned long long)(clock64() - t0) * K);
     }
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0 && cnt) atomicAdd(total, cnt);
-    if (kVC) {
+    if (kMode == kCountVertex) {
         __syncthreads();
         for (uint32_t i = tid; i < (uint32_t)kHubHist; i += blockDim.x)
             if (hist[i]) atomicAdd(&tri[i], (unsigned long long)hist[i]);
@@ -522,34 +550,20 @@ template <int MODE, bool kVC = false, bool kEC = false>
 __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* __restrict__ off,
                                                                 const int32_t* __restrict__ adj,
                                                                 const uint32_t* __restrict__ dplus,
-                                                                const int32_t* __restrict__ plist,
+                                                                const uint32_t* __restrict__ ooff,
                                                                 const Item* __restrict__ items,
                                                                 const uint32_t* __restrict__ nitems_p,
                                                                 uint32_t* __restrict__ next_item,
                                                                 unsigned long long* __restrict__ total,
                                                                 unsigned long long* __restrict__ unit_cost,
                                                                 const int32_t* __restrict__ unit_of,
-                                                                unsigned long long* __restrict__ tri = nullptr,
-                                                                uint32_t* __restrict__ ecnt = nullptr) {
-    __shared__ int32_t table[MODE == kModeHash ? kWarpCtaWarps : 1][MODE == kModeHash ? kHashSlots : 1];
-    __shared__ int32_t tpos[MODE == kModeHash && kEC ? kWarpCtaWarps : 1][MODE == kModeHash && kEC ? kHashSlots : 1];
-    // kEC: per warp, the hits of the pivot set's entries by rank, flushed to
-    // their slots once per item instead of one global atomic per triangle
-    __shared__ uint32_t rcnt[MODE == kModeHash && kEC ? kWarpCtaWarps : 1][MODE == kModeHash && kEC ? kHashCap : 1];
+                                                                unsigned long long* __restrict__ tri,
+                                                                uint32_t* __restrict__ ecnt) {
     __shared__ uint32_t hist[kVC ? kHubHist : 1];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t* T = table[MODE == kModeHash ? w : 0];
-    int32_t* TP = tpos[MODE == kModeHash && kEC ? w : 0];  // kEC: position of each key in N+(b)
-    uint32_t* RC = rcnt[MODE == kModeHash && kEC ? w : 0];
+    const int lane = threadIdx.x & 31;
     if (kVC) {
         for (int i = threadIdx.x; i < kHubHist; i += blockDim.x) hist[i] = 0;
         __syncthreads();
-    }
-    if (MODE == kModeHash) {
-        for (int s = lane; s < kHashSlots; s += 32) T[s] = -1;
-        if (kEC)
-            for (int s = lane; s < kHashCap; s += 32) RC[s] = 0;
-        __syncwarp();
     }
     const uint32_t nitems = *nitems_p;
     unsigned long long cnt = 0;
@@ -561,90 +575,17 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
         const long long t0 = unit_cost ? clock64() : 0;
         const unsigned long long cnt_item0 = cnt;
         const Item I = items[it];
-        const int32_t b = pivot_at(plist, I.pos);
-        const uint64_t rb = off[b], re = off[b + 1];
+        const int32_t b = I.b;
+        const uint64_t rb = off[b];
         const uint32_t dp = dplus[b];
-        const uint64_t in0 = rb + dp + (uint64_t)I.j0;
-        const uint64_t in1 = min(rb + dp + (uint64_t)I.j1, re);
+        const uint64_t in0 = I.in0, in1 = I.in0 + I.n;
         const int32_t* nb = adj + rb;
-        if (MODE == kModeHash && dp <= (uint32_t)kHashCap) {
-            for (uint32_t k = lane; k < dp; k += 32) {
-                const int32_t a = nb[k];
-                uint32_t s = hash_slot(a);
-                while (atomicCAS(&T[s], -1, a) != -1) s = (s + 1) & (kHashSlots - 1);
-                if (kEC) TP[s] = (int32_t)k;
-            }
-            __syncwarp();
-            for (uint64_t e = in0 + lane; e < in1; e += 32) {
-                const int32_t c = adj[e];
-                const uint64_t rc = off[c];
-                const int32_t* row = adj + rc;
-                const uint32_t lim = dplus[c];
-                // the lane's prefix scan, 4 ids per 16-byte load with the
-                // next load in flight (read from the 16-byte boundary at or
-                // below the row start; the padding after the last row keeps
-                // the up to 3 ids past lim in bounds)
-                uint32_t h = 0, i = lim;  // i: index of the first id >= b
-                const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(row) >> 2) & 3u;
-                const int4* q = reinterpret_cast<const int4*>(row - mis);
-                const uint32_t total = lim + mis;
-                int4 v = total ? __ldg(q) : make_int4(0, 0, 0, 0);
-                bool stop = false;
-                // one id of the prefix at index pos (masked outside [0, lim))
-                auto probe = [&](int32_t a, int64_t pos) {
-                    if (stop || pos < 0 || pos >= (int64_t)lim) return;
-                    if (a >= b) {
-                        stop = true;
-                        i = (uint32_t)pos;
-                        return;
-                    }
-                    uint32_t s = hash_slot(a);
-                    int32_t key;
-                    while ((key = T[s]) != -1) {
-                        if (key == a) {
-                            ++h;
-                            if (kVC) count_vertex(a, tri, hist);
-                            if (kEC) {
-                                atomicAdd(&ecnt[rc + pos], 1u);
-                                atomicAdd(&RC[TP[s]], 1u);
-                            }
-                            break;
-                        }
-                        s = (s + 1) & (kHashSlots - 1);
-                    }
-                };
-                for (uint32_t c0 = 0; c0 < total; c0 += 4) {
-                    const int4 vn = c0 + 4 < total ? __ldg(q + c0 / 4 + 1) : v;
-                    const int64_t p0 = (int64_t)c0 - (int64_t)mis;
-                    probe(v.x, p0);
-                    probe(v.y, p0 + 1);
-                    probe(v.z, p0 + 2);
-                    probe(v.w, p0 + 3);
-                    if (stop) break;
-                    v = vn;
-                }
-                cnt += h;
-                if (kVC && h) atomicAdd(&tri[c], (unsigned long long)h);
-                if (kEC && h && i < lim) atomicAdd(&ecnt[rc + i], h);  // row[i] == b
-            }
-            __syncwarp();
-            for (int s = lane; s < kHashSlots; s += 32) T[s] = -1;
-            if (kEC) {
-                for (uint32_t k = lane; k < dp; k += 32) {
-                    const uint32_t h = RC[k];
-                    if (h) {
-                        atomicAdd(&ecnt[rb + k], h);
-                        RC[k] = 0;
-                    }
-                }
-            }
-            __syncwarp();
-        } else if (MODE == kModeGallop) {
+        uint32_t* eb = kEC ? ecnt + slot_base(ooff, off, b) : nullptr;
+        if (MODE == kModeGallop) {
             for (uint64_t e = in0 + lane; e < in1; e += 32) {
                 const int32_t c = adj[e];
                 if (kEC) {
-                    const uint64_t rc = off[c];
-                    cnt += gallop_below_ec(adj + rc, dplus[c], nb, dp, b, ecnt + rc, ecnt + rb);
+                    cnt += gallop_below_ec(adj + off[c], dplus[c], nb, dp, b, ecnt + slot_base(ooff, off, c), eb);
                     continue;
                 }
                 const uint32_t h = gallop_below_vc<kVC>(adj + off[c], dplus[c], nb, dp, b, tri, hist);
@@ -655,8 +596,7 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
             for (uint64_t e = in0 + lane; e < in1; e += 32) {
                 const int32_t c = adj[e];
                 if (kEC) {
-                    const uint64_t rc = off[c];
-                    cnt += merge_below_ec(adj + rc, dplus[c], nb, dp, b, ecnt + rc, ecnt + rb);
+                    cnt += merge_below_ec(adj + off[c], dplus[c], nb, dp, b, ecnt + slot_base(ooff, off, c), eb);
                     continue;
                 }
                 const uint32_t h = merge_below_vc<kVC>(adj + off[c], dplus[c], nb, dp, b, tri, hist);
