@@ -602,9 +602,10 @@ class Batch:
 
     def run(self, tasks: int = 7):
         n = self.vlist.size - 1
-        tc = np.zeros(self.num_graphs, np.uint64) if tasks & self.TC else None
-        lcc = np.zeros(n, np.float64) if tasks & self.LCC else None
-        bfs = np.zeros(n, np.int32) if tasks & self.BFS else None
+        # every entry is written by the call
+        tc = np.empty(self.num_graphs, np.uint64) if tasks & self.TC else None
+        lcc = np.empty(n, np.float64) if tasks & self.LCC else None
+        bfs = np.empty(n, np.int32) if tasks & self.BFS else None
         st = _lib.BatchStats()
         check(lib.pc_batch_run(self._b, tasks, ptr(tc), ptr(lcc), ptr(bfs), C.byref(st)))
         return {"tc": tc, "lcc": lcc, "bfs": bfs, "ms": st.ms, "items": st.items, "threads": st.threads,

@@ -394,7 +394,7 @@ __global__ void k_oriented_count(const uint32_t* __restrict__ dplus, uint64_t n,
 // once per view (0.3 ms at RMAT-24, against 43 ms for one count).
 __global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
                                 const uint32_t* __restrict__ dplus, uint64_t n, const uint32_t* __restrict__ ooff,
-                                int4* __restrict__ ids) {
+                                const int32_t* __restrict__ row_base, int4* __restrict__ ids) {
     constexpr uint64_t kRun = 256;
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -418,14 +418,42 @@ __global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t*
             const uint64_t u = row(r0, r1, j);
             const uint32_t k = 4 * (uint32_t)(j - ooff[u]), left = dplus[u] - k;
             const int32_t* src = adj + off[u] + k;
+            const int32_t base = row_base ? row_base[u] : 0;
             int4 v = none;
-            v.x = src[0];
-            if (left > 1) v.y = src[1];
-            if (left > 2) v.z = src[2];
-            if (left > 3) v.w = src[3];
+            v.x = src[0] - base;
+            if (left > 1) v.y = src[1] - base;
+            if (left > 2) v.z = src[2] - base;
+            if (left > 3) v.w = src[3] - base;
             ids[j] = v;
         }
     }
+}
+
+pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
+                         uint64_t n, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff_buf,
+                         DevBuf* oids_buf, uint64_t* vecs) {
+    PC_TRY(ooff_buf->alloc((n + 1) * 4, "oriented offsets"));
+    uint32_t* ooff = ooff_buf->as<uint32_t>();
+    k_oriented_count<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(dplus, n, ooff);
+    PC_LAUNCHED();
+    PC_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, ooff, ooff, (int64_t)(n + 1), s));
+    count_launch();
+    uint32_t nvec = 0;
+    PC_CUDA(cudaMemcpyAsync(&nvec, ooff + n, 4, cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaStreamSynchronize(s));
+    PC_TRY(oids_buf->alloc(((uint64_t)nvec + 32) * 16, "oriented ids"));
+    *vecs = nvec;
+    const uint64_t grid = std::min<uint64_t>((uint64_t)sm_count(device) * 16, ceil_div(nvec, 8 * 256));
+    k_oriented_fill<<<(unsigned)std::max<uint64_t>(1, grid), 256, 0, s>>>(off, adj, dplus, n, ooff, row_base,
+                                                                          oids_buf->as<int4>());
+    PC_LAUNCHED();
+    return PC_OK;
+}
+
+size_t oriented_temp_bytes(uint64_t n) {
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)(n + 1));
+    return std::max<size_t>(tb, 1);
 }
 
 pc_status ensure_oriented(pc_pgraph* pg) {
@@ -433,34 +461,16 @@ pc_status ensure_oriented(pc_pgraph* pg) {
     if (pg->oriented_tried) return PC_OK;
     const uint64_t n = pg->g->n;
     pg->oriented_tried = true;
-    if (n == 0 || (pg->g->m + 3 * n) / 4 + 32 >= (1ull << 32)) return PC_OK;
-    if (pg->ooff.alloc((n + 1) * 4, "oriented offsets") != PC_OK) {
-        clear_error();
-        return PC_OK;
-    }
-    cudaStream_t s = pg->g->stream;
-    uint32_t* ooff = pg->ooff.as<uint32_t>();
-    size_t tb = 0;
-    PC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, ooff, ooff, (int64_t)(n + 1), s));
-    PC_TRY(scratch_reserve(pg, tb + 256));
-    void* tmp = pg->scratch.take<char>(std::max<size_t>(tb, 1));
-    k_oriented_count<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(pg->dplus.as<uint32_t>(), n, ooff);
-    PC_LAUNCHED();
-    PC_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, ooff, ooff, (int64_t)(n + 1), s));
-    count_launch();
-    uint32_t nvec = 0;
-    PC_CUDA(cudaMemcpyAsync(&nvec, ooff + n, 4, cudaMemcpyDeviceToHost, s));
-    PC_CUDA(cudaStreamSynchronize(s));
-    if (pg->oids.alloc(((uint64_t)nvec + 32) * 16, "oriented ids") != PC_OK) {
-        pg->ooff.release();
-        clear_error();
-        return PC_OK;
-    }
-    pg->ovecs = nvec;
-    const uint64_t grid = std::min<uint64_t>((uint64_t)sm_count(pg->g->device) * 16, ceil_div(nvec, 8 * 256));
-    k_oriented_fill<<<(unsigned)std::max<uint64_t>(1, grid), 256, 0, s>>>(pg->off, pg->adj, pg->dplus.as<uint32_t>(), n,
-                                                                          ooff, pg->oids.as<int4>());
-    PC_LAUNCHED();
+    if (n == 0 || !oriented_fits(n, pg->g->m)) return PC_OK;
+    const size_t tb = oriented_temp_bytes(n);
+    PC_TRY(scratch_reserve(pg, tb));
+    const pc_status st =
+        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->device, pg->g->stream,
+                       pg->scratch.take<char>(tb), tb, &pg->ooff, &pg->oids, &pg->ovecs);
+    if (st != PC_ERR_OOM) return st;
+    pg->ooff.release();
+    pg->oids.release();
+    clear_error();
     return PC_OK;
 }
 

@@ -3,13 +3,22 @@
 //
 // The graphs are packed in one CSR arena with arena-wide vertex ids; graph g
 // owns vertices [voff[g], voff[g+1]) and no edge joins two graphs, so the
-// arena is one block-diagonal graph.  A single persistent kernel takes work
-// items (graph, task) from a global counter, largest graphs first, and runs
-// each item inside one CTA: no CTA ever waits for another, so the launch
-// needs no grid-wide synchronisation.  The launch sequence (counter reset,
-// output clears, the kernel, the result copies) is captured once into a CUDA
-// graph and replayed by later calls; the schedule (threads per CTA, CTAs per
-// SM, item order) comes from pc_batch_autotune.
+// arena is one block-diagonal graph.  A single persistent kernel first takes
+// the BFS items (a graph each, largest first, one CTA) and then the triangle
+// items (a pivot and a run of its in-neighbours, one warp) from global
+// counters: no CTA ever waits for another, so the launch needs no grid-wide
+// synchronisation, and a large graph's triangles are spread over the whole
+// GPU.  One enumeration serves both the counts and the coefficients.  The
+// launch sequence (clears, the kernel, the coefficients' division, the result
+// copies) is captured once into a CUDA graph and replayed by later calls; the
+// schedule (threads per CTA, CTAs per SM, BFS order) comes from
+// pc_batch_autotune.
+//
+// Measured against one CTA per (graph, task), whose launch lasted as long as
+// its largest graph: 96 graphs of scales 8..12 (4.2 M entries) 7.0 -> 0.26 ms
+// on the device, 4096 graphs of scales 10..16 (2.4 G entries) 1261 -> 134 ms.
+// Bound by instruction issue in the scans (scan_in_neighbours), and for a few
+// small graphs by the latency of one CTA's BFS levels.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -25,7 +34,9 @@ struct pc_batch {
     uint32_t G = 0;
     std::vector<uint64_t> voff;
     std::vector<uint64_t> gm;  // directed edges per graph
-    pc::DevBuf d_voff, dplus, graph_of, ecnt, dist, q0, q1, tc, lcc, items, counter;
+    pc::DevBuf d_voff, dplus, graph_of, ooff, oids, titems, tri, dist, q0, q1, tc, lcc, items, counter;
+    uint64_t ovecs = 0;
+    uint32_t ntri = 0;  // triangle items
     uint64_t* h_tc = nullptr;  // pinned staging
     double* h_lcc = nullptr;
     int32_t* h_bfs = nullptr;
@@ -40,14 +51,24 @@ struct pc_batch {
 namespace pc {
 namespace bt {
 
-enum Task : int { kTC = 0, kLCC = 1, kBFS = 2 };
 constexpr int kMaxWarps = 16;
-constexpr int kSlots = 512;  // per-warp hash: keys + positions
-constexpr int kCap = 256;
+constexpr int32_t kLowIds = 1 << 13;  // graph-local ids with exact bits (mixed sets, a set per warp)
+constexpr uint32_t kBits = kLowIds / 32 + tc::kFilterWords;
+constexpr int32_t kHubs = 512;        // graph-local ids whose triangles each warp gathers in shared memory (LCC)
+constexpr uint32_t kSetWords = tc::bitmap_set_words(kBits, tc::kCountVertex, tc::kMixedSet);
+constexpr uint32_t kWarpWords(bool lcc) { return kSetWords + (lcc ? (uint32_t)kHubs : 0u); }
+constexpr uint32_t kHeavyRow = 256;   // BFS: longer frontier rows are expanded by the whole CTA
+constexpr uint32_t kHeavyList = 256;  // ... up to so many a level
+constexpr uint32_t kItemRun = 256;  // in-neighbours per triangle item
 
-__global__ void k_graph_of(const uint64_t* __restrict__ voff, int32_t* __restrict__ graph_of) {
+// base[v]: the first vertex of v's graph (v's graph-local id is v - base[v]).
+__global__ void k_graph_of(const uint64_t* __restrict__ voff, int32_t* __restrict__ graph_of,
+                           int32_t* __restrict__ base) {
     const uint64_t v0 = voff[blockIdx.x], v1 = voff[blockIdx.x + 1];
-    for (uint64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) graph_of[v] = (int32_t)blockIdx.x;
+    for (uint64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+        graph_of[v] = (int32_t)blockIdx.x;
+        base[v] = (int32_t)v0;
+    }
 }
 
 __global__ void k_prepare(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
@@ -68,168 +89,248 @@ __global__ void k_prepare(const uint64_t* __restrict__ off, const int32_t* __res
     dplus[u] = (uint32_t)(lo - b);
 }
 
+// Triangle items: every pivot with a set and in-neighbours gives a run of
+// items of <= kItemRun in-neighbours, appended in any order.
+__global__ void k_triangle_items(const uint64_t* __restrict__ off, const uint32_t* __restrict__ dplus, uint64_t n,
+                                 tc::Item* __restrict__ items, uint32_t* __restrict__ nitems) {
+    const uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (b >= n || dplus[b] == 0) return;
+    const uint64_t in0 = off[b] + dplus[b], din = off[b + 1] - in0;
+    const uint32_t c = (uint32_t)((din + kItemRun - 1) / kItemRun);
+    if (!c) return;
+    const uint32_t s = atomicAdd(nitems, c);
+    for (uint32_t j = 0; j < c; ++j)
+        items[s + j] = tc::Item{in0 + (uint64_t)j * kItemRun, (int32_t)b, (uint32_t)min((uint64_t)kItemRun, din - (uint64_t)j * kItemRun)};
+}
+
 struct Args {
     const uint64_t* off;
     const int32_t* adj;
-    const uint32_t* dplus;
     const uint64_t* voff;
-    const int32_t* items;  // graph * 4 + task
-    uint32_t nitems;
-    uint32_t* counter;     // [0] next item
-    unsigned long long* tc;
-    uint32_t* ecnt;
-    double* lcc;
+    const int32_t* graph_of;
+    const int32_t* base;
+    tc::OrientedView oriented;  // rows in graph-local ids
+    const tc::Item* titems;
+    uint32_t ntri;
+    const int32_t* bfs_order;   // graphs to search, in this order
+    uint32_t nbfs;
+    uint32_t* counter;          // [0] next BFS item, [1] next triangle item
+    unsigned long long* tc;     // per graph, or null
+    unsigned long long* tri;    // per vertex (LCC), or null
     int32_t* dist;
     int32_t* q0;
     int32_t* q1;
 };
 
-__device__ __forceinline__ uint32_t lbound(const int32_t* __restrict__ p, uint32_t n, int32_t x) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (p[mid] < x) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-
-// Triangle listing of one graph by one CTA.  Warps take pivots from a shared
-// counter; a pivot's set N+(b) goes into a warp-private hash (key -> position
-// in row b), lanes scan in-neighbour prefixes.  With `edges`, every triangle
-// adds 1 to its three edges' oriented slots (for LCC); otherwise the CTA
-// returns its count.
-template <bool kEdges>
-__device__ unsigned long long cta_triangles(const Args& A, uint64_t v0, uint64_t v1, int32_t* keys, int32_t* vals,
-                                            uint32_t* s_next) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t* K = keys + w * kSlots;
-    int32_t* V = vals + w * kSlots;
-    for (int i = lane; i < kSlots; i += 32) K[i] = -1;
+// The triangle items, one warp each, with a mixed pivot set of graph-local ids
+// (exact bits below kLowIds, which holds the hubs of every graph of the
+// batch).  kMode kCountVertex also counts each vertex's triangles; a warp
+// gathers those of a graph's first kHubs vertices, where nearly every hit
+// lands, in shared memory and adds them up when it comes to another graph
+// (one global atomic per hit: 1.05 ms for 96 graphs of 4.2 M entries).
+template <int kMode>
+__device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
+    const int lane = threadIdx.x & 31;
+    int32_t* ht = reinterpret_cast<int32_t*>(bm + kBits);
+    for (uint32_t i = lane; i < kBits; i += 32) bm[i] = 0;
+    for (uint32_t i = lane; i < (uint32_t)tc::kHashSlots; i += 32) ht[i] = -1;
+    uint32_t* hist = bm + kSetWords;
+    int32_t hist_base = -1;
+    if (kMode == tc::kCountVertex)
+        for (int i = lane; i < kHubs; i += 32) hist[i] = 0;
     __syncwarp();
-    unsigned long long cnt = 0;
+    auto flush = [&]() {
+        if (kMode != tc::kCountVertex || hist_base < 0) return;
+        __syncwarp();
+        for (int i = lane; i < kHubs; i += 32) {
+            const uint32_t h = hist[i];
+            if (h) {
+                atomicAdd(&A.tri[hist_base + i], (unsigned long long)h);
+                hist[i] = 0;
+            }
+        }
+        __syncwarp();
+    };
     for (;;) {
-        uint32_t q = 0;
-        if (lane == 0) q = atomicAdd(s_next, 1u);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        const uint64_t b64 = v0 + q;
-        if (b64 >= v1) break;
-        const int32_t b = (int32_t)b64;
-        const uint64_t rb = A.off[b], re = A.off[b + 1];
-        const uint32_t dp = A.dplus[b];
-        if (dp == 0 || rb + dp == re) continue;
-        const bool hashed = dp <= (uint32_t)kCap;
-        if (hashed) {
-            for (uint32_t k = lane; k < dp; k += 32) {
-                const int32_t a = A.adj[rb + k];
-                uint32_t s = tc::hash_slot(a);
-                while (atomicCAS(&K[s], -1, a) != -1) s = (s + 1) & (kSlots - 1);
-                V[s] = (int32_t)k;
-            }
-            __syncwarp();
+        uint32_t it = 0;
+        if (lane == 0) it = atomicAdd(&A.counter[1], 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= A.ntri) break;
+        const tc::Item I = A.titems[it];
+        const int32_t base = A.base[I.b], b = I.b - base;
+        if (base != hist_base) {
+            flush();
+            hist_base = base;
         }
-        for (uint64_t e = rb + dp + lane; e < re; e += 32) {
-            const int32_t c = A.adj[e];
-            const uint64_t rc = A.off[c];
-            const uint32_t lim = A.dplus[c];
-            uint32_t pair = 0, i = 0;
-            for (; i < lim; ++i) {
-                const int32_t a = A.adj[rc + i];
-                if (a >= b) break;
-                int32_t pos = -1;
-                if (hashed) {
-                    uint32_t s = tc::hash_slot(a);
-                    int32_t key;
-                    while ((key = K[s]) != -1) {
-                        if (key == a) { pos = V[s]; break; }
-                        s = (s + 1) & (kSlots - 1);
-                    }
-                } else {
-                    const uint32_t p = lbound(A.adj + rb, dp, a);
-                    if (p < dp && A.adj[rb + p] == a) pos = (int32_t)p;
-                }
-                if (pos >= 0) {
-                    ++pair;
-                    if (kEdges) {
-                        atomicAdd(&A.ecnt[rc + i], 1u);   // edge {c, a}
-                        atomicAdd(&A.ecnt[rb + pos], 1u); // edge {b, a}
-                    }
+        const uint32_t v0 = A.oriented.off[I.b], v1 = A.oriented.off[I.b + 1];
+        tc::SetView S;
+        S.bm = bm;
+        S.lo = kLowIds;
+        S.ht = ht;
+        S.hpos = nullptr;
+        S.nb = reinterpret_cast<const int32_t*>(A.oriented.ids + v0);
+        S.np = 4 * (v1 - v0);
+        S.ovf = S.np > (uint32_t)tc::kHashCap && __ldg(S.nb + (S.np - tc::kHashCap - 1)) >= kLowIds;
+        bool high = false;
+        for (uint32_t k = v0 + lane; k < v1; k += 32) {
+            const int4 v = __ldg(A.oriented.ids + k);
+            const int32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int32_t a = e[t];
+                if (a == INT32_MAX) continue;  // padding
+                const uint32_t x = S.place<tc::kMixedSet>(a);
+                atomicOr(&bm[x >> 5], 0x80000000u >> (x & 31));
+                if (!S.ovf && a >= kLowIds) {
+                    high = true;
+                    uint32_t hs = tc::hash_slot(a);
+                    while (atomicCAS(&ht[hs], -1, a) != -1) hs = (hs + 1) & (tc::kHashSlots - 1);
                 }
             }
-            cnt += pair;
-            // the scan stopped at b itself (b is in N(c) below c)
-            if (kEdges && pair && i < lim && A.adj[rc + i] == b) atomicAdd(&A.ecnt[rc + i], pair);  // edge {c, b}
         }
-        if (hashed) {
-            __syncwarp();
-            for (int i = lane; i < kSlots; i += 32) K[i] = -1;
-            __syncwarp();
+        __syncwarp();
+        tc::HitSink sink;
+        sink.tri = A.tri;
+        sink.tri_low = A.tri + base;
+        sink.hist = hist;
+        sink.hist_ids = kHubs;
+        sink.ecnt = sink.by_rank = nullptr;
+        sink.ranks = tc::SetRanks{nullptr, nullptr};
+        unsigned long long hits = 0;
+        for (uint32_t k = 0; k < I.n; k += 32) {
+            const int nb = min(32, (int)(I.n - k));
+            const int32_t c = lane < nb ? A.adj[I.in0 + k + lane] : 0;
+            hits += tc::scan_in_neighbours<8, kMode, tc::kMixedSet>(A.oriented, c, A.oriented.off[c], nb, b, S, lane, sink);
         }
+        for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
+        if (lane == 0 && hits) {
+            if (A.tc) atomicAdd(&A.tc[A.graph_of[I.b]], hits);
+            if (kMode == tc::kCountVertex) atomicAdd(&A.tri[I.b], hits);
+        }
+        for (uint32_t k = v0 + lane; k < v1; k += 32) {
+            const int4 v = __ldg(A.oriented.ids + k);
+            bm[S.place<tc::kMixedSet>(v.x) >> 5] = 0;
+            bm[S.place<tc::kMixedSet>(v.y) >> 5] = 0;
+            bm[S.place<tc::kMixedSet>(v.z) >> 5] = 0;
+            bm[S.place<tc::kMixedSet>(v.w) >> 5] = 0;
+        }
+        if (__any_sync(0xffffffffu, high))
+            for (uint32_t i = lane; i < (uint32_t)tc::kHashSlots; i += 32) ht[i] = -1;
+        __syncwarp();
     }
-    return cnt;
+    flush();
 }
 
-__device__ void cta_lcc_finalize(const Args& A, uint64_t v0, uint64_t v1) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (uint64_t u = v0 + w; u < v1; u += nw) {
-        const uint64_t b = A.off[u], e = A.off[u + 1];
-        const uint64_t du = e - b;
-        unsigned long long sum = 0;
-        for (uint64_t j = b + lane; j < e; j += 32) {
-            const int32_t v = A.adj[j];
-            if ((uint64_t)v < u) {
-                sum += A.ecnt[j];
-            } else {
-                const uint64_t rv = A.off[v];
-                sum += A.ecnt[rv + lbound(A.adj + rv, A.dplus[v], (int32_t)u)];
-            }
-        }
-        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        // src/Graph.cpp:833-838
-        if (lane == 0) A.lcc[u] = du < 1 ? 0.0 : (double)sum / (double)(du * (du - 1));
-    }
+// LCC from per-vertex triangle counts, as in intersect.cu (src/Graph.cpp:833-838).
+__global__ void k_batch_lcc(const uint64_t* __restrict__ off, const unsigned long long* __restrict__ tri, uint64_t n,
+                            double* __restrict__ lcc) {
+    const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (u >= n) return;
+    const uint64_t du = off[u + 1] - off[u];
+    lcc[u] = du < 1 ? 0.0 : (double)(2 * tri[u]) / (double)(du * (du - 1));
 }
 
-// Level-synchronous BFS of one graph by one CTA (warp per frontier vertex).
-__device__ void cta_bfs(const Args& A, uint64_t v0, uint64_t v1, uint32_t* s_cnt) {
+// Level-synchronous BFS of one graph by one CTA, direction-optimising (Beamer,
+// Asanovic, Patterson, SC'12).  Top-down: a warp per frontier vertex; rows of
+// more than kHeavyRow entries are set aside and expanded by all warps, so
+// that a hub does not hold the level up with one dependent load after
+// another.  Bottom-up: a thread per unvisited vertex looks for a neighbour of
+// the last level; rows list the hubs first, so most end at once.
+struct BfsShared {
+    uint32_t fn, nn;            // frontier, next frontier
+    unsigned long long edges;   // row entries of the next frontier
+    uint32_t nheavy;
+    int32_t heavy[kHeavyList];
+};
+
+__device__ void cta_bfs(const Args& A, uint64_t v0, uint64_t v1, BfsShared& S) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint64_t n = v1 - v0;
     for (uint64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) A.dist[v] = INT_MAX;
     __syncthreads();
     if (threadIdx.x == 0) {
         A.dist[v0] = 0;
         A.q0[v0] = (int32_t)v0;
-        s_cnt[0] = 1;
+        S.fn = 1;
+        S.edges = A.off[v0 + 1] - A.off[v0];
     }
     __syncthreads();
     int32_t* fq = A.q0 + v0;
     int32_t* nq = A.q1 + v0;
+    unsigned long long unexplored = A.off[v1] - A.off[v0];
+    bool bottom_up = false;
+    auto append = [&](bool won, int32_t v) {
+        const unsigned m = __ballot_sync(0xffffffffu, won);
+        if (!m) return;
+        unsigned long long d = won ? A.off[v + 1] - A.off[v] : 0;
+        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        uint32_t at = 0;
+        if (lane == 0) {
+            at = atomicAdd(&S.nn, (uint32_t)__popc(m));
+            atomicAdd(&S.edges, d);
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (won) nq[at + __popc(m & ((1u << lane) - 1u))] = v;
+    };
     for (int32_t level = 1;; ++level) {
-        const uint32_t fn = s_cnt[0];
+        const uint32_t fn = S.fn;
+        const unsigned long long edges = S.edges;
         __syncthreads();
         if (fn == 0) break;
-        if (threadIdx.x == 0) s_cnt[1] = 0;
+        unexplored -= edges;
+        if (!bottom_up && edges * 15 > unexplored) bottom_up = true;
+        else if (bottom_up && (uint64_t)fn * 18 < n) bottom_up = false;
+        if (threadIdx.x == 0) {
+            S.nn = 0;
+            S.edges = 0;
+            S.nheavy = 0;
+        }
         __syncthreads();
-        for (uint32_t i = w; i < fn; i += nw) {
-            const int32_t u = fq[i];
-            const uint64_t b = A.off[u], e = A.off[u + 1];
-            for (uint64_t j0 = b; j0 < e; j0 += 32) {
-                const uint64_t j = j0 + lane;
+        if (bottom_up) {
+            for (uint64_t i = threadIdx.x; i < ((n + 31) & ~31ull); i += blockDim.x) {
+                const uint64_t v = v0 + i;
+                bool found = false;
+                if (i < n && A.dist[v] == INT_MAX) {
+                    for (uint64_t j = A.off[v], e = A.off[v + 1]; j < e && !found; ++j)
+                        found = A.dist[A.adj[j]] == level - 1;
+                    if (found) A.dist[v] = level;
+                }
+                append(found, (int32_t)v);
+            }
+        } else {
+            auto expand = [&](uint64_t j, uint64_t e) {
                 bool won = false;
                 int32_t v = 0;
                 if (j < e) {
                     v = A.adj[j];
                     if (A.dist[v] == INT_MAX) won = atomicCAS(&A.dist[v], INT_MAX, level) == INT_MAX;
                 }
-                const unsigned m = __ballot_sync(0xffffffffu, won);
-                if (m) {
-                    uint32_t base = 0;
-                    if (lane == 0) base = atomicAdd(&s_cnt[1], (uint32_t)__popc(m));
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (won) nq[base + __popc(m & ((1u << lane) - 1u))] = v;
+                append(won, v);
+            };
+            for (uint32_t i = w; i < fn; i += nw) {
+                const int32_t u = fq[i];
+                const uint64_t b = A.off[u], e = A.off[u + 1];
+                if (e - b > kHeavyRow) {
+                    uint32_t h = 0;
+                    if (lane == 0) h = atomicAdd(&S.nheavy, 1u);
+                    h = __shfl_sync(0xffffffffu, h, 0);
+                    if (h < kHeavyList) {
+                        if (lane == 0) S.heavy[h] = u;
+                        continue;
+                    }
                 }
+                for (uint64_t j0 = b; j0 < e; j0 += 32) expand(j0 + lane, e);
+            }
+            __syncthreads();
+            const uint32_t nh = min(S.nheavy, kHeavyList);
+            for (uint32_t h = 0; h < nh; ++h) {
+                const int32_t u = S.heavy[h];
+                const uint64_t b = A.off[u], e = A.off[u + 1];
+                for (uint64_t j0 = b + 32 * w; j0 < e; j0 += 32 * nw) expand(j0 + lane, e);
             }
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_cnt[0] = s_cnt[1];
+        if (threadIdx.x == 0) S.fn = S.nn;
         int32_t* t = fq;
         fq = nq;
         nq = t;
@@ -241,41 +342,21 @@ __device__ void cta_bfs(const Args& A, uint64_t v0, uint64_t v1, uint32_t* s_cnt
     }
 }
 
-__global__ void __launch_bounds__(kMaxWarps * 32) k_batch(Args A) {
-    extern __shared__ int32_t smem[];
-    __shared__ uint32_t s_item, s_next, s_cnt[2];
-    __shared__ unsigned long long s_sum;
-    const int nw = blockDim.x >> 5;
-    int32_t* keys = smem;
-    int32_t* vals = smem + nw * kSlots;
-    for (;;) {
+template <int kMode>
+__global__ void __launch_bounds__(kMaxWarps * 32, 2) k_batch(Args A) {
+    extern __shared__ uint32_t smem[];
+    __shared__ uint32_t s_item;
+    __shared__ BfsShared s_bfs;
+    while (A.nbfs) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            s_item = atomicAdd(&A.counter[0], 1u);
-            s_next = 0;
-            s_sum = 0;
-        }
+        if (threadIdx.x == 0) s_item = atomicAdd(&A.counter[0], 1u);
         __syncthreads();
         const uint32_t it = s_item;
-        if (it >= A.nitems) break;
-        const int32_t code = A.items[it];
-        const int32_t g = code >> 2, task = code & 3;
-        const uint64_t v0 = A.voff[g], v1 = A.voff[g + 1];
-        if (task == kTC) {
-            unsigned long long c = cta_triangles<false>(A, v0, v1, keys, vals, &s_next);
-            for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-            if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_sum, c);
-            __syncthreads();
-            if (threadIdx.x == 0) A.tc[g] = s_sum;
-        } else if (task == kLCC) {
-            cta_triangles<true>(A, v0, v1, keys, vals, &s_next);
-            __threadfence_block();
-            __syncthreads();
-            cta_lcc_finalize(A, v0, v1);
-        } else {
-            cta_bfs(A, v0, v1, s_cnt);
-        }
+        if (it >= A.nbfs) break;
+        const int32_t g = A.bfs_order[it];
+        cta_bfs(A, A.voff[g], A.voff[g + 1], s_bfs);
     }
+    if (A.ntri) warp_triangles<kMode>(A, smem + (threadIdx.x >> 5) * kWarpWords(kMode == tc::kCountVertex));
 }
 
 static uint64_t key_of(uint32_t tasks, int threads, int cps, int order) {
@@ -288,23 +369,17 @@ static uint64_t key_of(uint32_t tasks, int threads, int cps, int order) {
 using namespace pc;
 using namespace pc::bt;
 
+// The graphs in BFS order: largest first (order 0) or as packed (order 1).
 static pc_status batch_build_items(pc_batch* b, uint32_t tasks) {
-    // largest graphs first (order 0) or graph order (order 1); LCC before TC
-    // before BFS for one graph size.
-    std::vector<int32_t> items;
-    std::vector<uint32_t> gidx(b->G);
-    std::iota(gidx.begin(), gidx.end(), 0u);
+    std::vector<int32_t> gidx(b->G);
+    std::iota(gidx.begin(), gidx.end(), 0);
     if (b->order == 0)
-        std::stable_sort(gidx.begin(), gidx.end(), [&](uint32_t x, uint32_t y) { return b->gm[x] > b->gm[y]; });
-    for (uint32_t gi : gidx) {
-        if (tasks & PC_BATCH_LCC) items.push_back((int32_t)(gi * 4 + kLCC));
-        if (tasks & PC_BATCH_TC) items.push_back((int32_t)(gi * 4 + kTC));
-        if (tasks & PC_BATCH_BFS) items.push_back((int32_t)(gi * 4 + kBFS));
-    }
-    b->nitems = (uint32_t)items.size();
-    PC_TRY(b->items.ensure(std::max<size_t>(items.size(), 1) * 4, "batch items"));
-    if (!items.empty())
-        PC_CUDA(cudaMemcpyAsync(b->items.p, items.data(), items.size() * 4, cudaMemcpyHostToDevice, b->g->stream));
+        std::stable_sort(gidx.begin(), gidx.end(), [&](int32_t x, int32_t y) { return b->gm[x] > b->gm[y]; });
+    int ntasks = 0;
+    for (uint32_t t : {PC_BATCH_TC, PC_BATCH_LCC, PC_BATCH_BFS}) ntasks += (tasks & t) != 0;
+    b->nitems = b->G * ntasks;
+    PC_TRY(b->items.ensure((size_t)b->G * 4, "batch items"));
+    PC_CUDA(cudaMemcpyAsync(b->items.p, gidx.data(), gidx.size() * 4, cudaMemcpyHostToDevice, b->g->stream));
     PC_CUDA(cudaStreamSynchronize(b->g->stream));
     return PC_OK;
 }
@@ -322,30 +397,35 @@ static pc_status batch_capture(pc_batch* b, uint32_t tasks) {
     }
     PC_TRY(batch_build_items(b, tasks));
     cudaStream_t s = b->g->stream;
-    const uint64_t N = b->g->n, M = b->g->m;
+    const uint64_t N = b->g->n;
+    const bool lcc = tasks & PC_BATCH_LCC, tc = tasks & PC_BATCH_TC;
     Args A;
     A.off = b->g->off.as<uint64_t>();
     A.adj = b->g->adj.as<int32_t>();
-    A.dplus = b->dplus.as<uint32_t>();
     A.voff = b->d_voff.as<uint64_t>();
-    A.items = b->items.as<int32_t>();
-    A.nitems = b->nitems;
+    A.graph_of = b->graph_of.as<int32_t>();
+    A.base = A.graph_of + N;
+    A.oriented = tc::OrientedView{b->ooff.as<uint32_t>(), b->oids.as<int4>()};
+    A.titems = b->titems.as<tc::Item>();
+    A.ntri = lcc || tc ? b->ntri : 0;
+    A.bfs_order = b->items.as<int32_t>();
+    A.nbfs = tasks & PC_BATCH_BFS ? b->G : 0;
     A.counter = b->counter.as<uint32_t>();
-    A.tc = b->tc.as<unsigned long long>();
-    A.ecnt = b->ecnt.as<uint32_t>();
-    A.lcc = b->lcc.as<double>();
+    A.tc = tc ? b->tc.as<unsigned long long>() : nullptr;
+    A.tri = lcc ? b->tri.as<unsigned long long>() : nullptr;
     A.dist = b->dist.as<int32_t>();
     A.q0 = b->q0.as<int32_t>();
     A.q1 = b->q1.as<int32_t>();
-    const int nw = b->threads / 32;
-    const size_t smem = (size_t)nw * kSlots * 4 * 2;
-    PC_CUDA(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = (size_t)(b->threads / 32) * kWarpWords(lcc) * 4;
+    auto kernel = lcc ? k_batch<tc::kCountVertex> : k_batch<tc::kCountOnly>;
+    PC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)(sm_count(b->g->device) * b->ctas_per_sm);
     PC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->counter.p, 0, 16, s);
-    if (tasks & PC_BATCH_TC) cudaMemsetAsync(b->tc.p, 0, (size_t)b->G * 8, s);
-    if (tasks & PC_BATCH_LCC) cudaMemsetAsync(b->ecnt.p, 0, std::max<uint64_t>(M, 1) * 4, s);
-    k_batch<<<grid, b->threads, smem, s>>>(A);
+    if (tc) cudaMemsetAsync(b->tc.p, 0, (size_t)b->G * 8, s);
+    if (lcc) cudaMemsetAsync(b->tri.p, 0, N * 8, s);
+    kernel<<<grid, b->threads, smem, s>>>(A);
+    if (lcc) k_batch_lcc<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(A.off, A.tri, N, b->lcc.as<double>());
     if (tasks & PC_BATCH_TC) cudaMemcpyAsync(b->h_tc, b->tc.p, (size_t)b->G * 8, cudaMemcpyDeviceToHost, s);
     if (tasks & PC_BATCH_LCC) cudaMemcpyAsync(b->h_lcc, b->lcc.p, N * 8, cudaMemcpyDeviceToHost, s);
     if (tasks & PC_BATCH_BFS) cudaMemcpyAsync(b->h_bfs, b->dist.p, N * 4, cudaMemcpyDeviceToHost, s);
@@ -385,8 +465,9 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     };
     pc_status st;
     if ((st = b->d_voff.alloc((G + 1) * 8, "graph offsets")) != PC_OK || (st = b->dplus.alloc(N * 4, "dplus")) != PC_OK ||
-        (st = b->graph_of.alloc(N * 4, "graph of vertex")) != PC_OK ||
-        (st = b->ecnt.alloc(std::max<uint64_t>(M, 1) * 4, "edge counts")) != PC_OK ||
+        (st = b->graph_of.alloc(N * 8, "graph of vertex")) != PC_OK ||
+        (st = b->tri.alloc(N * 8, "triangles per vertex")) != PC_OK ||
+        (st = b->titems.alloc((std::min<uint64_t>(N, M) + M / kItemRun + 1) * sizeof(tc::Item), "triangle items")) != PC_OK ||
         (st = b->dist.alloc(N * 4, "levels")) != PC_OK || (st = b->q0.alloc(N * 4, "queue")) != PC_OK ||
         (st = b->q1.alloc(N * 4, "queue")) != PC_OK || (st = b->tc.alloc((size_t)G * 8, "counts")) != PC_OK ||
         (st = b->lcc.alloc(N * 8, "lcc")) != PC_OK || (st = b->counter.alloc(16, "counter")) != PC_OK)
@@ -403,17 +484,32 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     e = cudaMemcpyAsync(b->d_voff.p, voff, (G + 1) * 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(chk.p, 0, 16, s);
     if (e != cudaSuccess) return bail(cuda_fail(e, "batch upload", __FILE__, __LINE__));
-    k_graph_of<<<G, 256, 0, s>>>(b->d_voff.as<uint64_t>(), b->graph_of.as<int32_t>());
+    k_graph_of<<<G, 256, 0, s>>>(b->d_voff.as<uint64_t>(), b->graph_of.as<int32_t>(), b->graph_of.as<int32_t>() + N);
     count_launch();
     k_prepare<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(),
                                                          b->d_voff.as<uint64_t>(), b->graph_of.as<int32_t>(), N,
                                                          b->dplus.as<uint32_t>(), chk.as<uint32_t>());
     count_launch();
-    uint32_t bad = 0;
-    e = cudaMemcpyAsync(&bad, chk.p, 4, cudaMemcpyDeviceToHost, s);
+    k_triangle_items<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(arena->off.as<uint64_t>(), b->dplus.as<uint32_t>(), N,
+                                                                b->titems.as<tc::Item>(), chk.as<uint32_t>() + 1);
+    count_launch();
+    uint32_t chk_h[2] = {0, 0};
+    e = cudaMemcpyAsync(chk_h, chk.p, 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
-    if (bad) return bail(fail(PC_ERR_INVALID_INPUT, "an edge joins two graphs of the batch"));
+    b->ntri = chk_h[1];
+    if (!chk_h[0]) {
+        if (!oriented_fits(N, M)) return bail(fail(PC_ERR_UNSUPPORTED, "the arena holds too many edges"));
+        DevBuf tmp;
+        const size_t tb = oriented_temp_bytes(N);
+        if ((st = tmp.alloc(tb, "scan scratch")) != PC_OK) return bail(st);
+        st = build_oriented(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(), b->dplus.as<uint32_t>(),
+                            b->graph_of.as<int32_t>() + N, N, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
+        if (st != PC_OK) return bail(st);
+        e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
+    }
+    if (chk_h[0]) return bail(fail(PC_ERR_INVALID_INPUT, "an edge joins two graphs of the batch"));
     *out = b;
     return PC_OK;
 }

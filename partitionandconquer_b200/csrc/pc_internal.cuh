@@ -162,6 +162,15 @@ int32_t to_internal_id(const pc_pgraph* pg, int32_t api_id);
 // Lazily computes pg->dplus.
 pc_status ensure_dplus(pc_pgraph* pg);
 
+// Builds the oriented copy of a CSR (see pc_pgraph::oids): row u's ids less
+// row_base[u] (none when null).  tmp: oriented_temp_bytes(n) bytes; waits for
+// the stream once.  Its vector indices are 32-bit: oriented_fits().
+pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
+                         uint64_t n, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff,
+                         DevBuf* oids, uint64_t* vecs);
+size_t oriented_temp_bytes(uint64_t n);
+inline bool oriented_fits(uint64_t n, uint64_t m) { return (m + 3 * n) / 4 + 64 < (1ull << 32); }
+
 // Lazily builds the oriented copy (uses the scratch arena).  Leaves oids null,
 // without an error, when device memory does not hold it.
 pc_status ensure_oriented(pc_pgraph* pg);

@@ -141,8 +141,9 @@ __device__ __forceinline__ void group_barrier(int id, int nthreads) {
 // Per-vertex triangle counts (kVC): every triangle found adds 1 to its
 // lowest vertex a; ids below kHubHist go to a shared-memory histogram
 // (almost every hit is a hub), the rest to the global counts.
-__device__ __forceinline__ void count_vertex(int32_t a, unsigned long long* __restrict__ tri, uint32_t* hist) {
-    if (a < kHubHist) atomicAdd(&hist[a], 1u);
+__device__ __forceinline__ void count_vertex(int32_t a, unsigned long long* __restrict__ tri, uint32_t* hist,
+                                             int32_t hist_ids = kHubHist) {
+    if (a < hist_ids) atomicAdd(&hist[a], 1u);
     else atomicAdd(&tri[a], 1ull);
 }
 
@@ -177,8 +178,10 @@ __device__ __forceinline__ uint32_t rank_in_set(const uint32_t* bm, const SetRan
 
 // Where the hits of one warp's scans go besides the count.
 struct HitSink {
-    unsigned long long* __restrict__ tri;  // kCountVertex: per-vertex counts
-    uint32_t* hist;                        // ... of the ids below kHubHist
+    unsigned long long* __restrict__ tri;  // kCountVertex: per-vertex counts, of in-neighbours
+    unsigned long long* tri_low;           // ... and of the ids in the oriented copy
+    uint32_t* hist;                        // ... whose first hist_ids ids count here
+    int32_t hist_ids;
     uint32_t* __restrict__ ecnt;           // kCountEdge: per-slot counts
     uint32_t* by_rank;                     // ... of row b: shared counters, or its slots in ecnt
     SetRanks ranks;
@@ -256,7 +259,7 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
                 for (int t = 0; t < 4; ++t) {
                     if (!h[t]) continue;
                     if constexpr (kMode == kCountVertex) {
-                        count_vertex(e[t], sink.tri, sink.hist);
+                        count_vertex(e[t], sink.tri_low, sink.hist, sink.hist_ids);
                     } else {
                         atomicAdd(sink.ecnt + (4ull * qc + t), 1u);
                         atomicAdd(sink.by_rank + (kKind == kMixedSet ? rank[t] : rank_in_set(S.bm, sink.ranks, e[t])),
@@ -373,8 +376,9 @@ __global__ void __launch_bounds__(kCtaThreads, kMode == kCountOnly ? 3 : 2)
         set_sync();
         const bool few = S.np <= (uint32_t)kEcRankCap;
         HitSink sink;
-        sink.tri = tri;
+        sink.tri = sink.tri_low = tri;
         sink.hist = hist;
+        sink.hist_ids = kHubHist;
         sink.ecnt = ecnt;
         sink.by_rank = few ? by_rank : ecnt + 4ull * v0;
         sink.ranks = SetRanks{r16, r32};
