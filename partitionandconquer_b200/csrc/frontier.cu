@@ -14,6 +14,7 @@
 #include "grid_sync.cuh"
 #include "pc_internal.cuh"
 #include "synth_rng.h"
+#include "tile_expand.cuh"
 
 namespace pc {
 namespace fr {
@@ -217,138 +218,214 @@ __global__ void k_bfs_finish(const int32_t* __restrict__ dist, uint64_t n, int32
 //
 // Both forms relax the rows of a frontier with atomicMin and queue every
 // vertex whose distance falls; they differ in which improved vertices are
-// relaxed next.  Bellman-Ford (kDelta = false) relaxes all of them in the
-// next round.  Delta-stepping (kDelta = true; Meyer and Sanders, "Delta-
-// stepping: a parallelizable shortest path algorithm", J. Algorithms 2003, in
-// the near/far-pile form of Davidson, Baxter, Garland and Owens, IPDPS 2014)
+// relaxed next.  Bellman-Ford (an unbounded bucket) relaxes all of them in the
+// next step.  Delta-stepping (Meyer and Sanders, "Delta-stepping: a
+// parallelizable shortest path algorithm", J. Algorithms 2003, in the
+// near/far-pile form of Davidson, Baxter, Garland and Owens, IPDPS 2014)
 // relaxes only vertices whose new distance is below the current bucket's
 // upper bound `thr` ("near"); the others go to a far pile that is split when
 // the bucket is exhausted.  Both are label-correcting: every improvement is
 // queued, so both end at the exact shortest distances (integer weights >= 0).
-struct SsspPush {
-    int32_t thr;                 // delta-stepping: near bound (exclusive)
-    int32_t* __restrict__ far;   // far pile and its length
-    uint32_t* __restrict__ farn;
-    int32_t* __restrict__ farflag;  // 1 while the vertex is in the far pile
+//
+// One persistent kernel runs all steps, a grid barrier between them, so a
+// bucket costs microseconds instead of launches and host reads, and narrow
+// buckets, which relax fewer edges in vain, pay.  A step is a relaxation of
+// the near frontier (tx::expand) or, when that is empty, the split of the far
+// pile.  Steps keep their state in three rotating records (see KState).
+//
+// Bound at RMAT-22 (6.1 -> 2.6-2.8 ms a call, 0.3 ms of it the copy back): the
+// gathers of the neighbours' distances, 2.9 m of them, from L1 and L2.
+struct __align__(16) SsspState {
+    uint32_t nl, nh;  // near queues' lengths
+    int32_t thr;      // near bound (exclusive)
+    int32_t par;      // near queues in use
+    int32_t splits;   // splits so far: the far pile is far[splits % 2], its counters those of splits % 3
+    int32_t pad[3];
+};
+struct SsspFar {
+    uint32_t n[3];
+    int32_t min[3];  // a bound on the pile's smallest distance
 };
 
-template <bool kDelta>
-__device__ __forceinline__ void sssp_relax_edge(int32_t du, int32_t v, int32_t wt, int32_t* __restrict__ dist,
-                                                int32_t* __restrict__ flag, const SsspPush& P, bool* near,
-                                                bool* far) {
-    const int32_t nd = du + wt;
-    if (nd < dist[v]) {
-        const int32_t old = atomicMin(&dist[v], nd);
-        if (nd < old) {
-            if (!kDelta || nd < P.thr) *near = atomicExch(&flag[v], 1) == 0;
-            else *far = atomicExch(&P.farflag[v], 1) == 0;
+// dist, stamps and flags cleared; the source queued.
+__global__ void k_sssp_init(const uint64_t* __restrict__ off, uint64_t n, int32_t src, int32_t bound,
+                            const int32_t* __restrict__ delta, int32_t* __restrict__ dist, int32_t* __restrict__ stamp,
+                            int32_t* __restrict__ farflag, tx::Queues Q, SsspState* S, SsspFar* F) {
+    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
+        dist[u] = u == (uint64_t)src ? 0 : INT_MAX / 2;  // src/test.cpp:202-203
+        stamp[u] = 0;
+        farflag[u] = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        if (threadIdx.x < 3) {
+            S[threadIdx.x] = SsspState{0, 0, bound ? bound : *delta, 0, 0, {0, 0, 0}};
+            F->n[threadIdx.x] = 0;
+            F->min[threadIdx.x] = INT_MAX;
         }
+        __syncwarp();
+        tx::enqueue(threadIdx.x == 0, src, off, Q, &S[0].nl, &S[0].nh);
     }
 }
 
-template <bool kDelta>
-__global__ void k_sssp_relax(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                             const int32_t* __restrict__ w, const int32_t* __restrict__ fq, uint32_t fn,
-                             int32_t* __restrict__ dist, int32_t* __restrict__ flag, int32_t* __restrict__ nq,
-                             uint32_t* __restrict__ nn, int32_t* __restrict__ hq, uint32_t* __restrict__ hn,
-                             SsspPush P) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = warp; i < fn; i += nwarps) {
-        const int32_t u = fq[i];
-        const uint64_t b = off[u], e = off[u + 1];
-        if (e - b > kHeavyDeg) {  // relaxed by k_sssp_relax_heavy
-            if (lane == 0) hq[atomicAdd(hn, 1u)] = u;
-            continue;
-        }
-        const int32_t du = dist[u];
-        for (uint64_t j0 = b; j0 < e; j0 += 32) {
-            const uint64_t j = j0 + lane;
-            bool near = false, far = false;
-            int32_t v = 0;
-            if (j < e) {
-                v = adj[j];
-                sssp_relax_edge<kDelta>(du, v, w[j], dist, flag, P, &near, &far);
-            }
-            warp_append(near, v, nq, nn);
-            if (kDelta) warp_append(far, v, P.far, P.farn);
-        }
-    }
-}
-
-// The heavy frontier vertices of a relaxation round, spread over the grid.
-// dist[u] may fall further while its row is being relaxed; any value read is
-// an achieved distance, and a vertex whose distance falls is queued again.
-template <bool kDelta>
-__global__ void k_sssp_relax_heavy(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                                   const int32_t* __restrict__ w, const int32_t* __restrict__ hq,
-                                   const uint32_t* __restrict__ hn, int32_t* __restrict__ dist,
-                                   int32_t* __restrict__ flag, int32_t* __restrict__ nq, uint32_t* __restrict__ nn,
-                                   SsspPush P) {
-    heavy_rows(off, hq, *hn, [&](int32_t u, uint64_t j, bool ok) {
-        bool near = false, far = false;
-        int32_t v = 0;
-        if (ok) {
-            v = adj[j];
-            sssp_relax_edge<kDelta>(dist[u], v, w[j], dist, flag, P, &near, &far);
-        }
-        warp_append(near, v, nq, nn);
-        if (kDelta) warp_append(far, v, P.far, P.farn);
-    });
-}
-
-// Smallest current distance in the far pile (entries at or above lo; lower
-// ones were relaxed in an earlier bucket), so empty buckets are skipped.
-__global__ void k_sssp_far_min(const int32_t* __restrict__ far, uint32_t fn, const int32_t* __restrict__ dist,
-                               int32_t lo, int32_t* __restrict__ out) {
-    int32_t mn = INT_MAX;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < fn; i += gridDim.x * blockDim.x) {
-        const int32_t d = dist[far[i]];
-        if (d >= lo) mn = min(mn, d);
-    }
-    for (int o = 16; o; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if ((threadIdx.x & 31) == 0 && mn != INT_MAX) atomicMin(out, mn);
-}
-
-// Splits the far pile at the new bucket [lo, hi): entries whose distance
-// fell below lo were relaxed when it fell and are dropped; entries in
-// [lo, hi) become the near frontier; the rest stay in the far pile.
-__global__ void k_sssp_far_split(const int32_t* __restrict__ far, uint32_t fn, const int32_t* __restrict__ dist,
-                                 int32_t lo, int32_t hi, int32_t* __restrict__ flag, int32_t* __restrict__ farflag,
-                                 int32_t* __restrict__ nq, uint32_t* __restrict__ nn, int32_t* __restrict__ far2,
-                                 uint32_t* __restrict__ far2n) {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t nr = (fn + 31) & ~31u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nr; i += stride) {
-        bool near = false, keep = false;
-        int32_t v = 0;
-        if (i < fn) {
-            v = far[i];
-            const int32_t d = dist[v];
-            keep = d >= hi;
-            if (!keep) {
-                farflag[v] = 0;
-                near = d >= lo && atomicExch(&flag[v], 1) == 0;
-            }
-        }
-        warp_append(near, v, nq, nn);
-        warp_append(keep, v, far2, far2n);
-    }
-}
-
-// Sum of m int32 values (non-negative weights) into *out.
-__global__ void k_sum_i32(const int32_t* __restrict__ a, uint64_t m, unsigned long long* __restrict__ out) {
+// The width chosen by the library (any width gives the same distances): the
+// mean of up to 2^16 weights taken at equal steps.  A step costs about 8 us
+// (barrier and one chain of dependent loads), and the wider a bucket, the more
+// edges are relaxed in vain.  Measured with weights 1..255 (mean 128), ms at
+// widths of 64 / 128 / 256 / 1024: RMAT-22 2.60 / 2.56 / 2.67 / 2.57, RMAT-18
+// 0.81 / 0.69 / 0.66 / 0.61, ER-20 1.64 / 1.36 / 1.92 / 2.08.  One CTA.
+__global__ void k_sssp_delta(const int32_t* __restrict__ w, uint64_t m, int32_t* __restrict__ delta) {
+    __shared__ unsigned long long sum;
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    const uint64_t step = m > 65536 ? m / 65536 : 1, cnt = (m + step - 1) / step;
     unsigned long long x = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
-        x += (unsigned long long)(uint32_t)a[i];
+    for (uint64_t i = threadIdx.x; i < cnt; i += blockDim.x) x += (unsigned long long)(uint32_t)w[i * step];
     x = warp_sum_u64(x);
-    if ((threadIdx.x & 31) == 0 && x) atomicAdd(out, x);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sum, x);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double mean = cnt ? (double)sum / (double)cnt : 1.0;
+        *delta = (int32_t)fmin((double)(1 << 30), fmax(1.0, round(mean)));
+    }
 }
 
-__global__ void k_clear_flags(const int32_t* __restrict__ q, uint32_t qn, int32_t* __restrict__ flag) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < qn) flag[q[i]] = 0;
+__global__ void __launch_bounds__(tx::kThreads, 5)
+    k_sssp_persistent(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, const int32_t* __restrict__ w,
+                      int32_t* dist, int32_t* stamp, int32_t* farflag, tx::Queues q0, tx::Queues q1, int32_t* far0,
+                      int32_t* far1, const int32_t* __restrict__ chosen, int32_t given, SsspState* S, SsspFar* F,
+                      GridBarrier* gb, uint64_t max_steps, uint64_t limit_ns) {
+    __shared__ tx::Tile s_tile[tx::kWarps];
+    __shared__ tx::Buffer s_near[tx::kWarps], s_far[tx::kWarps];
+    const int32_t delta = chosen ? *chosen : given;
+    tx::Tile& T = s_tile[threadIdx.x >> 5];
+    tx::Buffer& near_buf = s_near[threadIdx.x >> 5];
+    tx::Buffer& far_buf = s_far[threadIdx.x >> 5];
+    uint32_t nnear = 0, nfound_far = 0;
+    int32_t far_min = INT_MAX;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    const int lane = threadIdx.x & 31;
+    auto flush_far = [&](int32_t* far, int c) {
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < nfound_far; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            warp_append(i < nfound_far, i < nfound_far ? far_buf.v[i] : 0, far, &F->n[c]);
+        }
+        __syncwarp();
+        nfound_far = 0;
+    };
+    auto flush_far_min = [&](int c) {
+        const int32_t mn = __reduce_min_sync(0xffffffffu, far_min);
+        if (lane == 0 && mn != INT_MAX) atomicMin(&F->min[c], mn);
+        far_min = INT_MAX;
+    };
+    uint64_t step = 0;
+    for (; step < max_steps; ++step) {
+        const SsspState* in_p = &S[step % 3];
+        const int4 r0 = __ldcg(reinterpret_cast<const int4*>(in_p));
+        const uint32_t nl = (uint32_t)r0.x, nh = (uint32_t)r0.y;
+        const int32_t thr = r0.z, par = r0.w, splits = __ldcg(&in_p->splits);
+        SsspState* out = &S[(step + 1) % 3];
+        const int c = splits % 3;
+        int32_t* far = splits & 1 ? far1 : far0;
+        const bool relax = nl || nh;
+        const uint32_t nfar = relax ? 0u : __ldcg(&F->n[c]);
+        // every CTA reads the same record, so all leave at the same step
+        if (!relax && nfar == 0) break;
+        if (lead) {
+            SsspState* clr = &S[(step + 2) % 3];
+            clr->nl = clr->nh = 0;
+            out->par = 1 - par;
+        }
+        const tx::Queues& Q = par ? q1 : q0;
+        const tx::Queues& QN = par ? q0 : q1;
+        const int32_t mark = (int32_t)step + 1;  // stamp of the vertices queued in this step
+        if (relax) {
+            if (lead) {
+                out->thr = thr;
+                out->splits = splits;
+            }
+            tx::expand(
+                T, off, Q, nl, nh, [&](int32_t u) { return __ldcg(dist + u); },
+                [&](const uint64_t* j, const int32_t* du, const bool* ok) {
+                    int32_t v[tx::kPerLane], nd[tx::kPerLane];
+                    bool better[tx::kPerLane];
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        v[k] = ok[k] ? __ldcs(adj + j[k]) : 0;
+                        nd[k] = ok[k] ? du[k] + __ldcs(w + j[k]) : INT_MAX;
+                    }
+                    // A distance read here may be an older, larger one from L1:
+                    // atomicMin decides (reading L2 each time: 3.9 instead of
+                    // 2.6 ms at RMAT-22, the hubs' distances are hot).  Each
+                    // kind of access is issued for all edges before the first
+                    // answer is needed.
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) better[k] = nd[k] < dist[v[k]];
+                    if (!__any_sync(0xffffffffu, better[0] || better[1] || better[2] || better[3])) return;
+                    int32_t old[tx::kPerLane];
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) old[k] = better[k] ? atomicMin(&dist[v[k]], nd[k]) : INT_MIN;
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        better[k] = nd[k] < old[k];
+                        old[k] = better[k] ? atomicExch(nd[k] < thr ? &stamp[v[k]] : &farflag[v[k]], nd[k] < thr ? mark : 1)
+                                           : 0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        const bool near = better[k] && nd[k] < thr && old[k] != mark;
+                        const bool away = better[k] && nd[k] >= thr && old[k] == 0;
+                        tx::find(near_buf, nnear, near, v[k]);
+                        tx::find(far_buf, nfound_far, away, v[k]);
+                        if (away) far_min = min(far_min, nd[k]);
+                    }
+                },
+                [&]() {
+                    if (nnear > tx::kBuf - tx::kRound) tx::flush(near_buf, nnear, off, QN, &out->nl, &out->nh);
+                    if (nfound_far > tx::kBuf - tx::kRound) flush_far(far, c);
+                });
+            tx::flush(near_buf, nnear, off, QN, &out->nl, &out->nh);
+            flush_far(far, c);
+            flush_far_min(c);
+        } else {
+            // Split of the far pile at the next bucket [thr, hi): entries whose
+            // distance fell below thr were relaxed when it fell and are
+            // dropped; entries below hi become the near frontier; the rest
+            // go to the other pile.  Empty buckets are skipped.
+            const int32_t mn = max(__ldcg(&F->min[c]), thr);
+            const int32_t hi = (int32_t)min((int64_t)INT_MAX, (int64_t)mn + delta);
+            const int c2 = (splits + 1) % 3, c3 = (splits + 2) % 3;
+            int32_t* far2 = splits & 1 ? far0 : far1;
+            if (lead) {
+                out->thr = hi;
+                out->splits = splits + 1;
+                F->n[c3] = 0;  // last read in the split before, next written in the one after
+                F->min[c3] = INT_MAX;
+            }
+            const uint32_t gw = blockIdx.x * tx::kWarps + (threadIdx.x >> 5), nw = gridDim.x * tx::kWarps;
+            for (uint64_t i0 = gw * 32ull; i0 < nfar; i0 += nw * 32ull) {
+                const uint64_t i = i0 + lane;
+                bool near = false, keep = false;
+                int32_t v = 0;
+                if (i < nfar) {
+                    v = __ldcg(far + i);
+                    const int32_t d = __ldcg(dist + v);
+                    keep = d >= hi;
+                    if (!keep) {
+                        farflag[v] = 0;
+                        near = d >= thr;
+                    } else {
+                        far_min = min(far_min, d);
+                    }
+                }
+                tx::enqueue(near, v, off, QN, &out->nl, &out->nh);
+                warp_append(keep, v, far2, &F->n[c2]);
+            }
+            flush_far_min(c2);
+        }
+        if (!grid_sync(gb, limit_ns)) return;
+    }
+    if (lead && step == max_steps) atomicExch(&gb->err, 2);
 }
 
 // Hands the ids of adj[b, e) taken by lane gl of a group of L lanes to
@@ -1080,120 +1157,58 @@ pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, 
     const bool use_delta = method != PC_SSSP_BELLMAN_FORD;
     const int32_t isrc = to_internal_id(pg, src);
     cudaStream_t s = pg->g->stream;
-    const uint64_t hcap = heavy_cap(n, m);
-    PC_TRY(scratch_reserve(pg, n * 4 * (use_delta ? 9 : 5) + hcap * 4 + 1024));
+    const uint64_t hcap = tx::heavy_chunks(n, m);
+    PC_TRY(scratch_reserve(pg, n * 4 * 8 + hcap * 16 + 1024));
     int32_t* dist = pg->scratch.take<int32_t>(n);
-    int32_t* flag = pg->scratch.take<int32_t>(n);
-    int32_t* q0 = pg->scratch.take<int32_t>(n);
-    int32_t* q1 = pg->scratch.take<int32_t>(n);
+    int32_t* stamp = pg->scratch.take<int32_t>(n);
+    int32_t* farflag = pg->scratch.take<int32_t>(n);
+    tx::Queues q0{pg->scratch.take<int32_t>(n), nullptr}, q1{pg->scratch.take<int32_t>(n), nullptr};
+    q0.heavy = pg->scratch.take<int2>(hcap);
+    q1.heavy = pg->scratch.take<int2>(hcap);
+    int32_t* far0 = pg->scratch.take<int32_t>(n);
+    int32_t* far1 = pg->scratch.take<int32_t>(n);
     int32_t* out = pg->scratch.take<int32_t>(n);
-    int32_t* hq = pg->scratch.take<int32_t>(hcap);
-    uint32_t* cnt = pg->scratch.take<uint32_t>(8);  // [0] next frontier, [1] heavy list, [2] far, [3] far', [4] min
-    int32_t *farflag = nullptr, *far0 = nullptr, *far1 = nullptr;
-    unsigned long long* wsum = nullptr;
-    if (use_delta) {
-        farflag = pg->scratch.take<int32_t>(n);
-        far0 = pg->scratch.take<int32_t>(n);
-        far1 = pg->scratch.take<int32_t>(n);
-        wsum = pg->scratch.take<unsigned long long>(1);
+    SsspState* S = pg->scratch.take<SsspState>(3);
+    SsspFar* F = pg->scratch.take<SsspFar>(1);
+    GridBarrier* gb = pg->scratch.take<GridBarrier>(1);
+    int32_t* d_delta = pg->scratch.take<int32_t>(1);
+    if (!d_delta) return fail(PC_ERR_OOM, "SSSP scratch plan exceeds its reservation");
+    PC_CUDA(cudaMemsetAsync(gb, 0, sizeof(GridBarrier), s));
+    const bool choose = use_delta && delta == 0;
+    if (choose) {
+        k_sssp_delta<<<1, 1024, 0, s>>>(pg->w, m, d_delta);
+        PC_LAUNCHED();
     }
-    if (!cnt || (use_delta && !wsum)) return fail(PC_ERR_OOM, "SSSP scratch plan exceeds its reservation");
-    const unsigned nb = (unsigned)ceil_div(n, kThreads);
-    k_fill_i32<<<nb, kThreads, 0, s>>>(dist, n, INT_MAX / 2);  // src/test.cpp:202-203
+    // Bellman-Ford: one unbounded bucket
+    k_sssp_init<<<grid_for(pg), kThreads, 0, s>>>(pg->off, n, isrc, use_delta ? delta : INT_MAX, d_delta, dist, stamp,
+                                                  farflag, q0, S, F);
     PC_LAUNCHED();
-    PC_CUDA(cudaMemsetAsync(flag, 0, n * 4, s));
-    PC_CUDA(cudaMemsetAsync(cnt, 0, 32, s));
-    int32_t bucket = INT_MAX;  // Bellman-Ford: one unbounded bucket
-    if (use_delta) {
-        PC_CUDA(cudaMemsetAsync(farflag, 0, n * 4, s));
-        if (delta == 0) {
-            // Delta = 8 x mean weight.  Each relaxation round costs a launch and
-            // a host read of the queue size, so narrow buckets (many rounds per
-            // bucket) lose: on RMAT-22/24 with weights 1..255 the width of
-            // 32 x mean weight / mean degree (134; Davidson et al.) ran 1.3x
-            // slower than Bellman-Ford, while widths of 1024 and above ran 1-2 %
-            // faster than it.
-            PC_CUDA(cudaMemsetAsync(wsum, 0, 8, s));
-            k_sum_i32<<<grid_for(pg), kThreads, 0, s>>>(pg->w, m, wsum);
-            PC_LAUNCHED();
-            unsigned long long h = 0;
-            PC_CUDA(cudaMemcpyAsync(&h, wsum, 8, cudaMemcpyDeviceToHost, s));
-            PC_TRY(sync(pg));
-            const double mean_w = m ? (double)h / (double)m : 1.0;
-            delta = (int32_t)std::min<double>(1 << 30, std::max(1.0, std::round(8.0 * mean_w)));
-        }
-        bucket = delta;
+    int per_sm = 0;
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sssp_persistent, tx::kThreads, 0));
+    if (per_sm < 1) return fail(PC_ERR_CUDA, "SSSP kernel cannot be resident");
+    const unsigned grid = (unsigned)(sm_count(pg->g->device) * std::min(per_sm, 5));
+    uint64_t max_steps = 8 * (n + 1) + 64, limit_ns = kBarrierLimitNs;
+    const uint64_t* off = pg->off;
+    const int32_t* adj = pg->adj;
+    const int32_t* w = pg->w;
+    const int32_t* chosen = choose ? d_delta : nullptr;
+    int32_t given = use_delta ? delta : INT_MAX;
+    void* args[] = {(void*)&off, (void*)&adj,  (void*)&w,    (void*)&dist,   (void*)&stamp, (void*)&farflag,
+                    (void*)&q0,  (void*)&q1,   (void*)&far0, (void*)&far1,   (void*)&chosen, (void*)&given,
+                    (void*)&S,   (void*)&F,    (void*)&gb,   (void*)&max_steps, (void*)&limit_ns};
+    PC_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_persistent, dim3(grid), dim3(tx::kThreads), args, 0, s));
+    PC_LAUNCHED();
+    if (!api_is_internal(pg)) {
+        PC_TRY(gather_to_api_i32(pg, dist, out));
+        dist = out;
     }
-    const int32_t zero = 0;
-    PC_CUDA(cudaMemcpyAsync(dist + isrc, &zero, 4, cudaMemcpyHostToDevice, s));
-    PC_CUDA(cudaMemcpyAsync(q0, &isrc, 4, cudaMemcpyHostToDevice, s));
-    uint32_t fn = 1, farn = 0;
-    int32_t* fq = q0;
-    int32_t* nq = q1;
-    int32_t thr = bucket;
-    uint64_t rounds = 0;
-    const uint64_t round_cap = 4 * (n + 1) + 64;
-    for (;;) {
-        while (fn > 0) {
-            PC_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
-            SsspPush P{thr, far0, cnt + 2, farflag};
-            if (use_delta) {
-                k_sssp_relax<true><<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, pg->w, fq, fn, dist, flag, nq,
-                                                                    cnt, hq, cnt + 1, P);
-                PC_LAUNCHED();
-                k_sssp_relax_heavy<true><<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, pg->w, hq, cnt + 1, dist,
-                                                                          flag, nq, cnt, P);
-            } else {
-                k_sssp_relax<false><<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, pg->w, fq, fn, dist, flag,
-                                                                     nq, cnt, hq, cnt + 1, P);
-                PC_LAUNCHED();
-                k_sssp_relax_heavy<false><<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, pg->w, hq, cnt + 1,
-                                                                           dist, flag, nq, cnt, P);
-            }
-            PC_LAUNCHED();
-            PC_TRY(read_u32(pg, cnt, &fn));
-            if (fn) {
-                k_clear_flags<<<(unsigned)ceil_div(fn, kThreads), kThreads, 0, s>>>(nq, fn, flag);
-                PC_LAUNCHED();
-            }
-            std::swap(fq, nq);
-            if (++rounds > round_cap) return fail(PC_ERR_TIMEOUT, "SSSP did not converge");
-        }
-        if (!use_delta) break;
-        PC_TRY(read_u32(pg, cnt + 2, &farn));
-        if (farn == 0) break;
-        // next bucket: from the smallest far distance at or above thr (the
-        // entries below thr were relaxed when their distance fell)
-        const int32_t big = INT_MAX;
-        PC_CUDA(cudaMemcpyAsync(cnt + 4, &big, 4, cudaMemcpyHostToDevice, s));
-        k_sssp_far_min<<<(unsigned)std::min<uint64_t>(ceil_div(farn, kThreads), 1024), kThreads, 0, s>>>(
-            far0, farn, dist, thr, reinterpret_cast<int32_t*>(cnt + 4));
-        PC_LAUNCHED();
-        uint32_t mn_u = 0;
-        PC_TRY(read_u32(pg, cnt + 4, &mn_u));
-        const int32_t mn = (int32_t)mn_u;
-        const int32_t lo = thr;
-        const int32_t hi = mn == INT_MAX ? INT_MAX : (int32_t)std::min<int64_t>(INT_MAX, (int64_t)mn + delta);
-        PC_CUDA(cudaMemsetAsync(cnt, 0, 4, s));
-        PC_CUDA(cudaMemsetAsync(cnt + 3, 0, 4, s));
-        k_sssp_far_split<<<(unsigned)std::min<uint64_t>(ceil_div(farn, kThreads), 4096), kThreads, 0, s>>>(
-            far0, farn, dist, lo, hi, flag, farflag, fq, cnt, far1, cnt + 3);
-        PC_LAUNCHED();
-        PC_TRY(read_u32(pg, cnt, &fn));
-        PC_TRY(read_u32(pg, cnt + 3, &farn));
-        if (fn) {
-            k_clear_flags<<<(unsigned)ceil_div(fn, kThreads), kThreads, 0, s>>>(fq, fn, flag);
-            PC_LAUNCHED();
-        }
-        std::swap(far0, far1);
-        PC_CUDA(cudaMemcpyAsync(cnt + 2, &farn, 4, cudaMemcpyHostToDevice, s));
-        thr = hi;
-        if (fn == 0 && farn == 0) break;
-        if (++rounds > round_cap) return fail(PC_ERR_TIMEOUT, "SSSP did not converge");
-    }
-    PC_TRY(gather_to_api_i32(pg, dist, out));
-    PC_CUDA(cudaMemcpyAsync(dist_host, out, n * 4, cudaMemcpyDeviceToHost, s));
-    return sync(pg);
+    GridBarrier hb{};
+    PC_CUDA(cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaMemcpyAsync(dist_host, dist, n * 4, cudaMemcpyDeviceToHost, s));
+    PC_TRY(sync(pg));
+    if (hb.err == 1) return fail(PC_ERR_TIMEOUT, "SSSP: a grid barrier wait ran out of time");
+    if (hb.err) return fail(PC_ERR_TIMEOUT, "SSSP did not converge");
+    return PC_OK;
 }
 
 pc_status pc_pagerank(pc_pgraph* pg, float damping, int32_t iterations, const float* init, float* out) {
