@@ -126,92 +126,179 @@ __global__ void k_iota(int32_t* a, uint64_t n) {
     if (i < n) a[i] = (int32_t)i;
 }
 
-__global__ void k_fill_i32(int32_t* a, uint64_t n, int32_t v) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
+// Direction-optimising (Beamer, Asanovic, Patterson, SC'12) in one persistent
+// kernel, a grid barrier per level: top-down levels expand the frontier's
+// queues (tx::expand); bottom-up levels look for a neighbour of the last
+// level at every unvisited vertex and only count what they find.  Back from
+// bottom-up, one step collects the frontier's queues from the levels.
+// The state lives in three rotating records (see KState).
+//
+// Bound at RMAT-22: the copy of the levels to the host (0.3 of 0.6 ms), then
+// the dependent loads of seven levels and their barriers.  With two launches
+// and a host read per level, and a warp per row, 0.76-0.97 ms; ER-20 0.47 ->
+// 0.25 ms, RMAT-16 0.32 -> 0.14, RMAT-10 0.18 -> 0.06.
+struct __align__(16) BfsState {
+    uint32_t nl, nh;      // the frontier's queues (queued)
+    uint32_t fn;          // vertices in the frontier
+    int32_t level;        // of the frontier's unvisited neighbours
+    uint64_t edges;       // row entries of the frontier
+    uint64_t unexplored;  // ... and of it and every later vertex
+    int32_t bottom_up;    // direction of the level before
+    int32_t queued;       // the frontier is in the queues; 2: and top-down is decided
+    int32_t par;          // queues in use
+    int32_t pad;
+};
+
+__global__ void k_bfs_init(const uint64_t* __restrict__ off, uint64_t n, uint64_t m, int32_t src,
+                           int32_t* __restrict__ dist, tx::Queues Q, BfsState* S) {
+    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x)
+        dist[u] = u == (uint64_t)src ? 0 : kInf;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        if (threadIdx.x < 3)
+            S[threadIdx.x] = BfsState{0, 0, threadIdx.x == 0, 1, threadIdx.x ? 0 : off[src + 1] - off[src], m, 0, 1, 0, 0};
+        __syncwarp();
+        tx::enqueue<1>(&src, threadIdx.x == 0, off, Q, &S[0].nl, &S[0].nh);
+    }
 }
 
-// Top-down step: one warp per frontier vertex, lanes over its neighbours.
-__global__ void k_bfs_top_down(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                               const int32_t* __restrict__ fq, uint32_t fn, int32_t* __restrict__ dist,
-                               int32_t level, int32_t* __restrict__ nq, uint32_t* __restrict__ nn,
-                               unsigned long long* __restrict__ next_edges, int32_t* __restrict__ hq,
-                               uint32_t* __restrict__ hn) {
+__global__ void __launch_bounds__(tx::kThreads, 6)
+    k_bfs_persistent(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, int32_t src,
+                     int32_t* dist, tx::Queues q0, tx::Queues q1, BfsState* S, GridBarrier* gb, uint64_t max_steps,
+                     uint64_t limit_ns) {
+    __shared__ tx::Tile s_tile[tx::kWarps];
+    __shared__ tx::Buffer s_buf[tx::kWarps];
+    __shared__ unsigned long long s_edges;
+    __shared__ uint32_t s_fn;
+    tx::Tile& T = s_tile[threadIdx.x >> 5];
+    tx::Buffer& B = s_buf[threadIdx.x >> 5];
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint64_t edges = 0;
-    for (uint64_t i = warp; i < fn; i += nwarps) {
-        const int32_t u = fq[i];
-        const uint64_t b = off[u], e = off[u + 1];
-        if (e - b > kHeavyDeg) {  // expanded by k_bfs_top_down_heavy
-            if (lane == 0) hq[atomicAdd(hn, 1u)] = u;
-            continue;
-        }
-        for (uint64_t j0 = b; j0 < e; j0 += 32) {
-            const uint64_t j = j0 + lane;
-            bool won = false;
-            int32_t v = 0;
-            if (j < e) {
-                v = adj[j];
-                if (dist[v] == kInf) won = atomicCAS(&dist[v], kInf, level) == kInf;
-            }
-            if (won) edges += off[v + 1] - off[v];
-            warp_append(won, v, nq, nn);
-        }
+    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t nr = (n + 127) & ~127ull;  // whole warps of four vertices a lane
+    // levels of vertices v .. v + 3 (v a multiple of 4; -2 past the last one)
+    auto levels4 = [&](uint64_t v) {
+        if (v + 4 <= n) return __ldcg(reinterpret_cast<const int4*>(dist + v));
+        int4 d = make_int4(-2, -2, -2, -2);
+        if (v < n) d.x = __ldcg(dist + v);
+        if (v + 1 < n) d.y = __ldcg(dist + v + 1);
+        if (v + 2 < n) d.z = __ldcg(dist + v + 2);
+        return d;
+    };
+    if (threadIdx.x == 0) {
+        s_edges = 0;
+        s_fn = 0;
     }
-    edges = warp_sum_u64(edges);
-    if (lane == 0 && edges) atomicAdd(next_edges, (unsigned long long)edges);
-}
-
-// The heavy frontier vertices of a top-down step, spread over the grid.
-__global__ void k_bfs_top_down_heavy(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                                     const int32_t* __restrict__ hq, const uint32_t* __restrict__ hn,
-                                     int32_t* __restrict__ dist, int32_t level, int32_t* __restrict__ nq,
-                                     uint32_t* __restrict__ nn, unsigned long long* __restrict__ next_edges) {
-    uint64_t edges = 0;
-    heavy_rows(off, hq, *hn, [&](int32_t, uint64_t j, bool ok) {
-        bool won = false;
-        int32_t v = 0;
-        if (ok) {
-            v = adj[j];
-            if (dist[v] == kInf) won = atomicCAS(&dist[v], kInf, level) == kInf;
-        }
-        if (won) edges += off[v + 1] - off[v];
-        warp_append(won, v, nq, nn);
-    });
-    edges = warp_sum_u64(edges);
-    if ((threadIdx.x & 31) == 0 && edges) atomicAdd(next_edges, (unsigned long long)edges);
-}
-
-// Bottom-up step: every unvisited vertex looks for a neighbour at level-1.
-__global__ void k_bfs_bottom_up(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n,
-                                int32_t* __restrict__ dist, int32_t level, int32_t* __restrict__ nq,
-                                uint32_t* __restrict__ nn, unsigned long long* __restrict__ next_edges) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t nr = (n + 31) & ~31ull;
-    uint64_t edges = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nr; v += stride) {
-        bool found = false;
-        if (v < n && dist[v] == kInf) {
-            const uint64_t b = off[v], e = off[v + 1];
-            for (uint64_t j = b; j < e; ++j) {
-                if (dist[adj[j]] == level - 1) { found = true; break; }
-            }
-            if (found) {
-                dist[v] = level;
-                edges += e - b;
+    __syncthreads();
+    uint64_t step = 0;
+    for (; step < max_steps; ++step) {
+        const BfsState* in = &S[step % 3];
+        BfsState* out = &S[(step + 1) % 3];
+        const uint32_t nl = __ldcg(&in->nl), nh = __ldcg(&in->nh), fn = __ldcg(&in->fn);
+        const int32_t level = __ldcg(&in->level), queued = __ldcg(&in->queued), par = __ldcg(&in->par);
+        const uint64_t edges = __ldcg(&in->edges), unexplored = __ldcg(&in->unexplored) - edges;
+        // every CTA reads the same record, so all leave at the same step
+        if (fn == 0) break;
+        const int32_t was = __ldcg(&in->bottom_up);
+        const bool bottom_up = queued != 2 && (was ? fn * 18ull >= n : edges * 15 > unexplored);
+        const bool collect = !bottom_up && !queued;  // the frontier is not in the queues
+        // A level that expands a good part of what is left finds most of the
+        // graph, and the next one runs bottom-up: it is counted, not queued
+        // (RMAT-22, 0.8 M vertices found: 130 us for the level with queues).
+        const bool many = !bottom_up && !collect && edges * 64 > unexplored;
+        if (lead) {
+            BfsState* clr = &S[(step + 2) % 3];
+            clr->nl = clr->nh = clr->fn = 0;
+            clr->edges = 0;
+            out->bottom_up = bottom_up;
+            out->queued = collect ? 2 : !bottom_up && !many;
+            out->par = bottom_up ? par : 1 - par;
+            out->level = collect ? level : level + 1;
+            out->unexplored = collect ? unexplored + edges : unexplored;
+            if (collect) {
+                out->fn = fn;
+                out->edges = edges;
             }
         }
-        warp_append(found, (int32_t)v, nq, nn);
+        const tx::Queues& Q = par ? q1 : q0;
+        const tx::Queues& QN = par ? q0 : q1;
+        uint64_t found_edges = 0;
+        uint32_t found = 0;
+        if (collect) {
+            uint32_t nb = 0;
+            for (uint64_t v = 4 * tid; v < nr; v += 4 * stride) {
+                const int4 d = levels4(v);
+                tx::find(B, nb, d.x == level - 1, (int32_t)v);
+                tx::find(B, nb, d.y == level - 1, (int32_t)v + 1);
+                tx::find(B, nb, d.z == level - 1, (int32_t)v + 2);
+                tx::find(B, nb, d.w == level - 1, (int32_t)v + 3);
+                if (nb > tx::kBuf - 128) tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+            }
+            tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        } else if (bottom_up) {
+            // (four vertices a thread with their loads together: a quarter
+            // slower; the rows that go on then wait for one another)
+            for (uint64_t v = tid; v < n; v += stride) {
+                if (__ldcg(dist + v) != kInf) continue;
+                const uint64_t b = off[v], e = off[v + 1];
+                bool hit = false;
+                // four ids a load; the ids outside [b, e) are not looked at
+                for (uint64_t q = b & ~3ull; q < e && !hit; q += 4) {
+                    const int4 a = __ldg(reinterpret_cast<const int4*>(adj + q));
+                    hit = (q >= b && dist[a.x] == level - 1) || (q + 1 >= b && q + 1 < e && dist[a.y] == level - 1) ||
+                          (q + 2 >= b && q + 2 < e && dist[a.z] == level - 1) || (q + 3 < e && dist[a.w] == level - 1);
+                }
+                if (hit) {
+                    dist[v] = level;
+                    found_edges += e - b;
+                    ++found;
+                }
+            }
+        } else {
+            uint32_t nb = 0;
+            tx::expand(
+                T, off, Q, nl, nh, [](int32_t) { return 0; },
+                [&](const uint64_t* j, const int32_t*, const bool* ok) {
+                    int32_t v[tx::kPerLane];
+                    bool open[tx::kPerLane];
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) v[k] = ok[k] ? __ldcs(adj + j[k]) : 0;
+                    // a level read here may be an old "unvisited" from L1: atomicCAS decides
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) open[k] = ok[k] && dist[v[k]] == kInf;
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k)
+                        open[k] = open[k] && atomicCAS(&dist[v[k]], kInf, level) == kInf;
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        if (many) found_edges += open[k] ? off[v[k] + 1] - off[v[k]] : 0;
+                        else tx::find(B, nb, open[k], v[k]);
+                        found += open[k];
+                    }
+                },
+                [&]() {
+                    if (nb > tx::kBuf - tx::kRound) found_edges += tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+                });
+            found_edges += tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        }
+        found_edges = warp_sum_u64(found_edges);
+        found = __reduce_add_sync(0xffffffffu, found);
+        if (lane == 0 && found) {
+            atomicAdd(&s_edges, (unsigned long long)found_edges);
+            atomicAdd(&s_fn, found);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && s_fn) {
+            atomicAdd((unsigned long long*)&out->edges, s_edges);
+            atomicAdd(&out->fn, s_fn);
+            s_edges = 0;
+            s_fn = 0;
+        }
+        if (!grid_sync(gb, limit_ns)) return;
     }
-    edges = warp_sum_u64(edges);
-    if ((threadIdx.x & 31) == 0 && edges) atomicAdd(next_edges, (unsigned long long)edges);
-}
-
-__global__ void k_bfs_finish(const int32_t* __restrict__ dist, uint64_t n, int32_t* __restrict__ rank) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) rank[i] = dist[i] == 0 ? -1 : dist[i];
+    if (lead) {
+        dist[src] = -1;  // rank[src] = -1 (src/Graph.cpp:1704)
+        if (step == max_steps) atomicExch(&gb->err, 2);
+    }
 }
 
 // ---- SSSP: frontier Bellman-Ford and delta-stepping --------------------------
@@ -233,8 +320,10 @@ __global__ void k_bfs_finish(const int32_t* __restrict__ dist, uint64_t n, int32
 // the near frontier (tx::expand) or, when that is empty, the split of the far
 // pile.  Steps keep their state in three rotating records (see KState).
 //
-// Bound at RMAT-22 (6.1 -> 2.6-2.8 ms a call, 0.3 ms of it the copy back): the
-// gathers of the neighbours' distances, 2.9 m of them, from L1 and L2.
+// Bound at RMAT-22 (6.1 -> 2.2 ms a call, 0.3 ms of it the copy back): the
+// gathers of the neighbours' distances, 2.9 m of them, from L1 and L2.  Small
+// graphs: barriers and chains of atomics, 4-10 us a step (RMAT-16 0.90 -> 0.37
+// ms, RMAT-10 0.50 -> 0.15); ER-20 5.2 -> 0.92 ms.
 struct __align__(16) SsspState {
     uint32_t nl, nh;  // near queues' lengths
     int32_t thr;      // near bound (exclusive)
@@ -263,7 +352,7 @@ __global__ void k_sssp_init(const uint64_t* __restrict__ off, uint64_t n, int32_
             F->min[threadIdx.x] = INT_MAX;
         }
         __syncwarp();
-        tx::enqueue(threadIdx.x == 0, src, off, Q, &S[0].nl, &S[0].nh);
+        tx::enqueue<1>(&src, threadIdx.x == 0, off, Q, &S[0].nl, &S[0].nh);
     }
 }
 
@@ -272,7 +361,8 @@ __global__ void k_sssp_init(const uint64_t* __restrict__ off, uint64_t n, int32_
 // (barrier and one chain of dependent loads), and the wider a bucket, the more
 // edges are relaxed in vain.  Measured with weights 1..255 (mean 128), ms at
 // widths of 64 / 128 / 256 / 1024: RMAT-22 2.60 / 2.56 / 2.67 / 2.57, RMAT-18
-// 0.81 / 0.69 / 0.66 / 0.61, ER-20 1.64 / 1.36 / 1.92 / 2.08.  One CTA.
+// 0.81 / 0.69 / 0.66 / 0.61, ER-20 1.64 / 1.36 / 1.92 / 2.08 (with a dearer
+// step than now).  One CTA.
 __global__ void k_sssp_delta(const int32_t* __restrict__ w, uint64_t m, int32_t* __restrict__ delta) {
     __shared__ unsigned long long sum;
     if (threadIdx.x == 0) sum = 0;
@@ -305,11 +395,12 @@ __global__ void __launch_bounds__(tx::kThreads, 5)
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     const int lane = threadIdx.x & 31;
     auto flush_far = [&](int32_t* far, int c) {
+        if (nfound_far == 0) return;
         __syncwarp();
-        for (uint32_t i0 = 0; i0 < nfound_far; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            warp_append(i < nfound_far, i < nfound_far ? far_buf.v[i] : 0, far, &F->n[c]);
-        }
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&F->n[c], nfound_far);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (uint32_t i = lane; i < nfound_far; i += 32) far[at + i] = far_buf.v[i];
         __syncwarp();
         nfound_far = 0;
     };
@@ -418,9 +509,13 @@ __global__ void __launch_bounds__(tx::kThreads, 5)
                         far_min = min(far_min, d);
                     }
                 }
-                tx::enqueue(near, v, off, QN, &out->nl, &out->nh);
-                warp_append(keep, v, far2, &F->n[c2]);
+                tx::find(near_buf, nnear, near, v);
+                tx::find(far_buf, nfound_far, keep, v);
+                if (nnear > tx::kBuf - 32) tx::flush(near_buf, nnear, off, QN, &out->nl, &out->nh);
+                if (nfound_far > tx::kBuf - 32) flush_far(far2, c2);
             }
+            tx::flush(near_buf, nnear, off, QN, &out->nl, &out->nh);
+            flush_far(far2, c2);
             flush_far_min(c2);
         }
         if (!grid_sync(gb, limit_ns)) return;
@@ -981,66 +1076,56 @@ static pc_status read_u32(pc_pgraph* pg, const uint32_t* d, uint32_t* h) {
     return PC_OK;
 }
 
+// CTAs of a persistent kernel: every SM's share, fewer for a small graph,
+// whose barriers then have fewer arrivals; one per `work` vertices and quarter
+// entries.  BFS takes 2048 (RMAT-16: 0.14 ms, 0.20 with 256), SSSP, whose steps
+// wait on chains of atomics, 256 (RMAT-16: 0.37 ms, 0.41 with 2048).
+static pc_status persistent_grid(const pc_pgraph* pg, const void* kernel, int threads, int most_per_sm, uint64_t work,
+                                 unsigned* grid) {
+    int per_sm = 0;
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+    if (per_sm < 1) return fail(PC_ERR_CUDA, "persistent kernel cannot be resident");
+    const uint64_t all = (uint64_t)sm_count(pg->g->device) * std::min(per_sm, most_per_sm);
+    *grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(all, ceil_div(pg->g->n + pg->g->m / 4, work)));
+    return PC_OK;
+}
+
 static pc_status bfs_run(pc_pgraph* pg, int32_t src, int32_t* rank_host) {
     const uint64_t n = pg->g->n, m = pg->g->m;
     cudaStream_t s = pg->g->stream;
-    const uint64_t hcap = heavy_cap(n, m);
-    PC_TRY(scratch_reserve(pg, n * 4 * 4 + hcap * 4 + 256));
+    const uint64_t hcap = tx::heavy_chunks(n, m);
+    PC_TRY(scratch_reserve(pg, n * 4 * 4 + hcap * 16 + 1024));
     int32_t* dist = pg->scratch.take<int32_t>(n);
-    int32_t* q0 = pg->scratch.take<int32_t>(n);
-    int32_t* q1 = pg->scratch.take<int32_t>(n);
-    int32_t* hq = pg->scratch.take<int32_t>(hcap);
-    uint32_t* cnt = pg->scratch.take<uint32_t>(4);  // [0] next frontier, [1] heavy list
-    unsigned long long* edges = pg->scratch.take<unsigned long long>(2);
-    if (!edges) return fail(PC_ERR_OOM, "BFS scratch plan exceeds its reservation");
-    const unsigned nb = (unsigned)ceil_div(n, kThreads);
-    k_fill_i32<<<nb, kThreads, 0, s>>>(dist, n, kInf);
+    int32_t* out = pg->scratch.take<int32_t>(n);
+    tx::Queues q0{pg->scratch.take<int32_t>(n), nullptr}, q1{pg->scratch.take<int32_t>(n), nullptr};
+    q0.heavy = pg->scratch.take<int2>(hcap);
+    q1.heavy = pg->scratch.take<int2>(hcap);
+    BfsState* S = pg->scratch.take<BfsState>(3);
+    GridBarrier* gb = pg->scratch.take<GridBarrier>(1);
+    if (!gb) return fail(PC_ERR_OOM, "BFS scratch plan exceeds its reservation");
+    PC_CUDA(cudaMemsetAsync(gb, 0, sizeof(GridBarrier), s));
+    k_bfs_init<<<grid_for(pg), kThreads, 0, s>>>(pg->off, n, m, src, dist, q0, S);
     PC_LAUNCHED();
-    const int32_t zero = 0;
-    PC_CUDA(cudaMemcpyAsync(dist + src, &zero, 4, cudaMemcpyHostToDevice, s));
-    PC_CUDA(cudaMemcpyAsync(q0, &src, 4, cudaMemcpyHostToDevice, s));
-    // host-side state of the direction heuristic (Beamer, Asanovic, Patterson, SC'12)
-    std::vector<uint64_t> h_off(2);
-    PC_CUDA(cudaMemcpyAsync(h_off.data(), pg->off + src, 16, cudaMemcpyDeviceToHost, s));
-    PC_CUDA(cudaStreamSynchronize(s));
-    uint64_t frontier_edges = h_off[1] - h_off[0];
-    uint64_t unexplored = m - frontier_edges;
-    uint32_t fn = 1;
-    bool bottom_up = false;
-    const double alpha = 15.0, beta = 18.0;
-    int32_t* fq = q0;
-    int32_t* nq = q1;
-    for (int32_t level = 1; fn > 0; ++level) {
-        if (!bottom_up && (double)frontier_edges > (double)unexplored / alpha) bottom_up = true;
-        else if (bottom_up && (double)fn < (double)n / beta) bottom_up = false;
-        PC_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
-        PC_CUDA(cudaMemsetAsync(edges, 0, 8, s));
-        if (bottom_up) {
-            k_bfs_bottom_up<<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, n, dist, level, nq, cnt, edges);
-        } else {
-            k_bfs_top_down<<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, fq, fn, dist, level, nq, cnt, edges,
-                                                             hq, cnt + 1);
-            PC_LAUNCHED();
-            k_bfs_top_down_heavy<<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, hq, cnt + 1, dist, level, nq, cnt,
-                                                                   edges);
-        }
-        PC_LAUNCHED();
-        unsigned long long h_edges = 0;
-        PC_CUDA(cudaMemcpyAsync(&fn, cnt, 4, cudaMemcpyDeviceToHost, s));
-        PC_CUDA(cudaMemcpyAsync(&h_edges, edges, 8, cudaMemcpyDeviceToHost, s));
-        PC_CUDA(cudaStreamSynchronize(s));
-        frontier_edges = h_edges;
-        unexplored = unexplored > h_edges ? unexplored - h_edges : 0;
-        std::swap(fq, nq);
-        if (level > (int32_t)n + 1) return fail(PC_ERR_TIMEOUT, "BFS did not converge");
+    unsigned grid = 0;
+    PC_TRY(persistent_grid(pg, (const void*)k_bfs_persistent, tx::kThreads, 6, 2048, &grid));
+    uint64_t max_steps = 2 * (n + 1) + 64, limit_ns = kBarrierLimitNs, nn = n;
+    const uint64_t* off = pg->off;
+    const int32_t* adj = pg->adj;
+    void* args[] = {(void*)&off, (void*)&adj, (void*)&nn, (void*)&src, (void*)&dist,      (void*)&q0,
+                    (void*)&q1,  (void*)&S,   (void*)&gb, (void*)&max_steps, (void*)&limit_ns};
+    PC_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_persistent, dim3(grid), dim3(tx::kThreads), args, 0, s));
+    PC_LAUNCHED();
+    if (!api_is_internal(pg)) {
+        PC_TRY(gather_to_api_i32(pg, dist, out));
+        dist = out;
     }
-    int32_t* rank_int = q0 == fq ? q1 : q0;  // any free n-array
-    k_bfs_finish<<<nb, kThreads, 0, s>>>(dist, n, rank_int);
-    PC_LAUNCHED();
-    int32_t* rank_api = dist;
-    PC_TRY(gather_to_api_i32(pg, rank_int, rank_api));
-    PC_CUDA(cudaMemcpyAsync(rank_host, rank_api, n * 4, cudaMemcpyDeviceToHost, s));
-    return sync(pg);
+    GridBarrier hb{};
+    PC_CUDA(cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaMemcpyAsync(rank_host, dist, n * 4, cudaMemcpyDeviceToHost, s));
+    PC_TRY(sync(pg));
+    if (hb.err == 1) return fail(PC_ERR_TIMEOUT, "BFS: a grid barrier wait ran out of time");
+    if (hb.err) return fail(PC_ERR_TIMEOUT, "BFS did not converge");
+    return PC_OK;
 }
 
 template <class T>
@@ -1183,10 +1268,8 @@ pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, 
     k_sssp_init<<<grid_for(pg), kThreads, 0, s>>>(pg->off, n, isrc, use_delta ? delta : INT_MAX, d_delta, dist, stamp,
                                                   farflag, q0, S, F);
     PC_LAUNCHED();
-    int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sssp_persistent, tx::kThreads, 0));
-    if (per_sm < 1) return fail(PC_ERR_CUDA, "SSSP kernel cannot be resident");
-    const unsigned grid = (unsigned)(sm_count(pg->g->device) * std::min(per_sm, 5));
+    unsigned grid = 0;
+    PC_TRY(persistent_grid(pg, (const void*)k_sssp_persistent, tx::kThreads, 5, 256, &grid));
     uint64_t max_steps = 8 * (n + 1) + 64, limit_ns = kBarrierLimitNs;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;

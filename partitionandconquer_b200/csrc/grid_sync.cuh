@@ -11,9 +11,8 @@
 namespace pc {
 
 struct GridBarrier {
-    unsigned count;  // CTAs arrived in the current generation
-    unsigned gen;    // generation, bumped by the last CTA to arrive
-    int err;         // 1: a wait ran out of time; 2: a step bound was hit
+    unsigned long long arrived;  // CTAs arrived so far, over all barriers
+    int err;                     // 1: a wait ran out of time; 2: a step bound was hit
     int pad;
 };
 
@@ -23,9 +22,9 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -37,26 +36,23 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* gb, uint64_t limit_ns) {
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        // the generation is read before arriving: the last CTA can only bump
-        // it after this CTA's arrival
-        const unsigned g = ld_acquire_u32(&gb->gen);
+        // The counter only grows: the arrival that this barrier waits for is
+        // the next multiple of the grid's size, so nothing is reset and the
+        // waiting CTAs poll the counter itself (one round trip less than a
+        // generation word that the last CTA bumps).
         __threadfence();
-        const unsigned arrived = atomicAdd(&gb->count, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(&gb->count, 0u);
-            __threadfence();
-            atomicAdd(&gb->gen, 1u);
-        } else {
+        const unsigned long long mine = atomicAdd(&gb->arrived, 1ull);
+        const unsigned long long all = (mine / gridDim.x + 1) * gridDim.x;
+        if (mine + 1 != all) {
             const uint64_t t0 = global_ns();
-            for (;;) {
-                if (ld_acquire_u32(&gb->gen) != g) break;
+            while (ld_acquire_u64(&gb->arrived) < all) {
                 if (*(volatile int*)&gb->err) { ok = 0; break; }
                 if (global_ns() - t0 > limit_ns) {
                     atomicExch(&gb->err, 1);
                     ok = 0;
                     break;
                 }
-                __nanosleep(64);
+                __nanosleep(32);
             }
         }
         __threadfence();

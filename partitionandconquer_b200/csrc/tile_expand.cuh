@@ -58,41 +58,70 @@ __device__ __forceinline__ void find(Buffer& B, uint32_t& n, bool pred, int32_t 
     n += __popc(m);
 }
 
-// Appends one vertex per lane with pred set to the queues by its row's
-// length; all 32 lanes call it.
-__device__ __forceinline__ void enqueue(bool pred, int32_t v, const uint64_t* __restrict__ off, const Queues& Q,
-                                        uint32_t* nlight, uint32_t* nheavy) {
+// Appends v[0 .. k) of each lane to the queues by their rows' lengths; all 32
+// lanes call it (k may differ).  Returns the lane's row entries.  The lengths
+// are loaded together and each queue takes one atomic: appending 32 at a
+// time, a full buffer waited through eight chains of load and atomics.
+template <int kMost>
+__device__ __forceinline__ uint64_t enqueue(const int32_t* v, int k, const uint64_t* __restrict__ off, const Queues& Q,
+                                            uint32_t* nlight, uint32_t* nheavy) {
     const int lane = threadIdx.x & 31;
-    const uint64_t deg = pred ? off[v + 1] - off[v] : 0;
-    const unsigned m = __ballot_sync(0xffffffffu, pred && deg <= kLightRow);
-    if (m) {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(nlight, (uint32_t)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (m >> lane & 1) Q.light[at + __popc(m & ((1u << lane) - 1u))] = v;
+    uint64_t entries = 0;
+    uint32_t chunks[kMost];  // of a heavy row, 0 of a light one
+    uint32_t nl = 0, nh = 0;
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        const uint64_t deg = i < k ? off[v[i] + 1] - off[v[i]] : 0;
+        entries += deg;
+        chunks[i] = deg > kLightRow ? (uint32_t)((deg + kHeavyRun - 1) / kHeavyRun) : 0u;
+        nl += i < k && !chunks[i];
+        nh += chunks[i];
     }
-    unsigned h = __ballot_sync(0xffffffffu, pred && deg > kLightRow);
-    if (!h) return;
-    const uint32_t c = h >> lane & 1 ? (uint32_t)((deg + kHeavyRun - 1) / kHeavyRun) : 0u;
-    uint32_t at = c ? atomicAdd(nheavy, c) : 0u;
-    for (; h; h &= h - 1) {  // the warp writes a row's chunks together
-        const int src = __ffs(h) - 1;
-        const uint32_t cs = __shfl_sync(0xffffffffu, c, src), as = __shfl_sync(0xffffffffu, at, src);
-        const int32_t vs = __shfl_sync(0xffffffffu, v, src);
-        for (uint32_t i = lane; i < cs; i += 32) Q.heavy[as + i] = make_int2(vs, (int32_t)i);
+    uint32_t lend = nl, hend = nh;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, lend, o), y = __shfl_up_sync(0xffffffffu, hend, o);
+        if (lane >= o) {
+            lend += x;
+            hend += y;
+        }
     }
+    uint32_t lat = 0, hat = 0;
+    if (lane == 31 && lend) lat = atomicAdd(nlight, lend);
+    if (lane == 31 && hend) hat = atomicAdd(nheavy, hend);
+    lat = __shfl_sync(0xffffffffu, lat, 31) + lend - nl;
+    hat = __shfl_sync(0xffffffffu, hat, 31) + hend - nh;
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+        if (i < k && !chunks[i]) Q.light[lat++] = v[i];
+        for (unsigned h = __ballot_sync(0xffffffffu, chunks[i] != 0); h; h &= h - 1) {
+            // the warp writes a row's chunks together
+            const int src = __ffs(h) - 1;
+            const uint32_t cs = __shfl_sync(0xffffffffu, chunks[i], src), as = __shfl_sync(0xffffffffu, hat, src);
+            const int32_t vs = __shfl_sync(0xffffffffu, i < k ? v[i] : 0, src);
+            for (uint32_t c = lane; c < cs; c += 32) Q.heavy[as + c] = make_int2(vs, (int32_t)c);
+        }
+        hat += chunks[i];
+    }
+    return entries;
 }
 
-// Empties a buffer into the next queues.
-__device__ __forceinline__ void flush(Buffer& B, uint32_t& n, const uint64_t* __restrict__ off, const Queues& Q,
-                                      uint32_t* nlight, uint32_t* nheavy) {
+// Empties a buffer into the next queues; returns the row entries of this
+// lane's vertices.
+__device__ __forceinline__ uint64_t flush(Buffer& B, uint32_t& n, const uint64_t* __restrict__ off, const Queues& Q,
+                                          uint32_t* nlight, uint32_t* nheavy) {
+    constexpr int kMost = kBuf / 32;
+    const uint32_t lane = threadIdx.x & 31;
+    if (n == 0) return 0;
     __syncwarp();
-    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-        const uint32_t i = i0 + (threadIdx.x & 31);
-        enqueue(i < n, i < n ? B.v[i] : 0, off, Q, nlight, nheavy);
-    }
+    int32_t v[kMost];
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) v[i] = lane + 32 * i < n ? B.v[lane + 32 * i] : 0;
+    const int k = n > lane ? (int)((n - lane + 31) / 32) : 0;
+    const uint64_t entries = enqueue<kMost>(v, k, off, Q, nlight, nheavy);
     __syncwarp();
     n = 0;
+    return entries;
 }
 
 // Expands a frontier of nl light rows and nh chunks.  value(u) is taken once per row and chunk; visit(j, val,
@@ -122,13 +151,16 @@ __device__ __forceinline__ void expand(Tile& T, const uint64_t* __restrict__ off
             done();
         }
     }
-    // from the other end: the warps without a chunk begin
-    for (uint32_t t = nw - 1 - gw; (uint64_t)t * 32 < nl; t += nw) {
-        const uint32_t i = t * 32 + lane;
+    // Light rows, from the other end: the warps without a chunk begin.  A short
+    // queue is spread over all warps: 22 rows of up to 256 entries in one
+    // warp's hands held a level up for 80 us.
+    const uint32_t rows = min(32u, (nl + nw - 1) / nw);
+    for (uint32_t t = nw - 1 - gw; (uint64_t)t * rows < nl; t += nw) {
+        const uint32_t i = t * rows + lane;
         uint32_t len = 0;
         uint64_t b = 0;
         int32_t x = 0;
-        if (i < nl) {
+        if (lane < rows && i < nl) {
             const int32_t u = __ldcg(in.light + i);
             b = off[u];
             len = (uint32_t)(off[u + 1] - b);
