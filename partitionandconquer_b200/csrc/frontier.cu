@@ -25,9 +25,12 @@ constexpr int32_t kInf = INT_MAX;
 constexpr uint64_t kBarrierLimitNs = 4000000000ull;
 // k-core: ids below this have their degree decrements gathered per CTA
 constexpr int kKcoreHubs = 4096;
-constexpr uint32_t kLocalQ = 1024;       // k-core: per-CTA queue of vertices pushed in a step
+constexpr int kKcoreThreads = 512;       // k-core: threads per CTA
+constexpr int kKcorePerSm = 2;
+constexpr uint32_t kLocalQ = 2048;       // ... its queue of claimed vertices
 constexpr uint32_t kLocalEdges = 16384;  // ... peeled by the CTA itself while their rows stay below this
-static_assert(kKcoreHubs % kThreads == 0, "the flush loop needs a uniform trip count");
+constexpr size_t kKcoreSmem = 80 * 1024;
+static_assert(kKcoreHubs % kKcoreThreads == 0, "the flush loop needs a uniform trip count");
 
 // Appends `val` for every lane with pred set; all 32 lanes of the warp must
 // call it together.
@@ -47,66 +50,12 @@ __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t x) {
     return x;
 }
 
-// ---- rows longer than kHeavyDeg ------------------------------------------------
-// A warp-per-vertex loop serialises a hub's row on one warp (RMAT-22's largest
-// row has 163K entries: 5100 rounds of dependent loads on one warp).  The
-// frontier kernels set such vertices aside in a heavy list; heavy_rows() then
-// spreads the rows of the list over every warp of the grid in chunks of
-// kHeavyChunk entries, balanced by a block-local prefix of chunk counts.
-constexpr uint32_t kHeavyDeg = 1024;
-constexpr uint32_t kHeavyChunk = 256;
-constexpr uint32_t kHeavyBatch = 2048;  // list entries per shared-memory prefix
-static_assert(kHeavyBatch % kThreads == 0, "prefix items per thread");
 // Pull kernels (PageRank, CDLP): rows of more than kPullHeavyDeg entries get a
 // CTA; the others kPullLanes lanes, so a warp keeps 8 rows in flight (4 lanes
 // measured 10 % faster than 8 for PageRank at RMAT-22, 16 lanes 16 % slower).
 constexpr uint32_t kPullHeavyDeg = 256;
 constexpr int kPullLanes = 4;
 constexpr int kMisLanes = 8;  // MIS under id priorities: lanes per vertex
-
-// Calls body(u, j, valid) for the entries j of every row of hq[0..hn); the 32
-// lanes of a warp call it together (valid is false past a row's end), so the
-// body may use warp collectives.  All threads of every CTA must call it.
-template <class Body>
-__device__ __forceinline__ void heavy_rows(const uint64_t* __restrict__ off, const int32_t* hq, uint32_t hn,
-                                           Body&& body) {
-    using Scan = cub::BlockScan<uint32_t, kThreads>;
-    __shared__ typename Scan::TempStorage scan_tmp;
-    __shared__ uint32_t s_pref[kHeavyBatch + 1];
-    constexpr int kPer = kHeavyBatch / kThreads;
-    const int lane = threadIdx.x & 31;
-    const uint64_t wpb = blockDim.x >> 5;
-    const uint64_t gw = blockIdx.x * wpb + (threadIdx.x >> 5), nw = (uint64_t)gridDim.x * wpb;
-    for (uint32_t h0 = 0; h0 < hn; h0 += kHeavyBatch) {
-        const uint32_t hb = min(kHeavyBatch, hn - h0);
-        uint32_t cnt[kPer];
-        for (int t = 0; t < kPer; ++t) {
-            const uint32_t h = threadIdx.x * kPer + t;
-            cnt[t] = 0;
-            if (h < hb) {
-                const int32_t u = __ldcg(hq + h0 + h);
-                cnt[t] = (uint32_t)((off[u + 1] - off[u] + kHeavyChunk - 1) / kHeavyChunk);
-            }
-        }
-        __syncthreads();  // the previous batch is done with s_pref and scan_tmp
-        uint32_t total = 0;
-        Scan(scan_tmp).ExclusiveSum(cnt, cnt, total);
-        for (int t = 0; t < kPer; ++t) s_pref[threadIdx.x * kPer + t] = cnt[t];
-        if (threadIdx.x == 0) s_pref[kHeavyBatch] = total;
-        __syncthreads();
-        for (uint64_t c = gw; c < total; c += nw) {
-            uint32_t lo = 0, hi = hb - 1;  // last row whose chunks start at or before c
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (s_pref[mid] <= c) lo = mid; else hi = mid - 1;
-            }
-            const int32_t u = __ldcg(hq + h0 + lo);
-            const uint64_t rb = off[u] + (c - s_pref[lo]) * (uint64_t)kHeavyChunk;
-            const uint64_t re = min(rb + kHeavyChunk, off[u + 1]);
-            for (uint64_t j0 = rb; j0 < re; j0 += 32) body(u, j0 + lane, j0 + lane < re);
-        }
-    }
-}
 
 // Rows of more than thr entries (the pull kernels give each a whole CTA).
 __global__ void k_heavy_list(const uint64_t* __restrict__ off, uint64_t n, uint32_t thr, int32_t* __restrict__ hq,
@@ -628,245 +577,313 @@ __global__ void __launch_bounds__(kThreads) k_pr_iter(const uint64_t* __restrict
 
 // ---- k-core ----------------------------------------------------------------------
 
+// Device-driven peeling in one persistent kernel.  A step either scans the
+// remaining vertices at the next level or peels the frontier that an earlier
+// step of the level left in the queues; a grid barrier separates steps.
+//
+// Within a level the order of peeling does not matter, so a CTA peels what it
+// finds at once: vertices that the scan or a decrement takes below the level
+// go to the CTA's own queue, whose rows it lays end to end (a block scan) and
+// takes kPerLane entries per thread at a time, round after round until the
+// queue is dry.  A vertex is claimed by the compare-and-swap that sets its
+// core number, since the scan and the decrements of other CTAs may meet at
+// it.  What does not fit the queue, or would keep one CTA busy for long (rows
+// of more than `local_edges` entries together), goes to the next step's queues,
+// which all CTAs share (tx::expand).  So most levels take one step.
+//
+// The state lives in three rotating records: step i reads S[i % 3],
+// accumulates into S[(i+1) % 3] (counters cleared by step i-1) and clears
+// S[(i+2) % 3], which no CTA reads during step i.  Core numbers are read
+// through L1, which may hold an old "unpeeled": the entry then decrements a
+// peeled vertex's degree, which nobody looks at any more.
+//
+// Bound (RMAT-22): latency.  The 128 M entries are read once, but in some 300
+// dependent steps of a barrier and, per cascade round, one chain of row, id,
+// core number and decrement.  16.6 -> 8.5 ms a call (RMAT-16 3.2 -> 2.2, ER-20
+// 1.6 -> 0.88) against a step per scan and per round of spilled rows, with a
+// warp per row.  CTAs of 256 / 512 / 1024 threads, 1024 threads an SM: 9.0 /
+// 8.5 / 9.9 ms; local_edges of 4 K / 16 K / 64 K: 9.2 / 8.5 / 10.7 ms.
+struct __align__(16) KState {
+    uint32_t nl, nh;   // the frontier's queues
+    uint32_t rn;       // vertices on the remaining list
+    int32_t ml;        // minimum degree kept by a scan
+    int32_t k;         // level of the step that wrote this record
+    int32_t par;       // frontier queues in use
+    int32_t rpar;      // remaining list in use
+    int32_t dirty;     // whether the level claimed vertices before this step
+    uint32_t claimed;  // vertices the step claimed
+    int32_t top;       // largest core number before this step
+    int32_t pad[2];
+};
+
 __global__ void k_kcore_init(const uint64_t* __restrict__ off, uint64_t n, int32_t* __restrict__ deg,
-                             int32_t* __restrict__ core, int32_t* __restrict__ rem) {
-    uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+                             int32_t* __restrict__ core, int32_t* __restrict__ rem, KState* S, int32_t* d_top,
+                             GridBarrier* gb) {
+    const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (u < 3) S[u] = KState{0, 0, u ? 0u : (uint32_t)n, INT_MAX, 0, 0, 0, 1, 0, 0, {0, 0}};
+    if (u == 0) {
+        *d_top = 0;
+        *gb = GridBarrier{};
+    }
     if (u >= n) return;
     deg[u] = (int32_t)(off[u + 1] - off[u]);
     core[u] = -1;
     rem[u] = (int32_t)u;
 }
 
-// Device-driven peeling in one persistent kernel.  Each step is a peel round
-// at the current level when the frontier is not empty, else the scan of the
-// next level; a grid barrier separates steps.  The state lives in three
-// rotating records: step i reads S[i % 3], accumulates into S[(i+1) % 3]
-// (counters cleared by step i-1) and clears S[(i+2) % 3], which no CTA reads
-// during step i.  Mutable arrays are read with __ldcg: L1 is not coherent
-// across CTAs within one launch.  Frontier vertices with more than kHeavyDeg
-// neighbours are set aside (hq0/hq1 by step parity) and their rows are peeled
-// in the next step, spread over the grid; that step is still a peel round of
-// the same level, so every decrement of a level lands before its next scan.
-struct KState {
-    int32_t k;      // level of the step that wrote this record
-    uint32_t fn;    // frontier size it produced
-    uint32_t rn;    // remaining (unpeeled) vertices after it
-    int32_t ml;     // minimum degree left (scan steps)
-    int32_t phase;  // 0 scan, 1 peel
-    int32_t fpar;   // frontier buffer holding the frontier
-    int32_t rpar;   // remaining-list buffer
-    uint32_t hn;    // heavy frontier vertices it set aside for the next step
+struct KcoreTile {
+    uint64_t base[kKcoreThreads];
+    uint32_t start[kKcoreThreads];
 };
 
-__device__ __forceinline__ KState load_state(const KState* p) {
-    const int4 lo = __ldcg(reinterpret_cast<const int4*>(p));
-    const int4 hi = __ldcg(reinterpret_cast<const int4*>(p) + 1);
-    KState s;
-    s.k = lo.x;
-    s.fn = (uint32_t)lo.y;
-    s.rn = (uint32_t)lo.z;
-    s.ml = lo.w;
-    s.phase = hi.x;
-    s.fpar = hi.y;
-    s.rpar = hi.z;
-    s.hn = (uint32_t)hi.w;
-    return s;
-}
-
-__global__ void __launch_bounds__(kThreads) k_kcore_persistent(
+__global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent(
     const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, int32_t* deg, int32_t* core,
-    int32_t* rem0, int32_t* rem1, int32_t* f0, int32_t* f1, int32_t* hq0, int32_t* hq1, KState* S,
-    GridBarrier* gb, uint64_t max_steps, uint64_t limit_ns, uint64_t* steps_done, uint32_t local_edges) {
-    // decrements of the lowest ids (the hubs, once ids are degree-ordered)
-    // are gathered per CTA in shared memory and applied once per step
-    __shared__ int32_t s_dec[kKcoreHubs];
-    __shared__ int s_any;
-    __shared__ int32_t s_lq[2][kLocalQ];
-    __shared__ uint32_t s_lqn[2];  // entries pushed (may exceed kLocalQ: the rest went to the frontier)
-    __shared__ uint32_t s_lqe[2];  // row entries of the queued vertices
-    for (int i = threadIdx.x; i < kKcoreHubs; i += blockDim.x) s_dec[i] = 0;
+    int32_t* rem0, int32_t* rem1, tx::Queues q0, tx::Queues q1, KState* S, GridBarrier* gb, uint64_t max_steps,
+    uint64_t limit_ns, int32_t* d_top, uint32_t local_edges) {
+    constexpr int kWarps = kKcoreThreads / 32;
+    extern __shared__ __align__(16) unsigned char kcore_smem[];
+    struct Smem {
+        KcoreTile tile;                 // the local queue's rows
+        tx::Tile warp_tile[kWarps];     // tx::expand
+        tx::Buffer spill[kWarps];       // for the next step's queues
+        tx::Buffer keep[kWarps];        // for the remaining list
+        int32_t lq[2][kLocalQ];         // the CTA's own queue, two rounds
+        int32_t dec[kKcoreHubs];        // decrements of the lowest ids (the hubs, once ids are degree-ordered)
+        uint32_t warp_sum[kWarps];
+        uint32_t lqn[2];                // entries offered (those past kLocalQ went to spill)
+        uint32_t claimed;
+        int32_t ml;
+        int any_dec;
+    };
+    static_assert(sizeof(Smem) <= kKcoreSmem, "dynamic shared memory of the launch");
+    Smem& M = *reinterpret_cast<Smem*>(kcore_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    for (int i = threadIdx.x; i < kKcoreHubs; i += kKcoreThreads) M.dec[i] = 0;
     if (threadIdx.x == 0) {
-        s_any = 0;
-        s_lqn[0] = s_lqn[1] = 0;
-        s_lqe[0] = s_lqe[1] = 0;
+        M.lqn[0] = M.lqn[1] = 0;
+        M.claimed = 0;
+        M.ml = INT_MAX;
+        M.any_dec = 0;
     }
     __syncthreads();
-    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-    const int lane = threadIdx.x & 31;
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t warp = tid >> 5, nwarps = stride >> 5;
+    tx::Buffer& spill = M.spill[warp];
+    tx::Buffer& keep = M.keep[warp];
+    uint32_t nspill = 0, nkeep = 0;
     uint64_t step = 0;
     for (; step < max_steps; ++step) {
-        const KState in = load_state(&S[step % 3]);
+        const KState* in = &S[step % 3];
         KState* out = &S[(step + 1) % 3];
-        const bool peel = in.fn > 0 || in.hn > 0;
-        const int32_t k = peel ? in.k
-                               : ((in.phase == 1 || in.ml == INT_MAX) ? in.k + 1 : max(in.k + 1, in.ml + 1));
+        const int4 r0 = __ldcg(reinterpret_cast<const int4*>(in));
+        const int4 r1 = __ldcg(reinterpret_cast<const int4*>(in) + 1);
+        const int4 r2 = __ldcg(reinterpret_cast<const int4*>(in) + 2);
+        const uint32_t nl = (uint32_t)r0.x, nh = (uint32_t)r0.y, rn = (uint32_t)r0.z;
+        const int32_t par = r1.y, rpar = r1.z;
+        const bool peel = nl || nh;
+        const bool dirty = r1.w || r2.x;  // the level of the last step claimed something
+        const int32_t k = peel ? r1.x : (dirty || r0.w == INT_MAX ? r1.x + 1 : max(r1.x + 1, r0.w + 1));
+        const int32_t top = r2.x ? max(r2.y, r1.x - 1) : r2.y;
         // every CTA reads the same record, so all leave at the same step
-        if (!peel && (in.rn == 0 || (uint64_t)k >= n)) break;
+        if (!peel && (rn == 0 || (uint64_t)k >= n)) {
+            // vertices never peeled (only in a complete graph) keep core 0
+            if (rn)
+                for (uint64_t u = blockIdx.x * (uint64_t)kKcoreThreads + threadIdx.x; u < n;
+                     u += (uint64_t)gridDim.x * kKcoreThreads)
+                    if (__ldcg(core + u) < 0) core[u] = 0;
+            if (lead) *d_top = top;
+            return;
+        }
         if (lead) {
             KState* clr = &S[(step + 2) % 3];
-            clr->fn = 0;
-            clr->rn = 0;
+            clr->nl = clr->nh = clr->rn = clr->claimed = 0;
             clr->ml = INT_MAX;
-            clr->hn = 0;
-            if (peel) out->rn = in.rn;  // a peel round keeps the remaining list
+            if (peel) out->rn = rn;  // a peel step keeps the remaining list
             out->k = k;
-            out->phase = peel ? 1 : 0;
-            out->fpar = peel ? 1 - in.fpar : 0;
-            out->rpar = peel ? in.rpar : 1 - in.rpar;
+            out->par = 1 - par;
+            out->rpar = peel ? rpar : 1 - rpar;
+            out->dirty = peel && dirty;
+            out->top = top;
         }
+        const tx::Queues& Q = par ? q1 : q0;
+        const tx::Queues& QN = par ? q0 : q1;
+        uint32_t claimed = 0;
+        // a claimed vertex whose row is to be peeled, for every lane with pred set
+        auto push = [&](bool pred, int32_t v, int wr) {
+            const unsigned m = __ballot_sync(0xffffffffu, pred);
+            if (!m) return;
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&M.lqn[wr], (uint32_t)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (pred && at < kLocalQ) M.lq[wr][at] = v;
+            if (__any_sync(0xffffffffu, pred && at >= kLocalQ)) {
+                tx::find(spill, nspill, pred && at >= kLocalQ, v);
+                if (nspill > tx::kBuf - 32) tx::flush(spill, nspill, off, QN, &out->nl, &out->nh);
+            }
+        };
+        auto claim = [&](int32_t v) { return atomicCAS(&core[v], -1, k - 1) == -1; };
+        // kPerLane entries of peeled rows; each kind of access is issued for
+        // all of them before the first answer is needed
+        auto peel_entries = [&](const uint64_t* j, const bool* ok, int wr) {
+            int32_t v[tx::kPerLane], old[tx::kPerLane];
+            bool open[tx::kPerLane];
+#pragma unroll
+            for (int i = 0; i < tx::kPerLane; ++i) v[i] = ok[i] ? __ldcs(adj + j[i]) : 0;
+#pragma unroll
+            for (int i = 0; i < tx::kPerLane; ++i) open[i] = ok[i] && core[v[i]] < 0;
+#pragma unroll
+            for (int i = 0; i < tx::kPerLane; ++i) {
+                old[i] = 0;
+                if (!open[i]) continue;
+                if (v[i] < kKcoreHubs) {
+                    atomicAdd(&M.dec[v[i]], 1);
+                    M.any_dec = 1;
+                } else {
+                    old[i] = atomicSub(&deg[v[i]], 1);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < tx::kPerLane; ++i) {
+                const bool won = open[i] && old[i] == k && claim(v[i]);
+                claimed += won;
+                push(won, v[i], wr);
+            }
+        };
         if (peel) {
-            const int32_t* fq = in.fpar ? f1 : f0;
-            int32_t* nq = in.fpar ? f0 : f1;
-            int32_t* hq_next = (step & 1) ? hq1 : hq0;
-            const int32_t* hq_prev = (step & 1) ? hq0 : hq1;
-            // A vertex pushed at this level goes to this CTA's local queue
-            // (s_lq[wr]) while it has room, else to the next step's frontier;
-            // the CTA peels its local queue itself, so a level's cascade
-            // takes one step instead of one step per round.
-            int wr = 0;
-            auto push_v = [&](bool pred, int32_t v) {
-                const unsigned m = __ballot_sync(0xffffffffu, pred);
-                if (!m) return;
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&s_lqn[wr], (uint32_t)__popc(m));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                const uint32_t idx = base + __popc(m & ((1u << lane) - 1u));
-                const bool local = pred && idx < kLocalQ;
-                uint32_t len = 0;
-                if (local) {
-                    s_lq[wr][idx] = v;
-                    len = (uint32_t)min(off[v + 1] - off[v], (uint64_t)kHeavyDeg + 1);
-                }
-                for (int o = 16; o; o >>= 1) len += __shfl_xor_sync(0xffffffffu, len, o);
-                if (lane == 0 && len) atomicAdd(&s_lqe[wr], len);
-                warp_append(pred && !local, v, nq, &out->fn);
-            };
-            // one CSR entry (u, v) of a peeled vertex u; all lanes call it
-            auto peel_entry = [&](uint64_t j, bool ok) {
-                bool push = false;
-                int32_t v = 0;
-                if (ok) {
-                    v = adj[j];
-                    if (__ldcg(core + v) < 0) {
-                        if (v < kKcoreHubs) {
-                            atomicAdd(&s_dec[v], 1);
-                            s_any = 1;
-                        } else {
-                            const int32_t old = atomicSub(&deg[v], 1);
-                            if (old == k) {
-                                push = true;
-                                core[v] = k - 1;
-                            }
-                        }
-                    }
-                }
-                push_v(push, v);
-            };
-            // the row of a peeled vertex u, by one warp (set aside if heavy)
-            auto peel_row = [&](int32_t u) {
-                const uint64_t b = off[u], e = off[u + 1];
-                if (e - b > kHeavyDeg) {
-                    if (lane == 0) hq_next[atomicAdd(&out->hn, 1u)] = u;
-                    return;
-                }
-                for (uint64_t j0 = b; j0 < e; j0 += 32) peel_entry(j0 + lane, j0 + lane < e);
-            };
-            for (uint64_t i = warp; i < in.fn; i += nwarps) peel_row(__ldcg(fq + i));
-            heavy_rows(off, hq_prev, in.hn, [&](int32_t, uint64_t j, bool ok) { peel_entry(j, ok); });
-            // drain the local queues; when one runs dry, flush the gathered
-            // hub decrements (the one flush that takes a degree from >= k to
-            // < k pushes the vertex) and go on until nothing is left
-            int rd = 0;
-            for (;;) {
-                __syncthreads();
-                uint32_t cnt = min(s_lqn[rd], (uint32_t)kLocalQ);
-                if (cnt == 0) {
-                    if (s_any) {
-                        wr = rd;
-                        for (int i = threadIdx.x; i < kKcoreHubs; i += blockDim.x) {
-                            const int32_t c = s_dec[i];
-                            bool push = false;
-                            if (c) {
-                                s_dec[i] = 0;
-                                const int32_t old = atomicSub(&deg[i], c);
-                                if (old >= k && old - c < k) {
-                                    push = true;
-                                    core[i] = k - 1;
-                                }
-                            }
-                            push_v(push, i);
-                        }
-                        __syncthreads();
-                        if (threadIdx.x == 0) s_any = 0;
-                        __syncthreads();
-                        cnt = min(s_lqn[rd], (uint32_t)kLocalQ);
-                    }
-                    if (cnt == 0) break;
-                }
-                if (s_lqe[rd] > local_edges) {
-                    // too much for one CTA: the next step shares it among all
-                    const uint32_t cpad = (cnt + 31) & ~31u;
-                    for (uint32_t i = threadIdx.x; i < cpad; i += blockDim.x)
-                        warp_append(i < cnt, i < cnt ? s_lq[rd][i] : 0, nq, &out->fn);
-                    __syncthreads();
-                    if (threadIdx.x == 0) {
-                        s_lqn[rd] = 0;
-                        s_lqe[rd] = 0;
-                    }
-                    continue;
-                }
-                wr = rd ^ 1;
-                for (uint32_t i = threadIdx.x >> 5; i < cnt; i += blockDim.x >> 5) peel_row(s_lq[rd][i]);
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    s_lqn[rd] = 0;
-                    s_lqe[rd] = 0;
-                }
-                rd ^= 1;
-            }
-            if (threadIdx.x == 0) {
-                s_lqn[0] = s_lqn[1] = 0;
-                s_lqe[0] = s_lqe[1] = 0;
-            }
+            tx::expand(
+                M.warp_tile[warp], off, Q, nl, nh, [](int32_t) { return 0; },
+                [&](const uint64_t* j, const int32_t*, const bool* ok) { peel_entries(j, ok, 0); }, []() {});
         } else {
-            // scan of level k over the remaining list
-            const int32_t* rem = in.rpar ? rem1 : rem0;
-            int32_t* rem2 = in.rpar ? rem0 : rem1;
-            const uint64_t nr = ((uint64_t)in.rn + 31) & ~(uint64_t)31;
+            const int32_t* rem = rpar ? rem1 : rem0;
+            int32_t* rem2 = rpar ? rem0 : rem1;
+            auto flush_keep = [&]() {
+                if (nkeep == 0) return;
+                __syncwarp();
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&out->rn, nkeep);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                for (uint32_t i = lane; i < nkeep; i += 32) rem2[at + i] = keep.v[i];
+                __syncwarp();
+                nkeep = 0;
+            };
             int32_t mn = INT_MAX;
-            for (uint64_t i = tid; i < nr; i += stride) {
-                bool pl = false, keep = false;
+            const uint64_t nr = ((uint64_t)rn + 31) & ~(uint64_t)31;
+            for (uint64_t i = blockIdx.x * (uint64_t)kKcoreThreads + threadIdx.x; i < nr;
+                 i += (uint64_t)gridDim.x * kKcoreThreads) {
+                bool pl = false, stay = false;
                 int32_t u = 0;
-                if (i < in.rn) {
+                if (i < rn) {
                     u = __ldcg(rem + i);
-                    if (__ldcg(core + u) < 0) {
-                        const int32_t d = __ldcg(deg + u);
-                        if (d < k) {
+                    const int32_t c = __ldcg(core + u), d = __ldcg(deg + u);
+                    if (c < 0) {
+                        if (d >= k) {
+                            stay = true;
+                            mn = min(mn, d);
+                        } else if (claim(u)) {
+                            ++claimed;
                             // d counts the unpeeled neighbours: with none,
                             // peeling u would decrement nobody
                             pl = d > 0;
-                            core[u] = k - 1;
-                        } else {
-                            keep = true;
-                            mn = min(mn, d);
                         }
                     }
                 }
-                warp_append(pl, u, f0, &out->fn);
-                warp_append(keep, u, rem2, &out->rn);
+                push(pl, u, 0);
+                tx::find(keep, nkeep, stay, u);
+                if (nkeep > tx::kBuf - 32) flush_keep();
             }
-            for (int o = 16; o; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            if (lane == 0 && mn != INT_MAX) atomicMin(&out->ml, mn);
+            flush_keep();
+            mn = __reduce_min_sync(0xffffffffu, mn);
+            if (lane == 0 && mn != INT_MAX) atomicMin(&M.ml, mn);
+        }
+        // drain the CTA's queue; when it runs dry, flush the gathered hub
+        // decrements (the one flush that takes a degree from >= k to < k
+        // pushes the vertex) and go on until nothing is left
+        int rd = 0;
+        for (;;) {
+            __syncthreads();
+            uint32_t cnt = min(M.lqn[rd], (uint32_t)kLocalQ);
+            if (cnt == 0) {
+                if (!M.any_dec) break;
+                __syncthreads();  // every thread has read any_dec
+                if (threadIdx.x == 0) M.any_dec = 0;
+                for (int i = threadIdx.x; i < kKcoreHubs; i += kKcoreThreads) {
+                    const int32_t c = M.dec[i];
+                    bool won = false;
+                    if (c) {
+                        M.dec[i] = 0;
+                        const int32_t old = atomicSub(&deg[i], c);
+                        won = old >= k && old - c < k && claim(i);
+                        claimed += won;
+                    }
+                    push(won, i, rd);
+                }
+                __syncthreads();
+                cnt = min(M.lqn[rd], (uint32_t)kLocalQ);
+                if (cnt == 0) break;
+            }
+            const int wr = rd ^ 1;
+            for (uint32_t base = 0; base < cnt; base += kKcoreThreads) {
+                // rows of up to kKcoreThreads entries of the queue, end to end
+                const uint32_t i = base + threadIdx.x;
+                const int32_t u = i < cnt ? M.lq[rd][i] : 0;
+                const uint64_t b = i < cnt ? off[u] : 0;
+                const uint32_t len = i < cnt ? (uint32_t)min(off[u + 1] - b, (uint64_t)(1u << 21)) : 0;
+                uint32_t end = len;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+                    if (lane >= o) end += x;
+                }
+                if (lane == 31) M.warp_sum[warp] = end;
+                __syncthreads();
+                uint32_t total = 0;
+                for (int x = 0; x < kWarps; ++x) {
+                    const uint32_t y = M.warp_sum[x];
+                    if (x < warp) end += y;
+                    total += y;
+                }
+                M.tile.start[threadIdx.x] = end - len;
+                M.tile.base[threadIdx.x] = b - (end - len);
+                __syncthreads();
+                if (total > local_edges) {  // too much for one CTA: the next step shares it among all
+                    tx::find(spill, nspill, i < cnt, u);
+                    if (nspill > tx::kBuf - 32) tx::flush(spill, nspill, off, QN, &out->nl, &out->nh);
+                    continue;
+                }
+                for (uint32_t e0 = 0; e0 < total; e0 += kKcoreThreads * tx::kPerLane) {
+                    uint64_t j[tx::kPerLane];
+                    bool ok[tx::kPerLane];
+#pragma unroll
+                    for (int x = 0; x < tx::kPerLane; ++x) {
+                        const uint32_t e = e0 + x * kKcoreThreads + threadIdx.x;
+                        ok[x] = e < total;
+                        int lo = 0;
+#pragma unroll
+                        for (int s = kKcoreThreads / 2; s; s >>= 1)
+                            if (M.tile.start[lo + s] <= e) lo += s;
+                        j[x] = M.tile.base[lo] + e;
+                    }
+                    peel_entries(j, ok, wr);
+                }
+                __syncthreads();  // the tile is rewritten
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) M.lqn[rd] = 0;
+            rd = wr;
+        }
+        tx::flush(spill, nspill, off, QN, &out->nl, &out->nh);
+        claimed = __reduce_add_sync(0xffffffffu, claimed);
+        if (lane == 0 && claimed) atomicAdd(&M.claimed, claimed);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (M.claimed) atomicAdd(&out->claimed, M.claimed);
+            if (M.ml != INT_MAX) atomicMin(&out->ml, M.ml);
+            M.claimed = 0;
+            M.ml = INT_MAX;
+            M.lqn[0] = M.lqn[1] = 0;
         }
         if (!grid_sync(gb, limit_ns)) return;
     }
-    if (lead) {
-        *steps_done = step;
-        if (step == max_steps) atomicExch(&gb->err, 2);
-    }
+    if (lead) atomicExch(&gb->err, 2);
 }
 
 // Self-test of the grid barrier: `rounds` barriers, each CTA adding 1 to
@@ -882,18 +899,6 @@ __global__ void k_grid_sync_selftest(GridBarrier* gb, int rounds, int absent, ui
         if (threadIdx.x == 0 && __ldcg(tally) < (unsigned)(r + 1) * gridDim.x) atomicAdd(bad, 1u);
         if (!grid_sync(gb, limit_ns)) return;
     }
-}
-
-// Vertices never peeled get core 0; *top receives the largest core number.
-__global__ void k_kcore_finish(int32_t* __restrict__ core, uint64_t n, int32_t* __restrict__ top) {
-    const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    int32_t c = 0;
-    if (u < n) {
-        c = core[u];
-        if (c < 0) core[u] = c = 0;
-    }
-    for (int o = 16; o; o >>= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
-    if ((threadIdx.x & 31) == 0 && c > 0) atomicMax(top, c);
 }
 
 // ---- MIS -------------------------------------------------------------------------
@@ -1050,8 +1055,7 @@ using namespace fr;
 
 static unsigned grid_for(const pc_pgraph* pg, int per_sm = 8) { return (unsigned)(sm_count(pg->g->device) * per_sm); }
 
-// Entries a heavy list can need: rows of more than kHeavyDeg entries.
-static uint64_t heavy_cap(uint64_t n, uint64_t m) { return std::max<uint64_t>(1, std::min<uint64_t>(n, m / kHeavyDeg + 1)); }
+// Entries the list of heavy rows can need.
 static uint64_t pull_heavy_cap(uint64_t n, uint64_t m) {
     return std::max<uint64_t>(1, std::min<uint64_t>(n, m / kPullHeavyDeg + 1));
 }
@@ -1081,9 +1085,9 @@ static pc_status read_u32(pc_pgraph* pg, const uint32_t* d, uint32_t* h) {
 // entries.  BFS takes 2048 (RMAT-16: 0.14 ms, 0.20 with 256), SSSP, whose steps
 // wait on chains of atomics, 256 (RMAT-16: 0.37 ms, 0.41 with 2048).
 static pc_status persistent_grid(const pc_pgraph* pg, const void* kernel, int threads, int most_per_sm, uint64_t work,
-                                 unsigned* grid) {
+                                 unsigned* grid, size_t smem = 0) {
     int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (per_sm < 1) return fail(PC_ERR_CUDA, "persistent kernel cannot be resident");
     const uint64_t all = (uint64_t)sm_count(pg->g->device) * std::min(per_sm, most_per_sm);
     *grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(all, ceil_div(pg->g->n + pg->g->m / 4, work)));
@@ -1373,62 +1377,53 @@ pc_status pc_kcore(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
         if (largest) *largest = 0;
         return PC_OK;
     }
-    const uint64_t hcap = heavy_cap(n, pg->g->m);
-    PC_TRY(scratch_reserve(pg, n * 4 * 7 + hcap * 8 + sizeof(KState) * 3 + sizeof(GridBarrier) + 16));
+    const uint64_t hcap = tx::heavy_chunks(n, pg->g->m);
+    PC_TRY(scratch_reserve(pg, n * 4 * 7 + hcap * 16 + 1024));
     int32_t* deg = pg->scratch.take<int32_t>(n);
     int32_t* core = pg->scratch.take<int32_t>(n);
     int32_t* rem0 = pg->scratch.take<int32_t>(n);
     int32_t* rem1 = pg->scratch.take<int32_t>(n);
-    int32_t* f0 = pg->scratch.take<int32_t>(n);
-    int32_t* f1 = pg->scratch.take<int32_t>(n);
+    tx::Queues q0{pg->scratch.take<int32_t>(n), nullptr}, q1{pg->scratch.take<int32_t>(n), nullptr};
+    q0.heavy = pg->scratch.take<int2>(hcap);
+    q1.heavy = pg->scratch.take<int2>(hcap);
     int32_t* out = pg->scratch.take<int32_t>(n);
-    int32_t* hq0 = pg->scratch.take<int32_t>(hcap);
-    int32_t* hq1 = pg->scratch.take<int32_t>(hcap);
     KState* S = pg->scratch.take<KState>(3);
     GridBarrier* gb = pg->scratch.take<GridBarrier>(1);
-    uint64_t* d_steps = pg->scratch.take<uint64_t>(1);
     int32_t* d_top = pg->scratch.take<int32_t>(1);
     if (!d_top) return fail(PC_ERR_OOM, "k-core scratch plan exceeds its reservation");
-    const unsigned nb = (unsigned)ceil_div(n, kThreads);
-    k_kcore_init<<<nb, kThreads, 0, s>>>(pg->off, n, deg, core, rem0);
-    PC_LAUNCHED();
     // Levels k = 1 .. n-1, as the reference's loop (src/Graph.cpp:683, 1893):
     // at level k every remaining vertex of degree < k gets core k-1, and
     // peeling repeats until no degree crosses below k; empty levels jump to
     // the minimum degree left, as the reference does (src/Graph.cpp:1921).
     // Vertices never peeled (only in a complete graph) keep core 0.
-    KState init[3] = {};
-    init[0].rn = (uint32_t)n;
-    init[1].ml = INT_MAX;
-    PC_CUDA(cudaMemcpyAsync(S, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    PC_CUDA(cudaMemsetAsync(gb, 0, sizeof(GridBarrier), s));
-    PC_CUDA(cudaMemsetAsync(d_top, 0, 4, s));
-    int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_kcore_persistent, kThreads, 0));
-    if (per_sm < 1) return fail(PC_ERR_CUDA, "k-core kernel cannot be resident");
-    const unsigned grid = (unsigned)(sm_count(pg->g->device) * std::min(per_sm, 4));
-    // a step scans a level, peels a frontier or peels set-aside heavy rows;
-    // each vertex enters a frontier and a heavy list at most once, so n
-    // levels plus 2n peel rounds bound the steps
+    k_kcore_init<<<(unsigned)ceil_div(n, kThreads), kThreads, 0, s>>>(pg->off, n, deg, core, rem0, S, d_top, gb);
+    PC_LAUNCHED();
+    PC_CUDA(cudaFuncSetAttribute(k_kcore_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKcoreSmem));
+    unsigned grid = 0;
+    PC_TRY(persistent_grid(pg, (const void*)k_kcore_persistent, kKcoreThreads, kKcorePerSm, 4096, &grid, kKcoreSmem));
+    // a step scans a level or peels vertices claimed before it; each vertex
+    // is claimed once, so n levels plus 2n peel steps bound the steps
     uint64_t max_steps = 3 * n + 8;
     uint64_t limit_ns = kBarrierLimitNs;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     uint64_t nn = n;
     uint32_t local_edges = kcore_local_edges();
-    void* args[] = {(void*)&off,  (void*)&adj, (void*)&nn, (void*)&deg, (void*)&core, (void*)&rem0,
-                    (void*)&rem1, (void*)&f0,  (void*)&f1, (void*)&hq0, (void*)&hq1,  (void*)&S,
-                    (void*)&gb,   (void*)&max_steps, (void*)&limit_ns, (void*)&d_steps, (void*)&local_edges};
-    PC_CUDA(cudaLaunchCooperativeKernel((const void*)k_kcore_persistent, dim3(grid), dim3(kThreads), args, 0, s));
+    void* args[] = {(void*)&off, (void*)&adj, (void*)&nn, (void*)&deg, (void*)&core, (void*)&rem0, (void*)&rem1,
+                    (void*)&q0,  (void*)&q1,  (void*)&S,  (void*)&gb,  (void*)&max_steps, (void*)&limit_ns,
+                    (void*)&d_top, (void*)&local_edges};
+    PC_CUDA(cudaLaunchCooperativeKernel((const void*)k_kcore_persistent, dim3(grid), dim3(kKcoreThreads), args, kKcoreSmem,
+                                        s));
     PC_LAUNCHED();
-    k_kcore_finish<<<nb, kThreads, 0, s>>>(core, n, d_top);
-    PC_LAUNCHED();
-    PC_TRY(gather_to_api_i32(pg, core, out));
-    PC_CUDA(cudaMemcpyAsync(core_host, out, n * 4, cudaMemcpyDeviceToHost, s));
+    if (!api_is_internal(pg)) {
+        PC_TRY(gather_to_api_i32(pg, core, out));
+        core = out;
+    }
     GridBarrier hb{};
     int32_t top = 0;
     PC_CUDA(cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s));
     PC_CUDA(cudaMemcpyAsync(&top, d_top, 4, cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaMemcpyAsync(core_host, core, n * 4, cudaMemcpyDeviceToHost, s));
     PC_TRY(sync(pg));
     // the kernel's own status decides whether core_host holds a result
     if (hb.err == 1) return fail(PC_ERR_TIMEOUT, "k-core: a grid barrier wait ran out of time");

@@ -131,7 +131,7 @@ template <class Value, class Visit, class Done>
 __device__ __forceinline__ void expand(Tile& T, const uint64_t* __restrict__ off, const Queues& in, uint32_t nl,
                                            uint32_t nh, Value&& value, Visit&& visit, Done&& done) {
     const int lane = threadIdx.x & 31;
-    const uint32_t gw = blockIdx.x * kWarps + (threadIdx.x >> 5), nw = gridDim.x * kWarps;
+    const uint32_t wpb = blockDim.x >> 5, gw = blockIdx.x * wpb + (threadIdx.x >> 5), nw = gridDim.x * wpb;
     uint64_t j[kPerLane];
     int32_t val[kPerLane];
     bool ok[kPerLane];
