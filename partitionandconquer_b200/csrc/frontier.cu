@@ -55,7 +55,6 @@ __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t x) {
 // measured 10 % faster than 8 for PageRank at RMAT-22, 16 lanes 16 % slower).
 constexpr uint32_t kPullHeavyDeg = 256;
 constexpr int kPullLanes = 4;
-constexpr int kMisLanes = 8;  // MIS under id priorities: lanes per vertex
 
 // Rows of more than thr entries (the pull kernels give each a whole CTA).
 __global__ void k_heavy_list(const uint64_t* __restrict__ off, uint64_t n, uint32_t thr, int32_t* __restrict__ hq,
@@ -69,11 +68,6 @@ __global__ void k_heavy_list(const uint64_t* __restrict__ off, uint64_t n, uint3
 }
 
 // ---- BFS -------------------------------------------------------------------
-
-__global__ void k_iota(int32_t* a, uint64_t n) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) a[i] = (int32_t)i;
-}
 
 // Direction-optimising (Beamer, Asanovic, Patterson, SC'12) in one persistent
 // kernel, a grid barrier per level: top-down levels expand the frontier's
@@ -902,102 +896,154 @@ __global__ void k_grid_sync_selftest(GridBarrier* gb, int rounds, int absent, ui
 }
 
 // ---- MIS -------------------------------------------------------------------------
+//
+// The lexicographically-first set: u is in it when no neighbour of smaller
+// priority is.  Work-efficient form (Blelloch, Fineman, Shun, "Greedy
+// sequential maximal independent set and matching are parallel on average",
+// SPAA 2012): waits[u] counts the undecided neighbours of smaller priority; a
+// vertex that is decided is queued once, and its row tells its neighbours: a
+// member takes its undecided neighbours out, a vertex left out stops the
+// neighbours of larger priority from waiting, and the one that waits for
+// nobody any more is a member.  Every decision follows from final ones, so the
+// order does not matter and the set is unique.
+//
+// One persistent kernel: a step expands the queue of the vertices decided in
+// the step before (tx::expand); every entry is looked at once (and once more to
+// count, under priorities that are not the ids).  Bound by the steps' latency
+// on small graphs, by the gathers of states on large ones.  Rounds over the
+// undecided vertices' whole rows, a launch and a host read each, took 0.32 ms
+// at RMAT-16 and 3.1 at RMAT-22 (hashed), 4.2 at RMAT-22 under ids; this form
+// 0.19, 1.9 and 1.6 ms.
+struct __align__(16) MisState {
+    uint32_t nl, nh;  // the queues of the step that reads the record
+    int32_t par;
+    int32_t pad;
+};
 
-// Round over the undecided list: OUT if a neighbour is IN; IN if every
-// neighbour of smaller priority is OUT; otherwise undecided again.  Decisions
-// are final and only made from final neighbour states, so the in-place update
-// reaches the unique greedy (lexicographically-first) set.
-__global__ void k_mis_round(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                            const uint64_t* __restrict__ prio, const uint32_t* __restrict__ dplus,
-                            const int32_t* __restrict__ uq, uint32_t un, int32_t* __restrict__ state,
-                            int32_t* __restrict__ nq, uint32_t* __restrict__ nn) {
+// Priorities: a hash of the caller's id, or that id; ties by internal id.
+struct MisPriority {
+    uint64_t key;
+    int hashed;
+    const int32_t* __restrict__ int2api;  // null: the same ids
+    __device__ __forceinline__ bool less(int32_t v, int32_t u) const {  // v before u
+        const uint32_t a = int2api ? (uint32_t)int2api[v] : (uint32_t)v, b = int2api ? (uint32_t)int2api[u] : (uint32_t)u;
+        const uint64_t pv = hashed ? pc_vertex_priority(key, a) : a, pu = hashed ? pc_vertex_priority(key, b) : b;
+        return pv < pu || (pv == pu && v < u);
+    }
+};
+
+// state: -1 undecided, 0 left out, 1 member.  dplus (id priorities): the
+// neighbours to wait for; else every vertex is queued to have them counted.
+__global__ void k_mis_init(const uint64_t* __restrict__ off, uint64_t n, const uint32_t* __restrict__ dplus,
+                           int32_t* __restrict__ state, int32_t* __restrict__ waits, tx::Queues Q, MisState* S,
+                           GridBarrier* gb) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *gb = GridBarrier{};
+    __shared__ tx::Buffer buf[kThreads / 32];
+    tx::Buffer& B = buf[threadIdx.x >> 5];
+    uint32_t nb = 0;
+    for (uint64_t u0 = blockIdx.x * (uint64_t)blockDim.x; u0 < n; u0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t u = u0 + threadIdx.x;
+        if (u < n) {
+            state[u] = -1;
+            waits[u] = dplus ? (int32_t)dplus[u] : 0;
+        }
+        if (!dplus) {
+            tx::find(B, nb, u < n, (int32_t)u);
+            if (nb > tx::kBuf - 32) tx::flush(B, nb, off, Q, &S[0].nl, &S[0].nh);
+        }
+    }
+    tx::flush(B, nb, off, Q, &S[0].nl, &S[0].nh);
+}
+
+__global__ void __launch_bounds__(tx::kThreads, 6)
+    k_mis_persistent(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, MisPriority P,
+                     int count_first, int32_t* state, int32_t* waits, tx::Queues q0, tx::Queues q1, MisState* S,
+                     GridBarrier* gb, uint64_t max_steps, uint64_t limit_ns) {
+    __shared__ tx::Tile s_tile[tx::kWarps];
+    __shared__ tx::Buffer s_buf[tx::kWarps];
+    tx::Tile& T = s_tile[threadIdx.x >> 5];
+    tx::Buffer& B = s_buf[threadIdx.x >> 5];
+    uint32_t nb = 0;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    if (dplus) {
-        // With id priorities only the neighbours below u matter: an IN
-        // neighbour v > u would need u OUT first, and only v < u block (rows
-        // are sorted, so those are the first dplus[u] entries).  Those lists
-        // are short, so kMisLanes lanes take a vertex, 32 / kMisLanes at once.
-        constexpr int kRows = 32 / kMisLanes;
-        const int g = lane / kMisLanes, gl = lane % kMisLanes;
-        const unsigned gm = ((1u << kMisLanes) - 1u) << (g * kMisLanes);
-        for (uint64_t i0 = warp * kRows; i0 < un; i0 += nwarps * kRows) {
-            const uint64_t i = i0 + g;
-            const bool have = i < un;
-            int32_t u = 0;
-            uint64_t b = 0, e = 0;
-            if (have) {
-                u = uq[i];
-                b = off[u];
-                e = b + dplus[u];
-            }
-            bool in_nbr = false, blocked = false;
-            for (uint64_t k = 0;; k += kMisLanes) {
-                const uint64_t j = b + k + gl;
-                bool a = false, c = false;
-                if (have && !in_nbr && j < e) {
-                    const int32_t v = adj[j];
-                    const int32_t sv = state[v];
-                    a = sv == 1;
-                    c = sv == 0;  // every v here is below u
-                }
-                // every lane votes (a short-circuit here would skip the
-                // vote on some lanes and leave the others waiting)
-                const unsigned va = __ballot_sync(0xffffffffu, a);
-                const unsigned vc = __ballot_sync(0xffffffffu, c);
-                in_nbr = in_nbr || (va & gm) != 0;
-                blocked = blocked || (vc & gm) != 0;
-                const bool more = have && !in_nbr && b + k + kMisLanes < e;
-                if (!__any_sync(0xffffffffu, more)) break;
-            }
-            if (have && gl == 0) {
-                if (in_nbr) state[u] = 2;
-                else if (!blocked) state[u] = 1;
-            }
-            warp_append(have && gl == 0 && !in_nbr && blocked, u, nq, nn);
+    const uint64_t first = count_first ? 1 : 0;  // step in which the vertices that wait for nobody join
+    uint64_t step = 0;
+    for (; step < max_steps; ++step) {
+        const MisState* in = &S[step % 3];
+        MisState* out = &S[(step + 1) % 3];
+        const int4 r = __ldcg(reinterpret_cast<const int4*>(in));
+        const uint32_t nl = (uint32_t)r.x, nh = (uint32_t)r.y;
+        const int32_t par = r.z;
+        // every CTA reads the same record, so all leave at the same step
+        if (step > first && !nl && !nh) return;
+        if (lead) {
+            MisState* clr = &S[(step + 2) % 3];
+            clr->nl = clr->nh = 0;
+            out->par = 1 - par;
         }
-        return;
+        const tx::Queues& Q = par ? q1 : q0;
+        const tx::Queues& QN = par ? q0 : q1;
+        auto room = [&]() {
+            if (nb > tx::kBuf - tx::kRound) tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        };
+        if (step < first) {
+            // neighbours of smaller priority, a vote per run of lanes with the same row
+            tx::expand(
+                T, off, Q, nl, nh, [](int32_t u) { return u; },
+                [&](const uint64_t* j, const int32_t* u, const bool* ok) {
+                    int32_t v[tx::kPerLane];
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) v[k] = ok[k] ? __ldcs(adj + j[k]) : 0;
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        const unsigned m = __ballot_sync(0xffffffffu, ok[k] && P.less(v[k], u[k]));
+                        if (!m) continue;
+                        const unsigned run = __match_any_sync(0xffffffffu, u[k]);
+                        if (lane == __ffs(run) - 1 && (m & run)) atomicAdd(&waits[u[k]], __popc(m & run));
+                    }
+                },
+                []() {});
+        } else if (step == first) {
+            for (uint64_t u0 = blockIdx.x * (uint64_t)tx::kThreads; u0 < n; u0 += (uint64_t)gridDim.x * tx::kThreads) {
+                const uint64_t u = u0 + threadIdx.x;
+                const bool in_set = u < n && __ldcg(waits + u) == 0;
+                if (in_set) state[u] = 1;
+                tx::find(B, nb, in_set && off[u + 1] > off[u], (int32_t)u);
+                room();
+            }
+        } else {
+            tx::expand(
+                T, off, Q, nl, nh, [&](int32_t u) { return __ldcg(state + u) ? u : ~u; },
+                [&](const uint64_t* j, const int32_t* val, const bool* ok) {
+                    int32_t v[tx::kPerLane];
+                    bool hit[tx::kPerLane];
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) v[k] = ok[k] ? __ldcs(adj + j[k]) : 0;
+                    // a state read here may be an old "undecided" from L1: a member's
+                    // row settles that by compare-and-swap, and a decided
+                    // vertex's count is not looked at any more
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) hit[k] = ok[k] && state[v[k]] < 0;
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        if (!hit[k]) continue;
+                        if (val[k] >= 0) hit[k] = atomicCAS(&state[v[k]], -1, 0) == -1;
+                        else hit[k] = P.less(~val[k], v[k]) && atomicSub(&waits[v[k]], 1) == 1;
+                    }
+#pragma unroll
+                    for (int k = 0; k < tx::kPerLane; ++k) {
+                        // a vertex with a member among the neighbours it waits for
+                        // never stops waiting, so no other step decides this one
+                        if (hit[k] && val[k] < 0) state[v[k]] = 1;
+                        tx::find(B, nb, hit[k], v[k]);
+                    }
+                },
+                room);
+        }
+        tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        if (!grid_sync(gb, limit_ns)) return;
     }
-    for (uint64_t i = warp; i < un; i += nwarps) {
-        const int32_t u = uq[i];
-        const uint64_t pu = prio ? prio[u] : (uint64_t)u;
-        const uint64_t b = off[u], e = off[u + 1];
-        bool in_nbr = false, blocked = false;
-        for (uint64_t j0 = b; j0 < e; j0 += 32) {
-            const uint64_t j = j0 + lane;
-            bool a = false, c = false;
-            if (j < e) {
-                const int32_t v = adj[j];
-                const int32_t sv = state[v];
-                a = sv == 1;
-                const uint64_t pv = prio ? prio[v] : (uint64_t)v;
-                c = sv == 0 && (pv < pu || (pv == pu && v < u));
-            }
-            in_nbr = __any_sync(0xffffffffu, a) || in_nbr;
-            blocked = __any_sync(0xffffffffu, c) || blocked;
-            if (in_nbr) break;
-        }
-        if (lane == 0) {
-            if (in_nbr) state[u] = 2;
-            else if (!blocked) state[u] = 1;
-        }
-        const bool again = !in_nbr && blocked;
-        if (lane == 0 && again) nq[atomicAdd(nn, 1u)] = u;
-    }
-}
-
-__global__ void k_mis_prio(uint64_t n, const int32_t* __restrict__ int2api, uint64_t key, int hashed,
-                           uint64_t* __restrict__ prio) {
-    uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    const uint32_t api = int2api ? (uint32_t)int2api[u] : (uint32_t)u;
-    prio[u] = hashed ? pc_vertex_priority(key, api) : (uint64_t)api;
-}
-
-__global__ void k_mis_finish(const int32_t* __restrict__ state, uint64_t n, int32_t* __restrict__ res) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) res[i] = state[i] == 1 ? 1 : 0;
+    if (lead) atomicExch(&gb->err, 2);
 }
 
 // ---- CDLP --------------------------------------------------------------------------
@@ -1073,17 +1119,11 @@ static pc_status list_heavy_rows(pc_pgraph* pg, int32_t* hq, uint32_t* d_hn, uin
     return PC_OK;
 }
 
-// Reads a device counter (synchronising the stream).
-static pc_status read_u32(pc_pgraph* pg, const uint32_t* d, uint32_t* h) {
-    PC_CUDA(cudaMemcpyAsync(h, d, 4, cudaMemcpyDeviceToHost, pg->g->stream));
-    PC_CUDA(cudaStreamSynchronize(pg->g->stream));
-    return PC_OK;
-}
-
 // CTAs of a persistent kernel: every SM's share, fewer for a small graph,
 // whose barriers then have fewer arrivals; one per `work` vertices and quarter
 // entries.  BFS takes 2048 (RMAT-16: 0.14 ms, 0.20 with 256), SSSP, whose steps
-// wait on chains of atomics, 256 (RMAT-16: 0.37 ms, 0.41 with 2048).
+// wait on chains of atomics, 256 (RMAT-16: 0.37 ms, 0.41 with 2048), MIS 1024,
+// k-core's larger CTAs 4096.
 static pc_status persistent_grid(const pc_pgraph* pg, const void* kernel, int threads, int most_per_sm, uint64_t work,
                                  unsigned* grid, size_t smem = 0) {
     int per_sm = 0;
@@ -1171,47 +1211,51 @@ static pc_status pagerank_run(pc_pgraph* pg, T damping, int32_t iters, const T* 
 }
 
 static pc_status mis_run(pc_pgraph* pg, bool hashed, uint64_t seed, int32_t* res_host) {
-    const uint64_t n = pg->g->n;
+    const uint64_t n = pg->g->n, m = pg->g->m;
     cudaStream_t s = pg->g->stream;
-    PC_TRY(scratch_reserve(pg, n * 4 * 4 + n * 8 + 256));
-    int32_t* state = pg->scratch.take<int32_t>(n);
-    int32_t* q0 = pg->scratch.take<int32_t>(n);
-    int32_t* q1 = pg->scratch.take<int32_t>(n);
-    int32_t* out = pg->scratch.take<int32_t>(n);
-    uint64_t* prio = nullptr;
-    uint32_t* cnt = pg->scratch.take<uint32_t>(2);
-    const unsigned nb = (unsigned)ceil_div(n, kThreads);
     const int32_t* int2api = api_is_internal(pg) ? nullptr : pg->old2new.as<int32_t>();
-    if (hashed || int2api) {
-        prio = pg->scratch.take<uint64_t>(n);
-        k_mis_prio<<<nb, kThreads, 0, s>>>(n, int2api, pc_graph_key(seed, PC_GEN_PRIORITY), hashed ? 1 : 0, prio);
-        PC_LAUNCHED();
-    }
-    const uint32_t* dp = nullptr;
-    if (!prio) {
-        PC_TRY(ensure_dplus(pg));
-        dp = pg->dplus.as<uint32_t>();
-    }
-    PC_CUDA(cudaMemsetAsync(state, 0, n * 4, s));
-    // all vertices start undecided
-    k_iota<<<nb, kThreads, 0, s>>>(q0, n);
+    // under the internal ids themselves the neighbours to wait for are the
+    // first dplus[u] of a row
+    const bool count_first = hashed || int2api;
+    if (!count_first) PC_TRY(ensure_dplus(pg));
+    const uint64_t hcap = tx::heavy_chunks(n, m);
+    PC_TRY(scratch_reserve(pg, n * 4 * 5 + hcap * 16 + 1024));
+    int32_t* state = pg->scratch.take<int32_t>(n);
+    int32_t* waits = pg->scratch.take<int32_t>(n);
+    int32_t* out = pg->scratch.take<int32_t>(n);
+    tx::Queues q0{pg->scratch.take<int32_t>(n), nullptr}, q1{pg->scratch.take<int32_t>(n), nullptr};
+    q0.heavy = pg->scratch.take<int2>(hcap);
+    q1.heavy = pg->scratch.take<int2>(hcap);
+    MisState* S = pg->scratch.take<MisState>(3);
+    GridBarrier* gb = pg->scratch.take<GridBarrier>(1);
+    if (!gb) return fail(PC_ERR_OOM, "MIS scratch plan exceeds its reservation");
+    PC_CUDA(cudaMemsetAsync(S, 0, 3 * sizeof(MisState), s));
+    const unsigned nb = (unsigned)std::min<uint64_t>(grid_for(pg), ceil_div(n, kThreads));
+    k_mis_init<<<nb, kThreads, 0, s>>>(pg->off, n, count_first ? nullptr : pg->dplus.as<uint32_t>(), state, waits, q0, S,
+                                       gb);
     PC_LAUNCHED();
-    uint32_t un = (uint32_t)n;
-    int32_t* fq = q0;
-    int32_t* nq = q1;
-    for (uint64_t round = 0; un > 0; ++round) {
-        PC_CUDA(cudaMemsetAsync(cnt, 0, 4, s));
-        k_mis_round<<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->adj, prio, dp, fq, un, state, nq, cnt);
-        PC_LAUNCHED();
-        PC_TRY(read_u32(pg, cnt, &un));
-        std::swap(fq, nq);
-        if (round > n + 1) return fail(PC_ERR_TIMEOUT, "MIS did not converge");
-    }
-    k_mis_finish<<<nb, kThreads, 0, s>>>(state, n, q0);
+    unsigned grid = 0;
+    PC_TRY(persistent_grid(pg, (const void*)k_mis_persistent, tx::kThreads, 6, 1024, &grid));
+    uint64_t max_steps = 2 * n + 8, limit_ns = kBarrierLimitNs, nn = n;
+    const uint64_t* off = pg->off;
+    const int32_t* adj = pg->adj;
+    MisPriority P{pc_graph_key(seed, PC_GEN_PRIORITY), hashed ? 1 : 0, int2api};
+    int first = count_first ? 1 : 0;
+    void* args[] = {(void*)&off, (void*)&adj, (void*)&nn, (void*)&P, (void*)&first, (void*)&state, (void*)&waits,
+                    (void*)&q0,  (void*)&q1,  (void*)&S,  (void*)&gb, (void*)&max_steps, (void*)&limit_ns};
+    PC_CUDA(cudaLaunchCooperativeKernel((const void*)k_mis_persistent, dim3(grid), dim3(tx::kThreads), args, 0, s));
     PC_LAUNCHED();
-    PC_TRY(gather_to_api_i32(pg, q0, out));
-    PC_CUDA(cudaMemcpyAsync(res_host, out, n * 4, cudaMemcpyDeviceToHost, s));
-    return sync(pg);
+    if (!api_is_internal(pg)) {
+        PC_TRY(gather_to_api_i32(pg, state, out));
+        state = out;
+    }
+    GridBarrier hb{};
+    PC_CUDA(cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaMemcpyAsync(res_host, state, n * 4, cudaMemcpyDeviceToHost, s));
+    PC_TRY(sync(pg));
+    if (hb.err == 1) return fail(PC_ERR_TIMEOUT, "MIS: a grid barrier wait ran out of time");
+    if (hb.err) return fail(PC_ERR_TIMEOUT, "MIS did not converge");
+    return PC_OK;
 }
 
 }  // namespace pc

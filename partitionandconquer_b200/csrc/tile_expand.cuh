@@ -152,11 +152,14 @@ __device__ __forceinline__ void expand(Tile& T, const uint64_t* __restrict__ off
         }
     }
     // Light rows, from the other end: the warps without a chunk begin.  A short
-    // queue is spread over all warps: 22 rows of up to 256 entries in one
-    // warp's hands held a level up for 80 us.
+    // queue is spread over all warps (22 rows of up to 256 entries in one warp's
+    // hands held a level up for 80 us), and a tile's rows are a tile count
+    // apart: neighbours in a queue tend to have rows of the same length, above
+    // all under degree-ordered ids.
     const uint32_t rows = min(32u, (nl + nw - 1) / nw);
-    for (uint32_t t = nw - 1 - gw; (uint64_t)t * rows < nl; t += nw) {
-        const uint32_t i = t * rows + lane;
+    const uint32_t tiles = rows ? (nl + rows - 1) / rows : 0u;
+    for (uint32_t t = nw - 1 - gw; t < tiles; t += nw) {
+        const uint32_t i = t + lane * tiles;
         uint32_t len = 0;
         uint64_t b = 0;
         int32_t x = 0;
