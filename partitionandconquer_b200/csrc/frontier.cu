@@ -50,22 +50,9 @@ __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t x) {
     return x;
 }
 
-// Pull kernels (PageRank, CDLP): rows of more than kPullHeavyDeg entries get a
-// CTA; the others kPullLanes lanes, so a warp keeps 8 rows in flight (4 lanes
-// measured 10 % faster than 8 for PageRank at RMAT-22, 16 lanes 16 % slower).
-constexpr uint32_t kPullHeavyDeg = 256;
+// Pull sweeps (PageRank, CDLP): lanes of a short row (4 lanes measured 10 %
+// faster than 8 for PageRank at RMAT-22, 16 lanes 16 % slower).
 constexpr int kPullLanes = 4;
-
-// Rows of more than thr entries (the pull kernels give each a whole CTA).
-__global__ void k_heavy_list(const uint64_t* __restrict__ off, uint64_t n, uint32_t thr, int32_t* __restrict__ hq,
-                             uint32_t* __restrict__ hn) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t nr = (n + 31) & ~31ull;
-    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < nr; u += stride) {
-        const bool heavy = u < n && off[u + 1] - off[u] > thr;
-        warp_append(heavy, (int32_t)u, hq, hn);
-    }
-}
 
 // ---- BFS -------------------------------------------------------------------
 
@@ -464,109 +451,6 @@ __global__ void __launch_bounds__(tx::kThreads, 5)
         if (!grid_sync(gb, limit_ns)) return;
     }
     if (lead && step == max_steps) atomicExch(&gb->err, 2);
-}
-
-// Hands the ids of adj[b, e) taken by lane gl of a group of L lanes to
-// f(ok, id), four per 16-byte load: the loads start at the 16-byte boundary
-// at or below b and step by 4 L ids, so one dependent round gives each lane
-// four independent gathers; ok is false for the positions of a load outside
-// [b, e), which the caller skips.  A load may run up to 3 ids past e, which
-// the 64 ids of padding after the last row keep inside the adjacency array.
-// The adjacency is read once per sweep, so its loads carry the streaming
-// hint (evict first): the gathered vectors keep their L2 lines.
-template <int L, class F>
-__device__ __forceinline__ void row_ids_vec4(const int32_t* __restrict__ adj, uint64_t b, uint64_t e, int gl,
-                                             F&& f) {
-    for (uint64_t q = (b & ~3ull) + 4ull * (uint64_t)gl; q < e; q += 4ull * L) {
-        const int4 v = __ldcs(reinterpret_cast<const int4*>(adj + q));
-        f(q >= b, v.x);
-        f(q + 1 >= b && q + 1 < e, v.y);
-        f(q + 2 >= b && q + 2 < e, v.z);
-        f(q + 3 < e, v.w);
-    }
-}
-
-// ---- PageRank (pull) -----------------------------------------------------------
-
-template <class T>
-__global__ void k_pr_init(const uint64_t* __restrict__ off, uint64_t n, T damping, const T* __restrict__ init,
-                          T* __restrict__ degs, T* __restrict__ contrib) {
-    uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    // degs[u] = d(u) / damping; x0 = degs / n (src/Graph.cpp:1563-1570)
-    const T dg = (T)(off[u + 1] - off[u]) / damping;
-    degs[u] = dg;
-    const T x0 = init ? init[u] : dg / (T)n;
-    contrib[u] = dg > (T)0 ? x0 / dg : (T)0;
-}
-
-// One iteration: x'[v] = base + sum_{u in N(v)} contrib[u]; contrib'[v] = x'[v] / degs[v].
-// T is the storage type of the vectors; the row sums, x' and the division
-// run in fp64 for both instances, so the fp32 vectors carry only their own
-// storage rounding (within 1e-6 relative of the FP64 recurrence at 20
-// iterations; fp32 row sums over hub in-lists drift past that).
-template <class T>
-__device__ __forceinline__ void pr_epilogue(uint64_t v, double base, double sum, const T* __restrict__ degs,
-                                            T* __restrict__ x_out, T* __restrict__ contrib_out) {
-    const double x = base + sum;
-    x_out[v] = (T)x;
-    const double dg = (double)degs[v];
-    contrib_out[v] = dg > 0.0 ? (T)(x / dg) : (T)0;
-}
-
-// One iteration: x'[v] = base + sum_{u in N(v)} contrib[u]; contrib'[v] = x'[v] / degs[v].
-// T is the storage type of the vectors; the row sums, x' and the division
-// run in fp64 for both instances, so the fp32 vectors carry only their own
-// storage rounding (within 1e-6 relative of the FP64 recurrence at 20
-// iterations; fp32 row sums over hub in-lists drift past that).  Rows listed
-// in hq (more than kPullHeavyDeg entries) get a whole CTA each; the others
-// kPullLanes lanes.  Both reductions run in a fixed order, so results are
-// reproducible.
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_pr_iter(const uint64_t* __restrict__ off,
-                                                      const int32_t* __restrict__ adj, uint64_t n, double base,
-                                                      const T* __restrict__ degs, const T* __restrict__ contrib,
-                                                      T* __restrict__ x_out, T* __restrict__ contrib_out,
-                                                      const int32_t* __restrict__ hq, uint32_t hn) {
-    __shared__ double s_part[kThreads / 32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (uint32_t h = blockIdx.x; h < hn; h += gridDim.x) {
-        const int32_t v = hq[h];
-        const uint64_t b = off[v], e = off[v + 1];
-        double s = 0.0;
-        row_ids_vec4<kThreads>(adj, b, e, threadIdx.x, [&](bool ok, int32_t u) {
-            if (ok) s += (double)__ldg(contrib + u);
-        });
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) s_part[wib] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int i = 0; i < kThreads / 32; ++i) t += s_part[i];
-            pr_epilogue(v, base, t, degs, x_out, contrib_out);
-        }
-        __syncthreads();
-    }
-    // the other rows: kPullLanes lanes each, 32 / kPullLanes rows per warp at once
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    constexpr int kRows = 32 / kPullLanes;
-    const int g = lane / kPullLanes, gl = lane % kPullLanes;
-    for (uint64_t v0 = warp * kRows; v0 < n; v0 += nwarps * kRows) {
-        const uint64_t v = v0 + g;
-        uint64_t b = 0, e = 0;
-        if (v < n) {
-            b = off[v];
-            e = off[v + 1];
-            if (e - b > kPullHeavyDeg) e = b;  // a CTA row
-        }
-        double s = 0.0;
-        row_ids_vec4<kPullLanes>(adj, b, e, gl, [&](bool ok, int32_t u) {
-            if (ok) s += (double)__ldg(contrib + u);
-        });
-        for (int o = kPullLanes / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (v < n && gl == 0 && off[v + 1] - off[v] <= kPullHeavyDeg) pr_epilogue(v, base, s, degs, x_out, contrib_out);
-    }
 }
 
 // ---- k-core ----------------------------------------------------------------------
@@ -1046,78 +930,168 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
     if (lead) atomicExch(&gb->err, 2);
 }
 
-// ---- CDLP --------------------------------------------------------------------------
+// ---- pull sweeps: PageRank and CDLP ---------------------------------------------
+//
+// A sweep combines, for every row, the values its ids have in a vector.  The
+// gathers bound it: at RMAT-22 a third of the 128 M hit L1 and the others move
+// a 32-byte sector each from L2.  (A copy of the hubs' values in shared memory
+// takes up to 58 % of them, but costs the resident warps that hide the rest's
+// latency: 64 / 128 / 192 KB 9.0 / 10.3 / 10.8 ms for 20 iterations against
+// 8.1 without; cache hints that keep hubs in L1 and others out: 8.2-9.0.)
+//
+// Rows longer than PullRows::warp_deg get a warp and than cta_deg a CTA, the
+// others kPullLanes lanes.  The bounds follow the graph's size (pull_rows): a
+// large sweep wants few lanes per row, a small one has lanes to spare and ends
+// when its longest row does.  A CTA for every row past 256 entries spent a
+// third of its time in barriers: RMAT-22 10.9 ms, now 7.6.  Every reduction runs in a
+// fixed order, so results are reproducible.
+struct PullRows {
+    const int32_t* __restrict__ cta;
+    const int32_t* __restrict__ warp;
+    uint32_t ncta, nwarp;
+    uint32_t cta_deg, warp_deg;
+};
 
-// One iteration: out[v] = max label over N(v), 0 for an isolated vertex
-// (src/Graph.cpp:650: labels start at 0 for every vertex).  Rows listed in hq
-// get a whole CTA each; the others kPullLanes lanes.
-__global__ void __launch_bounds__(kThreads) k_cdlp_iter(const uint64_t* __restrict__ off,
-                                                        const int32_t* __restrict__ adj, uint64_t n,
-                                                        const int32_t* __restrict__ lab, int32_t* __restrict__ out,
-                                                        const int32_t* __restrict__ hq, uint32_t hn) {
-    __shared__ int32_t s_part[kThreads / 32];
+// cnt[0], cnt[1]: lengths of the lists.
+__global__ void k_pull_rows(const uint64_t* __restrict__ off, uint64_t n, uint32_t cta_deg, uint32_t warp_deg,
+                            int32_t* __restrict__ cta, int32_t* __restrict__ warp, uint32_t* __restrict__ cnt) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t nr = (n + 31) & ~31ull;
+    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < nr; u += stride) {
+        const uint64_t d = u < n ? off[u + 1] - off[u] : 0;
+        warp_append(d > cta_deg, (int32_t)u, cta, &cnt[0]);
+        warp_append(d > warp_deg && d <= cta_deg, (int32_t)u, warp, &cnt[1]);
+    }
+}
+
+// Combines the values of the ids of adj[b, e) taken by lane gl of L lanes into
+// acc, four ids per 16-byte load: the loads start at the 16-byte boundary at
+// or below b and step by 4 L ids; ids outside [b, e) are not looked up.  A load may
+// run up to 3 ids past e, which the 64 ids of padding after the last row keep
+// inside the adjacency array.  The adjacency is read once per sweep, so its
+// loads carry the streaming hint (evict first): the gathered vector keeps its
+// L2 lines.
+template <int L, class Op>
+__device__ __forceinline__ void pull_row(const int32_t* __restrict__ adj, uint64_t b, uint64_t e, int gl, const Op& op,
+                                         typename Op::A& acc) {
+    // positions are relative to the boundary; the ids at [lo, lo + len) are the row's
+    const int4* p = reinterpret_cast<const int4*>(adj + (b & ~3ull));
+    const uint32_t lo = (uint32_t)b & 3u, len = (uint32_t)(e - b), hi = lo + len;
+    for (uint32_t q = gl; 4 * q < hi; q += L) {
+        const int4 v = __ldcs(p + q);
+        const int32_t id[4] = {v.x, v.y, v.z, v.w};
+        typename Op::V x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = 4 * q + k - lo < len ? __ldg(op.in + id[k]) : Op::none();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) op.add(acc, x[k]);
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(kThreads)
+    k_pull(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, Op op, PullRows R) {
+    using A = typename Op::A;
+    __shared__ A s_part[kThreads / 32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (uint32_t h = blockIdx.x; h < hn; h += gridDim.x) {
-        const int32_t v = hq[h];
-        const uint64_t b = off[v], e = off[v + 1];
-        int32_t mx = 0;
-        row_ids_vec4<kThreads>(adj, b, e, threadIdx.x, [&](bool ok, int32_t u) {
-            if (ok) mx = max(mx, __ldg(lab + u));
-        });
-        for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) s_part[wib] = mx;
+    for (uint32_t h = blockIdx.x; h < R.ncta; h += gridDim.x) {
+        const int32_t v = R.cta[h];
+        A acc = Op::zero();
+        pull_row<kThreads>(adj, off[v], off[v + 1], threadIdx.x, op, acc);
+        for (int o = 16; o; o >>= 1) acc = Op::merge(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+        if (lane == 0) s_part[wib] = acc;
         __syncthreads();
         if (threadIdx.x == 0) {
-            int32_t t = 0;
-            for (int i = 0; i < kThreads / 32; ++i) t = max(t, s_part[i]);
-            out[v] = t;
+            A t = Op::zero();
+            for (int i = 0; i < kThreads / 32; ++i) t = Op::merge(t, s_part[i]);
+            op.finish(v, off[v + 1] - off[v], t);
         }
         __syncthreads();
     }
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t warp = (blockIdx.x * (uint64_t)kThreads + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * kThreads) >> 5;
+    for (uint64_t h = warp; h < R.nwarp; h += nwarps) {
+        const int32_t v = R.warp[h];
+        const uint64_t b = off[v], e = off[v + 1];
+        A acc = Op::zero();
+        pull_row<32>(adj, b, e, lane, op, acc);
+        for (int o = 16; o; o >>= 1) acc = Op::merge(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+        if (lane == 0) op.finish(v, e - b, acc);
+    }
+    // the other rows: kPullLanes lanes each, 32 / kPullLanes rows per warp at once
     constexpr int kRows = 32 / kPullLanes;
     const int g = lane / kPullLanes, gl = lane % kPullLanes;
     for (uint64_t v0 = warp * kRows; v0 < n; v0 += nwarps * kRows) {
         const uint64_t v = v0 + g;
-        uint64_t b = 0, e = 0;
-        if (v < n) {
-            b = off[v];
-            e = off[v + 1];
-            if (e - b > kPullHeavyDeg) e = b;  // a CTA row
-        }
-        int32_t mx = 0;
-        row_ids_vec4<kPullLanes>(adj, b, e, gl, [&](bool ok, int32_t u) {
-            if (ok) mx = max(mx, __ldg(lab + u));
-        });
-        for (int o = kPullLanes / 2; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (v < n && gl == 0 && off[v + 1] - off[v] <= kPullHeavyDeg) out[v] = mx;
+        const uint64_t b = v < n ? off[v] : 0, e = v < n ? off[v + 1] : 0;
+        const bool mine = v < n && e - b <= R.warp_deg;
+        A acc = Op::zero();
+        pull_row<kPullLanes>(adj, b, mine ? e : b, gl, op, acc);
+        for (int o = kPullLanes / 2; o; o >>= 1) acc = Op::merge(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+        if (mine && gl == 0) op.finish(v, e - b, acc);
     }
 }
+
+// ---- PageRank (pull) -----------------------------------------------------------
+
+template <class T>
+__global__ void k_pr_init(const uint64_t* __restrict__ off, uint64_t n, T damping, const T* __restrict__ init,
+                          T* __restrict__ contrib) {
+    uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (u >= n) return;
+    // degs[u] = d(u) / damping; x0 = degs / n (src/Graph.cpp:1563-1570)
+    const T dg = (T)(off[u + 1] - off[u]) / damping;
+    const T x0 = init ? init[u] : dg / (T)n;
+    contrib[u] = dg > (T)0 ? x0 / dg : (T)0;
+}
+
+// One iteration: x'[v] = base + sum_{u in N(v)} contrib[u]; contrib'[v] = x'[v] / degs[v].
+// T is the storage type of the vectors; the row sums, x' and the division
+// run in fp64 for both instances, so the fp32 vectors carry only their own
+// storage rounding (within 1e-6 relative of the FP64 recurrence at 20
+// iterations; fp32 row sums over hub in-lists drift past that).  The last
+// iteration writes x' (out_x), the others the contributions.
+template <class T>
+struct PageRankOp {
+    using V = T;
+    using A = double;
+    const T* __restrict__ in;
+    T* __restrict__ out;
+    double base;
+    T damping;
+    bool out_x;
+    static __device__ __forceinline__ A zero() { return 0.0; }
+    static __device__ __forceinline__ V none() { return (V)0; }
+    static __device__ __forceinline__ void add(A& a, V v) { a += (double)v; }
+    static __device__ __forceinline__ A merge(A a, A b) { return a + b; }
+    __device__ __forceinline__ void finish(uint64_t v, uint64_t degree, A sum) const {
+        const double x = base + sum;
+        const double dg = (double)((T)degree / damping);
+        out[v] = out_x ? (T)x : (dg > 0.0 ? (T)(x / dg) : (T)0);
+    }
+};
+
+// ---- CDLP --------------------------------------------------------------------------
+
+// One iteration: out[v] = max label over N(v), 0 for an isolated vertex
+// (src/Graph.cpp:650: labels start at 0 for every vertex).
+struct CdlpOp {
+    using V = int32_t;
+    using A = int32_t;
+    const int32_t* __restrict__ in;
+    int32_t* __restrict__ out;
+    static __device__ __forceinline__ A zero() { return 0; }
+    static __device__ __forceinline__ V none() { return 0; }
+    static __device__ __forceinline__ void add(A& a, V v) { a = max(a, v); }
+    static __device__ __forceinline__ A merge(A a, A b) { return max(a, b); }
+    __device__ __forceinline__ void finish(uint64_t v, uint64_t, A m) const { out[v] = m; }
+};
 
 }  // namespace fr
 
 using namespace fr;
 
 static unsigned grid_for(const pc_pgraph* pg, int per_sm = 8) { return (unsigned)(sm_count(pg->g->device) * per_sm); }
-
-// Entries the list of heavy rows can need.
-static uint64_t pull_heavy_cap(uint64_t n, uint64_t m) {
-    return std::max<uint64_t>(1, std::min<uint64_t>(n, m / kPullHeavyDeg + 1));
-}
-
-// Lists the rows of more than kPullHeavyDeg entries into hq (room for
-// pull_heavy_cap entries) and reads their number back.
-static pc_status list_heavy_rows(pc_pgraph* pg, int32_t* hq, uint32_t* d_hn, uint32_t* hn) {
-    if (!hq || !d_hn) return fail(PC_ERR_OOM, "scratch plan exceeds its reservation");
-    cudaStream_t s = pg->g->stream;
-    PC_CUDA(cudaMemsetAsync(d_hn, 0, 4, s));
-    k_heavy_list<<<grid_for(pg), kThreads, 0, s>>>(pg->off, pg->g->n, kPullHeavyDeg, hq, d_hn);
-    PC_LAUNCHED();
-    PC_CUDA(cudaMemcpyAsync(hn, d_hn, 4, cudaMemcpyDeviceToHost, s));
-    PC_CUDA(cudaStreamSynchronize(s));
-    return PC_OK;
-}
 
 // CTAs of a persistent kernel: every SM's share, fewer for a small graph,
 // whose barriers then have fewer arrivals; one per `work` vertices and quarter
@@ -1172,41 +1146,79 @@ static pc_status bfs_run(pc_pgraph* pg, int32_t src, int32_t* rank_host) {
     return PC_OK;
 }
 
+// Bounds of the row classes, measured with PageRank's 20 iterations on RMAT
+// graphs (ms): warp_deg 32 / 64 / 128 / 256 / 512 at scale 14 (0.5 M entries)
+// 0.26 / 0.22 / 0.28 / 0.35 / -, at 18 (8 M) 0.57 / 0.56 / 0.55 / 0.61 / -, at 22
+// (128 M) - / - / 8.04 / 8.09 / 7.53; cta_deg 512 / 1024 / 2048 / 4096 at 16
+// 0.29 / 0.29 / 0.31 / 0.31, at 20 2.39 / 2.35 / 1.91 / 2.06.
+static uint32_t pull_warp_deg(uint64_t m) { return m >= (1ull << 26) ? 512 : (m >= (1ull << 22) ? 128 : 64); }
+static uint32_t pull_cta_deg(uint64_t m) { return m >= (1ull << 24) ? 2048 : 1024; }
+
+// Device bytes pull_rows() takes from the scratch arena.
+static uint64_t pull_rows_bytes(uint64_t n, uint64_t m) {
+    return (std::min<uint64_t>(n, m / pull_cta_deg(m)) + std::min<uint64_t>(n, m / pull_warp_deg(m)) + 2) * 4 + 1024;
+}
+
+// Lists the long rows; waits for the stream.
+static pc_status pull_rows(pc_pgraph* pg, PullRows* rows) {
+    const uint64_t n = pg->g->n, m = pg->g->m;
+    const uint32_t cta_deg = pull_cta_deg(m), warp_deg = pull_warp_deg(m);
+    cudaStream_t s = pg->g->stream;
+    int32_t* cta = pg->scratch.take<int32_t>(std::min<uint64_t>(n, m / cta_deg) + 1);
+    int32_t* warp = pg->scratch.take<int32_t>(std::min<uint64_t>(n, m / warp_deg) + 1);
+    uint32_t* cnt = pg->scratch.take<uint32_t>(2);
+    if (!cnt) return fail(PC_ERR_OOM, "scratch plan exceeds its reservation");
+    PC_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
+    k_pull_rows<<<(unsigned)std::min<uint64_t>(grid_for(pg), ceil_div(n, kThreads)), kThreads, 0, s>>>(
+        pg->off, n, cta_deg, warp_deg, cta, warp, cnt);
+    PC_LAUNCHED();
+    uint32_t h[2] = {0, 0};
+    PC_CUDA(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, s));
+    PC_CUDA(cudaStreamSynchronize(s));
+    *rows = PullRows{cta, warp, h[0], h[1], cta_deg, warp_deg};
+    return PC_OK;
+}
+
+template <class Op>
+static pc_status pull_sweep(pc_pgraph* pg, const Op& op, const PullRows& rows) {
+    const uint64_t n = pg->g->n;
+    const uint64_t grid = std::min<uint64_t>(grid_for(pg, 16), ceil_div(n, kThreads / kPullLanes));
+    k_pull<Op><<<(unsigned)grid, kThreads, 0, pg->g->stream>>>(pg->off, pg->adj, n, op, rows);
+    PC_LAUNCHED();
+    return PC_OK;
+}
+
 template <class T>
 static pc_status pagerank_run(pc_pgraph* pg, T damping, int32_t iters, const T* init, T* out_host) {
     const uint64_t n = pg->g->n;
     cudaStream_t s = pg->g->stream;
-    const uint64_t hcap = pull_heavy_cap(n, pg->g->m);
-    PC_TRY(scratch_reserve(pg, n * sizeof(T) * 6 + hcap * 4 + 512));
-    int32_t* hq = pg->scratch.take<int32_t>(hcap);
-    uint32_t* d_hn = pg->scratch.take<uint32_t>(1);
-    T* degs = pg->scratch.take<T>(n);
+    PC_TRY(scratch_reserve(pg, n * sizeof(T) * 4 + pull_rows_bytes(n, pg->g->m)));
     T* c0 = pg->scratch.take<T>(n);
     T* c1 = pg->scratch.take<T>(n);
-    T* x = pg->scratch.take<T>(n);
     T* xapi = pg->scratch.take<T>(n);
     T* ini = nullptr;
-    const unsigned nb = (unsigned)ceil_div(n, kThreads);
     if (init) {
         ini = pg->scratch.take<T>(n);
         PC_CUDA(cudaMemcpyAsync(xapi, init, n * sizeof(T), cudaMemcpyHostToDevice, s));
         if (sizeof(T) == 4) PC_TRY(gather_to_internal_f32(pg, (const float*)xapi, (float*)ini));
         else PC_TRY(gather_to_internal_f64(pg, (const double*)xapi, (double*)ini));
     }
-    k_pr_init<T><<<nb, kThreads, 0, s>>>(pg->off, n, damping, ini, degs, c0);
+    k_pr_init<T><<<(unsigned)ceil_div(n, kThreads), kThreads, 0, s>>>(pg->off, n, damping, ini, c0);
     PC_LAUNCHED();
-    uint32_t hn = 0;
-    PC_TRY(list_heavy_rows(pg, hq, d_hn, &hn));
+    PullRows rows;
+    PC_TRY(pull_rows(pg, &rows));
     // (1 - damping) / n (src/Graph.cpp:1558), in fp64 like the row sums
     const double base = (1.0 - (double)damping) / (double)n;
     for (int32_t it = 0; it < iters; ++it) {
-        k_pr_iter<T><<<grid_for(pg, 16), kThreads, 0, s>>>(pg->off, pg->adj, n, base, degs, c0, x, c1, hq, hn);
-        PC_LAUNCHED();
+        PC_TRY(pull_sweep(pg, PageRankOp<T>{c0, c1, base, damping, it + 1 == iters}, rows));
         std::swap(c0, c1);
     }
-    if (sizeof(T) == 4) PC_TRY(gather_to_api_f32(pg, (const float*)x, (float*)xapi));
-    else PC_TRY(gather_to_api_f64(pg, (const double*)x, (double*)xapi));
-    PC_CUDA(cudaMemcpyAsync(out_host, xapi, n * sizeof(T), cudaMemcpyDeviceToHost, s));
+    if (!api_is_internal(pg)) {
+        if (sizeof(T) == 4) PC_TRY(gather_to_api_f32(pg, (const float*)c0, (float*)xapi));
+        else PC_TRY(gather_to_api_f64(pg, (const double*)c0, (double*)xapi));
+        c0 = xapi;
+    }
+    PC_CUDA(cudaMemcpyAsync(out_host, c0, n * sizeof(T), cudaMemcpyDeviceToHost, s));
     return sync(pg);
 }
 
@@ -1500,24 +1512,22 @@ pc_status pc_cdlp(pc_pgraph* pg, int32_t iterations, int32_t* labels) {
     const uint64_t n = pg->g->n;
     if (n == 0 || iterations == 0) return PC_OK;
     cudaStream_t s = pg->g->stream;
-    const uint64_t hcap = pull_heavy_cap(n, pg->g->m);
-    PC_TRY(scratch_reserve(pg, n * 4 * 3 + hcap * 4 + 512));
+    PC_TRY(scratch_reserve(pg, n * 4 * 3 + pull_rows_bytes(n, pg->g->m)));
     int32_t* a = pg->scratch.take<int32_t>(n);
     int32_t* b = pg->scratch.take<int32_t>(n);
     int32_t* c = pg->scratch.take<int32_t>(n);
-    int32_t* hq = pg->scratch.take<int32_t>(hcap);
-    uint32_t* d_hn = pg->scratch.take<uint32_t>(1);
-    if (!d_hn) return fail(PC_ERR_OOM, "CDLP scratch plan exceeds its reservation");
-    PC_CUDA(cudaMemcpyAsync(c, labels, n * 4, cudaMemcpyHostToDevice, s));
-    PC_TRY(gather_to_internal_i32(pg, c, a));
-    uint32_t hn = 0;
-    PC_TRY(list_heavy_rows(pg, hq, d_hn, &hn));
+    if (!c) return fail(PC_ERR_OOM, "CDLP scratch plan exceeds its reservation");
+    const bool same_ids = api_is_internal(pg);
+    PC_CUDA(cudaMemcpyAsync(same_ids ? a : c, labels, n * 4, cudaMemcpyHostToDevice, s));
+    if (!same_ids) PC_TRY(gather_to_internal_i32(pg, c, a));
+    PullRows rows;
+    PC_TRY(pull_rows(pg, &rows));
     for (int32_t it = 0; it < iterations; ++it) {
-        k_cdlp_iter<<<grid_for(pg, 16), kThreads, 0, s>>>(pg->off, pg->adj, n, a, b, hq, hn);
-        PC_LAUNCHED();
+        PC_TRY(pull_sweep(pg, CdlpOp{a, b}, rows));
         std::swap(a, b);
     }
-    PC_TRY(gather_to_api_i32(pg, a, c));
+    if (same_ids) c = a;
+    else PC_TRY(gather_to_api_i32(pg, a, c));
     PC_CUDA(cudaMemcpyAsync(labels, c, n * 4, cudaMemcpyDeviceToHost, s));
     return sync(pg);
 }
