@@ -150,24 +150,30 @@ __device__ __forceinline__ int64_t range_pos(const int64_t* __restrict__ ranges,
     return ranges[2 * lo] + (int64_t)(q - (uint64_t)rprefix[lo]);
 }
 
+// First CSR entry of pivot b's in-neighbours at or above c_min (0: of all).
+__device__ __forceinline__ uint64_t first_in_neighbour(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                                                       const uint32_t* __restrict__ dplus, int32_t b, int32_t c_min) {
+    const uint64_t in0 = off[b] + dplus[b];
+    return c_min > b ? in0 + lower_bound_i32(adj + in0, (uint32_t)(off[b + 1] - in0), c_min) : in0;
+}
+
 // Work items: pivot q (a linear position in the launch's position ranges)
-// gives ceil(din / chunk) items, each a run of <= chunk of its in-neighbours;
-// pivots without a set or without in-neighbours give none.
-__global__ void k_item_count(const uint64_t* __restrict__ off, const uint32_t* __restrict__ dplus,
-                             const int32_t* __restrict__ plist, const int64_t* __restrict__ ranges,
+// gives ceil(din / chunk) items, each a run of <= chunk of its in-neighbours
+// at or above c_min; pivots without a set or without in-neighbours give none.
+__global__ void k_item_count(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                             const uint32_t* __restrict__ dplus, const int32_t* __restrict__ plist, int32_t c_min, const int64_t* __restrict__ ranges,
                              const int64_t* __restrict__ rprefix, uint32_t nranges, uint64_t npos, uint32_t chunk,
                              uint32_t* __restrict__ cnt) {
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t > npos) return;
     if (t == npos) { cnt[t] = 0; return; }
     const int32_t b = pivot_at(plist, range_pos(ranges, rprefix, nranges, t));
-    const uint32_t dp = dplus[b];
-    const uint32_t din = (uint32_t)(off[b + 1] - off[b]) - dp;
-    cnt[t] = dp == 0 ? 0u : (din + chunk - 1) / chunk;
+    const uint32_t din = (uint32_t)(off[b + 1] - first_in_neighbour(off, adj, dplus, b, c_min));
+    cnt[t] = dplus[b] == 0 ? 0u : (din + chunk - 1) / chunk;
 }
 
-__global__ void k_item_fill(const uint64_t* __restrict__ off, const uint32_t* __restrict__ dplus,
-                            const int32_t* __restrict__ plist, const int64_t* __restrict__ ranges,
+__global__ void k_item_fill(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                            const uint32_t* __restrict__ dplus, const int32_t* __restrict__ plist, int32_t c_min, const int64_t* __restrict__ ranges,
                             const int64_t* __restrict__ rprefix, uint32_t nranges, uint64_t npos, uint32_t chunk,
                             const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ start,
                             Item* __restrict__ items, uint32_t cap, uint32_t* __restrict__ nitems) {
@@ -178,7 +184,7 @@ __global__ void k_item_fill(const uint64_t* __restrict__ off, const uint32_t* __
     if (!c) return;
     const int64_t p = range_pos(ranges, rprefix, nranges, t);
     const int32_t b = pivot_at(plist, p);
-    const uint64_t in0 = off[b] + dplus[b];
+    const uint64_t in0 = first_in_neighbour(off, adj, dplus, b, c_min);
     const uint32_t din = (uint32_t)(off[b + 1] - in0);
     const uint32_t s = start[t];
     for (uint32_t j = 0; j < c && s + j < cap; ++j)
@@ -200,39 +206,6 @@ __global__ void k_matrix_rows(const uint64_t* __restrict__ off, const int32_t* _
             atomicOr(&h[a >> 5], 1u << (a & 31));
         }
     }
-}
-
-// ---- asynchronous staging of an in-neighbour's span into shared memory ----
-//
-// cp.async (LDGSTS) copies 16-byte pieces global -> shared without passing
-// through registers; a lane waits for its own groups (wait_group), and a
-// __syncwarp() after the wait makes every lane's pieces visible to the warp.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// A warp-private stage holds up to kStageIds ids of a span (or the smaller
-// stage a launch chooses, svec uint4): the copy starts
-// at the 16-byte boundary at or below the span (up to 3 ids early) and may
-// end up to 3 ids past it, which the 64 ids of padding after the last row
-// keep inside the adjacency array.
-constexpr uint32_t kStageIds = 256;
-
-// Issues the copies of ids [r, r + k) of adj into stage; returns the offset
-// of id r inside it, or -1 when the span does not fit (it is then read from
-// global memory).
-__device__ __forceinline__ int stage_span(const int32_t* __restrict__ adj, uint64_t r, uint32_t k, uint4* stage,
-                                          uint32_t svec, int lane) {
-    const uint32_t shift = (uint32_t)(r & 3);
-    const uint32_t nvec = (shift + k + 3) >> 2;
-    if (nvec > svec) return -1;
-    const uint4* src = reinterpret_cast<const uint4*>(adj + (r - shift));
-    for (uint32_t x = lane; x < nvec; x += 32) cp_async16(stage + x, src + x);
-    return (int)shift;
 }
 
 // Word form of a block whose last pivot b sits at position jl: ceil(b/128)
@@ -323,39 +296,28 @@ __device__ __forceinline__ void matrix_span(const uint64_t* __restrict__ off, co
     *klo = lower_bound_i32(adj + *r, *khi, lo);
 }
 
-// In-neighbours c run in two phases.  The first kMatrixHeavy ids after lo
-// (the hubs, with the longest S_c) are taken one per warp from counter
-// next[0], their spans read from global memory; the rest 32 at a time from
-// next[1], lanes locating the 32 spans at once.  In the second phase the
-// spans are staged into two warp-private shared-memory buffers by cp.async:
-// the next span's copies are in flight while the current one is counted.
-// One-at-a-time for the hubs keeps a single warp from holding a batch of 32
-// hubs at the end of the launch.
-constexpr uint64_t kMatrixHeavy = 65536;
-
+// The in-neighbours c in (lo, c1), taken one per warp: they are the hubs, with
+// long spans S_c (c1: kMatrixFrom).
 template <int U>
 __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t* __restrict__ off,
                                                                const int32_t* __restrict__ adj,
                                                                const uint32_t* __restrict__ dplus, int32_t lo,
-                                                               int32_t hi, uint64_t n, uint32_t hstride,
+                                                               int32_t hi, uint64_t c1, uint32_t hstride,
                                                                const uint32_t* __restrict__ H,
                                                                unsigned long long* __restrict__ next,
                                                                unsigned long long* __restrict__ total,
                                                                unsigned long long* __restrict__ unit_cost,
-                                                               int32_t unit, uint32_t svec) {
+                                                               int32_t unit) {
     extern __shared__ uint4 msm4[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t nwarps = blockDim.x >> 5;  // kMatrixWarps or fewer
     uint32_t* Sb = reinterpret_cast<uint32_t*>(msm4) + (size_t)w * hstride;  // warp-private bitmap of S_c
-    uint4* stage = msm4 + (size_t)nwarps * (hstride / 4) + (size_t)w * 2 * svec;
     for (uint32_t i = lane; i < hstride; i += 32) Sb[i] = 0;
     __syncwarp();
     const long long t0 = unit_cost ? clock64() : 0;
     unsigned long long cnt = 0;
-    const uint64_t c1 = (uint64_t)lo + 1 + kMatrixHeavy < n ? (uint64_t)lo + 1 + kMatrixHeavy : n;
-    for (;;) {  // phase 1: one hub in-neighbour per grab
+    for (;;) {
         unsigned long long q = 0;
-        if (lane == 0) q = atomicAdd(&next[0], 1ull);
+        if (lane == 0) q = atomicAdd(next, 1ull);
         const uint64_t c = __shfl_sync(0xffffffffu, q, 0) + (uint64_t)lo + 1;
         if (c >= c1) break;
         uint64_t r = 0;
@@ -366,47 +328,6 @@ __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t*
         khi = __shfl_sync(0xffffffffu, khi, 0);
         if (khi > klo) cnt += matrix_block_pairs<U>(adj + r, klo, khi, lo, hstride, H, Sb, lane);
     }
-    for (;;) {  // phase 2: 32 in-neighbours per grab, spans staged two deep
-        unsigned long long q = 0;
-        if (lane == 0) q = atomicAdd(&next[1], 32ull);
-        const uint64_t base = __shfl_sync(0xffffffffu, q, 0) + c1;
-        if (base >= n) break;
-        const uint64_t c = base + lane;
-        uint64_t r = 0;
-        uint32_t klo = 0, khi = 0;
-        if (c < n) matrix_span(off, adj, dplus, lo, hi, c, &r, &klo, &khi);
-        unsigned todo = __ballot_sync(0xffffffffu, khi > klo);
-        if (!todo) continue;
-        int src = __ffs(todo) - 1;
-        todo &= todo - 1;
-        int buf = 0;
-        int shift = stage_span(adj, __shfl_sync(0xffffffffu, r, src), __shfl_sync(0xffffffffu, khi, src),
-                               stage, svec, lane);
-        cp_async_commit();
-        for (;;) {
-            const int nxt = todo ? __ffs(todo) - 1 : -1;
-            if (nxt >= 0) todo &= todo - 1;
-            int nshift = -1;
-            if (nxt >= 0)
-                nshift = stage_span(adj, __shfl_sync(0xffffffffu, r, nxt), __shfl_sync(0xffffffffu, khi, nxt),
-                                    stage + (buf ^ 1) * svec, svec, lane);
-            cp_async_commit();
-            cp_async_wait<1>();  // every group but the one just issued: the current span is in place
-            __syncwarp();
-            const uint64_t rs = __shfl_sync(0xffffffffu, r, src);
-            const uint32_t j0 = __shfl_sync(0xffffffffu, klo, src);
-            const uint32_t k = __shfl_sync(0xffffffffu, khi, src);
-            const int32_t* S = shift >= 0 ? reinterpret_cast<const int32_t*>(stage + buf * svec) + shift
-                                          : adj + rs;
-            cnt += matrix_block_pairs<U>(S, j0, k, lo, hstride, H, Sb, lane);
-            __syncwarp();  // the buffer just read is the next stage's target
-            if (nxt < 0) break;
-            src = nxt;
-            shift = nshift;
-            buf ^= 1;
-        }
-    }
-    cp_async_wait<0>();
     if (unit_cost) {
         __syncwarp();
         if (lane == 0) atomicAdd(&unit_cost[unit], (unsigned long long)(clock64() - t0));
@@ -414,6 +335,11 @@ __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t*
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0 && cnt) atomicAdd(total, cnt);
 }
+
+// A matrix unit's in-neighbours from this id on run through the bitmap kernel:
+// their spans are short, and the probes of a short span into rows of L2 are
+// slower than a scan against a bitmap in shared memory.
+constexpr int32_t kMatrixFrom = 1 << 16;
 
 constexpr uint32_t kBitmapCapBits = 1u << 20;  // 128 KB of shared memory
 
@@ -632,6 +558,8 @@ struct LaunchGroup {
     double ein = 0;
     size_t units = 0;
     std::vector<int32_t> unit_ids;  // matrix groups: one launch per unit (ranges not merged)
+    int32_t c_min = 0;              // in-neighbours below this are not taken
+    std::vector<LaunchGroup> tails; // matrix groups: the in-neighbours from kMatrixFrom on, per bitmap shape
 };
 
 // Words per resident pivot bitmap row of a matrix unit with ids below hi:
@@ -662,39 +590,17 @@ static int matrix_pivot_block() {
     return u;
 }
 
-// Matrix launch shape: warps per CTA (kMatrixWarps, or PC_MATRIX_WARPS=4) and
-// ids per span stage (kStageIds, or PC_MATRIX_STAGE_IDS=128|512|1024), read
-// once from the environment; switches for measurements.
-static int matrix_env(const char* name, int dflt, std::initializer_list<int> allowed) {
-    const char* e = getenv(name);
-    if (!e) return dflt;
-    const int v = atoi(e);
-    for (int a : allowed)
-        if (a == v) return v;
-    return dflt;
-}
-static int matrix_warps() {
-    static const int w = matrix_env("PC_MATRIX_WARPS", kMatrixWarps, {4, 8});
-    return w;
-}
-static uint32_t matrix_stage_vec() {
-    static const uint32_t v = (uint32_t)matrix_env("PC_MATRIX_STAGE_IDS", (int)kStageIds, {128, 256, 512, 1024}) / 4 + 1;
-    return v;
-}
-
 template <int U>
 static pc_status launch_matrix(pc_pgraph* pg, int64_t lo, int64_t hi, uint32_t hstride, const uint32_t* H,
                                unsigned long long* d_next, unsigned long long* d_total, unsigned long long* d_cost,
                                int32_t unit, int sms, cudaStream_t s) {
-    const int warps = matrix_warps();
-    const uint32_t svec = matrix_stage_vec();
-    const size_t smem = (size_t)warps * hstride * 4 + (size_t)warps * 2 * svec * sizeof(uint4);
+    const size_t smem = (size_t)kMatrixWarps * hstride * 4;
     PC_CUDA(cudaFuncSetAttribute(k_tc_matrix<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_matrix<U>, warps * 32, smem));
-    k_tc_matrix<U><<<(unsigned)(sms * std::max(1, per_sm)), warps * 32, smem, s>>>(
-        pg->off, pg->adj, pg->dplus.as<uint32_t>(), (int32_t)lo, (int32_t)hi, pg->g->n, hstride, H, d_next, d_total,
-        d_cost, unit, svec);
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_matrix<U>, kMatrixWarps * 32, smem));
+    const uint64_t c1 = std::min<uint64_t>(pg->g->n, (uint64_t)kMatrixFrom);
+    k_tc_matrix<U><<<(unsigned)(sms * std::max(1, per_sm)), kMatrixWarps * 32, smem, s>>>(
+        pg->off, pg->adj, pg->dplus.as<uint32_t>(), (int32_t)lo, (int32_t)hi, c1, hstride, H, d_next, d_total, d_cost, unit);
     PC_LAUNCHED();
     return PC_OK;
 }
@@ -727,6 +633,9 @@ static void finish_group(LaunchGroup* gr) {
     gr->item_bound = std::min<uint64_t>(gr->npos, ein) + ein / 256 + 1;
 }
 
+static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long long* d_total, uint64_t* launches,
+                           unsigned long long* d_cost, unsigned long long* d_tri, uint32_t* d_ecnt);
+
 // Launches one group (all asynchronous).
 static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long long* d_total, uint64_t* launches,
                            unsigned long long* d_cost, unsigned long long* d_tri, uint32_t* d_ecnt) {
@@ -739,8 +648,15 @@ static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
         for (size_t i = 0; i < gr.unit_ids.size(); ++i)
             PC_TRY(run_matrix_unit(pg, gr.ranges[2 * i], gr.ranges[2 * i + 1], gr.unit_ids[i], H, d_next, d_total,
                                    d_cost, launches));
+        for (const LaunchGroup& t : gr.tails) PC_TRY(run_items(pg, t, d_total, launches, d_cost, d_tri, d_ecnt));
         return PC_OK;
     }
+    return run_items(pg, gr, d_total, launches, d_cost, d_tri, d_ecnt);
+}
+
+// The groups whose work is a list of items.
+static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long long* d_total, uint64_t* launches,
+                           unsigned long long* d_cost, unsigned long long* d_tri, uint32_t* d_ecnt) {
     const int32_t* unit_of = pg->unit_of.as<int32_t>();
     cudaStream_t s = pg->g->stream;
     const int v = gr.v;
@@ -771,13 +687,13 @@ static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
     Item* d_items = pg->scratch.take<Item>(gr.item_bound);
     if (!d_cnt || !d_start || !d_tmp || !d_next || !d_items)
         return fail(PC_ERR_OOM, "scratch arena too small (internal sizing error)");
-    k_item_count<<<(unsigned)ceil_div(npos + 1, 256), 256, 0, s>>>(pg->off, dp, plist, d_ranges, d_pref, nr, npos,
-                                                                   chunk, d_cnt);
+    k_item_count<<<(unsigned)ceil_div(npos + 1, 256), 256, 0, s>>>(pg->off, pg->adj, dp, plist, gr.c_min, d_ranges, d_pref,
+                                                                   nr, npos, chunk, d_cnt);
     PC_LAUNCHED();
     PC_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp, tmpb, d_cnt, d_start, (int64_t)(npos + 1), s));
     count_launch();
-    k_item_fill<<<(unsigned)ceil_div(npos, 256), 256, 0, s>>>(pg->off, dp, plist, d_ranges, d_pref, nr, npos, chunk,
-                                                              d_cnt, d_start, d_items, (uint32_t)gr.item_bound,
+    k_item_fill<<<(unsigned)ceil_div(npos, 256), 256, 0, s>>>(pg->off, pg->adj, dp, plist, gr.c_min, d_ranges, d_pref,
+                                                              nr, npos, chunk, d_cnt, d_start, d_items, (uint32_t)gr.item_bound,
                                                               d_next + 1);
     PC_LAUNCHED();
     PC_CUDA(cudaMemsetAsync(d_next, 0, 4, s));
@@ -852,32 +768,54 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         if (v < 0) continue;
         if ((is_bitmap(v) || v == PC_VARIANT_HASH_WARP) && !pg->oids.p) v = PC_VARIANT_MERGE_LANE;  // no room for the oriented copy
         const uint32_t mid = (uint32_t)feat[u * kNumFeatures + 4];
-        int c = 0;
-        if (is_bitmap(v)) {
+        auto bitmap_class = [&]() {
             const uint32_t w = std::max<uint32_t>(1, (mid + 31) / 32);
+            int c = 0;
             while ((1u << c) < w && c < kClasses - 1) ++c;
-            if (split_ok && mid > kSplitFrom) c = kClasses;
-        }
+            return split_ok && mid > kSplitFrom ? kClasses : c;
+        };
+        auto add_unit = [&](LaunchGroup& gr, bool merge) {
+            if (merge && !gr.ranges.empty() && gr.ranges.back() == lo[u]) {
+                gr.ranges.back() = hi[u];
+            } else {
+                gr.ranges.push_back(lo[u]);
+                gr.ranges.push_back(hi[u]);
+            }
+            gr.npos += (uint64_t)(hi[u] - lo[u]);
+            gr.ein += feat[u * kNumFeatures + 1];
+            gr.units += 1;
+        };
+        const int c = is_bitmap(v) ? bitmap_class() : 0;
         LaunchGroup& gr = groups[v * (kClasses + 1) + c];
         group_of[u] = v * (kClasses + 1) + c;
         gr.v = v;
         gr.split = c == kClasses;
         gr.words = gr.split ? 0 : 1u << c;
-        if (v == PC_VARIANT_MATRIX) {
-            gr.ranges.push_back(lo[u]);
-            gr.ranges.push_back(hi[u]);
-            gr.unit_ids.push_back((int32_t)u);
-        } else if (!gr.ranges.empty() && gr.ranges.back() == lo[u]) {
-            gr.ranges.back() = hi[u];
-        } else {
-            gr.ranges.push_back(lo[u]);
-            gr.ranges.push_back(hi[u]);
+        add_unit(gr, v != PC_VARIANT_MATRIX);
+        if (v != PC_VARIANT_MATRIX) continue;
+        gr.unit_ids.push_back((int32_t)u);
+        if ((uint64_t)kMatrixFrom >= pg->g->n) continue;
+        const int tc = bitmap_class();
+        LaunchGroup* tail = nullptr;
+        for (LaunchGroup& t : gr.tails)
+            if (t.words == 1u << tc) tail = &t;
+        if (!tail) {
+            gr.tails.emplace_back();
+            tail = &gr.tails.back();
+            tail->v = pg->oids.p ? PC_VARIANT_BITMAP_GROUP8 : PC_VARIANT_MERGE_LANE;
+            tail->words = 1u << tc;
+            tail->c_min = kMatrixFrom;
         }
-        gr.npos += (uint64_t)(hi[u] - lo[u]);
-        gr.ein += feat[u * kNumFeatures + 1];
-        gr.units += 1;
+        add_unit(*tail, true);
     }
     size_t need = 1024;
+    auto items_need = [&](LaunchGroup& gr) {
+        finish_group(&gr);
+        size_t tmpb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tmpb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)(gr.npos + 1),
+                                      s);
+        need += gr.ranges.size() * 16 + 64 + (gr.npos + 1) * 8 + tmpb + gr.item_bound * sizeof(Item) + 8 * 256;
+    };
     for (LaunchGroup& gr : groups) {
         if (gr.ranges.empty()) continue;
         if (gr.v == PC_VARIANT_MATRIX) {
@@ -885,13 +823,10 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
             for (size_t i = 0; i < gr.unit_ids.size(); ++i)
                 hb = std::max(hb, matrix_bytes(gr.ranges[2 * i], gr.ranges[2 * i + 1]));
             need += hb + 2 * 256;
+            for (LaunchGroup& t : gr.tails) items_need(t);
             continue;
         }
-        finish_group(&gr);
-        size_t tmpb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tmpb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)(gr.npos + 1),
-                                      s);
-        need += gr.ranges.size() * 16 + 64 + (gr.npos + 1) * 8 + tmpb + gr.item_bound * sizeof(Item) + 8 * 256;
+        items_need(gr);
     }
     if (unit_ms) need += U * 8 + 256;
     PC_TRY(scratch_reserve(pg, need));
