@@ -167,9 +167,9 @@ pc_status pc_pgraph_evaluate(pc_pgraph* pg, int64_t* max_part_deg, int64_t* max_
 #define PC_VARIANT_AUTO -1       /* learned selector if trained, else heuristic */
 #define PC_VARIANT_HEURISTIC -2  /* plain autotuned heuristic                    */
 #define PC_VARIANT_BITMAP_WARP 0 /* pivot bitmap in smem, warp per in-neighbour  */
-#define PC_VARIANT_BITMAP_GROUP8 1 /* pivot bitmap, 8 lanes per in-neighbour     */
+#define PC_VARIANT_BITMAP_GROUP8 1 /* pivot bitmap, a few lanes per in-neighbour */
 #define PC_VARIANT_BITMAP_LANE 2 /* pivot bitmap, one lane per in-neighbour      */
-#define PC_VARIANT_HASH_WARP 3   /* warp-private pivot hash, 8 lanes per in-nbr   */
+#define PC_VARIANT_HASH_WARP 3   /* warp-private pivot hash, 4 lanes per in-nbr  */
 #define PC_VARIANT_MERGE_LANE 4  /* threshold merge, lane per edge (reference)   */
 #define PC_VARIANT_GALLOP_LANE 5 /* binary search, lane per edge                 */
 #define PC_VARIANT_MATRIX 6      /* hub units (ids < 2^16, contiguous partitions):

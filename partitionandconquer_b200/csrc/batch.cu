@@ -200,7 +200,7 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
         for (uint32_t k = 0; k < I.n; k += 32) {
             const int nb = min(32, (int)(I.n - k));
             const int32_t c = lane < nb ? A.adj[I.in0 + k + lane] : 0;
-            hits += tc::scan_in_neighbours<8, kMode, tc::kMixedSet>(A.oriented, c, A.oriented.off[c], nb, b, S, lane, sink);
+            hits += tc::scan_in_neighbours<4, 1, kMode, tc::kMixedSet>(A.oriented, c, A.oriented.off[c], nb, b, S, lane, sink);
         }
         for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
         if (lane == 0 && hits) {

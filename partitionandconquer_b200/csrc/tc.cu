@@ -453,11 +453,11 @@ struct BitmapLaunch {
     uint32_t* ecnt;           // per-edge counts at the oriented slots (Jaccard), or null
 };
 
-template <int K, int G, int kMode, int kKind>
+template <int K, int G, int V, int kMode, int kKind>
 static pc_status launch_bitmap_kgm(const BitmapLaunch& L) {
-    PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, kMode, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, V, kMode, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)L.smem));
-    k_tc_bitmap<K, G, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.next,
+    k_tc_bitmap<K, G, V, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.next,
                                                                         L.total, L.words, L.cost, L.unit_of, L.tri,
                                                                         L.ecnt);
     return PC_OK;
@@ -465,9 +465,9 @@ static pc_status launch_bitmap_kgm(const BitmapLaunch& L) {
 
 template <int K, int kMode, int kKind>
 static pc_status launch_bitmap_kmode(int G, const BitmapLaunch& L) {
-    if (G == 32) return launch_bitmap_kgm<K, 32, kMode, kKind>(L);
-    if (G == 8) return launch_bitmap_kgm<K, 8, kMode, kKind>(L);
-    return launch_bitmap_kgm<K, 1, kMode, kKind>(L);
+    if (G == 32) return launch_bitmap_kgm<K, 32, 1, kMode, kKind>(L);
+    if (G == 8) return launch_bitmap_kgm<K, 4, kMode == kCountEdge ? 1 : 2, kMode, kKind>(L);
+    return launch_bitmap_kgm<K, 1, 1, kMode, kKind>(L);
 }
 
 template <int K>
@@ -479,9 +479,9 @@ static pc_status launch_bitmap_k(int G, const BitmapLaunch& L) {
 
 static pc_status launch_bitmap(int K, int G, int kind, const BitmapLaunch& L) {
     if (kind == kMixedSet) {  // fixed-size sets (mixed_shape)
-        if (K == 1 && L.ecnt) return launch_bitmap_kgm<1, 8, kCountEdge, kMixedSet>(L);
-        if (K == 1 && L.tri) return launch_bitmap_kgm<1, 8, kCountVertex, kMixedSet>(L);
-        if (K == 1) return launch_bitmap_kgm<1, 8, kCountOnly, kMixedSet>(L);
+        if (K == 1 && L.ecnt) return launch_bitmap_kgm<1, 4, 1, kCountEdge, kMixedSet>(L);
+        if (K == 1 && L.tri) return launch_bitmap_kgm<1, 4, 1, kCountVertex, kMixedSet>(L);
+        if (K == 1) return launch_bitmap_kgm<1, 4, 1, kCountOnly, kMixedSet>(L);
         if (L.ecnt || K != 2) return fail(PC_ERR_UNSUPPORTED, "mixed pivot sets: unexpected launch shape");
         if (L.tri) return launch_bitmap_kmode<2, kCountVertex, kMixedSet>(G, L);
         return launch_bitmap_kmode<2, kCountOnly, kMixedSet>(G, L);

@@ -190,8 +190,8 @@ struct HitSink {
 // Scans the prefixes of up to 32 in-neighbours of pivot b: lane j < nb holds
 // in-neighbour j's id (c) and row start; returns this lane's hits.
 //
-// A group of G lanes takes one in-neighbour at a time, 4 ids per lane and
-// step, and goes on to its next one (NG apart) as soon as its row reaches an
+// A group of G lanes takes one in-neighbour at a time, V vectors of 4 ids per
+// lane and step, and goes on to its next one (NG apart) as soon as its row reaches an
 // id >= b -- b itself is in the row, so a scan ends inside it -- while the
 // other groups go on with theirs: no lane waits for the longest of the 32 / G
 // rows in flight.  All groups step together, so the vote that ends a row is
@@ -207,8 +207,15 @@ struct HitSink {
 // warp instructions per 128 ids; the earlier scan, which tested each id's
 // position and kept a group waiting for the longest of its warp's rows, took
 // about 130.  Bitmap kernels of RMAT-20: 2.07 -> 0.83 ms; RMAT-24's unit of ids
-// 49-65 K (2.0e9 ids): 3.23 -> 1.92 ms.
-template <int G, int kMode, int kKind>
+// 49-65 K (2.0e9 ids): 3.23 -> 1.92 ms with G = 8 and V = 1.
+//
+// Two vectors a step keep twice the bytes in flight and halve the votes per id
+// where prefixes are long; short ones waste the second.  RMAT-24 by (G, V), ms:
+// that unit (8, 1) 1.95, (4, 1) 2.05, (4, 2) 1.82, (8, 2) 1.65, (2, 2) 2.21; the
+// first unit's tail with its matrix part 8.3 / 8.0 / 7.4 / 8.4 / 7.0; RMAT-20's
+// light pivots, ER-20: 0.98 / 0.83 / 1.01 / 1.41 / 0.95.  So bitmap sets scan with
+// (4, 2), light pivots with (4, 1).
+template <int G, int V, int kMode, int kKind>
 __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, int32_t c, uint32_t start, int nb,
                                                        int32_t b, const SetView& S, int lane,
                                                        const HitSink& sink) {
@@ -220,53 +227,71 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
     int j = lane / G;
     uint32_t q = __shfl_sync(0xffffffffu, start, j) + gl;
     bool act = j < nb;
-    int4 v = act ? __ldg(O.ids + q) : none;
+    int4 v[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = act ? __ldg(O.ids + q + i * G) : none;
     uint32_t cnt = 0, pair = 0;
     while (__any_sync(0xffffffffu, act)) {
-        const unsigned stop = __ballot_sync(0xffffffffu, v.w >= b);
-        const bool done = G == 1 ? v.w >= b : (stop & gmask) != 0;
+        // vector i of the group's lanes precedes vector i + 1: the row's stop is
+        // the lowest lane of the first vector that has one
+        unsigned stop[V];
+        bool past[V];  // this lane's vector lies behind the stop
+        bool done = false;
+        int4 a[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            stop[i] = __ballot_sync(0xffffffffu, v[i].w >= b);
+            past[i] = done || (G > 1 && (stop[i] & below) != 0);
+            done = done || (G == 1 ? v[i].w >= b : (stop[i] & gmask) != 0);
+            a[i] = v[i];
+            if (past[i]) a[i].x = INT32_MAX;
+        }
         const uint32_t qc = q;
         const int jc = j;
-        int4 a = v;
-        if (G > 1 && (stop & below)) a.x = INT32_MAX;
         if (done) j += NG;
         const uint32_t s = __shfl_sync(0xffffffffu, start, j & 31);
-        q = done ? s + gl : q + G;
+        q = done ? s + gl : q + V * G;
         const bool had = act;
         act = j < nb;
-        v = act ? __ldg(O.ids + q) : none;
-        a.y = max(a.x, a.y);
-        a.z = max(a.y, a.z);
-        a.w = max(a.z, a.w);
-        uint32_t h[4];
-        uint32_t rank[4];  // kMixedSet with lo = 0: of the hits
-        h[0] = bit_of(S.bm, S.place<kKind>(min(a.x, b)));
-        h[1] = bit_of(S.bm, S.place<kKind>(min(a.y, b)));
-        h[2] = bit_of(S.bm, S.place<kKind>(min(a.z, b)));
-        h[3] = bit_of(S.bm, S.place<kKind>(min(a.w, b)));
-        if constexpr (kKind == kMixedSet) {
-            if (h[0] && a.x >= S.lo) h[0] = a.x < b && S.find(a.x, &rank[0]);
-            if (h[1] && a.y >= S.lo) h[1] = a.y < b && S.find(a.y, &rank[1]);
-            if (h[2] && a.z >= S.lo) h[2] = a.z < b && S.find(a.z, &rank[2]);
-            if (h[3] && a.w >= S.lo) h[3] = a.w < b && S.find(a.w, &rank[3]);
-        }
-        const uint32_t hits = h[0] + h[1] + h[2] + h[3];
-        cnt += hits;
-        if constexpr (kMode != kCountOnly) {
-            const int32_t e[4] = {a.x, a.y, a.z, a.w};
-            if (hits) {
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    if (!h[t]) continue;
-                    if constexpr (kMode == kCountVertex) {
-                        count_vertex(e[t], sink.tri_low, sink.hist, sink.hist_ids);
-                    } else {
-                        atomicAdd(sink.ecnt + (4ull * qc + t), 1u);
-                        atomicAdd(sink.by_rank + (kKind == kMixedSet ? rank[t] : rank_in_set(S.bm, sink.ranks, e[t])),
-                                  1u);
+        for (int i = 0; i < V; ++i) v[i] = act ? __ldg(O.ids + q + i * G) : none;
+        uint32_t hits = 0;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            a[i].y = max(a[i].x, a[i].y);
+            a[i].z = max(a[i].y, a[i].z);
+            a[i].w = max(a[i].z, a[i].w);
+            const int32_t e[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+            uint32_t h[4];
+            uint32_t rank[4];  // kMixedSet with lo = 0: of the hits
+#pragma unroll
+            for (int t = 0; t < 4; ++t) h[t] = bit_of(S.bm, S.place<kKind>(min(e[t], b)));
+            if constexpr (kKind == kMixedSet) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (h[t] && e[t] >= S.lo) h[t] = e[t] < b && S.find(e[t], &rank[t]);
+            }
+            const uint32_t here = h[0] + h[1] + h[2] + h[3];
+            hits += here;
+            if constexpr (kMode != kCountOnly) {
+                if (here) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        if (!h[t]) continue;
+                        if constexpr (kMode == kCountVertex) {
+                            count_vertex(e[t], sink.tri_low, sink.hist, sink.hist_ids);
+                        } else {
+                            atomicAdd(sink.ecnt + (4ull * (qc + i * G) + t), 1u);
+                            atomicAdd(sink.by_rank +
+                                          (kKind == kMixedSet ? rank[t] : rank_in_set(S.bm, sink.ranks, e[t])),
+                                      1u);
+                        }
                     }
                 }
             }
+        }
+        cnt += hits;
+        if constexpr (kMode != kCountOnly) {
             pair += hits;
             if (__any_sync(0xffffffffu, done && had)) {
                 uint32_t sum = pair;
@@ -275,15 +300,25 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
                     const int32_t cj = __shfl_sync(0xffffffffu, c, jc & 31);
                     if (done && had && gl == 0 && sum) atomicAdd(&sink.tri[cj], (unsigned long long)sum);
                 } else {
-                    // the first lane to stop holds b: after the ids below it
-                    if (done && had && sum && ((stop >> lane) & 1u) && !(stop & below))
-                        atomicAdd(sink.ecnt + (4ull * qc + (a.x < b) + (a.y < b) + (a.z < b)), sum);
+                    // the stop holds b: after the ids below it
+#pragma unroll
+                    for (int i = 0; i < V; ++i)
+                        if (done && had && sum && ((stop[i] >> lane) & 1u) && !past[i])
+                            atomicAdd(sink.ecnt + (4ull * (qc + i * G) + (a[i].x < b) + (a[i].y < b) + (a[i].z < b)), sum);
                 }
                 if (done) pair = 0;
             }
         }
     }
     return cnt;
+}
+
+// CTAs per SM a bitmap kernel's registers leave room for.  Three for the count;
+// two for split sets with two vectors a step, whose look-ups spill at 40
+// registers (RMAT-24's unit of ids 65-82 K: 1.10 ms, 1.28 with three), and for the
+// other modes.
+constexpr int bitmap_ctas(int V, int mode, int kind) {
+    return mode == kCountOnly && !(kind == kMixedSet && V > 1) ? 3 : 2;
 }
 
 // Bitmap kernel: a CTA of kCtaThreads threads holds 16/K pivot sets in
@@ -295,8 +330,8 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
 // Mixed sets have (bm_words - kFilterWords) * 32 = lo bits for the low ids,
 // whatever the pivots' ids (0 in the per-edge mode, which needs every hit's
 // rank).
-template <int K, int G, int kMode, int kKind>
-__global__ void __launch_bounds__(kCtaThreads, kMode == kCountOnly ? 3 : 2)
+template <int K, int G, int V, int kMode, int kKind>
+__global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
     k_tc_bitmap(OrientedView O, const int32_t* __restrict__ adj, const Item* __restrict__ items,
                 const uint32_t* __restrict__ nitems_p, uint32_t* __restrict__ next_item,
                 unsigned long long* __restrict__ total, uint32_t bm_words, unsigned long long* __restrict__ unit_cost,
@@ -387,7 +422,7 @@ __global__ void __launch_bounds__(kCtaThreads, kMode == kCountOnly ? 3 : 2)
             const int nb = min(32, (int)(I.n - k));
             const int32_t c = lane < nb ? adj[I.in0 + k + lane] : 0;
             const uint32_t start = O.off[c];
-            cnt += scan_in_neighbours<G, kMode, kKind>(O, c, start, nb, b, S, lane, sink);
+            cnt += scan_in_neighbours<G, V, kMode, kKind>(O, c, start, nb, b, S, lane, sink);
         }
         if (kMode == kCountVertex) {
             unsigned long long hb = cnt - cnt0;  // this item's triangles at pivot b
