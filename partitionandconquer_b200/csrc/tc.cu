@@ -1,7 +1,5 @@
 // Triangle counting: planning units, per-unit features, variant selection
 // (forced / heuristic / learned) and the pc_tc entry points.
-#include <cub/device/device_scan.cuh>
-
 #include <algorithm>
 #include <initializer_list>
 #include <cmath>
@@ -139,17 +137,6 @@ __global__ void k_unit_scan_stats(const uint64_t* __restrict__ off, const int32_
     }
 }
 
-// Locates linear position q inside a list of position ranges.
-__device__ __forceinline__ int64_t range_pos(const int64_t* __restrict__ ranges, const int64_t* __restrict__ rprefix,
-                                             uint32_t nranges, uint64_t q) {
-    uint32_t lo = 0, hi = nranges;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((uint64_t)rprefix[mid] <= q) lo = mid; else hi = mid;
-    }
-    return ranges[2 * lo] + (int64_t)(q - (uint64_t)rprefix[lo]);
-}
-
 // First CSR entry of pivot b's in-neighbours at or above c_min (0: of all).
 __device__ __forceinline__ uint64_t first_in_neighbour(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
                                                        const uint32_t* __restrict__ dplus, int32_t b, int32_t c_min) {
@@ -157,38 +144,173 @@ __device__ __forceinline__ uint64_t first_in_neighbour(const uint64_t* __restric
     return c_min > b ? in0 + lower_bound_i32(adj + in0, (uint32_t)(off[b + 1] - in0), c_min) : in0;
 }
 
-// Work items: pivot q (a linear position in the launch's position ranges)
-// gives ceil(din / chunk) items, each a run of <= chunk of its in-neighbours
-// at or above c_min; pivots without a set or without in-neighbours give none.
-__global__ void k_item_count(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                             const uint32_t* __restrict__ dplus, const int32_t* __restrict__ plist, int32_t c_min, const int64_t* __restrict__ ranges,
-                             const int64_t* __restrict__ rprefix, uint32_t nranges, uint64_t npos, uint32_t chunk,
-                             uint32_t* __restrict__ cnt) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t > npos) return;
-    if (t == npos) { cnt[t] = 0; return; }
-    const int32_t b = pivot_at(plist, range_pos(ranges, rprefix, nranges, t));
-    const uint32_t din = (uint32_t)(off[b + 1] - first_in_neighbour(off, adj, dplus, b, c_min));
-    cnt[t] = dplus[b] == 0 ? 0u : (din + chunk - 1) / chunk;
+// One launch's list of work items.
+struct ItemList {
+    Item* items;
+    uint32_t* count;  // zeroed before
+    uint32_t cap;     // room of items: an upper bound of the count
+    uint32_t chunk;   // in-neighbours per item
+    int32_t c_min;    // in-neighbours below this are not taken
+};
+
+// Work items of all launches of a count: pivot b gives its list (list_of[its
+// unit], -1: none) ceil(din / chunk) items, each a run of <= chunk of its
+// in-neighbours; pivots without a set or without in-neighbours give none.
+//
+// A warp takes a block of 32 kRows consecutive pivots.  The lists are in pivot
+// order wherever a block has pivots of one list only: kItemsCount writes the
+// blocks' items, k_item_offsets adds them up per list, kItemsOrdered fills them
+// in.  (In the order of an atomic per block the bitmap kernels of RMAT-20 took
+// 873 instead of 798 us: sets of neighbouring pivots are scanned by rows that
+// L2 still holds.)  Blocks with several lists, and all blocks of small graphs
+// (kItemsAny, a single pass), take an atomic per list instead.  A count, a scan
+// and a fill per launch cost 20 us for each of them.
+enum ItemPass { kItemsCount, kItemsOrdered, kItemsAny };
+struct __align__(16) ItemBlock {
+    uint32_t n;     // items
+    uint32_t at;    // the block's first place in its list
+    int32_t list;   // -1: none, -2: several
+    int32_t pad;
+};
+// The items of a block of hubs (100 K for RMAT-24's first one) are written by
+// kRows warps, a row of pivots each.
+constexpr uint32_t kItemsSplit = 256;
+
+template <int kRows, int kPass>
+__global__ void k_items(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                        const uint32_t* __restrict__ dplus, const int32_t* __restrict__ unit_of,
+                        const int16_t* __restrict__ list_of, const ItemList* __restrict__ lists, uint64_t n,
+                        ItemBlock* __restrict__ blocks) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const int part = blockIdx.y;  // kItemsOrdered: 0 .. kRows - 1
+    for (uint64_t blk = warp; blk * 32 * kRows < n; blk += nwarps) {
+        const bool split = kPass == kItemsOrdered && blocks[blk].n > kItemsSplit;
+        if (part && !split) continue;
+        const uint64_t b0 = blk * 32 * kRows;
+        uint64_t in0[kRows];
+        uint32_t din[kRows], c[kRows];
+        int32_t l[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const uint64_t b = min(b0 + 32 * i + lane, n - 1);
+            const uint32_t dp = dplus[b];
+            in0[i] = off[b] + dp;
+            din[i] = (uint32_t)(off[b + 1] - in0[i]);
+            l[i] = unit_of[b];
+            if (dp == 0 || b0 + 32 * i + lane >= n) din[i] = 0;
+        }
+        uint32_t sum = 0;
+        int32_t mine = -1;  // the lane's list, -2: more than one
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            c[i] = 0;
+            l[i] = din[i] ? list_of[l[i]] : -1;
+            if (l[i] < 0) continue;
+            const int32_t c_min = lists[l[i]].c_min;
+            if (c_min) {
+                const uint64_t b = b0 + 32 * i + lane;
+                in0[i] = first_in_neighbour(off, adj, dplus, (int32_t)b, c_min);
+                din[i] = (uint32_t)(off[b + 1] - in0[i]);
+            }
+            const uint32_t chunk = lists[l[i]].chunk;
+            c[i] = (din[i] + chunk - 1) / chunk;
+            if (!c[i]) continue;
+            sum += c[i];
+            mine = mine == -1 || mine == l[i] ? l[i] : -2;
+        }
+        const unsigned have = __ballot_sync(0xffffffffu, sum != 0);
+        const int32_t l0 = have ? __shfl_sync(0xffffffffu, mine, __ffs(have) - 1) : -1;
+        const bool one = __all_sync(0xffffffffu, sum == 0 || mine == l0) && l0 >= 0;
+        if (kPass == kItemsCount) {
+            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0) blocks[blk] = ItemBlock{one ? sum : 0u, 0u, have ? (one ? l0 : -2) : -1, 0};
+            continue;
+        }
+        if (!have) continue;
+        // the lists of the block one after the other
+        for (unsigned left = have; left;) {
+            int32_t cur = 0x7fffffff;  // the smallest list not done yet
+#pragma unroll
+            for (int i = 0; i < kRows; ++i)
+                if (c[i]) cur = min(cur, l[i]);
+            cur = __reduce_min_sync(0xffffffffu, cur);
+            uint32_t own = 0;
+#pragma unroll
+            for (int i = 0; i < kRows; ++i)
+                if (c[i] && l[i] == cur) own += c[i];
+            uint32_t end = own;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += x;
+            }
+            const ItemList L = lists[cur];
+            uint32_t at = 0;
+            if (lane == 31) at = kPass == kItemsOrdered && one ? blocks[blk].at : atomicAdd(L.count, end);
+            at = __shfl_sync(0xffffffffu, at, 31) + end - own;
+            bool more = false;
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const int32_t b = (int32_t)(b0 + 32 * i + lane);
+                const uint32_t ci = l[i] == cur ? c[i] : 0u;
+                const bool here = !split || i == part;
+                if (here && ci && ci <= 8)
+                    for (uint32_t j = 0; j < ci && at + j < L.cap; ++j)
+                        L.items[at + j] = Item{in0[i] + (uint64_t)j * L.chunk, b, min(L.chunk, din[i] - j * L.chunk)};
+                // a hub's items are written by the warp together
+                for (unsigned hubs = __ballot_sync(0xffffffffu, here && ci > 8); hubs; hubs &= hubs - 1) {
+                    const int src = __ffs(hubs) - 1;
+                    const uint32_t cs = __shfl_sync(0xffffffffu, ci, src), as = __shfl_sync(0xffffffffu, at, src);
+                    const uint32_t ds = __shfl_sync(0xffffffffu, din[i], src);
+                    const uint64_t is = __shfl_sync(0xffffffffu, in0[i], src);
+                    for (uint32_t j = lane; j < cs && as + j < L.cap; j += 32)
+                        L.items[as + j] = Item{is + (uint64_t)j * L.chunk, b - lane + src, min(L.chunk, ds - j * L.chunk)};
+                }
+                at += ci;
+                if (ci) c[i] = 0;
+                more |= c[i] != 0;
+            }
+            left = __ballot_sync(0xffffffffu, more);
+        }
+    }
 }
 
-__global__ void k_item_fill(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                            const uint32_t* __restrict__ dplus, const int32_t* __restrict__ plist, int32_t c_min, const int64_t* __restrict__ ranges,
-                            const int64_t* __restrict__ rprefix, uint32_t nranges, uint64_t npos, uint32_t chunk,
-                            const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ start,
-                            Item* __restrict__ items, uint32_t cap, uint32_t* __restrict__ nitems) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t == 0) *nitems = min(start[npos], cap);
-    if (t >= npos) return;
-    const uint32_t c = cnt[t];
-    if (!c) return;
-    const int64_t p = range_pos(ranges, rprefix, nranges, t);
-    const int32_t b = pivot_at(plist, p);
-    const uint64_t in0 = first_in_neighbour(off, adj, dplus, b, c_min);
-    const uint32_t din = (uint32_t)(off[b + 1] - in0);
-    const uint32_t s = start[t];
-    for (uint32_t j = 0; j < c && s + j < cap; ++j)
-        items[s + j] = Item{in0 + (uint64_t)j * chunk, b, min(chunk, din - j * chunk)};
+// Finds the blocks' first places in their list and writes the list's length
+// (of the ordered blocks).  A CTA per list, a run of blocks per warp.
+__global__ void __launch_bounds__(1024) k_item_offsets(ItemBlock* __restrict__ blocks, uint32_t nblocks,
+                                                       const ItemList* __restrict__ lists) {
+    __shared__ uint32_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l = blockIdx.x;
+    const uint32_t per = ((nblocks + 1023) / 1024) * 32, k0 = min(nblocks, warp * per), k1 = min(nblocks, k0 + per);
+    uint32_t own = 0;
+#pragma unroll 8
+    for (uint32_t k = k0 + lane; k < k1; k += 32) {
+        const ItemBlock B = blocks[k];
+        if (B.list == l) own += B.n;
+    }
+    own = __reduce_add_sync(0xffffffffu, own);
+    if (lane == 0) s_warp[warp] = own;
+    __syncthreads();
+    uint32_t at = 0, total = 0;
+    for (int w = 0; w < 32; ++w) {
+        if (w < warp) at += s_warp[w];
+        total += s_warp[w];
+    }
+    if (threadIdx.x == 0) *lists[l].count = total;
+    if (own == 0) return;
+    for (uint32_t kk = k0; kk < k1; kk += 32) {
+        const uint32_t k = kk + lane;
+        const bool mine = k < k1 && blocks[k].list == l;
+        const uint32_t c = mine ? blocks[k].n : 0u;
+        uint32_t end = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+        }
+        if (mine) blocks[k].at = at + end - c;
+        at += __shfl_sync(0xffffffffu, end, 31);
+    }
 }
 
 // H[b - lo][a >> 5] |= bit(a) for a in N+(b), one warp per pivot.
@@ -444,6 +566,7 @@ struct BitmapLaunch {
     const int32_t* adj;
     const Item* items;
     const uint32_t* nitems;
+    uint32_t cap;
     uint32_t* next;
     unsigned long long* total;
     uint32_t words;
@@ -457,7 +580,7 @@ template <int K, int G, int V, int kMode, int kKind>
 static pc_status launch_bitmap_kgm(const BitmapLaunch& L) {
     PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, V, kMode, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)L.smem));
-    k_tc_bitmap<K, G, V, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.next,
+    k_tc_bitmap<K, G, V, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.cap, L.next,
                                                                         L.total, L.words, L.cost, L.unit_of, L.tri,
                                                                         L.ecnt);
     return PC_OK;
@@ -560,6 +683,11 @@ struct LaunchGroup {
     std::vector<int32_t> unit_ids;  // matrix groups: one launch per unit (ranges not merged)
     int32_t c_min = 0;              // in-neighbours below this are not taken
     std::vector<LaunchGroup> tails; // matrix groups: the in-neighbours from kMatrixFrom on, per bitmap shape
+    // launches of item lists (finish_group)
+    BitmapShape shape{};
+    uint32_t chunk = 0;
+    int list = -1;                  // index among the count's lists
+    ItemList dev{};
 };
 
 // Words per resident pivot bitmap row of a matrix unit with ids below hi:
@@ -626,11 +754,28 @@ static pc_status run_matrix_unit(pc_pgraph* pg, int64_t lo, int64_t hi, int32_t 
     return PC_OK;
 }
 
+// Shape and item size of a launch.  An item is up to 256 in-neighbours per warp
+// of its set, less where that would leave sets without one: RMAT-10's 11 K
+// in-edges in runs of 256 kept one warp busy for 30 us, in runs of 32 for 13.
 // Items never exceed min(pivots, in-edges) + in-edges / chunk; the float
 // in-edge feature is widened by 256 per unit for its rounding.
-static void finish_group(LaunchGroup* gr) {
+static void finish_group(LaunchGroup* gr, int mode, int sms) {
     const uint64_t ein = (uint64_t)gr->ein + 256 * gr->units;
-    gr->item_bound = std::min<uint64_t>(gr->npos, ein) + ein / 256 + 1;
+    uint64_t per_set = 0, sets = 0, most = 0;
+    if (is_bitmap(gr->v) || gr->v == PC_VARIANT_HASH_WARP) {
+        if (gr->v == PC_VARIANT_HASH_WARP) gr->shape = mixed_shape(mode, 1, mode == kCountEdge ? 0u : kLightLo);
+        else gr->shape = gr->split ? mixed_shape(mode, 2, kSplitLo) : bitmap_shape(gr->words, mode);
+        per_set = 32u * (uint32_t)gr->shape.K;
+        sets = (uint64_t)sms * gr->shape.ctas_per_sm * (16 / gr->shape.K);
+        most = 256u * (uint32_t)gr->shape.K;
+    } else {
+        per_set = 32;
+        sets = (uint64_t)sms * 8 * kWarpCtaWarps;
+        most = (uint64_t)kChunkWarp;
+    }
+    const uint64_t want = ceil_div(ceil_div(ein, 2 * sets), per_set) * per_set;
+    gr->chunk = (uint32_t)std::min(most, std::max(per_set, want));
+    gr->item_bound = std::min<uint64_t>(gr->npos, ein) + ein / gr->chunk + 1;
 }
 
 static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long long* d_total, uint64_t* launches,
@@ -654,52 +799,22 @@ static pc_status run_group(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
     return run_items(pg, gr, d_total, launches, d_cost, d_tri, d_ecnt);
 }
 
-// The groups whose work is a list of items.
+
+// The groups whose work is a list of items (built by k_items).
 static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long long* d_total, uint64_t* launches,
                            unsigned long long* d_cost, unsigned long long* d_tri, uint32_t* d_ecnt) {
     const int32_t* unit_of = pg->unit_of.as<int32_t>();
     cudaStream_t s = pg->g->stream;
     const int v = gr.v;
     const uint32_t* dp = pg->dplus.as<uint32_t>();
-    const int32_t* plist = pg->contiguous ? nullptr : pg->new2old.as<int32_t>();
     const int sms = sm_count(pg->g->device);
-    const uint32_t nr = (uint32_t)(gr.ranges.size() / 2);
-    std::vector<int64_t> pref(nr + 1, 0);
-    for (uint32_t i = 0; i < nr; ++i) pref[i + 1] = pref[i] + (gr.ranges[2 * i + 1] - gr.ranges[2 * i]);
-    const uint64_t npos = (uint64_t)pref[nr];
-    if (npos == 0) return PC_OK;
-    int64_t* d_ranges = nullptr;
-    int64_t* d_pref = nullptr;
-    PC_TRY(upload(pg, gr.ranges.data(), gr.ranges.size(), &d_ranges));
-    PC_TRY(upload(pg, pref.data(), nr + 1, &d_pref));
-    const int mode = d_tri ? kCountVertex : (d_ecnt ? kCountEdge : kCountOnly);
-    const bool sets = is_bitmap(v) || v == PC_VARIANT_HASH_WARP;  // run by k_tc_bitmap
+    if (gr.npos == 0) return PC_OK;
+    const BitmapShape& sh = gr.shape;
     const bool light = v == PC_VARIANT_HASH_WARP;
-    const BitmapShape sh = light ? mixed_shape(mode, 1, mode == kCountEdge ? 0u : kLightLo)
-                                 : (gr.split ? mixed_shape(mode, 2, kSplitLo) : bitmap_shape(gr.words, mode));
-    const uint32_t chunk = sets ? 256u * (uint32_t)sh.K : (uint32_t)kChunkWarp;
-    uint32_t* d_cnt = pg->scratch.take<uint32_t>(npos + 1);
-    uint32_t* d_start = pg->scratch.take<uint32_t>(npos + 1);
-    size_t tmpb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmpb, d_cnt, d_start, (int64_t)(npos + 1), s);
-    void* d_tmp = pg->scratch.take<char>(tmpb);
-    uint32_t* d_next = pg->scratch.take<uint32_t>(2);
-    Item* d_items = pg->scratch.take<Item>(gr.item_bound);
-    if (!d_cnt || !d_start || !d_tmp || !d_next || !d_items)
-        return fail(PC_ERR_OOM, "scratch arena too small (internal sizing error)");
-    k_item_count<<<(unsigned)ceil_div(npos + 1, 256), 256, 0, s>>>(pg->off, pg->adj, dp, plist, gr.c_min, d_ranges, d_pref,
-                                                                   nr, npos, chunk, d_cnt);
-    PC_LAUNCHED();
-    PC_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp, tmpb, d_cnt, d_start, (int64_t)(npos + 1), s));
-    count_launch();
-    k_item_fill<<<(unsigned)ceil_div(npos, 256), 256, 0, s>>>(pg->off, pg->adj, dp, plist, gr.c_min, d_ranges, d_pref,
-                                                              nr, npos, chunk, d_cnt, d_start, d_items, (uint32_t)gr.item_bound,
-                                                              d_next + 1);
-    PC_LAUNCHED();
-    PC_CUDA(cudaMemsetAsync(d_next, 0, 4, s));
-    *launches += 3;
-    const uint32_t* d_nitems = d_next + 1;
-    if (sets) {
+    const Item* d_items = gr.dev.items;
+    const uint32_t* d_nitems = gr.dev.count;
+    uint32_t* d_next = gr.dev.count + 1;
+    if (is_bitmap(v) || light) {  // run by k_tc_bitmap
         BitmapLaunch L;
         L.smem = sh.smem;
         L.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * sh.ctas_per_sm, gr.item_bound));
@@ -708,6 +823,7 @@ static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
         L.adj = pg->adj;
         L.items = d_items;
         L.nitems = d_nitems;
+        L.cap = gr.dev.cap;
         L.next = d_next;
         L.total = d_total;
         L.words = sh.words;
@@ -723,7 +839,7 @@ static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
         const unsigned bs = kWarpCtaWarps * 32;
         const uint32_t* ooff = pg->oids.p ? pg->ooff.as<uint32_t>() : nullptr;
         auto launch = [&](auto* kernel) {
-            kernel<<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, ooff, d_items, d_nitems, d_next, d_total, d_cost, unit_of,
+            kernel<<<grid, bs, 0, s>>>(pg->off, pg->adj, dp, ooff, d_items, d_nitems, gr.dev.cap, d_next, d_total, d_cost, unit_of,
                                        d_tri, d_ecnt);
         };
         if (v == PC_VARIANT_MERGE_LANE) {
@@ -808,13 +924,15 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         }
         add_unit(*tail, true);
     }
-    size_t need = 1024;
-    auto items_need = [&](LaunchGroup& gr) {
-        finish_group(&gr);
-        size_t tmpb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tmpb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)(gr.npos + 1),
-                                      s);
-        need += gr.ranges.size() * 16 + 64 + (gr.npos + 1) * 8 + tmpb + gr.item_bound * sizeof(Item) + 8 * 256;
+    const int mode = d_tri ? kCountVertex : (d_ecnt ? kCountEdge : kCountOnly);
+    const int sms = sm_count(pg->g->device);
+    std::vector<LaunchGroup*> listed;  // the groups with an item list
+    size_t need = 4096;
+    auto add_list = [&](LaunchGroup& gr) {
+        finish_group(&gr, mode, sms);
+        gr.list = (int)listed.size();
+        listed.push_back(&gr);
+        need += gr.item_bound * sizeof(Item) + 256;
     };
     for (LaunchGroup& gr : groups) {
         if (gr.ranges.empty()) continue;
@@ -823,14 +941,42 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
             for (size_t i = 0; i < gr.unit_ids.size(); ++i)
                 hb = std::max(hb, matrix_bytes(gr.ranges[2 * i], gr.ranges[2 * i + 1]));
             need += hb + 2 * 256;
-            for (LaunchGroup& t : gr.tails) items_need(t);
+            for (LaunchGroup& t : gr.tails) add_list(t);
             continue;
         }
-        items_need(gr);
+        add_list(gr);
     }
+    // the list of every unit (a matrix unit's is its tail's)
+    std::vector<int16_t> list_of(std::max<size_t>(U, 1), -1);
+    for (const LaunchGroup* gr : listed)
+        for (size_t i = 0; i < gr->ranges.size(); i += 2) {
+            const size_t u0 = std::lower_bound(lo.begin(), lo.end(), gr->ranges[i]) - lo.begin();
+            for (size_t u = u0; u < U && lo[u] < gr->ranges[i + 1]; ++u) list_of[u] = (int16_t)gr->list;
+        }
+    // ordered lists from 2^17 vertices on; below, three launches cost more
+    // (RMAT-16 0.15 ms with them, 0.11 without)
+    const uint64_t n = pg->g->n;
+    const uint64_t item_blocks = n >= (1u << 17) ? ceil_div(n, 256) : 0;
+    need += U * 2 + listed.size() * (sizeof(ItemList) + 8) + item_blocks * sizeof(ItemBlock) + 1024;
     if (unit_ms) need += U * 8 + 256;
     PC_TRY(scratch_reserve(pg, need));
-    unsigned long long* d_total = pg->scratch.take<unsigned long long>(1);
+    // the total, then a count and a taken-items counter per list
+    unsigned long long* d_total = pg->scratch.take<unsigned long long>(1 + listed.size());
+    int16_t* d_list_of = nullptr;
+    ItemList* d_lists = nullptr;
+    ItemBlock* d_blocks = item_blocks ? pg->scratch.take<ItemBlock>(item_blocks) : nullptr;
+    if (item_blocks && !d_blocks) return fail(PC_ERR_OOM, "scratch arena too small (internal sizing error)");
+    std::vector<ItemList> lists(listed.size());
+    for (size_t i = 0; i < listed.size(); ++i) {
+        ItemList& L = listed[i]->dev;
+        L.items = pg->scratch.take<Item>(listed[i]->item_bound);
+        if (!L.items) return fail(PC_ERR_OOM, "scratch arena too small (internal sizing error)");
+        L.count = reinterpret_cast<uint32_t*>(d_total + 1 + i);
+        L.cap = (uint32_t)listed[i]->item_bound;
+        L.chunk = listed[i]->chunk;
+        L.c_min = listed[i]->c_min;
+        lists[i] = L;
+    }
     unsigned long long* d_cost = unit_ms ? pg->scratch.take<unsigned long long>(std::max<size_t>(U, 1)) : nullptr;
     std::vector<cudaEvent_t> gev;
     auto drop_events = [&]() {
@@ -848,7 +994,28 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     }
     uint64_t launches = 0;
     PC_CUDA(cudaEventRecord(pg->ev0, s));
-    PC_CUDA(cudaMemsetAsync(d_total, 0, 8, s));
+    PC_CUDA(cudaMemsetAsync(d_total, 0, 8 * (1 + listed.size()), s));
+    if (!listed.empty()) {
+        PC_TRY(upload(pg, list_of.data(), U, &d_list_of));
+        PC_TRY(upload(pg, lists.data(), lists.size(), &d_lists));
+        auto launch = [&](auto* kernel, int rows, unsigned parts) {  // rows: pivots per lane
+            const dim3 grid((unsigned)std::min<uint64_t>((uint64_t)sms * 16, ceil_div(n, 128 * rows)), parts);
+            kernel<<<grid, 128, 0, s>>>(
+                pg->off, pg->adj, pg->dplus.as<uint32_t>(), pg->unit_of.as<int32_t>(), d_list_of, d_lists, n, d_blocks);
+        };
+        if (item_blocks) {
+            launch(k_items<8, kItemsCount>, 8, 1);
+            PC_LAUNCHED();
+            k_item_offsets<<<(unsigned)listed.size(), 1024, 0, s>>>(d_blocks, (uint32_t)item_blocks, d_lists);
+            PC_LAUNCHED();
+            launch(k_items<8, kItemsOrdered>, 8, 8);
+            launches += 2;
+        } else {
+            launch(k_items<1, kItemsAny>, 1, 1);
+        }
+        PC_LAUNCHED();
+        ++launches;
+    }
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const LaunchGroup& gr = groups[gi];
         if (gr.ranges.empty()) continue;

@@ -333,7 +333,7 @@ constexpr int bitmap_ctas(int V, int mode, int kind) {
 template <int K, int G, int V, int kMode, int kKind>
 __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
     k_tc_bitmap(OrientedView O, const int32_t* __restrict__ adj, const Item* __restrict__ items,
-                const uint32_t* __restrict__ nitems_p, uint32_t* __restrict__ next_item,
+                const uint32_t* __restrict__ nitems_p, uint32_t cap, uint32_t* __restrict__ next_item,
                 unsigned long long* __restrict__ total, uint32_t bm_words, unsigned long long* __restrict__ unit_cost,
                 const int32_t* __restrict__ unit_of, unsigned long long* __restrict__ tri,
                 uint32_t* __restrict__ ecnt) {
@@ -353,19 +353,18 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
     uint16_t* r16 = reinterpret_cast<uint16_t*>(r32 + (kHash ? 0u : (bm_words + 63) / 64));
     uint32_t* by_rank = bm + set_words - kEcRankCap;
     uint32_t* hist = smem + (size_t)nsets * set_words;        // kCountVertex: kHubHist counters after the sets
-    const uint32_t zero_words = (uint32_t)nsets * set_words + (kMode == kCountVertex ? (uint32_t)kHubHist : 0u);
-    for (uint32_t i = tid; i < zero_words; i += blockDim.x)
-        smem[i] = (kHash && i < (uint32_t)nsets * set_words && i % set_words >= bm_words &&
-                   i % set_words < bm_words + kHashSlots)
-                      ? 0xffffffffu
-                      : 0u;
+    for (uint32_t i = tis; i < set_words; i += set_threads) bm[i] = 0;
+    if (kHash)
+        for (uint32_t i = tis; i < (uint32_t)kHashSlots; i += set_threads) ht[i] = -1;
+    if (kMode == kCountVertex)
+        for (uint32_t i = tid; i < (uint32_t)kHubHist; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     auto set_sync = [&]() {
         if constexpr (K == 1) __syncwarp();
         else group_barrier(1 + set, set_threads);
     };
     const int32_t lo = kHash ? (int32_t)(bm_words - kFilterWords) * 32 : 0;
-    const uint32_t nitems = *nitems_p;
+    const uint32_t nitems = min(*nitems_p, cap);
     unsigned long long cnt = 0;
     for (;;) {
         if (tis == 0) s_item[set] = atomicAdd(next_item, 1u);
@@ -592,6 +591,7 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
                                                                 const uint32_t* __restrict__ ooff,
                                                                 const Item* __restrict__ items,
                                                                 const uint32_t* __restrict__ nitems_p,
+                                                                uint32_t cap,
                                                                 uint32_t* __restrict__ next_item,
                                                                 unsigned long long* __restrict__ total,
                                                                 unsigned long long* __restrict__ unit_cost,
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
         for (int i = threadIdx.x; i < kHubHist; i += blockDim.x) hist[i] = 0;
         __syncthreads();
     }
-    const uint32_t nitems = *nitems_p;
+    const uint32_t nitems = min(*nitems_p, cap);
     unsigned long long cnt = 0;
     for (;;) {
         uint32_t it = 0;
