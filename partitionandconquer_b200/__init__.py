@@ -448,7 +448,7 @@ class Partitioned_Graph:
     def triangle_count(self, method: int = METHOD_MERGE, variant: int = VARIANT_AUTO, stats: bool = False):
         out = C.c_uint64()
         st = TCStats()
-        check(lib.pc_tc_ex(self._pg, method, variant, C.byref(out), C.byref(st)))
+        check(lib.pc_tc_ex(self._pg, method, variant, C.byref(out), C.byref(st) if stats else None))
         return (int(out.value), st) if stats else int(out.value)
 
     def solve_triangle_counting_merge(self) -> int:

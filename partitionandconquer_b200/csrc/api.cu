@@ -94,6 +94,18 @@ void DevBuf::release() {
     bytes = 0;
 }
 
+void DevBuf::release_idle() {
+    if (p) {
+        int cur = -1;
+        cudaGetDevice(&cur);
+        if (cur != dev) cudaSetDevice(dev);
+        cudaFreeAsync(p, 0);
+        if (cur != dev && cur >= 0) cudaSetDevice(cur);
+    }
+    p = nullptr;
+    bytes = 0;
+}
+
 int sm_count(int device) {
     static std::mutex mu;
     static std::vector<int> cache;
@@ -118,7 +130,8 @@ pc_status scratch_reserve(pc_pgraph* pg, size_t bytes) {
     size_t want = bytes + 64 * 256;
     if (want > pg->scratch.buf.bytes) {
         PC_CUDA(cudaStreamSynchronize(pg->g->stream));
-        PC_TRY(pg->scratch.buf.alloc(want + want / 4, "scratch arena"));
+        // small calls of a new view would grow it again and again: 4 MB at least
+        PC_TRY(pg->scratch.buf.alloc(std::max<size_t>(want + want / 4, 4u << 20), "scratch arena"));
     }
     return PC_OK;
 }
@@ -430,7 +443,7 @@ __global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t*
 }
 
 pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
-                         uint64_t n, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff_buf,
+                         uint64_t n, uint64_t m, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff_buf,
                          DevBuf* oids_buf, uint64_t* vecs) {
     PC_TRY(ooff_buf->alloc((n + 1) * 4, "oriented offsets"));
     uint32_t* ooff = ooff_buf->as<uint32_t>();
@@ -438,9 +451,13 @@ pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t
     PC_LAUNCHED();
     PC_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, ooff, ooff, (int64_t)(n + 1), s));
     count_launch();
-    uint32_t nvec = 0;
-    PC_CUDA(cudaMemcpyAsync(&nvec, ooff + n, 4, cudaMemcpyDeviceToHost, s));
-    PC_CUDA(cudaStreamSynchronize(s));
+    uint64_t nvec = (m + 3 * n) / 4;
+    if (nvec > (1u << 18)) {
+        uint32_t exact = 0;
+        PC_CUDA(cudaMemcpyAsync(&exact, ooff + n, 4, cudaMemcpyDeviceToHost, s));
+        PC_CUDA(cudaStreamSynchronize(s));
+        nvec = exact;
+    }
     PC_TRY(oids_buf->alloc(((uint64_t)nvec + 32) * 16, "oriented ids"));
     *vecs = nvec;
     const uint64_t grid = std::min<uint64_t>((uint64_t)sm_count(device) * 16, ceil_div(nvec, 8 * 256));
@@ -465,7 +482,7 @@ pc_status ensure_oriented(pc_pgraph* pg) {
     const size_t tb = oriented_temp_bytes(n);
     PC_TRY(scratch_reserve(pg, tb));
     const pc_status st =
-        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->device, pg->g->stream,
+        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->m, pg->g->device, pg->g->stream,
                        pg->scratch.take<char>(tb), tb, &pg->ooff, &pg->oids, &pg->ovecs);
     if (st != PC_ERR_OOM) return st;
     pg->ooff.release();
@@ -621,9 +638,9 @@ pc_status pc_graph_destroy(pc_graph* g) {
     if (g->live_views) return fail(PC_ERR_INVALID_INPUT, "destroy the partitioned views of this graph first");
     cudaSetDevice(g->device);
     cudaStreamSynchronize(g->stream);
-    g->off.release();
-    g->adj.release();
-    g->w.release();
+    g->off.release_idle();
+    g->adj.release_idle();
+    g->w.release_idle();
     cudaStreamDestroy(g->stream);
     delete g;
     return PC_OK;
@@ -741,6 +758,12 @@ pc_status pc_pgraph_destroy(pc_pgraph* pg) {
     cudaStreamSynchronize(pg->g->stream);
     if (pg->ev0) cudaEventDestroy(pg->ev0);
     if (pg->ev1) cudaEventDestroy(pg->ev1);
+    if (pg->copy_stream) cudaStreamDestroy(pg->copy_stream);  // idle: its calls wait for it
+    for (cudaEvent_t e : pg->part_done)
+        if (e) cudaEventDestroy(e);
+    for (DevBuf* b : {&pg->old2new, &pg->new2old, &pg->v2p, &pg->d_pstart, &pg->dplus, &pg->ooff, &pg->oids, &pg->unit_of,
+                      &pg->scratch.buf})
+        b->release_idle();
     pg->g->live_views--;
     delete pg;
     return PC_OK;

@@ -504,7 +504,7 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
         const size_t tb = oriented_temp_bytes(N);
         if ((st = tmp.alloc(tb, "scan scratch")) != PC_OK) return bail(st);
         st = build_oriented(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(), b->dplus.as<uint32_t>(),
-                            b->graph_of.as<int32_t>() + N, N, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
+                            b->graph_of.as<int32_t>() + N, N, M, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
         if (st != PC_OK) return bail(st);
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));

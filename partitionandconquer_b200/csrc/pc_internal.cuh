@@ -53,6 +53,7 @@ struct DevBuf {
     pc_status alloc(size_t nbytes, const char* what);
     pc_status ensure(size_t nbytes, const char* what);  // grow-only
     void release();
+    void release_idle();  // the caller has waited for every stream that used it
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
@@ -114,6 +115,9 @@ struct pc_pgraph {
     pc::DevBuf unit_of;           // int32 [n]: planning unit of each vertex (tc.cu)
     pc::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // copies of a large result's parts beside the kernels of the later parts (intersect.cu)
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t part_done[8] = {};
     // planner state (tc.cu)
     std::vector<float> part_features;  // per-unit features (lazy)
     std::vector<int64_t> unit_lo, unit_hi;  // planning units (plist position ranges)
@@ -163,10 +167,12 @@ int32_t to_internal_id(const pc_pgraph* pg, int32_t api_id);
 pc_status ensure_dplus(pc_pgraph* pg);
 
 // Builds the oriented copy of a CSR (see pc_pgraph::oids): row u's ids less
-// row_base[u] (none when null).  tmp: oriented_temp_bytes(n) bytes; waits for
-// the stream once.  Its vector indices are 32-bit: oriented_fits().
+// row_base[u] (none when null).  tmp: oriented_temp_bytes(n) bytes.  Waits for
+// the stream once, for the copy's size, except for a small graph, whose copy
+// gets the room that it can need at most.  Its vector indices are 32-bit:
+// oriented_fits().
 pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
-                         uint64_t n, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff,
+                         uint64_t n, uint64_t m, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff,
                          DevBuf* oids, uint64_t* vecs);
 size_t oriented_temp_bytes(uint64_t n);
 inline bool oriented_fits(uint64_t n, uint64_t m) { return (m + 3 * n) / 4 + 64 < (1ull << 32); }

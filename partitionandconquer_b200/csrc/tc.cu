@@ -993,11 +993,17 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         PC_CUDA(cudaMemsetAsync(d_cost, 0, std::max<size_t>(U, 1) * 8, s));
     }
     uint64_t launches = 0;
-    PC_CUDA(cudaEventRecord(pg->ev0, s));
+    if (stats) PC_CUDA(cudaEventRecord(pg->ev0, s));
     PC_CUDA(cudaMemsetAsync(d_total, 0, 8 * (1 + listed.size()), s));
     if (!listed.empty()) {
-        PC_TRY(upload(pg, list_of.data(), U, &d_list_of));
-        PC_TRY(upload(pg, lists.data(), lists.size(), &d_lists));
+        // one copy: the lists, then the units' list numbers
+        std::vector<char> tables(lists.size() * sizeof(ItemList) + U * 2);
+        memcpy(tables.data(), lists.data(), lists.size() * sizeof(ItemList));
+        memcpy(tables.data() + lists.size() * sizeof(ItemList), list_of.data(), U * 2);
+        char* d_tables = nullptr;
+        PC_TRY(upload(pg, tables.data(), tables.size(), &d_tables));
+        d_lists = reinterpret_cast<ItemList*>(d_tables);
+        d_list_of = reinterpret_cast<int16_t*>(d_tables + lists.size() * sizeof(ItemList));
         auto launch = [&](auto* kernel, int rows, unsigned parts) {  // rows: pivots per lane
             const dim3 grid((unsigned)std::min<uint64_t>((uint64_t)sms * 16, ceil_div(n, 128 * rows)), parts);
             kernel<<<grid, 128, 0, s>>>(
@@ -1023,7 +1029,7 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         PC_TRY(run_group(pg, gr, d_total, &launches, d_cost, d_tri, d_ecnt));
         if (unit_ms) PC_CUDA(cudaEventRecord(gev[2 * gi + 1], s));
     }
-    PC_CUDA(cudaEventRecord(pg->ev1, s));
+    if (stats) PC_CUDA(cudaEventRecord(pg->ev1, s));
     unsigned long long h = 0;
     PC_CUDA(cudaMemcpyAsync(&h, d_total, 8, cudaMemcpyDeviceToHost, s));
     std::vector<unsigned long long> cyc(unit_ms ? U : 0);
