@@ -340,19 +340,20 @@ __device__ __forceinline__ bool matrix_words_win(int32_t b, uint32_t jl) {
 // The pairs (b, c) of one in-neighbour c: S = N(c) & [0, min(hi, c)), pivots
 // at positions [j0, k).  Pivots are taken U consecutive positions at a time,
 // so each step of the warp has U independent row loads in flight per lane and
-// shares one load of S (or of its bitmap) between them:
+// shares one load of S (or of its bitmap) between them (RMAT-24 count with
+// U = 4: 27.7 ms, 8: 27.1; RMAT-22: 4.51 and 4.50):
 //  - probe form: lanes read S[i] for i below the block's last position and
 //    test bit S[i] of each pivot's row (i < j of that pivot);
 //  - word form: lanes AND 16-byte words of each row with the warp's
 //    shared-memory bitmap of S and count bits.  A row b has bits only below
 //    b, so words past a pivot's own length read zeros.
 // The form is chosen per block by the rounds each needs; the bitmap is built
-// only when some block uses it.  S may point to shared or global memory.
-template <int U>
+// only when some block uses it.
 __device__ __forceinline__ unsigned long long matrix_block_pairs(const int32_t* S, uint32_t j0, uint32_t k,
                                                                  int32_t lo, uint32_t hstride,
                                                                  const uint32_t* __restrict__ H, uint32_t* Sb,
                                                                  int lane) {
+    constexpr int U = kMatrixBlock;
     unsigned long long cnt = 0;
     bool want = false;
     for (uint32_t jb = j0 + (uint32_t)lane * U; jb < k; jb += 32u * U) {
@@ -420,7 +421,6 @@ __device__ __forceinline__ void matrix_span(const uint64_t* __restrict__ off, co
 
 // The in-neighbours c in (lo, c1), taken one per warp: they are the hubs, with
 // long spans S_c (c1: kMatrixFrom).
-template <int U>
 __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t* __restrict__ off,
                                                                const int32_t* __restrict__ adj,
                                                                const uint32_t* __restrict__ dplus, int32_t lo,
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t*
         r = __shfl_sync(0xffffffffu, r, 0);
         klo = __shfl_sync(0xffffffffu, klo, 0);
         khi = __shfl_sync(0xffffffffu, khi, 0);
-        if (khi > klo) cnt += matrix_block_pairs<U>(adj + r, klo, khi, lo, hstride, H, Sb, lane);
+        if (khi > klo) cnt += matrix_block_pairs(adj + r, klo, khi, lo, hstride, H, Sb, lane);
     }
     if (unit_cost) {
         __syncwarp();
@@ -460,7 +460,10 @@ __global__ void __launch_bounds__(kMatrixWarps * 32) k_tc_matrix(const uint64_t*
 
 // A matrix unit's in-neighbours from this id on run through the bitmap kernel:
 // their spans are short, and the probes of a short span into rows of L2 are
-// slower than a scan against a bitmap in shared memory.
+// slower than a scan against a bitmap in shared memory.  RMAT-24 / RMAT-22
+// counts in ms with the line at 2^13: 33.6 / 5.15, 2^14: 31.6 / 4.85,
+// 2^15: 30.0 / 4.55, 2^16: 27.1 / 4.50, 2^17: 27.1 / 4.57, 2^18: 27.3 / 4.66,
+// 2^19: 28.0 / 4.80.
 constexpr int32_t kMatrixFrom = 1 << 16;
 
 constexpr uint32_t kBitmapCapBits = 1u << 20;  // 128 KB of shared memory
@@ -708,26 +711,15 @@ static bool bitmap_split_enabled() {
     return on;
 }
 
-// Pivots per block of the matrix kernel: 4, or 8 with PC_MATRIX_PIVOT_BLOCK=8
-// in the environment (read once; a tuning override for measurements).
-static int matrix_pivot_block() {
-    static const int u = [] {
-        const char* e = getenv("PC_MATRIX_PIVOT_BLOCK");
-        return (e && atoi(e) == 8) ? 8 : 4;
-    }();
-    return u;
-}
-
-template <int U>
 static pc_status launch_matrix(pc_pgraph* pg, int64_t lo, int64_t hi, uint32_t hstride, const uint32_t* H,
                                unsigned long long* d_next, unsigned long long* d_total, unsigned long long* d_cost,
                                int32_t unit, int sms, cudaStream_t s) {
     const size_t smem = (size_t)kMatrixWarps * hstride * 4;
-    PC_CUDA(cudaFuncSetAttribute(k_tc_matrix<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PC_CUDA(cudaFuncSetAttribute(k_tc_matrix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_matrix<U>, kMatrixWarps * 32, smem));
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_matrix, kMatrixWarps * 32, smem));
     const uint64_t c1 = std::min<uint64_t>(pg->g->n, (uint64_t)kMatrixFrom);
-    k_tc_matrix<U><<<(unsigned)(sms * std::max(1, per_sm)), kMatrixWarps * 32, smem, s>>>(
+    k_tc_matrix<<<(unsigned)(sms * std::max(1, per_sm)), kMatrixWarps * 32, smem, s>>>(
         pg->off, pg->adj, pg->dplus.as<uint32_t>(), (int32_t)lo, (int32_t)hi, c1, hstride, H, d_next, d_total, d_cost, unit);
     PC_LAUNCHED();
     return PC_OK;
@@ -746,10 +738,7 @@ static pc_status run_matrix_unit(pc_pgraph* pg, int64_t lo, int64_t hi, int32_t 
     k_matrix_rows<<<sms * 8, 256, 0, s>>>(pg->off, pg->adj, pg->dplus.as<uint32_t>(), (int32_t)lo, (int32_t)hi, hstride,
                                           H);
     PC_LAUNCHED();
-    if (matrix_pivot_block() == 8)
-        PC_TRY(launch_matrix<8>(pg, lo, hi, hstride, H, d_next, d_total, d_cost, unit, sms, s));
-    else
-        PC_TRY(launch_matrix<4>(pg, lo, hi, hstride, H, d_next, d_total, d_cost, unit, sms, s));
+    PC_TRY(launch_matrix(pg, lo, hi, hstride, H, d_next, d_total, d_cost, unit, sms, s));
     *launches += 2;
     return PC_OK;
 }

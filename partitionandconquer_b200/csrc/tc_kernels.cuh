@@ -675,10 +675,12 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
 // either by j bit probes into H[b] or by ceil(b/32) word-wise ANDs of H[b]
 // with a shared-memory bitmap of S_c and popcounts, whichever is cheaper.
 // Every (pivot, in-neighbour) pair of the unit is one pair (b, c) here, so the
-// count equals the pivot form's; what changes is that N(c) comes from DRAM
-// once per c instead of once per pivot.
+// count equals the pivot form's; what changes is that N(c) is read once per c
+// instead of once per pivot.  Only the hubs' pairs run this way (kMatrixFrom in
+// tc.cu); the other in-neighbours of the unit are items of the bitmap kernels.
 constexpr int kMatrixMaxId = 1 << 16;      // hi bound: rows of <= 8 KB, H <= 512 MB
 constexpr int kMatrixWarps = 8;            // warps per CTA
+constexpr int kMatrixBlock = 8;            // pivots a warp takes at a time
 constexpr int kMatrixWordsMax = kMatrixMaxId / 32;
 
 __device__ __forceinline__ uint32_t lower_bound_i32(const int32_t* __restrict__ p, uint32_t n, int32_t x) {
