@@ -162,14 +162,14 @@ __global__ void k_check_offsets(const uint64_t* __restrict__ off, uint64_t n, ui
     if (blockIdx.x == 0 && threadIdx.x == 0 && (off[0] != 0 || off[n] != m)) atomicOr(err, BAD_OFFSETS);
 }
 
-// Warp-chunked edge walk: each warp takes a chunk of 1024 consecutive edge
-// slots; lane 0 finds the row of the chunk start by binary search, then lanes
-// walk forward to the row of their own slot.
-__device__ __forceinline__ uint64_t row_of(const uint64_t* __restrict__ off, uint64_t n, uint64_t e) {
-    uint64_t lo = 0, hi = n;  // off[lo] <= e < off[hi]
+// The row of entry e (off[row] <= e < off[row + 1]), found by a warp: 32 rows a
+// round trip.
+__device__ __forceinline__ uint64_t row_of(const uint64_t* __restrict__ off, uint64_t n, uint64_t e, int lane) {
+    uint64_t lo = 0, hi = n;
     while (hi - lo > 1) {
-        uint64_t mid = (lo + hi) >> 1;
-        if (off[mid] <= e) lo = mid; else hi = mid;
+        const uint64_t step = (hi - lo + 31) / 32, mid = lo + (lane + 1) * step;
+        lo += step * __popc(__ballot_sync(0xffffffffu, mid < hi && off[mid] <= e));
+        hi = min(hi, lo + step);
     }
     return lo;
 }
@@ -183,38 +183,94 @@ __device__ __forceinline__ uint64_t fp_mix(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-__global__ void k_check_edges(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n,
-                              uint64_t m, uint32_t* err, unsigned long long* fp) {
+// A warp takes a run of chunks of kCheckChunk entries, four of a chunk's
+// 16-byte vectors per lane, all loaded before the first is looked at.  The rows
+// that start in the chunk leave a mark (row + 1) at their first entry's place
+// in shared memory, and a running maximum over the marks gives every entry its
+// row: no lane walks the offsets on its own.
+//
+// Bound: instruction issue, the two hashes' multiplications.  An entry per
+// lane, whose row was looked for from the row of the 32 entries before, waited
+// on dependent loads: RMAT-20's 31 M entries 234 -> 150 us.
+constexpr int kCheckChunk = 512;
+constexpr int kCheckWarps = 8;
+
+__global__ void __launch_bounds__(kCheckWarps * 32) k_check_edges(const uint64_t* __restrict__ off,
+                                                                  const int32_t* __restrict__ adj, uint64_t n,
+                                                                  uint64_t m, uint32_t* err, unsigned long long* fp) {
+    constexpr int kSteps = kCheckChunk / 128;
+    __shared__ uint4 marks[kCheckWarps][kCheckChunk / 4];
     const int lane = threadIdx.x & 31;
+    uint4* mk4 = marks[threadIdx.x >> 5];
+    uint32_t* mk = reinterpret_cast<uint32_t*>(mk4);
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t chunks = (m + kCheckChunk - 1) / kCheckChunk, per = (chunks + nwarps - 1) / nwarps;
+    const uint64_t c0 = min(warp * per, chunks), c1 = min(c0 + per, chunks);
     uint64_t acc0 = 0, acc1 = 0;
     uint32_t bad = 0;
-    for (uint64_t c = warp; c * 1024 < m; c += nwarps) {
-        uint64_t base = c * 1024, end = min(base + 1024, m);
-        uint64_t r = 0;
-        if (lane == 0) r = row_of(off, n, base);
-        r = __shfl_sync(0xffffffffu, r, 0);
-        for (uint64_t e0 = base; e0 < end; e0 += 32) {
-            uint64_t e = e0 + lane;
-            uint64_t u = r;
-            if (e < end) {
-                while (off[u + 1] <= e) ++u;
-                int32_t v = adj[e];
-                if (v < 0 || (uint64_t)v >= n) {
+    for (int i = lane; i < kCheckChunk / 4; i += 32) mk4[i] = make_uint4(0, 0, 0, 0);
+    uint64_t first = 0;  // the first row that may start in the chunk
+    uint32_t last = 0;   // 1 + the row of the entry before the ones in hand
+    if (c0 < c1) {
+        const uint64_t r = row_of(off, n, c0 * kCheckChunk, lane);
+        last = (uint32_t)r + 1;
+        first = off[r] == c0 * kCheckChunk ? r : r + 1;
+    }
+    __syncwarp();
+    for (uint64_t c = c0; c < c1; ++c) {
+        const uint64_t base = c * kCheckChunk, end = min(base + kCheckChunk, m);
+        int4 v[kSteps];  // the ids past the last entry are the array's padding
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+            const uint64_t p = base + i * 128 + lane * 4;
+            v[i] = p < end ? __ldcs(reinterpret_cast<const int4*>(adj + p)) : make_int4(0, 0, 0, 0);
+        }
+        int32_t before = lane == 0 && base ? adj[base - 1] : 0;
+        for (uint64_t row = first + lane;; row += 32) {
+            const uint64_t o = row < n ? off[row] : m, next = row < n ? off[row + 1] : m;
+            if (o < end && next > o) mk[o - base] = (uint32_t)row + 1;
+            if (__any_sync(0xffffffffu, o >= end)) break;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+            const uint4 k = mk4[i * 32 + lane];
+            mk4[i * 32 + lane] = make_uint4(0, 0, 0, 0);
+            uint32_t top = max(max(k.x, k.y), max(k.z, k.w));
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, top, o);
+                if (lane >= o) top = max(top, x);
+            }
+            uint32_t row = __shfl_up_sync(0xffffffffu, top, 1);
+            row = lane ? max(row, last) : last;
+            last = max(last, __shfl_sync(0xffffffffu, top, 31));
+            int32_t prev = __shfl_up_sync(0xffffffffu, v[i].w, 1);
+            if (lane == 0) prev = before;
+            before = __shfl_sync(0xffffffffu, v[i].w, 31);
+            const int32_t id[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+            const uint32_t mark[4] = {k.x, k.y, k.z, k.w};
+            const uint64_t p = base + i * 128 + lane * 4;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                row = max(row, mark[t]);
+                if (p + t >= end) break;
+                const uint32_t u = row - 1, w = (uint32_t)id[t];
+                if (id[t] < 0 || w >= n) {
                     bad |= BAD_RANGE;
                 } else {
-                    if ((uint64_t)v == u) bad |= BAD_SELF;
-                    if (e > off[u] && adj[e - 1] >= v) bad |= BAD_ORDER;
-                    const uint64_t uv = (uint64_t)v;
-                    const uint64_t lo = u < uv ? u : uv, hi = u < uv ? uv : u;
-                    uint64_t key = (lo << 32) | hi;
-                    uint64_t h0 = fp_mix(key ^ 0x243F6A8885A308D3ULL), h1 = fp_mix(key + 0x13198A2E03707344ULL);
-                    if (u < (uint64_t)v) { acc0 += h0; acc1 += h1; } else { acc0 -= h0; acc1 -= h1; }
+                    if (w == u) bad |= BAD_SELF;
+                    if (mark[t] == 0 && prev >= id[t]) bad |= BAD_ORDER;
+                    const uint64_t key = ((uint64_t)min(u, w) << 32) | max(u, w);
+                    const uint64_t h0 = fp_mix(key ^ 0x243F6A8885A308D3ULL), h1 = fp_mix(key + 0x13198A2E03707344ULL);
+                    acc0 += u < w ? h0 : 0 - h0;
+                    acc1 += u < w ? h1 : 0 - h1;
                 }
+                prev = id[t];
             }
-            r = __shfl_sync(0xffffffffu, u, 31);
         }
+        first = last;
+        __syncwarp();  // the marks are cleared before the next chunk's are set
     }
     for (int o = 16; o; o >>= 1) {
         acc0 += __shfl_xor_sync(0xffffffffu, acc0, o);
@@ -226,6 +282,13 @@ __global__ void k_check_edges(const uint64_t* __restrict__ off, const int32_t* _
         if (acc1) atomicAdd(&fp[1], (unsigned long long)acc1);
         if (bad) atomicOr(err, bad);
     }
+}
+
+// A chunk a warp, runs of chunks only where there are more than 64 CTAs per SM
+// (RMAT-16 / 20 / 22: 15 / 150 / 530 us; two a warp and 32 CTAs 22 / 147 / 542;
+// always one 15 / 150 / 586, for each run starts with the search of its row).
+static unsigned check_grid(uint64_t m, int sms) {
+    return (unsigned)std::min<uint64_t>(ceil_div(m, kCheckWarps * kCheckChunk), (uint64_t)sms * 64);
 }
 
 // Weights must be in [0, 2^30): non-negative for the shortest-path semantics,
@@ -606,7 +669,7 @@ pc_status pc_graph_create(const uint64_t* vlist, const int32_t* elist, const int
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "offset validation", __FILE__, __LINE__));
         if (h_err) return cleanup(fail(PC_ERR_INVALID_INPUT, "csr_vlist must start at 0, be non-decreasing and end at m"));
         if (m) {
-            k_check_edges<<<sms * 8, 256, 0, g->stream>>>(g->off.as<uint64_t>(), g->adj.as<int32_t>(), n, m, d_err, d_fp);
+            k_check_edges<<<check_grid(m, sms), kCheckWarps * 32, 0, g->stream>>>(g->off.as<uint64_t>(), g->adj.as<int32_t>(), n, m, d_err, d_fp);
             count_launch();
             if (g->weighted) {
                 k_check_weights<<<sms * 4, 256, 0, g->stream>>>(g->w.as<int32_t>(), m, d_err);
