@@ -313,6 +313,64 @@ __global__ void __launch_bounds__(1024) k_item_offsets(ItemBlock* __restrict__ b
     }
 }
 
+// The items of bitmap lists by where their in-neighbours' rows lie in the
+// oriented copy: kBins parts of equal size, in list order (about) within a part.
+// In pivot order every pivot sweeps the rows of all its in-neighbours, and on a
+// graph whose rows L2 does not hold the scans of the hub units wait on DRAM
+// (4.5-5.9 TB/s in RMAT-24's).  An item builds its pivot's set either way.
+constexpr int kBins = 64;
+__device__ __forceinline__ int bin_of(const Item& I, const int32_t* __restrict__ adj, const uint32_t* __restrict__ ooff,
+                                      uint64_t vecs) {
+    return min((int)((uint64_t)ooff[adj[I.in0]] * kBins / vecs), kBins - 1);
+}
+
+__global__ void k_bin_count(const Item* __restrict__ items, const uint32_t* __restrict__ nitems, uint32_t cap,
+                            const int32_t* __restrict__ adj, const uint32_t* __restrict__ ooff, uint64_t vecs,
+                            uint32_t* __restrict__ bins) {
+    __shared__ uint32_t h[kBins];
+    if (threadIdx.x < kBins) h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t n = min(*nitems, cap);
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        atomicAdd(&h[bin_of(items[i], adj, ooff, vecs)], 1u);
+    __syncthreads();
+    if (threadIdx.x < kBins && h[threadIdx.x]) atomicAdd(&bins[threadIdx.x], h[threadIdx.x]);
+}
+
+// bins: the counts, then kBins zeroed words (items placed so far).
+__global__ void k_bin_scatter(const Item* __restrict__ items, const uint32_t* __restrict__ nitems, uint32_t cap,
+                              const int32_t* __restrict__ adj, const uint32_t* __restrict__ ooff, uint64_t vecs,
+                              uint32_t* __restrict__ bins, Item* __restrict__ out) {
+    __shared__ uint32_t base[kBins], h[kBins], at[kBins];
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+        for (int k = 0; k < kBins; ++k) {
+            base[k] = sum;
+            sum += bins[k];
+        }
+    }
+    const uint32_t n = min(*nitems, cap);
+    for (uint64_t tile = blockIdx.x * (uint64_t)blockDim.x; tile < n; tile += (uint64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x < kBins) h[threadIdx.x] = 0;
+        __syncthreads();
+        const uint64_t i = tile + threadIdx.x;
+        Item I{};
+        int k = 0;
+        uint32_t rank = 0;
+        if (i < n) {
+            I = items[i];
+            k = bin_of(I, adj, ooff, vecs);
+            rank = atomicAdd(&h[k], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < kBins)
+            at[threadIdx.x] = base[threadIdx.x] +
+                              (h[threadIdx.x] ? atomicAdd(&bins[kBins + threadIdx.x], h[threadIdx.x]) : 0u);
+        __syncthreads();
+        if (i < n) out[at[k] + rank] = I;
+    }
+}
+
 // H[b - lo][a >> 5] |= bit(a) for a in N+(b), one warp per pivot.
 __global__ void k_matrix_rows(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj,
                               const uint32_t* __restrict__ dplus, int32_t lo, int32_t hi, uint32_t hstride,
@@ -673,6 +731,11 @@ pc_status tc_ensure_features(pc_pgraph* pg) {
     return PC_OK;
 }
 
+// Item lists are binned where L2 (126 MB) does not hold the oriented copy: counts
+// of RMAT-24 27.1 -> 25.0 ms, RMAT-22 (0.27 GB) 4.50 -> 4.40, but RMAT-20 (65 MB)
+// 0.99 -> 1.02, where the rows stay in L2 in any order.
+constexpr uint64_t kBinFrom = 126ull << 20;
+
 // One launch: a variant and its bitmap shape (words rounded up to a power
 // of two).
 struct LaunchGroup {
@@ -689,6 +752,7 @@ struct LaunchGroup {
     // launches of item lists (finish_group)
     BitmapShape shape{};
     uint32_t chunk = 0;
+    bool binned = false;            // items in order of their in-neighbours' rows
     int list = -1;                  // index among the count's lists
     ItemList dev{};
 };
@@ -917,11 +981,15 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     const int sms = sm_count(pg->g->device);
     std::vector<LaunchGroup*> listed;  // the groups with an item list
     size_t need = 4096;
+    // lists put in order of their in-neighbours' rows
+    const uint64_t n = pg->g->n;
+    const bool bin = n >= (1u << 17) && pg->oids.p && pg->ovecs * 16 > kBinFrom;
     auto add_list = [&](LaunchGroup& gr) {
         finish_group(&gr, mode, sms);
         gr.list = (int)listed.size();
         listed.push_back(&gr);
-        need += gr.item_bound * sizeof(Item) + 256;
+        gr.binned = bin && is_bitmap(gr.v);
+        need += (gr.binned ? 2 : 1) * (gr.item_bound * sizeof(Item) + 256 + kBins * 8);
     };
     for (LaunchGroup& gr : groups) {
         if (gr.ranges.empty()) continue;
@@ -944,7 +1012,6 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         }
     // ordered lists from 2^17 vertices on; below, three launches cost more
     // (RMAT-16 0.15 ms with them, 0.11 without)
-    const uint64_t n = pg->g->n;
     const uint64_t item_blocks = n >= (1u << 17) ? ceil_div(n, 256) : 0;
     need += U * 2 + listed.size() * (sizeof(ItemList) + 8) + item_blocks * sizeof(ItemBlock) + 1024;
     if (unit_ms) need += U * 8 + 256;
@@ -1010,6 +1077,22 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         }
         PC_LAUNCHED();
         ++launches;
+        for (LaunchGroup* gr : listed) {
+            if (!gr->binned) continue;
+            Item* sorted = pg->scratch.take<Item>(gr->item_bound);
+            uint32_t* bins = pg->scratch.take<uint32_t>(2 * kBins);
+            if (!sorted || !bins) return fail(PC_ERR_OOM, "scratch arena too small (internal sizing error)");
+            PC_CUDA(cudaMemsetAsync(bins, 0, 2 * kBins * 4, s));
+            const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sms * 8, ceil_div(gr->item_bound, 256));
+            const uint32_t* ooff = pg->ooff.as<uint32_t>();
+            k_bin_count<<<grid, 256, 0, s>>>(gr->dev.items, gr->dev.count, gr->dev.cap, pg->adj, ooff, pg->ovecs, bins);
+            PC_LAUNCHED();
+            k_bin_scatter<<<grid, 256, 0, s>>>(gr->dev.items, gr->dev.count, gr->dev.cap, pg->adj, ooff, pg->ovecs, bins,
+                                               sorted);
+            PC_LAUNCHED();
+            gr->dev.items = sorted;
+            launches += 2;
+        }
     }
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const LaunchGroup& gr = groups[gi];
