@@ -47,7 +47,8 @@ typedef struct pc_pgraph pc_pgraph; /* partitioned view of a pc_graph */
 
 /* ---- library ---------------------------------------------------------- */
 
-/* Message of the last failed call on this thread ("" if none). */
+/* Message of the last failed call on this thread ("" if none).  Calls that
+ * release a handle leave it as it is. */
 const char* pc_last_error(void);
 /* Library version string. */
 const char* pc_version(void);

@@ -695,8 +695,9 @@ pc_status pc_graph_create(const uint64_t* vlist, const int32_t* elist, const int
     return PC_OK;
 }
 
+// The destroy calls leave the thread's message alone: a caller's garbage
+// collector may make them between a failed call and its pc_last_error().
 pc_status pc_graph_destroy(pc_graph* g) {
-    clear_error();
     if (!g) return PC_OK;
     if (g->live_views) return fail(PC_ERR_INVALID_INPUT, "destroy the partitioned views of this graph first");
     cudaSetDevice(g->device);
@@ -815,7 +816,6 @@ pc_status pc_partition(pc_graph* g, const int32_t* v2p, pc_pgraph** out) {
 }
 
 pc_status pc_pgraph_destroy(pc_pgraph* pg) {
-    clear_error();
     if (!pg) return PC_OK;
     cudaSetDevice(pg->g->device);
     cudaStreamSynchronize(pg->g->stream);

@@ -455,7 +455,7 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     b->gm.resize(G);
     for (uint32_t g = 0; g < G; ++g) b->gm[g] = vlist[voff[g + 1]] - vlist[voff[g]];
     auto bail = [&](pc_status st) {
-        const std::string msg = pc_last_error();  // pc_graph_destroy clears it
+        const std::string msg = pc_last_error();
         if (b->h_tc) cudaFreeHost(b->h_tc);
         if (b->h_lcc) cudaFreeHost(b->h_lcc);
         if (b->h_bfs) cudaFreeHost(b->h_bfs);
@@ -517,7 +517,6 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
 }
 
 pc_status pc_batch_destroy(pc_batch* b) {
-    clear_error();
     if (!b) return PC_OK;
     cudaSetDevice(b->g->device);
     cudaStreamSynchronize(b->g->stream);

@@ -118,7 +118,6 @@ pc_status pc_host_csr_from_arrays(const uint64_t* vlist, const int32_t* elist, c
 }
 
 pc_status pc_host_csr_free(pc_host_csr* g) {
-    pc::clear_error();
     delete g;
     return PC_OK;
 }
