@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include <cub/block/block_scan.cuh>
@@ -21,14 +22,13 @@ namespace fr {
 
 constexpr int kThreads = 256;
 constexpr int32_t kInf = INT_MAX;
-// bound on any grid-barrier wait of the persistent kernels (4 s)
-constexpr uint64_t kBarrierLimitNs = 4000000000ull;
 // k-core: ids below this have their degree decrements gathered per CTA
 constexpr int kKcoreHubs = 4096;
 constexpr int kKcoreThreads = 512;       // k-core: threads per CTA
 constexpr int kKcorePerSm = 2;
 constexpr uint32_t kLocalQ = 2048;       // ... its queue of claimed vertices
 constexpr uint32_t kLocalEdges = 16384;  // ... peeled by the CTA itself while their rows stay below this
+constexpr int kLocalRounds = 1024;       // ... and for so many rounds a step, while the others wait
 constexpr size_t kKcoreSmem = 80 * 1024;
 static_assert(kKcoreHubs % kKcoreThreads == 0, "the flush loop needs a uniform trip count");
 
@@ -466,8 +466,10 @@ __global__ void __launch_bounds__(tx::kThreads, 5)
 // queue is dry.  A vertex is claimed by the compare-and-swap that sets its
 // core number, since the scan and the decrements of other CTAs may meet at
 // it.  What does not fit the queue, or would keep one CTA busy for long (rows
-// of more than `local_edges` entries together), goes to the next step's queues,
-// which all CTAs share (tx::expand).  So most levels take one step.
+// of more than `local_edges` entries together, or more than kLocalRounds rounds:
+// a chain peels one vertex a round), goes to the next step's queues, which all
+// CTAs share (tx::expand).  So most levels take one step, and no step keeps the
+// others at the barrier for more than a few milliseconds.
 //
 // The state lives in three rotating records: step i reads S[i % 3],
 // accumulates into S[(i+1) % 3] (counters cleared by step i-1) and clears
@@ -676,7 +678,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
         // decrements (the one flush that takes a degree from >= k to < k
         // pushes the vertex) and go on until nothing is left
         int rd = 0;
-        for (;;) {
+        for (int round = 0;; ++round) {
             __syncthreads();
             uint32_t cnt = min(M.lqn[rd], (uint32_t)kLocalQ);
             if (cnt == 0) {
@@ -722,7 +724,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
                 M.tile.start[threadIdx.x] = end - len;
                 M.tile.base[threadIdx.x] = b - (end - len);
                 __syncthreads();
-                if (total > local_edges) {  // too much for one CTA: the next step shares it among all
+                if (total > local_edges || round >= kLocalRounds) {  // too much for one CTA: the next step shares it among all
                     tx::find(spill, nspill, i < cnt, u);
                     if (nspill > tx::kBuf - 32) tx::flush(spill, nspill, off, QN, &out->nl, &out->nh);
                     continue;
@@ -1091,6 +1093,14 @@ struct CdlpOp {
 
 using namespace fr;
 
+// Bound on any grid-barrier wait of the persistent kernels: 4 s, or
+// PC_BARRIER_LIMIT_MS from the environment (read on every call).
+static uint64_t barrier_limit_ns() {
+    const char* e = getenv("PC_BARRIER_LIMIT_MS");
+    const long ms = e ? std::max(1L, std::min(atol(e), 600000L)) : 4000L;
+    return (uint64_t)ms * 1000000ull;
+}
+
 static unsigned grid_for(const pc_pgraph* pg, int per_sm = 8) { return (unsigned)(sm_count(pg->g->device) * per_sm); }
 
 // CTAs of a persistent kernel: every SM's share, fewer for a small graph,
@@ -1126,7 +1136,7 @@ static pc_status bfs_run(pc_pgraph* pg, int32_t src, int32_t* rank_host) {
     PC_LAUNCHED();
     unsigned grid = 0;
     PC_TRY(persistent_grid(pg, (const void*)k_bfs_persistent, tx::kThreads, 6, 2048, &grid));
-    uint64_t max_steps = 2 * (n + 1) + 64, limit_ns = kBarrierLimitNs, nn = n;
+    uint64_t max_steps = 2 * (n + 1) + 64, limit_ns = barrier_limit_ns(), nn = n;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     void* args[] = {(void*)&off, (void*)&adj, (void*)&nn, (void*)&src, (void*)&dist,      (void*)&q0,
@@ -1248,7 +1258,7 @@ static pc_status mis_run(pc_pgraph* pg, bool hashed, uint64_t seed, int32_t* res
     PC_LAUNCHED();
     unsigned grid = 0;
     PC_TRY(persistent_grid(pg, (const void*)k_mis_persistent, tx::kThreads, 6, 1024, &grid));
-    uint64_t max_steps = 2 * n + 8, limit_ns = kBarrierLimitNs, nn = n;
+    uint64_t max_steps = 2 * n + 8, limit_ns = barrier_limit_ns(), nn = n;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     MisPriority P{pc_graph_key(seed, PC_GEN_PRIORITY), hashed ? 1 : 0, int2api};
@@ -1330,7 +1340,7 @@ pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, 
     PC_LAUNCHED();
     unsigned grid = 0;
     PC_TRY(persistent_grid(pg, (const void*)k_sssp_persistent, tx::kThreads, 5, 256, &grid));
-    uint64_t max_steps = 8 * (n + 1) + 64, limit_ns = kBarrierLimitNs;
+    uint64_t max_steps = 8 * (n + 1) + 64, limit_ns = barrier_limit_ns();
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     const int32_t* w = pg->w;
@@ -1460,7 +1470,7 @@ pc_status pc_kcore(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
     // a step scans a level or peels vertices claimed before it; each vertex
     // is claimed once, so n levels plus 2n peel steps bound the steps
     uint64_t max_steps = 3 * n + 8;
-    uint64_t limit_ns = kBarrierLimitNs;
+    uint64_t limit_ns = barrier_limit_ns();
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     uint64_t nn = n;
