@@ -167,6 +167,8 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
         } else if (bottom_up) {
             // (four vertices a thread with their loads together: a quarter
             // slower; the rows that go on then wait for one another)
+            // The plain loads of the neighbours' levels see all of the last
+            // step's (grid_sync); this step's, old or new, are not looked for.
             for (uint64_t v = tid; v < n; v += stride) {
                 if (__ldcg(dist + v) != kInf) continue;
                 const uint64_t b = off[v], e = off[v + 1];
@@ -1094,7 +1096,10 @@ struct CdlpOp {
 using namespace fr;
 
 // Bound on any grid-barrier wait of the persistent kernels: 4 s, or
-// PC_BARRIER_LIMIT_MS from the environment (read on every call).
+// PC_BARRIER_LIMIT_MS from the environment (read on every call).  A cooperative
+// grid is placed as a whole, so no CTA waits for one that has no room yet
+// (measured: behind a kernel that left half of the SMs after 5 ms and the others
+// after 60 ms, all CTAs began at 60 ms).
 static uint64_t barrier_limit_ns() {
     const char* e = getenv("PC_BARRIER_LIMIT_MS");
     const long ms = e ? std::max(1L, std::min(atol(e), 600000L)) : 4000L;

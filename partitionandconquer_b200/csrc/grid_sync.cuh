@@ -1,12 +1,15 @@
 // Grid-wide barrier for persistent kernels started with a cooperative launch
 // (every CTA of the grid is resident, so every CTA can reach the barrier).
 //
-// Every wait is bounded by a wall-clock limit read from %globaltimer: a CTA
-// that waits longer, or that sees another CTA's error, records the error and
-// the barrier returns false, so the kernel can return and the host can read
-// the status instead of the GPU spinning for ever.
+// Every wait is bounded by a limit on the time from %globaltimer (less the time
+// in which another program had the GPU, see WaitClock): a CTA that waits longer,
+// or that sees another CTA's error, records the error and the barrier returns
+// false, so the kernel can return and the host can read the status instead of
+// the GPU spinning for ever.
 #pragma once
 #include <cstdint>
+
+#include "wait_clock.h"
 
 namespace pc {
 
@@ -29,8 +32,11 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 }
 
 // All threads of every CTA call it.  Writes made before it (plain stores and
-// atomics) are visible to every CTA after it, to loads that bypass L1
-// (__ldcg) or to atomics.
+// atomics) are visible to every CTA after it, plain loads included: thread 0's
+// fence and arrival release its CTA's writes (ordered before them by the CTA
+// barrier), its acquiring read of the counter and the fence after it take the
+// others' in and drop what L1 holds, and the second CTA barrier passes that on.
+// During a step a plain load may still return what L1 took in earlier in it.
 __device__ __forceinline__ bool grid_sync(GridBarrier* gb, uint64_t limit_ns) {
     __shared__ int s_ok;
     __syncthreads();
@@ -44,10 +50,10 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* gb, uint64_t limit_ns) {
         const unsigned long long mine = atomicAdd(&gb->arrived, 1ull);
         const unsigned long long all = (mine / gridDim.x + 1) * gridDim.x;
         if (mine + 1 != all) {
-            const uint64_t t0 = global_ns();
+            WaitClock clock(global_ns());
             while (ld_acquire_u64(&gb->arrived) < all) {
                 if (*(volatile int*)&gb->err) { ok = 0; break; }
-                if (global_ns() - t0 > limit_ns) {
+                if (clock.over(global_ns(), limit_ns)) {
                     atomicExch(&gb->err, 1);
                     ok = 0;
                     break;
