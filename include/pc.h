@@ -76,7 +76,12 @@ pc_status pc_selftest_grid_barrier(int32_t device, int32_t rounds, int32_t absen
 
 /* ---- graph (class Graph, src/Graph.hpp:38-103) ------------------------- */
 
-#define PC_GRAPH_NO_VALIDATE 1u /* skip the device-side CSR checks */
+/* Skip the device-side CSR checks.  The caller then vouches for them: offsets or
+ * ids out of range lead to accesses out of range.  An adjacency that is not
+ * symmetric is never left by an access, but algorithms that rely on the symmetry
+ * (per-edge and matrix counts, bottom-up BFS, k-core, MIS) return no defined
+ * result for it. */
+#define PC_GRAPH_NO_VALIDATE 1u
 
 /* Upload a symmetric CSR (rows strictly ascending, no self-loops, ids in
  * [0,n)).  weights may be NULL.  Replaces Graph::Graph(csrdir, is_weighted)

@@ -457,10 +457,12 @@ pc_status ensure_dplus(pc_pgraph* pg) {
     return PC_OK;
 }
 
-// ooff[u] = vectors of row u in the oriented copy, for the exclusive sum.
-__global__ void k_oriented_count(const uint32_t* __restrict__ dplus, uint64_t n, uint32_t* __restrict__ ooff) {
+// ooff[u] = vectors of row u in the oriented copy, for the exclusive sum
+// (pad 3: whole vectors, 4: and an INT_MAX in each).
+__global__ void k_oriented_count(const uint32_t* __restrict__ dplus, uint64_t n, uint32_t pad,
+                                 uint32_t* __restrict__ ooff) {
     const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (u <= n) ooff[u] = u < n ? (dplus[u] + 3) / 4 : 0u;
+    if (u <= n) ooff[u] = u < n ? (dplus[u] + pad) / 4 : 0u;
 }
 
 // Fills the oriented copy, a vector per thread; the work is split by vectors,
@@ -496,7 +498,7 @@ __global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t*
             const int32_t* src = adj + off[u] + k;
             const int32_t base = row_base ? row_base[u] : 0;
             int4 v = none;
-            v.x = src[0] - base;
+            if (left > 0) v.x = src[0] - base;
             if (left > 1) v.y = src[1] - base;
             if (left > 2) v.z = src[2] - base;
             if (left > 3) v.w = src[3] - base;
@@ -506,15 +508,15 @@ __global__ void k_oriented_fill(const uint64_t* __restrict__ off, const int32_t*
 }
 
 pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
-                         uint64_t n, uint64_t m, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff_buf,
-                         DevBuf* oids_buf, uint64_t* vecs) {
+                         uint64_t n, uint64_t m, bool checked, int device, cudaStream_t s, void* tmp, size_t tmp_bytes,
+                         DevBuf* ooff_buf, DevBuf* oids_buf, uint64_t* vecs) {
     PC_TRY(ooff_buf->alloc((n + 1) * 4, "oriented offsets"));
     uint32_t* ooff = ooff_buf->as<uint32_t>();
-    k_oriented_count<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(dplus, n, ooff);
+    k_oriented_count<<<(unsigned)ceil_div(n + 1, 256), 256, 0, s>>>(dplus, n, checked ? 3u : 4u, ooff);
     PC_LAUNCHED();
     PC_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, ooff, ooff, (int64_t)(n + 1), s));
     count_launch();
-    uint64_t nvec = (m + 3 * n) / 4;
+    uint64_t nvec = oriented_most(n, m, checked);
     if (nvec > (1u << 18)) {
         uint32_t exact = 0;
         PC_CUDA(cudaMemcpyAsync(&exact, ooff + n, 4, cudaMemcpyDeviceToHost, s));
@@ -541,11 +543,11 @@ pc_status ensure_oriented(pc_pgraph* pg) {
     if (pg->oriented_tried) return PC_OK;
     const uint64_t n = pg->g->n;
     pg->oriented_tried = true;
-    if (n == 0 || !oriented_fits(n, pg->g->m)) return PC_OK;
+    if (n == 0 || !oriented_fits(n, pg->g->m, pg->g->checked)) return PC_OK;
     const size_t tb = oriented_temp_bytes(n);
     PC_TRY(scratch_reserve(pg, tb));
     const pc_status st =
-        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->m, pg->g->device, pg->g->stream,
+        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->m, pg->g->checked, pg->g->device, pg->g->stream,
                        pg->scratch.take<char>(tb), tb, &pg->ooff, &pg->oids, &pg->ovecs);
     if (st != PC_ERR_OOM) return st;
     pg->ooff.release();
@@ -687,6 +689,7 @@ pc_status pc_graph_create(const uint64_t* vlist, const int32_t* elist, const int
             return cleanup(fail(PC_ERR_INVALID_INPUT, "neighbour lists must be strictly ascending (sorted, no duplicates)"));
         if (h_fp[0] || h_fp[1]) return cleanup(fail(PC_ERR_INVALID_INPUT, "the adjacency is not symmetric"));
         if (h_err & BAD_WEIGHT) return cleanup(fail(PC_ERR_INVALID_INPUT, "edge weights must be in [0, 2^30)"));
+        g->checked = true;
     } else {
         e = cudaStreamSynchronize(g->stream);
         if (e != cudaSuccess) return cleanup(cuda_fail(e, "upload", __FILE__, __LINE__));

@@ -499,14 +499,13 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
     b->ntri = chk_h[1];
     if (!chk_h[0]) {
-        // the arena was checked to be symmetric, so the copy holds M / 2 ids; more
-        // than fit here do not fit the device's memory either
-        if (!oriented_fits(N, M / 2)) return bail(fail(PC_ERR_UNSUPPORTED, "the arena holds too many edges"));
+        // more than fit here do not fit the device's memory either
+        if (!oriented_fits(N, M, true)) return bail(fail(PC_ERR_UNSUPPORTED, "the arena holds too many edges"));
         DevBuf tmp;
         const size_t tb = oriented_temp_bytes(N);
         if ((st = tmp.alloc(tb, "scan scratch")) != PC_OK) return bail(st);
         st = build_oriented(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(), b->dplus.as<uint32_t>(),
-                            b->graph_of.as<int32_t>() + N, N, M, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
+                            b->graph_of.as<int32_t>() + N, N, M, true, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
         if (st != PC_OK) return bail(st);
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));

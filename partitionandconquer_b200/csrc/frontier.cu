@@ -1245,12 +1245,14 @@ static pc_status mis_run(pc_pgraph* pg, bool hashed, uint64_t seed, int32_t* res
     // first dplus[u] of a row
     const bool count_first = hashed || int2api;
     if (!count_first) PC_TRY(ensure_dplus(pg));
-    const uint64_t hcap = tx::heavy_chunks(n, m);
-    PC_TRY(scratch_reserve(pg, n * 4 * 5 + hcap * 16 + 1024));
+    // a step decides a vertex once; where an adjacency that was not checked is
+    // not symmetric, it may do so twice, as left out and as waiting for nobody
+    const uint64_t twice = pg->g->checked ? 1 : 2, lcap = twice * n, hcap = twice * tx::heavy_chunks(n, m);
+    PC_TRY(scratch_reserve(pg, n * 4 * 3 + lcap * 8 + hcap * 16 + 1024));
     int32_t* state = pg->scratch.take<int32_t>(n);
     int32_t* waits = pg->scratch.take<int32_t>(n);
     int32_t* out = pg->scratch.take<int32_t>(n);
-    tx::Queues q0{pg->scratch.take<int32_t>(n), nullptr}, q1{pg->scratch.take<int32_t>(n), nullptr};
+    tx::Queues q0{pg->scratch.take<int32_t>(lcap), nullptr}, q1{pg->scratch.take<int32_t>(lcap), nullptr};
     q0.heavy = pg->scratch.take<int2>(hcap);
     q1.heavy = pg->scratch.take<int2>(hcap);
     MisState* S = pg->scratch.take<MisState>(3);

@@ -128,6 +128,7 @@ static pc_status new_handle(uint64_t n, pc_graph** out) {
         return cuda_fail(e, "graph handle", __FILE__, __LINE__);
     }
     g->n = n;
+    g->checked = true;  // every builder writes both directions, sorted and once
     *out = g;
     return PC_OK;
 }

@@ -211,6 +211,7 @@ pc_status pc_jaccard_edges(pc_pgraph* pg, float* out) {
     DevBuf ecnt;
     uint64_t slots = 0;
     PC_TRY(tc_edge_slots(pg, &slots));
+    slots += 4;  // an edge without its twin, in an adjacency that was not checked, may have its slot past the last row
     PC_TRY(ecnt.alloc(slots * 4, "triangles per edge"));
     PC_CUDA(cudaMemsetAsync(ecnt.p, 0, slots * 4, s));
     uint64_t T = 0;

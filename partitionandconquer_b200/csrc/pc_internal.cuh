@@ -86,6 +86,7 @@ struct pc_graph {
     cudaStream_t stream = nullptr;
     uint64_t n = 0, m = 0;
     bool weighted = false;
+    bool checked = false;  // rows ascending and the adjacency symmetric: validated, or built here
     pc::DevBuf off;   // uint64 [n+1]
     pc::DevBuf adj;   // int32  [m + pad]
     pc::DevBuf w;     // int32  [m] or empty
@@ -108,9 +109,10 @@ struct pc_pgraph {
     pc::DevBuf dplus;             // uint32 [n]: |N(u) & [0,u)| (internal ids)
     // oriented copy (ensure_oriented): row u = N(u) & [0,u) in ascending order,
     // from 16-byte vector ooff[u] of oids, padded with INT_MAX to whole vectors
+    // (of a graph that was not checked, with one INT_MAX at least)
     pc::DevBuf ooff;              // uint32 [n+1]
     pc::DevBuf oids;              // int4 [ovecs + 32]; null when there was no room for it
-    uint64_t ovecs = 0;           // vectors of all rows
+    uint64_t ovecs = 0;           // vectors of all rows (a small copy's: at most)
     bool oriented_tried = false;
     pc::DevBuf unit_of;           // int32 [n]: planning unit of each vertex (tc.cu)
     pc::Scratch scratch;
@@ -167,15 +169,22 @@ int32_t to_internal_id(const pc_pgraph* pg, int32_t api_id);
 pc_status ensure_dplus(pc_pgraph* pg);
 
 // Builds the oriented copy of a CSR (see pc_pgraph::oids): row u's ids less
-// row_base[u] (none when null).  tmp: oriented_temp_bytes(n) bytes.  Waits for
-// the stream once, for the copy's size, except for a small graph, whose copy
-// gets the room that it can need at most.  Its vector indices are 32-bit:
-// oriented_fits().
+// row_base[u] (none when null).  With `checked` rows may end without an INT_MAX:
+// the scans of a symmetric adjacency stop at an id inside the row.  tmp:
+// oriented_temp_bytes(n) bytes.  Waits for the stream once, for the copy's size,
+// except for a small graph, whose copy gets the room that it can need at most.
+// Its vector indices are 32-bit: oriented_fits().
 pc_status build_oriented(const uint64_t* off, const int32_t* adj, const uint32_t* dplus, const int32_t* row_base,
-                         uint64_t n, uint64_t m, int device, cudaStream_t s, void* tmp, size_t tmp_bytes, DevBuf* ooff,
-                         DevBuf* oids, uint64_t* vecs);
+                         uint64_t n, uint64_t m, bool checked, int device, cudaStream_t s, void* tmp, size_t tmp_bytes,
+                         DevBuf* ooff, DevBuf* oids, uint64_t* vecs);
 size_t oriented_temp_bytes(uint64_t n);
-inline bool oriented_fits(uint64_t n, uint64_t m) { return (m + 3 * n) / 4 + 64 < (1ull << 32); }
+// Vectors of the copy at most (half of a symmetric adjacency's entries are in it).
+inline uint64_t oriented_most(uint64_t n, uint64_t m, bool checked) {
+    return checked ? (m / 2 + 3 * n) / 4 : m / 4 + n;
+}
+inline bool oriented_fits(uint64_t n, uint64_t m, bool checked) {
+    return oriented_most(n, m, checked) + 64 < (1ull << 32);
+}
 
 // Lazily builds the oriented copy (uses the scratch arena).  Leaves oids null,
 // without an error, when device memory does not hold it.
