@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -543,6 +544,8 @@ pc_status ensure_oriented(pc_pgraph* pg) {
     if (pg->oriented_tried) return PC_OK;
     const uint64_t n = pg->g->n;
     pg->oriented_tried = true;
+    const char* wanted = getenv("PC_ORIENTED_COPY");  // 0: count on the CSR (a switch for measurements)
+    if (wanted && atoi(wanted) == 0) return PC_OK;
     if (n == 0 || !oriented_fits(n, pg->g->m, pg->g->checked)) return PC_OK;
     const size_t tb = oriented_temp_bytes(n);
     PC_TRY(scratch_reserve(pg, tb));

@@ -162,18 +162,17 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
             flush();
             hist_base = base;
         }
-        const uint32_t v0 = A.oriented.off[I.b], v1 = A.oriented.off[I.b + 1];
+        const tc::OrientedView::Row row = A.oriented.row(I.b);
         tc::SetView S;
         S.bm = bm;
         S.lo = kLowIds;
         S.ht = ht;
         S.hpos = nullptr;
-        S.nb = reinterpret_cast<const int32_t*>(A.oriented.ids + v0);
-        S.np = 4 * (v1 - v0);
+        A.oriented.sorted(row, &S);
         S.ovf = S.np > (uint32_t)tc::kHashCap && __ldg(S.nb + (S.np - tc::kHashCap - 1)) >= kLowIds;
         bool high = false;
-        for (uint32_t k = v0 + lane; k < v1; k += 32) {
-            const int4 v = __ldg(A.oriented.ids + k);
+        for (uint32_t k = lane; k < row.n; k += 32) {
+            const int4 v = A.oriented.vector(row, k);
             const int32_t e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
@@ -200,15 +199,15 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
         for (uint32_t k = 0; k < I.n; k += 32) {
             const int nb = min(32, (int)(I.n - k));
             const int32_t c = lane < nb ? A.adj[I.in0 + k + lane] : 0;
-            hits += tc::scan_in_neighbours<4, 1, kMode, tc::kMixedSet>(A.oriented, c, A.oriented.off[c], nb, b, S, lane, sink);
+            hits += tc::scan_in_neighbours<4, 1, kMode, tc::kMixedSet>(A.oriented, c, nb, b, S, lane, sink);
         }
         for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
         if (lane == 0 && hits) {
             if (A.tc) atomicAdd(&A.tc[A.graph_of[I.b]], hits);
             if (kMode == tc::kCountVertex) atomicAdd(&A.tri[I.b], hits);
         }
-        for (uint32_t k = v0 + lane; k < v1; k += 32) {
-            const int4 v = __ldg(A.oriented.ids + k);
+        for (uint32_t k = lane; k < row.n; k += 32) {
+            const int4 v = A.oriented.vector(row, k);
             bm[S.place<tc::kMixedSet>(v.x) >> 5] = 0;
             bm[S.place<tc::kMixedSet>(v.y) >> 5] = 0;
             bm[S.place<tc::kMixedSet>(v.z) >> 5] = 0;

@@ -623,7 +623,8 @@ struct BitmapLaunch {
     unsigned grid;
     size_t smem;
     cudaStream_t s;
-    OrientedView oriented;
+    OrientedView oriented;    // ids null: scans of the CSR
+    CsrView csr;
     const int32_t* adj;
     const Item* items;
     const uint32_t* nitems;
@@ -637,38 +638,50 @@ struct BitmapLaunch {
     uint32_t* ecnt;           // per-edge counts at the oriented slots (Jaccard), or null
 };
 
-template <int K, int G, int V, int kMode, int kKind>
-static pc_status launch_bitmap_kgm(const BitmapLaunch& L) {
-    PC_CUDA(cudaFuncSetAttribute(k_tc_bitmap<K, G, V, kMode, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)L.smem));
-    k_tc_bitmap<K, G, V, kMode, kKind><<<L.grid, kCtaThreads, L.smem, L.s>>>(L.oriented, L.adj, L.items, L.nitems, L.cap, L.next,
-                                                                        L.total, L.words, L.cost, L.unit_of, L.tri,
-                                                                        L.ecnt);
+template <int K, int G, int V, int kMode, int kKind, class Rows>
+static pc_status launch_bitmap_rows(const Rows& R, const BitmapLaunch& L) {
+    auto* kernel = k_tc_bitmap<K, G, V, kMode, kKind, Rows>;
+    PC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
+    kernel<<<L.grid, kCtaThreads, L.smem, L.s>>>(R, L.adj, L.items, L.nitems, L.cap, L.next, L.total, L.words, L.cost,
+                                                 L.unit_of, L.tri, L.ecnt);
     return PC_OK;
 }
 
+// G: lanes per in-neighbour on the copy (the CSR is scanned with 4); light: one vector a step.
 template <int K, int kMode, int kKind>
-static pc_status launch_bitmap_kmode(int G, const BitmapLaunch& L) {
-    if (G == 32) return launch_bitmap_kgm<K, 32, 1, kMode, kKind>(L);
-    if (G == 8) return launch_bitmap_kgm<K, 4, kMode == kCountEdge ? 1 : 2, kMode, kKind>(L);
-    return launch_bitmap_kgm<K, 1, 1, kMode, kKind>(L);
+static pc_status launch_bitmap_kmode(int G, bool light, const BitmapLaunch& L) {
+    constexpr int V = kMode == kCountEdge ? 1 : 2;
+    if (light) {
+        if constexpr (K == 1 && kKind == kMixedSet) {
+            if (!L.oriented.ids) return launch_bitmap_rows<1, 4, 1, kMode, kMixedSet>(L.csr, L);
+            return launch_bitmap_rows<1, 4, 1, kMode, kMixedSet>(L.oriented, L);
+        }
+        return fail(PC_ERR_UNSUPPORTED, "light pivot sets: unexpected launch shape");
+    }
+    if constexpr (!(K == 1 && kKind == kMixedSet)) {
+        if (!L.oriented.ids) return launch_bitmap_rows<K, 4, V, kMode, kKind>(L.csr, L);
+        if (G == 32) return launch_bitmap_rows<K, 32, 1, kMode, kKind>(L.oriented, L);
+        if (G == 8) return launch_bitmap_rows<K, 4, V, kMode, kKind>(L.oriented, L);
+        return launch_bitmap_rows<K, 1, 1, kMode, kKind>(L.oriented, L);
+    }
+    return fail(PC_ERR_UNSUPPORTED, "mixed pivot sets: unexpected launch shape");
 }
 
 template <int K>
 static pc_status launch_bitmap_k(int G, const BitmapLaunch& L) {
-    if (L.tri) return launch_bitmap_kmode<K, kCountVertex, kPlainSet>(G, L);
-    if (L.ecnt) return launch_bitmap_kmode<K, kCountEdge, kPlainSet>(G, L);
-    return launch_bitmap_kmode<K, kCountOnly, kPlainSet>(G, L);
+    if (L.tri) return launch_bitmap_kmode<K, kCountVertex, kPlainSet>(G, false, L);
+    if (L.ecnt) return launch_bitmap_kmode<K, kCountEdge, kPlainSet>(G, false, L);
+    return launch_bitmap_kmode<K, kCountOnly, kPlainSet>(G, false, L);
 }
 
 static pc_status launch_bitmap(int K, int G, int kind, const BitmapLaunch& L) {
-    if (kind == kMixedSet) {  // fixed-size sets (mixed_shape)
-        if (K == 1 && L.ecnt) return launch_bitmap_kgm<1, 4, 1, kCountEdge, kMixedSet>(L);
-        if (K == 1 && L.tri) return launch_bitmap_kgm<1, 4, 1, kCountVertex, kMixedSet>(L);
-        if (K == 1) return launch_bitmap_kgm<1, 4, 1, kCountOnly, kMixedSet>(L);
+    if (kind == kMixedSet) {  // fixed-size sets (mixed_shape): light pivots with a set per warp
+        if (K == 1 && L.ecnt) return launch_bitmap_kmode<1, kCountEdge, kMixedSet>(G, true, L);
+        if (K == 1 && L.tri) return launch_bitmap_kmode<1, kCountVertex, kMixedSet>(G, true, L);
+        if (K == 1) return launch_bitmap_kmode<1, kCountOnly, kMixedSet>(G, true, L);
         if (L.ecnt || K != 2) return fail(PC_ERR_UNSUPPORTED, "mixed pivot sets: unexpected launch shape");
-        if (L.tri) return launch_bitmap_kmode<2, kCountVertex, kMixedSet>(G, L);
-        return launch_bitmap_kmode<2, kCountOnly, kMixedSet>(G, L);
+        if (L.tri) return launch_bitmap_kmode<2, kCountVertex, kMixedSet>(G, false, L);
+        return launch_bitmap_kmode<2, kCountOnly, kMixedSet>(G, false, L);
     }
     switch (K) {
         case 1: return launch_bitmap_k<1>(G, L);
@@ -678,7 +691,6 @@ static pc_status launch_bitmap(int K, int G, int kind, const BitmapLaunch& L) {
         default: return launch_bitmap_k<16>(G, L);
     }
 }
-
 
 }  // namespace tc
 
@@ -873,6 +885,7 @@ static pc_status run_items(pc_pgraph* pg, const LaunchGroup& gr, unsigned long l
         L.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * sh.ctas_per_sm, gr.item_bound));
         L.s = s;
         L.oriented = OrientedView{pg->ooff.as<uint32_t>(), pg->oids.as<int4>()};
+        L.csr = CsrView{pg->off, pg->adj, dp, 0};
         L.adj = pg->adj;
         L.items = d_items;
         L.nitems = d_nitems;
@@ -933,9 +946,8 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     std::vector<LaunchGroup> groups(PC_NUM_VARIANTS * (kClasses + 1));
     std::vector<int> group_of(U, -1);
     for (size_t u = 0; u < U; ++u) {
-        int v = assign[u];
+        const int v = assign[u];
         if (v < 0) continue;
-        if ((is_bitmap(v) || v == PC_VARIANT_HASH_WARP) && !pg->oids.p) v = PC_VARIANT_MERGE_LANE;  // no room for the oriented copy
         const uint32_t mid = (uint32_t)feat[u * kNumFeatures + 4];
         auto bitmap_class = [&]() {
             const uint32_t w = std::max<uint32_t>(1, (mid + 31) / 32);
@@ -971,7 +983,7 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         if (!tail) {
             gr.tails.emplace_back();
             tail = &gr.tails.back();
-            tail->v = pg->oids.p ? PC_VARIANT_BITMAP_GROUP8 : PC_VARIANT_MERGE_LANE;
+            tail->v = PC_VARIANT_BITMAP_GROUP8;
             tail->words = 1u << tc;
             tail->c_min = kMatrixFrom;
         }

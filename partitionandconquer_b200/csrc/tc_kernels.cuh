@@ -90,7 +90,8 @@ struct SetView {
     int32_t lo;                      // kMixedSet
     const int32_t* ht;               // kHashSlots slots, -1 = empty
     const uint16_t* hpos;            // per-edge counts: the rank of each slot's key
-    const int32_t* __restrict__ nb;  // N+(b), padded with INT_MAX to np entries (overflow path)
+    const int32_t* __restrict__ nb;  // N+(b) + base, np entries with the copy's padding (overflow path)
+    int32_t base;
     uint32_t np;
     bool ovf;
     // the bit an id is tested at
@@ -105,10 +106,10 @@ struct SetView {
             uint32_t lo = 0, hi = np;
             while (lo < hi) {
                 const uint32_t mid = (lo + hi) >> 1;
-                if (__ldg(nb + mid) < a) lo = mid + 1; else hi = mid;
+                if (__ldg(nb + mid) - base < a) lo = mid + 1; else hi = mid;
             }
             *rank = lo;
-            return lo < np && __ldg(nb + lo) == a;
+            return lo < np && __ldg(nb + lo) - base == a;
         }
         uint32_t s = hash_slot(a);
         for (int32_t key; (key = ht[s]) != -1; s = (s + 1) & (kHashSlots - 1))
@@ -155,13 +156,66 @@ __device__ __forceinline__ void count_vertex(int32_t a, unsigned long long* __re
 // {x, y}, y < x, is the position of y in row x of the oriented copy.
 enum CountMode { kCountOnly = 0, kCountVertex = 1, kCountEdge = 2 };
 
-// The oriented copy of the graph the bitmap kernels scan (Oriented in
-// tc.cu): row x holds N+(x) in ascending order, starts at 16-byte vector
-// off[x] of ids and is padded with INT_MAX to whole vectors; at least 32 vectors of
-// INT_MAX follow the last row.
+// The rows N+(x) that the set kernels scan.
+//
+// OrientedView is the oriented copy (build_oriented): row x holds N+(x) in
+// ascending order, starts at 16-byte vector off[x] of ids and is padded with
+// INT_MAX to whole vectors; at least 32 vectors of INT_MAX follow the last row.
+//
+// CsrView is the CSR itself, for graphs whose copy has no room: the vectors that
+// hold a row begin up to 3 ids before it and end after it, so every id's place is
+// compared with the row's bounds.  With groups of 4 lanes only.
 struct OrientedView {
+    static constexpr bool kCsr = false;
+    using Pos = uint32_t;
     const uint32_t* __restrict__ off;
     const int4* __restrict__ ids;
+    // a row as a pivot set: n vectors from v0, the k-th of them, the id before
+    // it, all as a sorted array, and the slot of the first id
+    struct Row {
+        uint32_t v0, n;
+    };
+    __device__ __forceinline__ Row row(int32_t b) const { return Row{off[b], off[b + 1] - off[b]}; }
+    __device__ __forceinline__ int4 vector(const Row& r, uint32_t k) const { return __ldg(ids + (r.v0 + k)); }
+    __device__ __forceinline__ int32_t before(const Row& r, uint32_t k) const { return __ldg(&ids[r.v0 + k - 1].w); }
+    __device__ __forceinline__ void sorted(const Row& r, SetView* S) const {
+        S->nb = reinterpret_cast<const int32_t*>(ids + r.v0);
+        S->np = 4 * r.n;
+        S->base = 0;
+    }
+    __device__ __forceinline__ uint64_t slot(const Row& r) const { return 4ull * r.v0; }
+};
+
+struct CsrView {
+    static constexpr bool kCsr = true;
+    using Pos = uint64_t;
+    const uint64_t* __restrict__ off;
+    const int32_t* __restrict__ adj;
+    const uint32_t* __restrict__ dplus;
+    int32_t base;  // subtracted from the ids
+    struct Row {
+        uint64_t e0;
+        uint32_t n, len;  // n vectors for len entries
+    };
+    __device__ __forceinline__ Row row(int32_t b) const { return Row{off[b], (dplus[b] + 3) / 4, dplus[b]}; }
+    __device__ __forceinline__ int4 vector(const Row& r, uint32_t k) const {
+        const int32_t* p = adj + r.e0 + 4ull * k;
+        const uint32_t left = r.len - 4 * k;
+        int4 v = make_int4(__ldg(p) - base, INT32_MAX, INT32_MAX, INT32_MAX);
+        if (left > 1) v.y = __ldg(p + 1) - base;
+        if (left > 2) v.z = __ldg(p + 2) - base;
+        if (left > 3) v.w = __ldg(p + 3) - base;
+        return v;
+    }
+    __device__ __forceinline__ int32_t before(const Row& r, uint32_t k) const {
+        return __ldg(adj + r.e0 + 4ull * k - 1) - base;
+    }
+    __device__ __forceinline__ void sorted(const Row& r, SetView* S) const {
+        S->nb = adj + r.e0;
+        S->np = r.len;
+        S->base = base;
+    }
+    __device__ __forceinline__ uint64_t slot(const Row& r) const { return r.e0; }
 };
 
 // Ranks in a pivot set (per-edge counts): r16[w] is the rank, modulo 2^16, of
@@ -215,23 +269,54 @@ struct HitSink {
 // first unit's tail with its matrix part 8.3 / 8.0 / 7.4 / 8.4 / 7.0; RMAT-20's
 // light pivots, ER-20: 0.98 / 0.83 / 1.01 / 1.41 / 0.95.  So bitmap sets scan with
 // (4, 2), light pivots with (4, 1).
-template <int G, int V, int kMode, int kKind>
-__device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, int32_t c, uint32_t start, int nb,
-                                                       int32_t b, const SetView& S, int lane,
-                                                       const HitSink& sink) {
+//
+// On the CSR (CsrView) a step also masks the ids outside the row, and rows start
+// anywhere in a sector: counts of RMAT-24 / 22 / 20 / 16 take 35.0 / 6.2 / 1.83 /
+// 0.16 ms, on the copy 24.9 / 4.3 / 0.99 / 0.12.
+template <int G, int V, int kMode, int kKind, class Rows>
+__device__ __forceinline__ uint32_t scan_in_neighbours(const Rows& R, int32_t c, int nb, int32_t b, const SetView& S,
+                                                       int lane, const HitSink& sink) {
+    constexpr bool kCsr = Rows::kCsr;
+    using Pos = typename Rows::Pos;
+    static_assert(!kCsr || G == 4, "scans of the CSR take groups of 4 lanes");
     constexpr int NG = 32 / G;
     const int gl = lane % G;
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
     const unsigned below = gmask & ((1u << lane) - 1u);
     const int4 none = make_int4(INT32_MAX, INT32_MAX, INT32_MAX, INT32_MAX);
     int j = lane / G;
-    uint32_t q = __shfl_sync(0xffffffffu, start, j) + gl;
+    // the row starts: vectors of the copy, entries of the CSR (with the rows' lengths)
+    const Pos start = R.off[c];
+    uint32_t len = 0;
+    if constexpr (kCsr) len = R.dplus[c];
+    Pos e0 = __shfl_sync(0xffffffffu, start, j), e1 = 0;  // CSR: the current row's entries are [e0, e1)
+    Pos q = (kCsr ? e0 / 4 : e0) + gl;
+    if constexpr (kCsr) e1 = e0 + __shfl_sync(0xffffffffu, len, j);
     bool act = j < nb;
     int4 v[V];
+    auto load = [&](int i) {
+        if constexpr (kCsr) return act && 4 * (q + i * G) < e1 ? __ldg(reinterpret_cast<const int4*>(R.adj) + q + i * G) : none;
+        else return act ? __ldg(R.ids + q + i * G) : none;
+    };
 #pragma unroll
-    for (int i = 0; i < V; ++i) v[i] = act ? __ldg(O.ids + q + i * G) : none;
+    for (int i = 0; i < V; ++i) v[i] = load(i);
     uint32_t cnt = 0, pair = 0;
     while (__any_sync(0xffffffffu, act)) {
+        // CSR: ids before the row become the smallest id, those after it the
+        // largest; lead ids of the vector are before it (0 to 3)
+        int lead[kCsr ? V : 1];
+        if constexpr (kCsr) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const Pos p = 4 * (q + i * G);
+                lead[i] = act && p < e0 ? (int)(e0 - p) : 0;
+                const int end = act && p < e1 ? (int)min(e1 - p, (Pos)4) : 0;
+                v[i].x = lead[i] > 0 ? INT32_MIN : (end > 0 ? v[i].x - R.base : INT32_MAX);
+                v[i].y = lead[i] > 1 ? INT32_MIN : (end > 1 ? v[i].y - R.base : INT32_MAX);
+                v[i].z = lead[i] > 2 ? INT32_MIN : (end > 2 ? v[i].z - R.base : INT32_MAX);
+                v[i].w = end > 3 ? v[i].w - R.base : INT32_MAX;
+            }
+        }
         // vector i of the group's lanes precedes vector i + 1: the row's stop is
         // the lowest lane of the first vector that has one
         unsigned stop[V];
@@ -246,22 +331,34 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
             a[i] = v[i];
             if (past[i]) a[i].x = INT32_MAX;
         }
-        const uint32_t qc = q;
+        const Pos qc = q;
         const int jc = j;
         if (done) j += NG;
-        const uint32_t s = __shfl_sync(0xffffffffu, start, j & 31);
-        q = done ? s + gl : q + V * G;
+        const Pos s = __shfl_sync(0xffffffffu, start, j & 31);
+        q = done ? (kCsr ? s / 4 : s) + gl : q + V * G;
+        if constexpr (kCsr) {
+            const uint32_t l = __shfl_sync(0xffffffffu, len, j & 31);
+            if (done) {
+                e0 = s;
+                e1 = s + l;
+            }
+        }
         const bool had = act;
         act = j < nb;
 #pragma unroll
-        for (int i = 0; i < V; ++i) v[i] = act ? __ldg(O.ids + q + i * G) : none;
+        for (int i = 0; i < V; ++i) v[i] = load(i);
         uint32_t hits = 0;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
             a[i].y = max(a[i].x, a[i].y);
             a[i].z = max(a[i].y, a[i].z);
             a[i].w = max(a[i].z, a[i].w);
-            const int32_t e[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+            int32_t e[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+            if constexpr (kCsr) {
+#pragma unroll
+                for (int t = 0; t < 3; ++t)
+                    if (t < lead[i]) e[t] = INT32_MAX;
+            }
             uint32_t h[4];
             uint32_t rank[4];  // kMixedSet with lo = 0: of the hits
 #pragma unroll
@@ -315,10 +412,10 @@ __device__ __forceinline__ uint32_t scan_in_neighbours(const OrientedView& O, in
 
 // CTAs per SM a bitmap kernel's registers leave room for.  Three for the count;
 // two for split sets with two vectors a step, whose look-ups spill at 40
-// registers (RMAT-24's unit of ids 65-82 K: 1.10 ms, 1.28 with three), and for the
-// other modes.
-constexpr int bitmap_ctas(int V, int mode, int kind) {
-    return mode == kCountOnly && !(kind == kMixedSet && V > 1) ? 3 : 2;
+// registers (RMAT-24's unit of ids 65-82 K: 1.10 ms, 1.28 with three), for scans of
+// the CSR with two vectors a step, which spill too, and for the other modes.
+constexpr int bitmap_ctas(int V, int mode, int kind, bool csr) {
+    return mode == kCountOnly && !((kind == kMixedSet || csr) && V > 1) ? 3 : 2;
 }
 
 // Bitmap kernel: a CTA of kCtaThreads threads holds 16/K pivot sets in
@@ -330,9 +427,9 @@ constexpr int bitmap_ctas(int V, int mode, int kind) {
 // Mixed sets have (bm_words - kFilterWords) * 32 = lo bits for the low ids,
 // whatever the pivots' ids (0 in the per-edge mode, which needs every hit's
 // rank).
-template <int K, int G, int V, int kMode, int kKind>
-__global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
-    k_tc_bitmap(OrientedView O, const int32_t* __restrict__ adj, const Item* __restrict__ items,
+template <int K, int G, int V, int kMode, int kKind, class Rows>
+__global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind, Rows::kCsr))
+    k_tc_bitmap(Rows R, const int32_t* __restrict__ adj, const Item* __restrict__ items,
                 const uint32_t* __restrict__ nitems_p, uint32_t cap, uint32_t* __restrict__ next_item,
                 unsigned long long* __restrict__ total, uint32_t bm_words, unsigned long long* __restrict__ unit_cost,
                 const int32_t* __restrict__ unit_of, unsigned long long* __restrict__ tri,
@@ -374,24 +471,23 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
         const long long t0 = unit_cost ? clock64() : 0;
         const Item I = items[it];
         const int32_t b = I.b;
-        const uint32_t v0 = O.off[b], v1 = O.off[b + 1];
+        const typename Rows::Row row = R.row(b);
         SetView S;
         S.bm = bm;
         S.lo = lo;
         S.ht = ht;
         S.hpos = kHash && kMode == kCountEdge ? r16 : nullptr;
-        S.nb = reinterpret_cast<const int32_t*>(O.ids + v0);
-        S.np = 4 * (v1 - v0);
+        R.sorted(row, &S);
         // the hash takes ranks np - kHashCap and up: all high ids, or it is not used
-        S.ovf = kHash && S.np > (uint32_t)kHashCap && __ldg(S.nb + (S.np - kHashCap - 1)) >= lo;
-        for (uint32_t k = v0 + tis; k < v1; k += set_threads) {
-            const int4 v = __ldg(O.ids + k);
+        S.ovf = kHash && S.np > (uint32_t)kHashCap && __ldg(S.nb + (S.np - kHashCap - 1)) - S.base >= lo;
+        for (uint32_t k = tis; k < row.n; k += set_threads) {
+            const int4 v = R.vector(row, k);
             const int32_t e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const int32_t a = e[t];
                 if (a == INT32_MAX) continue;  // padding
-                const uint32_t rank = 4 * (k - v0) + t;
+                const uint32_t rank = 4 * k + t;
                 const uint32_t x = S.place<kKind>(a);
                 atomicOr(&bm[x >> 5], 0x80000000u >> (x & 31));
                 if (kHash && !S.ovf && a >= lo) {
@@ -401,7 +497,7 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
                     if (kMode == kCountEdge) r16[hs] = (uint16_t)rank;
                 }
                 if (kMode == kCountEdge && kKind == kPlainSet) {
-                    const int32_t prev = t ? e[t - 1] : (k > v0 ? __ldg(&O.ids[k - 1].w) : -1);
+                    const int32_t prev = t ? e[t - 1] : (k ? R.before(row, k) : -1);
                     if (prev < 0 || (prev >> 5) != (a >> 5)) r16[a >> 5] = (uint16_t)rank;
                     if (prev < 0 || (prev >> 11) != (a >> 11)) r32[a >> 11] = rank;
                 }
@@ -414,14 +510,13 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
         sink.hist = hist;
         sink.hist_ids = kHubHist;
         sink.ecnt = ecnt;
-        sink.by_rank = few ? by_rank : ecnt + 4ull * v0;
+        sink.by_rank = few ? by_rank : ecnt + R.slot(row);
         sink.ranks = SetRanks{r16, r32};
         const unsigned long long cnt0 = cnt;
         for (uint32_t k = wi * 32; k < I.n; k += set_threads) {
             const int nb = min(32, (int)(I.n - k));
             const int32_t c = lane < nb ? adj[I.in0 + k + lane] : 0;
-            const uint32_t start = O.off[c];
-            cnt += scan_in_neighbours<G, V, kMode, kKind>(O, c, start, nb, b, S, lane, sink);
+            cnt += scan_in_neighbours<G, V, kMode, kKind>(R, c, nb, b, S, lane, sink);
         }
         if (kMode == kCountVertex) {
             unsigned long long hb = cnt - cnt0;  // this item's triangles at pivot b
@@ -429,17 +524,17 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind))
             if (lane == 0 && hb) atomicAdd(&tri[b], hb);
         }
         set_sync();
-        for (uint32_t k = v0 + tis; k < v1; k += set_threads) {
-            const int4 v = __ldg(O.ids + k);
+        for (uint32_t k = tis; k < row.n; k += set_threads) {
+            const int4 v = R.vector(row, k);
             const int32_t e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 if (kHash || e[t] != INT32_MAX) bm[S.place<kKind>(e[t]) >> 5] = 0;
                 if (kMode == kCountEdge && few) {
-                    const uint32_t h = by_rank[4 * (k - v0) + t];
+                    const uint32_t h = by_rank[4 * k + t];
                     if (h) {
-                        atomicAdd(ecnt + (4ull * k + t), h);
-                        by_rank[4 * (k - v0) + t] = 0;
+                        atomicAdd(ecnt + (R.slot(row) + 4 * k + t), h);
+                        by_rank[4 * k + t] = 0;
                     }
                 }
             }
