@@ -60,11 +60,38 @@ static cudaError_t prepare_pool(int dev) {
     return e;
 }
 
+// Bytes of each device that DevBufs hold, and the most they may hold:
+// PC_MEMORY_LIMIT_MB from the environment (read at every allocation), else what
+// the device has.
+constexpr int kMaxDevices = 64;
+static std::atomic<uint64_t> g_held[kMaxDevices];
+
+static std::atomic<uint64_t>& held(int dev) { return g_held[dev < kMaxDevices ? dev : kMaxDevices - 1]; }
+
+static uint64_t memory_limit() {
+    const char* e = getenv("PC_MEMORY_LIMIT_MB");
+    return e ? (uint64_t)(std::max(0.0, atof(e)) * 1048576.0) : ~0ull;
+}
+
+uint64_t available_bytes(int device) {
+    size_t room = 0, all = 0;
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemGetInfo(&room, &all) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        room += reserved > used ? reserved - used : 0;
+    else cudaGetLastError();
+    const uint64_t limit = memory_limit(), have = held(device).load();
+    return std::min<uint64_t>(room, limit > have ? limit - have : 0);
+}
+
 pc_status DevBuf::alloc(size_t nbytes, const char* what) {
     release();
     if (nbytes == 0) return PC_OK;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = prepare_pool(dev);
+    if (e == cudaSuccess && held(dev).load() + nbytes > memory_limit()) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) e = cudaMallocAsync(&p, nbytes, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) {
@@ -75,6 +102,7 @@ pc_status DevBuf::alloc(size_t nbytes, const char* what) {
         return fail(e == cudaErrorMemoryAllocation ? PC_ERR_OOM : PC_ERR_CUDA, buf);
     }
     bytes = nbytes;
+    held(dev) += nbytes;
     return PC_OK;
 }
 pc_status DevBuf::ensure(size_t nbytes, const char* what) {
@@ -89,6 +117,7 @@ void DevBuf::release() {
         cudaDeviceSynchronize();
         cudaFreeAsync(p, 0);
         cudaStreamSynchronize(0);
+        held(dev) -= bytes;
         if (cur != dev && cur >= 0) cudaSetDevice(cur);
     }
     p = nullptr;
@@ -101,6 +130,7 @@ void DevBuf::release_idle() {
         cudaGetDevice(&cur);
         if (cur != dev) cudaSetDevice(dev);
         cudaFreeAsync(p, 0);
+        held(dev) -= bytes;
         if (cur != dev && cur >= 0) cudaSetDevice(cur);
     }
     p = nullptr;
@@ -541,22 +571,39 @@ size_t oriented_temp_bytes(uint64_t n) {
 
 pc_status ensure_oriented(pc_pgraph* pg) {
     PC_TRY(ensure_dplus(pg));
-    if (pg->oriented_tried) return PC_OK;
-    const uint64_t n = pg->g->n;
-    pg->oriented_tried = true;
+    if (pg->oids.p) return PC_OK;
+    const uint64_t n = pg->g->n, m = pg->g->m;
     const char* wanted = getenv("PC_ORIENTED_COPY");  // 0: count on the CSR (a switch for measurements)
-    if (wanted && atoi(wanted) == 0) return PC_OK;
-    if (n == 0 || !oriented_fits(n, pg->g->m, pg->g->checked)) return PC_OK;
+    if (n == 0 || !oriented_fits(n, m, pg->g->checked) || (wanted && atoi(wanted) == 0)) return PC_OK;
+    // A large copy is built only where as much again stays free, for the calls'
+    // temporaries and for other handles (the CSR's scans take 1.4 times as long,
+    // a call without memory fails); a small one whenever it fits.
+    const uint64_t bytes = oriented_most(n, m, pg->g->checked) * 16 + (n + 1) * 4;
+    const uint64_t from = std::max<uint64_t>(pg->oriented_from, bytes > (256ull << 20) ? 2 * bytes : 0);
+    if (from && available_bytes(pg->g->device) < from) return PC_OK;
     const size_t tb = oriented_temp_bytes(n);
-    PC_TRY(scratch_reserve(pg, tb));
-    const pc_status st =
-        build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, pg->g->m, pg->g->checked, pg->g->device, pg->g->stream,
-                       pg->scratch.take<char>(tb), tb, &pg->ooff, &pg->oids, &pg->ovecs);
-    if (st != PC_ERR_OOM) return st;
+    pc_status st = scratch_reserve(pg, tb);
+    if (st == PC_OK)
+        st = build_oriented(pg->off, pg->adj, pg->dplus.as<uint32_t>(), nullptr, n, m, pg->g->checked, pg->g->device,
+                            pg->g->stream, pg->scratch.take<char>(tb), tb, &pg->ooff, &pg->oids, &pg->ovecs);
+    if (st == PC_OK) return PC_OK;
+    PC_CUDA(cudaStreamSynchronize(pg->g->stream));
     pg->ooff.release();
     pg->oids.release();
+    if (st != PC_ERR_OOM) return st;
+    pg->oriented_from = available_bytes(pg->g->device) + bytes / 4;
     clear_error();
     return PC_OK;
+}
+
+bool release_oriented(pc_pgraph* pg) {
+    if (!pg->oids.p || cudaStreamSynchronize(pg->g->stream) != cudaSuccess) return false;
+    const uint64_t bytes = pg->oids.bytes;
+    pg->ooff.release();
+    pg->oids.release();
+    // not again until there is more room than now, without it
+    pg->oriented_from = available_bytes(pg->g->device) + bytes / 4;
+    return true;
 }
 
 }  // namespace pc
@@ -867,10 +914,7 @@ pc_status pc_pgraph_vertex_map(const pc_pgraph* pg, int32_t* old2new) {
     return PC_OK;
 }
 
-pc_status pc_pgraph_layout(pc_pgraph* pg, uint64_t* vlist, int32_t* elist, int32_t* weights) {
-    clear_error();
-    if (!pg || !vlist || (pg->g->m && !elist)) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    PC_TRY(use_device(pg->g));
+static pc_status layout_run(pc_pgraph* pg, uint64_t* vlist, int32_t* elist, int32_t* weights) {
     const uint64_t n = pg->g->n, m = pg->g->m, PN = (uint64_t)pg->P * n;
     if (PN > (1ull << 31)) return fail(PC_ERR_INVALID_INPUT, "P*n too large for a materialised layout (limit 2^31)");
     if (n == 0) {
@@ -904,6 +948,13 @@ pc_status pc_pgraph_layout(pc_pgraph* pg, uint64_t* vlist, int32_t* elist, int32
     if (m) PC_CUDA(cudaMemcpyAsync(elist, oe, m * 4, cudaMemcpyDeviceToHost, s));
     if (want_w && m) PC_CUDA(cudaMemcpyAsync(weights, ow, m * 4, cudaMemcpyDeviceToHost, s));
     return sync(pg);
+}
+
+pc_status pc_pgraph_layout(pc_pgraph* pg, uint64_t* vlist, int32_t* elist, int32_t* weights) {
+    clear_error();
+    if (!pg || !vlist || (pg->g->m && !elist)) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return layout_run(pg, vlist, elist, weights); });
 }
 
 pc_status pc_pgraph_evaluate(pc_pgraph* pg, int64_t* max_part_deg, int64_t* max_deg, double* balance_ratio) {

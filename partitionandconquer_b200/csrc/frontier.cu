@@ -1287,37 +1287,9 @@ static pc_status mis_run(pc_pgraph* pg, bool hashed, uint64_t seed, int32_t* res
     return PC_OK;
 }
 
-}  // namespace pc
-
-using namespace pc;
-
-extern "C" {
-
-pc_status pc_bfs(pc_pgraph* pg, int32_t src, int32_t* rank) {
-    clear_error();
-    if (!pg || !rank) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    const uint64_t n = pg->g->n;
-    if (src < 0 || (uint64_t)src >= n) return fail(PC_ERR_INVALID_INPUT, "source vertex out of range");
-    PC_TRY(use_device(pg->g));
-    return bfs_run(pg, to_internal_id(pg, src), rank);
-}
-
-pc_status pc_sssp(pc_pgraph* pg, int32_t src, int32_t* dist_host) {
-    return pc_sssp_ex(pg, src, PC_SSSP_AUTO, 0, dist_host);
-}
-
-pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, int32_t* dist_host) {
-    clear_error();
-    if (!pg || !dist_host) return fail(PC_ERR_INVALID_INPUT, "null argument");
+static pc_status sssp_run(pc_pgraph* pg, int32_t isrc, int32_t method, int32_t delta, int32_t* dist_host) {
     const uint64_t n = pg->g->n, m = pg->g->m;
-    if (!pg->w) return fail(PC_ERR_INVALID_INPUT, "SSSP needs a weighted graph");
-    if (src < 0 || (uint64_t)src >= n) return fail(PC_ERR_INVALID_INPUT, "source vertex out of range");
-    if (method != PC_SSSP_AUTO && method != PC_SSSP_BELLMAN_FORD && method != PC_SSSP_DELTA_STEPPING)
-        return fail(PC_ERR_INVALID_INPUT, "unknown SSSP method");
-    if (delta < 0) return fail(PC_ERR_INVALID_INPUT, "delta must be >= 0 (0: chosen from the graph)");
-    PC_TRY(use_device(pg->g));
     const bool use_delta = method != PC_SSSP_BELLMAN_FORD;
-    const int32_t isrc = to_internal_id(pg, src);
     cudaStream_t s = pg->g->stream;
     const uint64_t hcap = tx::heavy_chunks(n, m);
     PC_TRY(scratch_reserve(pg, n * 4 * 8 + hcap * 16 + 1024));
@@ -1371,63 +1343,6 @@ pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, 
     return PC_OK;
 }
 
-pc_status pc_pagerank(pc_pgraph* pg, float damping, int32_t iterations, const float* init, float* out) {
-    clear_error();
-    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    if (iterations <= 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be positive");
-    if (!(damping > 0.f && damping <= 1.f)) return fail(PC_ERR_INVALID_INPUT, "damping must be in (0, 1]");
-    PC_TRY(use_device(pg->g));
-    return pagerank_run<float>(pg, damping, iterations, init, out);
-}
-
-pc_status pc_pagerank_f64(pc_pgraph* pg, double damping, int32_t iterations, const double* init, double* out) {
-    clear_error();
-    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    if (iterations <= 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be positive");
-    if (!(damping > 0.0 && damping <= 1.0)) return fail(PC_ERR_INVALID_INPUT, "damping must be in (0, 1]");
-    PC_TRY(use_device(pg->g));
-    return pagerank_run<double>(pg, damping, iterations, init, out);
-}
-
-pc_status pc_selftest_grid_barrier(int32_t device, int32_t rounds, int32_t absent_cta, uint32_t limit_ms,
-                                   uint32_t* mismatches) {
-    clear_error();
-    if (rounds < 0 || !mismatches || limit_ms == 0) return fail(PC_ERR_INVALID_INPUT, "bad argument");
-    PC_TRY(pc_set_device(device));
-    int per_sm = 0;
-    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grid_sync_selftest, kThreads, 0));
-    if (per_sm < 1) return fail(PC_ERR_CUDA, "self-test kernel cannot be resident");
-    const int grid = sm_count(device) * std::min(per_sm, 2);
-    if (absent_cta >= grid) return fail(PC_ERR_INVALID_INPUT, "absent_cta is outside the grid");
-    cudaStream_t s = nullptr;
-    PC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    DevBuf buf;
-    pc_status st = buf.alloc(sizeof(GridBarrier) + 16, "self-test state");
-    if (st != PC_OK) {
-        cudaStreamDestroy(s);
-        return st;
-    }
-    GridBarrier* gb = buf.as<GridBarrier>();
-    unsigned* tally = reinterpret_cast<unsigned*>(gb + 1);
-    unsigned* bad = tally + 1;
-    uint64_t limit_ns = (uint64_t)limit_ms * 1000000ull;
-    void* args[] = {(void*)&gb, (void*)&rounds, (void*)&absent_cta, (void*)&limit_ns, (void*)&tally, (void*)&bad};
-    GridBarrier hb{};
-    unsigned hbad = 0;
-    cudaError_t e = cudaMemsetAsync(buf.p, 0, sizeof(GridBarrier) + 16, s);
-    if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel((const void*)k_grid_sync_selftest, dim3(grid), dim3(kThreads), args, 0, s);
-    count_launch();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-    if (e != cudaSuccess) return cuda_fail(e, "grid barrier self-test", __FILE__, __LINE__);
-    *mismatches = hbad;
-    if (hb.err) return fail(PC_ERR_TIMEOUT, "grid barrier: a wait ran out of time");
-    return PC_OK;
-}
-
 // Row entries of a CTA's local queue above which the queue goes to the next
 // step's frontier (shared by every CTA): kLocalEdges, or PC_KCORE_LOCAL_EDGES
 // from the environment (read once; a switch for measurements).
@@ -1440,16 +1355,9 @@ static uint32_t kcore_local_edges() {
     return v;
 }
 
-pc_status pc_kcore(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
-    clear_error();
-    if (!pg || !core_host) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    PC_TRY(use_device(pg->g));
+static pc_status kcore_run(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
     const uint64_t n = pg->g->n;
     cudaStream_t s = pg->g->stream;
-    if (n == 0) {
-        if (largest) *largest = 0;
-        return PC_OK;
-    }
     const uint64_t hcap = tx::heavy_chunks(n, pg->g->m);
     PC_TRY(scratch_reserve(pg, n * 4 * 7 + hcap * 16 + 1024));
     int32_t* deg = pg->scratch.take<int32_t>(n);
@@ -1505,29 +1413,8 @@ pc_status pc_kcore(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
     return PC_OK;
 }
 
-pc_status pc_mis(pc_pgraph* pg, int32_t* res) {
-    clear_error();
-    if (!pg || !res) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    PC_TRY(use_device(pg->g));
-    if (pg->g->n == 0) return PC_OK;
-    return mis_run(pg, false, 0, res);
-}
-
-pc_status pc_mis_hashed(pc_pgraph* pg, uint64_t seed, int32_t* res) {
-    clear_error();
-    if (!pg || !res) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    PC_TRY(use_device(pg->g));
-    if (pg->g->n == 0) return PC_OK;
-    return mis_run(pg, true, seed, res);
-}
-
-pc_status pc_cdlp(pc_pgraph* pg, int32_t iterations, int32_t* labels) {
-    clear_error();
-    if (!pg || !labels) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    if (iterations < 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be non-negative");
-    PC_TRY(use_device(pg->g));
+static pc_status cdlp_run(pc_pgraph* pg, int32_t iterations, int32_t* labels) {
     const uint64_t n = pg->g->n;
-    if (n == 0 || iterations == 0) return PC_OK;
     cudaStream_t s = pg->g->stream;
     PC_TRY(scratch_reserve(pg, n * 4 * 3 + pull_rows_bytes(n, pg->g->m)));
     int32_t* a = pg->scratch.take<int32_t>(n);
@@ -1547,6 +1434,132 @@ pc_status pc_cdlp(pc_pgraph* pg, int32_t iterations, int32_t* labels) {
     else PC_TRY(gather_to_api_i32(pg, a, c));
     PC_CUDA(cudaMemcpyAsync(labels, c, n * 4, cudaMemcpyDeviceToHost, s));
     return sync(pg);
+}
+
+}  // namespace pc
+
+using namespace pc;
+
+extern "C" {
+
+pc_status pc_bfs(pc_pgraph* pg, int32_t src, int32_t* rank) {
+    clear_error();
+    if (!pg || !rank) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    const uint64_t n = pg->g->n;
+    if (src < 0 || (uint64_t)src >= n) return fail(PC_ERR_INVALID_INPUT, "source vertex out of range");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return bfs_run(pg, to_internal_id(pg, src), rank); });
+}
+
+pc_status pc_sssp(pc_pgraph* pg, int32_t src, int32_t* dist_host) {
+    return pc_sssp_ex(pg, src, PC_SSSP_AUTO, 0, dist_host);
+}
+
+pc_status pc_sssp_ex(pc_pgraph* pg, int32_t src, int32_t method, int32_t delta, int32_t* dist_host) {
+    clear_error();
+    if (!pg || !dist_host) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    const uint64_t n = pg->g->n;
+    if (!pg->w) return fail(PC_ERR_INVALID_INPUT, "SSSP needs a weighted graph");
+    if (src < 0 || (uint64_t)src >= n) return fail(PC_ERR_INVALID_INPUT, "source vertex out of range");
+    if (method != PC_SSSP_AUTO && method != PC_SSSP_BELLMAN_FORD && method != PC_SSSP_DELTA_STEPPING)
+        return fail(PC_ERR_INVALID_INPUT, "unknown SSSP method");
+    if (delta < 0) return fail(PC_ERR_INVALID_INPUT, "delta must be >= 0 (0: chosen from the graph)");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return sssp_run(pg, to_internal_id(pg, src), method, delta, dist_host); });
+}
+
+pc_status pc_pagerank(pc_pgraph* pg, float damping, int32_t iterations, const float* init, float* out) {
+    clear_error();
+    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    if (iterations <= 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be positive");
+    if (!(damping > 0.f && damping <= 1.f)) return fail(PC_ERR_INVALID_INPUT, "damping must be in (0, 1]");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return pagerank_run<float>(pg, damping, iterations, init, out); });
+}
+
+pc_status pc_pagerank_f64(pc_pgraph* pg, double damping, int32_t iterations, const double* init, double* out) {
+    clear_error();
+    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    if (iterations <= 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be positive");
+    if (!(damping > 0.0 && damping <= 1.0)) return fail(PC_ERR_INVALID_INPUT, "damping must be in (0, 1]");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return pagerank_run<double>(pg, damping, iterations, init, out); });
+}
+
+pc_status pc_selftest_grid_barrier(int32_t device, int32_t rounds, int32_t absent_cta, uint32_t limit_ms,
+                                   uint32_t* mismatches) {
+    clear_error();
+    if (rounds < 0 || !mismatches || limit_ms == 0) return fail(PC_ERR_INVALID_INPUT, "bad argument");
+    PC_TRY(pc_set_device(device));
+    int per_sm = 0;
+    PC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grid_sync_selftest, kThreads, 0));
+    if (per_sm < 1) return fail(PC_ERR_CUDA, "self-test kernel cannot be resident");
+    const int grid = sm_count(device) * std::min(per_sm, 2);
+    if (absent_cta >= grid) return fail(PC_ERR_INVALID_INPUT, "absent_cta is outside the grid");
+    cudaStream_t s = nullptr;
+    PC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    DevBuf buf;
+    pc_status st = buf.alloc(sizeof(GridBarrier) + 16, "self-test state");
+    if (st != PC_OK) {
+        cudaStreamDestroy(s);
+        return st;
+    }
+    GridBarrier* gb = buf.as<GridBarrier>();
+    unsigned* tally = reinterpret_cast<unsigned*>(gb + 1);
+    unsigned* bad = tally + 1;
+    uint64_t limit_ns = (uint64_t)limit_ms * 1000000ull;
+    void* args[] = {(void*)&gb, (void*)&rounds, (void*)&absent_cta, (void*)&limit_ns, (void*)&tally, (void*)&bad};
+    GridBarrier hb{};
+    unsigned hbad = 0;
+    cudaError_t e = cudaMemsetAsync(buf.p, 0, sizeof(GridBarrier) + 16, s);
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel((const void*)k_grid_sync_selftest, dim3(grid), dim3(kThreads), args, 0, s);
+    count_launch();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    if (e != cudaSuccess) return cuda_fail(e, "grid barrier self-test", __FILE__, __LINE__);
+    *mismatches = hbad;
+    if (hb.err) return fail(PC_ERR_TIMEOUT, "grid barrier: a wait ran out of time");
+    return PC_OK;
+}
+
+pc_status pc_kcore(pc_pgraph* pg, int32_t* core_host, int32_t* largest) {
+    clear_error();
+    if (!pg || !core_host) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    if (pg->g->n == 0) {
+        if (largest) *largest = 0;
+        return PC_OK;
+    }
+    return with_room(pg, [&] { return kcore_run(pg, core_host, largest); });
+}
+
+pc_status pc_mis(pc_pgraph* pg, int32_t* res) {
+    clear_error();
+    if (!pg || !res) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    if (pg->g->n == 0) return PC_OK;
+    return with_room(pg, [&] { return mis_run(pg, false, 0, res); });
+}
+
+pc_status pc_mis_hashed(pc_pgraph* pg, uint64_t seed, int32_t* res) {
+    clear_error();
+    if (!pg || !res) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    if (pg->g->n == 0) return PC_OK;
+    return with_room(pg, [&] { return mis_run(pg, true, seed, res); });
+}
+
+pc_status pc_cdlp(pc_pgraph* pg, int32_t iterations, int32_t* labels) {
+    clear_error();
+    if (!pg || !labels) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    if (iterations < 0) return fail(PC_ERR_INVALID_INPUT, "iterations must be non-negative");
+    PC_TRY(use_device(pg->g));
+    const uint64_t n = pg->g->n;
+    if (n == 0 || iterations == 0) return PC_OK;
+    return with_room(pg, [&] { return cdlp_run(pg, iterations, labels); });
 }
 
 }  // extern "C"

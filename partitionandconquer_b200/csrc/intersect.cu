@@ -174,13 +174,7 @@ __global__ void k_lcc_from_triangles(const uint64_t* __restrict__ off, const uns
     lcc[u] = du < 1 ? 0.0 : (double)(2 * tri[u]) / (double)(du * (du - 1));
 }
 
-pc_status pc_lcc(pc_pgraph* pg, int32_t method, double* out) {
-    clear_error();
-    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    if (method != PC_METHOD_MERGE && method != PC_METHOD_GALLOPING) return fail(PC_ERR_INVALID_INPUT, "unknown method");
-    PC_TRY(use_device(pg->g));
-    const uint64_t n = pg->g->n;
-    if (n == 0) return PC_OK;
+static pc_status lcc_run(pc_pgraph* pg, uint64_t n, double* out) {
     cudaStream_t s = pg->g->stream;
     // per-vertex triangle counts with the triangle-count plan (its variants,
     // the learned or heuristic choice per unit) in per-vertex mode
@@ -199,12 +193,17 @@ pc_status pc_lcc(pc_pgraph* pg, int32_t method, double* out) {
     return sync(pg);
 }
 
-pc_status pc_jaccard_edges(pc_pgraph* pg, float* out) {
+pc_status pc_lcc(pc_pgraph* pg, int32_t method, double* out) {
     clear_error();
     if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    if (method != PC_METHOD_MERGE && method != PC_METHOD_GALLOPING) return fail(PC_ERR_INVALID_INPUT, "unknown method");
     PC_TRY(use_device(pg->g));
-    const uint64_t n = pg->g->n, m = pg->g->m;
-    if (m == 0) return PC_OK;
+    const uint64_t n = pg->g->n;
+    if (n == 0) return PC_OK;
+    return with_room(pg, [&] { return lcc_run(pg, n, out); });
+}
+
+static pc_status jaccard_run(pc_pgraph* pg, uint64_t n, uint64_t m, float* out) {
     cudaStream_t s = pg->g->stream;
     // per-edge triangle counts with the triangle-count plan (its variants,
     // the learned or heuristic choice per unit) in per-edge mode
@@ -258,6 +257,28 @@ pc_status pc_jaccard_edges(pc_pgraph* pg, float* out) {
     return sync(pg);
 }
 
+pc_status pc_jaccard_edges(pc_pgraph* pg, float* out) {
+    clear_error();
+    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    const uint64_t n = pg->g->n, m = pg->g->m;
+    if (m == 0) return PC_OK;
+    return with_room(pg, [&] { return jaccard_run(pg, n, m, out); });
+}
+
+static pc_status pairs_run(pc_pgraph* pg, const int32_t* pairs, uint64_t nq, uint64_t* out) {
+    cudaStream_t s = pg->g->stream;
+    PC_TRY(scratch_reserve(pg, nq * 8 + nq * 8 + 512));
+    int32_t* d_pairs = nullptr;
+    PC_TRY(upload(pg, pairs, 2 * nq, &d_pairs));
+    PC_TRY(map_ids_to_internal(pg, d_pairs, 2 * nq));
+    unsigned long long* d_out = pg->scratch.take<unsigned long long>(nq);
+    k_pair_counts<<<sm_count(pg->g->device) * 16, 256, 0, s>>>(pg->off, pg->adj, d_pairs, nq, d_out);
+    PC_LAUNCHED();
+    PC_CUDA(cudaMemcpyAsync(out, d_out, nq * 8, cudaMemcpyDeviceToHost, s));
+    return sync(pg);
+}
+
 pc_status pc_batch_count_pairs(pc_pgraph* pg, const int32_t* pairs, uint64_t nq, uint64_t* out) {
     clear_error();
     if (!pg || (nq && (!pairs || !out))) return fail(PC_ERR_INVALID_INPUT, "null argument");
@@ -266,13 +287,19 @@ pc_status pc_batch_count_pairs(pc_pgraph* pg, const int32_t* pairs, uint64_t nq,
     for (uint64_t i = 0; i < 2 * nq; ++i)
         if (pairs[i] < 0 || (uint64_t)pairs[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
     PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return pairs_run(pg, pairs, nq, out); });
+}
+
+static pc_status sets_run(pc_pgraph* pg, const int32_t* ids, const uint64_t* offsets, uint64_t tot, uint64_t nq, uint64_t* out) {
     cudaStream_t s = pg->g->stream;
-    PC_TRY(scratch_reserve(pg, nq * 8 + nq * 8 + 512));
-    int32_t* d_pairs = nullptr;
-    PC_TRY(upload(pg, pairs, 2 * nq, &d_pairs));
-    PC_TRY(map_ids_to_internal(pg, d_pairs, 2 * nq));
+    PC_TRY(scratch_reserve(pg, tot * 4 + (nq + 1) * 8 + nq * 8 + 512));
+    int32_t* d_ids = nullptr;
+    uint64_t* d_off = nullptr;
+    PC_TRY(upload(pg, ids, tot, &d_ids));
+    PC_TRY(upload(pg, offsets, nq + 1, &d_off));
+    PC_TRY(map_ids_to_internal(pg, d_ids, tot));
     unsigned long long* d_out = pg->scratch.take<unsigned long long>(nq);
-    k_pair_counts<<<sm_count(pg->g->device) * 16, 256, 0, s>>>(pg->off, pg->adj, d_pairs, nq, d_out);
+    k_set_counts<<<sm_count(pg->g->device) * 16, 256, 0, s>>>(pg->off, pg->adj, d_ids, d_off, nq, d_out);
     PC_LAUNCHED();
     PC_CUDA(cudaMemcpyAsync(out, d_out, nq * 8, cudaMemcpyDeviceToHost, s));
     return sync(pg);
@@ -290,28 +317,10 @@ pc_status pc_batch_count_sets(pc_pgraph* pg, const int32_t* ids, const uint64_t*
     for (uint64_t i = 0; i < tot; ++i)
         if (ids[i] < 0 || (uint64_t)ids[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
     PC_TRY(use_device(pg->g));
-    cudaStream_t s = pg->g->stream;
-    PC_TRY(scratch_reserve(pg, tot * 4 + (nq + 1) * 8 + nq * 8 + 512));
-    int32_t* d_ids = nullptr;
-    uint64_t* d_off = nullptr;
-    PC_TRY(upload(pg, ids, tot, &d_ids));
-    PC_TRY(upload(pg, offsets, nq + 1, &d_off));
-    PC_TRY(map_ids_to_internal(pg, d_ids, tot));
-    unsigned long long* d_out = pg->scratch.take<unsigned long long>(nq);
-    k_set_counts<<<sm_count(pg->g->device) * 16, 256, 0, s>>>(pg->off, pg->adj, d_ids, d_off, nq, d_out);
-    PC_LAUNCHED();
-    PC_CUDA(cudaMemcpyAsync(out, d_out, nq * 8, cudaMemcpyDeviceToHost, s));
-    return sync(pg);
+    return with_room(pg, [&] { return sets_run(pg, ids, offsets, tot, nq, out); });
 }
 
-pc_status pc_jaccard_queries(pc_pgraph* pg, const int32_t* queries, int32_t nq, double* out) {
-    clear_error();
-    if (!pg || nq < 0 || (nq && (!queries || !out))) return fail(PC_ERR_INVALID_INPUT, "bad argument");
-    if (nq == 0) return PC_OK;
-    const uint64_t n = pg->g->n;
-    for (int32_t i = 0; i < nq; ++i)
-        if (queries[i] < 0 || (uint64_t)queries[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
-    PC_TRY(use_device(pg->g));
+static pc_status jaccard_queries_run(pc_pgraph* pg, const int32_t* queries, int32_t nq, double* out) {
     cudaStream_t s = pg->g->stream;
     const uint64_t np = (uint64_t)nq * nq;
     PC_TRY(scratch_reserve(pg, nq * 4 + np * 8 + np * 8 + np * 8 + 512));
@@ -329,6 +338,17 @@ pc_status pc_jaccard_queries(pc_pgraph* pg, const int32_t* queries, int32_t nq, 
     PC_LAUNCHED();
     PC_CUDA(cudaMemcpyAsync(out, d_out, np * 8, cudaMemcpyDeviceToHost, s));
     return sync(pg);
+}
+
+pc_status pc_jaccard_queries(pc_pgraph* pg, const int32_t* queries, int32_t nq, double* out) {
+    clear_error();
+    if (!pg || nq < 0 || (nq && (!queries || !out))) return fail(PC_ERR_INVALID_INPUT, "bad argument");
+    if (nq == 0) return PC_OK;
+    const uint64_t n = pg->g->n;
+    for (int32_t i = 0; i < nq; ++i)
+        if (queries[i] < 0 || (uint64_t)queries[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
+    PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return jaccard_queries_run(pg, queries, nq, out); });
 }
 
 }  // extern "C"

@@ -113,7 +113,7 @@ struct pc_pgraph {
     pc::DevBuf ooff;              // uint32 [n+1]
     pc::DevBuf oids;              // int4 [ovecs + 32]; null when there was no room for it
     uint64_t ovecs = 0;           // vectors of all rows (a small copy's: at most)
-    bool oriented_tried = false;
+    uint64_t oriented_from = 0;   // build it only with so many bytes free (after it had no room or was given back)
     pc::DevBuf unit_of;           // int32 [n]: planning unit of each vertex (tc.cu)
     pc::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -186,9 +186,28 @@ inline bool oriented_fits(uint64_t n, uint64_t m, bool checked) {
     return oriented_most(n, m, checked) + 64 < (1ull << 32);
 }
 
-// Lazily builds the oriented copy (uses the scratch arena).  Leaves oids null,
-// without an error, when device memory does not hold it.
+// Lazily builds the oriented copy (uses the scratch arena) and dplus.  Leaves
+// oids null, without an error, when device memory does not hold the copy.
 pc_status ensure_oriented(pc_pgraph* pg);
+
+// Gives the oriented copy back; whether there was one.
+bool release_oriented(pc_pgraph* pg);
+
+// Runs a call on a view; when it runs out of device memory, gives the view's
+// oriented copy back and runs it again: no call needs more memory than it would
+// without the copy.  f must not have written its results before it allocates.
+template <class F>
+pc_status with_room(pc_pgraph* pg, F&& f) {
+    pc_status st = f();
+    if (st == PC_ERR_OOM && release_oriented(pg)) {
+        clear_error();
+        st = f();
+    }
+    return st;
+}
+
+// Device memory that an allocation could get now.
+uint64_t available_bytes(int device);
 
 // Synchronises the handle's stream and converts a device error to a status.
 pc_status sync(pc_pgraph* pg);

@@ -187,16 +187,7 @@ using namespace pc::qry;
 
 extern "C" {
 
-pc_status pc_friend_triangle(pc_pgraph* pg, int32_t root, const int32_t* nodes, uint64_t nn, uint64_t* out) {
-    clear_error();
-    if (!pg || !out || (nn && !nodes)) return fail(PC_ERR_INVALID_INPUT, "null argument");
-    const uint64_t n = pg->g->n;
-    if (root < 0 || (uint64_t)root >= n) return fail(PC_ERR_INVALID_INPUT, "root vertex out of range");
-    for (uint64_t i = 0; i < nn; ++i)
-        if (nodes[i] < 0 || (uint64_t)nodes[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
-    *out = 0;
-    if (nn < 2) return PC_OK;
-    PC_TRY(use_device(pg->g));
+static pc_status friend_run(pc_pgraph* pg, int32_t root, const int32_t* nodes, uint64_t nn, uint64_t* out) {
     cudaStream_t s = pg->g->stream;
     const int32_t iroot = to_internal_id(pg, root);
     uint64_t dr = 0;
@@ -230,15 +221,23 @@ pc_status pc_friend_triangle(pc_pgraph* pg, int32_t root, const int32_t* nodes, 
     return PC_OK;
 }
 
-pc_status pc_square_count(pc_pgraph* pg, uint64_t* out) {
+pc_status pc_friend_triangle(pc_pgraph* pg, int32_t root, const int32_t* nodes, uint64_t nn, uint64_t* out) {
     clear_error();
-    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    if (!pg || !out || (nn && !nodes)) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    const uint64_t n = pg->g->n;
+    if (root < 0 || (uint64_t)root >= n) return fail(PC_ERR_INVALID_INPUT, "root vertex out of range");
+    for (uint64_t i = 0; i < nn; ++i)
+        if (nodes[i] < 0 || (uint64_t)nodes[i] >= n) return fail(PC_ERR_INVALID_INPUT, "query vertex out of range");
+    *out = 0;
+    if (nn < 2) return PC_OK;
     PC_TRY(use_device(pg->g));
+    return with_room(pg, [&] { return friend_run(pg, root, nodes, nn, out); });
+}
+
+static pc_status square_run(pc_pgraph* pg, uint64_t* out) {
     cudaStream_t s = pg->g->stream;
     const uint64_t n = pg->g->n, m = pg->g->m;
     const int sms = sm_count(pg->g->device);
-    *out = 0;
-    if (n == 0 || m == 0) return PC_OK;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
     DevBuf roff, radj, keys, dp;
@@ -280,6 +279,15 @@ pc_status pc_square_count(pc_pgraph* pg, uint64_t* out) {
     PC_TRY(sync(pg));
     *out = h;
     return PC_OK;
+}
+
+pc_status pc_square_count(pc_pgraph* pg, uint64_t* out) {
+    clear_error();
+    if (!pg || !out) return fail(PC_ERR_INVALID_INPUT, "null argument");
+    PC_TRY(use_device(pg->g));
+    *out = 0;
+    if (pg->g->n == 0 || pg->g->m == 0) return PC_OK;
+    return with_room(pg, [&] { return square_run(pg, out); });
 }
 
 }  // extern "C"

@@ -697,7 +697,7 @@ static pc_status launch_bitmap(int K, int G, int kind, const BitmapLaunch& L) {
 using namespace tc;
 
 static pc_status tc_features(pc_pgraph* pg) {
-    PC_TRY(ensure_oriented(pg));
+    PC_TRY(ensure_dplus(pg));
     build_units(pg, &pg->unit_lo, &pg->unit_hi);
     const size_t U = pg->unit_lo.size();
     const uint64_t n = pg->g->n;
@@ -992,7 +992,7 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     const int mode = d_tri ? kCountVertex : (d_ecnt ? kCountEdge : kCountOnly);
     const int sms = sm_count(pg->g->device);
     std::vector<LaunchGroup*> listed;  // the groups with an item list
-    size_t need = 4096;
+    size_t need = 4096, need_binned = 0;
     // lists put in order of their in-neighbours' rows
     const uint64_t n = pg->g->n;
     const bool bin = n >= (1u << 17) && pg->oids.p && pg->ovecs * 16 > kBinFrom;
@@ -1001,7 +1001,9 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
         gr.list = (int)listed.size();
         listed.push_back(&gr);
         gr.binned = bin && is_bitmap(gr.v);
-        need += (gr.binned ? 2 : 1) * (gr.item_bound * sizeof(Item) + 256 + kBins * 8);
+        const size_t room = gr.item_bound * sizeof(Item) + 256 + kBins * 8;
+        need += room;
+        if (gr.binned) need_binned += room;
     };
     for (LaunchGroup& gr : groups) {
         if (gr.ranges.empty()) continue;
@@ -1027,7 +1029,13 @@ static pc_status tc_execute(pc_pgraph* pg, const std::vector<int8_t>& assign, ui
     const uint64_t item_blocks = n >= (1u << 17) ? ceil_div(n, 256) : 0;
     need += U * 2 + listed.size() * (sizeof(ItemList) + 8) + item_blocks * sizeof(ItemBlock) + 1024;
     if (unit_ms) need += U * 8 + 256;
-    PC_TRY(scratch_reserve(pg, need));
+    pc_status reserved = scratch_reserve(pg, need + need_binned);
+    if (reserved == PC_ERR_OOM && need_binned) {  // the lists in pivot order need half the room
+        for (LaunchGroup* gr : listed) gr->binned = false;
+        clear_error();
+        reserved = scratch_reserve(pg, need);
+    }
+    PC_TRY(reserved);
     // the total, then a count and a taken-items counter per list
     unsigned long long* d_total = pg->scratch.take<unsigned long long>(1 + listed.size());
     int16_t* d_list_of = nullptr;
@@ -1205,7 +1213,8 @@ pc_status tc_assign(pc_pgraph* pg, int32_t variant, const std::vector<float>& fe
     return PC_OK;
 }
 
-pc_status tc_count(pc_pgraph* pg, int32_t variant, uint64_t* count, pc_tc_stats* stats) {
+static pc_status tc_count_run(pc_pgraph* pg, int32_t variant, uint64_t* count, pc_tc_stats* stats) {
+    PC_TRY(ensure_oriented(pg));
     PC_TRY(tc_ensure_features(pg));
     const size_t U = pg->unit_lo.size();
     if (U == 0 || pg->g->m == 0) {
@@ -1221,11 +1230,16 @@ pc_status tc_count(pc_pgraph* pg, int32_t variant, uint64_t* count, pc_tc_stats*
     return PC_OK;
 }
 
+pc_status tc_count(pc_pgraph* pg, int32_t variant, uint64_t* count, pc_tc_stats* stats) {
+    return with_room(pg, [&] { return tc_count_run(pg, variant, count, stats); });
+}
+
 // Per-vertex triangle counts (each triangle adds 1 to each of its three
 // vertices) into d_tri (n zeroed counters, outside the scratch arena) under
 // the plan of `variant`; the matrix form has no per-vertex mode, so its units
 // run with the 32-lane bitmap kernel.  Returns the triangle count.
 pc_status tc_vertex_triangles(pc_pgraph* pg, int32_t variant, unsigned long long* d_tri, uint64_t* count) {
+    PC_TRY(ensure_oriented(pg));
     PC_TRY(tc_ensure_features(pg));
     const size_t U = pg->unit_lo.size();
     *count = 0;
@@ -1241,8 +1255,10 @@ pc_status tc_vertex_triangles(pc_pgraph* pg, int32_t variant, unsigned long long
     return tc_execute(pg, assign, count, nullptr, nullptr, d_tri);
 }
 
-// Counters tc_edge_triangles needs.
+// Counters tc_edge_triangles needs.  Builds the oriented copy or not, which
+// decides where the slots are, so tc_edge_triangles itself leaves that alone.
 pc_status tc_edge_slots(pc_pgraph* pg, uint64_t* slots) {
+    PC_TRY(ensure_oriented(pg));
     PC_TRY(tc_ensure_features(pg));
     *slots = pg->oids.p ? 4 * pg->ovecs : pg->g->m;
     return PC_OK;
@@ -1273,7 +1289,8 @@ pc_status tc_edge_triangles(pc_pgraph* pg, int32_t variant, uint32_t* d_ecnt, ui
 // variants only where the ids fit) in one profiled call; returns the per-unit
 // cost inside that full run, -1 where the variant cannot run, and the count
 // over the units it ran.
-pc_status tc_profile_variant(pc_pgraph* pg, int variant, std::vector<double>* unit_ms, uint64_t* count) {
+static pc_status tc_profile_variant_run(pc_pgraph* pg, int variant, std::vector<double>* unit_ms, uint64_t* count) {
+    PC_TRY(ensure_oriented(pg));
     PC_TRY(tc_ensure_features(pg));
     const size_t U = pg->unit_lo.size();
     std::vector<int8_t> assign(U, -1);
@@ -1288,8 +1305,13 @@ pc_status tc_profile_variant(pc_pgraph* pg, int variant, std::vector<double>* un
     return PC_OK;
 }
 
+pc_status tc_profile_variant(pc_pgraph* pg, int variant, std::vector<double>* unit_ms, uint64_t* count) {
+    return with_room(pg, [&] { return tc_profile_variant_run(pg, variant, unit_ms, count); });
+}
+
 // Times one variant on one unit alone (selector training data).
-pc_status tc_time_unit(pc_pgraph* pg, size_t unit, int variant, double* ms, uint64_t* count) {
+static pc_status tc_time_unit_run(pc_pgraph* pg, size_t unit, int variant, double* ms, uint64_t* count) {
+    PC_TRY(ensure_oriented(pg));
     PC_TRY(tc_ensure_features(pg));
     const size_t U = pg->unit_lo.size();
     if (unit >= U) return fail(PC_ERR_INVALID_INPUT, "unit index out of range");
@@ -1299,6 +1321,10 @@ pc_status tc_time_unit(pc_pgraph* pg, size_t unit, int variant, double* ms, uint
     PC_TRY(tc_execute(pg, assign, count, &st));
     *ms = st.kernel_ms;
     return PC_OK;
+}
+
+pc_status tc_time_unit(pc_pgraph* pg, size_t unit, int variant, double* ms, uint64_t* count) {
+    return with_room(pg, [&] { return tc_time_unit_run(pg, unit, variant, ms, count); });
 }
 
 }  // namespace pc
