@@ -569,18 +569,26 @@ size_t oriented_temp_bytes(uint64_t n) {
     return std::max<size_t>(tb, 1);
 }
 
+static uint64_t oriented_bytes(uint64_t n, uint64_t m, bool checked) {
+    return oriented_most(n, m, checked) * 16 + (n + 1) * 4;
+}
+
+bool oriented_wanted(uint64_t n, uint64_t m, bool checked, int device, uint64_t from) {
+    const char* e = getenv("PC_ORIENTED_COPY");  // 0: count on the CSR (a switch for measurements)
+    if (n == 0 || !oriented_fits(n, m, checked) || (e && atoi(e) == 0)) return false;
+    // A large copy is built only where as much again stays free, for the calls'
+    // temporaries and for other handles (the CSR's scans take 1.4 times as long,
+    // a call without memory fails); a small one whenever it fits.
+    const uint64_t bytes = oriented_bytes(n, m, checked);
+    from = std::max<uint64_t>(from, bytes > (256ull << 20) ? 2 * bytes : 0);
+    return from == 0 || available_bytes(device) >= from;
+}
+
 pc_status ensure_oriented(pc_pgraph* pg) {
     PC_TRY(ensure_dplus(pg));
     if (pg->oids.p) return PC_OK;
     const uint64_t n = pg->g->n, m = pg->g->m;
-    const char* wanted = getenv("PC_ORIENTED_COPY");  // 0: count on the CSR (a switch for measurements)
-    if (n == 0 || !oriented_fits(n, m, pg->g->checked) || (wanted && atoi(wanted) == 0)) return PC_OK;
-    // A large copy is built only where as much again stays free, for the calls'
-    // temporaries and for other handles (the CSR's scans take 1.4 times as long,
-    // a call without memory fails); a small one whenever it fits.
-    const uint64_t bytes = oriented_most(n, m, pg->g->checked) * 16 + (n + 1) * 4;
-    const uint64_t from = std::max<uint64_t>(pg->oriented_from, bytes > (256ull << 20) ? 2 * bytes : 0);
-    if (from && available_bytes(pg->g->device) < from) return PC_OK;
+    if (!oriented_wanted(n, m, pg->g->checked, pg->g->device, pg->oriented_from)) return PC_OK;
     const size_t tb = oriented_temp_bytes(n);
     pc_status st = scratch_reserve(pg, tb);
     if (st == PC_OK)
@@ -591,7 +599,7 @@ pc_status ensure_oriented(pc_pgraph* pg) {
     pg->ooff.release();
     pg->oids.release();
     if (st != PC_ERR_OOM) return st;
-    pg->oriented_from = available_bytes(pg->g->device) + bytes / 4;
+    pg->oriented_from = available_bytes(pg->g->device) + oriented_bytes(n, m, pg->g->checked) / 4;
     clear_error();
     return PC_OK;
 }

@@ -34,7 +34,7 @@ struct pc_batch {
     uint32_t G = 0;
     std::vector<uint64_t> voff;
     std::vector<uint64_t> gm;  // directed edges per graph
-    pc::DevBuf d_voff, dplus, graph_of, ooff, oids, titems, tri, dist, q0, q1, tc, lcc, items, counter;
+    pc::DevBuf d_voff, dplus, ooff, oids, titems, tri, dist, q0, q1, tc, items, counter;
     uint64_t ovecs = 0;
     uint32_t ntri = 0;  // triangle items
     uint64_t* h_tc = nullptr;  // pinned staging
@@ -62,6 +62,7 @@ constexpr uint32_t kHeavyList = 256;  // ... up to so many a level
 constexpr uint32_t kItemRun = 256;  // in-neighbours per triangle item
 
 // base[v]: the first vertex of v's graph (v's graph-local id is v - base[v]).
+// Needed for the preparation only, in the memory of the BFS queues.
 __global__ void k_graph_of(const uint64_t* __restrict__ voff, int32_t* __restrict__ graph_of,
                            int32_t* __restrict__ base) {
     const uint64_t v0 = voff[blockIdx.x], v1 = voff[blockIdx.x + 1];
@@ -90,27 +91,35 @@ __global__ void k_prepare(const uint64_t* __restrict__ off, const int32_t* __res
 }
 
 // Triangle items: every pivot with a set and in-neighbours gives a run of
-// items of <= kItemRun in-neighbours, appended in any order.
-__global__ void k_triangle_items(const uint64_t* __restrict__ off, const uint32_t* __restrict__ dplus, uint64_t n,
-                                 tc::Item* __restrict__ items, uint32_t* __restrict__ nitems) {
+// items of <= kItemRun in-neighbours, appended in any order (items null: counted
+// only).  The in-neighbours are found from the pivot, so that a sparse arena's
+// items take no more room than the counts and coefficients leave.
+struct TriItem {
+    int32_t b;     // pivot
+    int32_t g;     // its graph
+    uint32_t run;  // in-neighbours from run * kItemRun on
+};
+
+__global__ void k_triangle_items(const uint64_t* __restrict__ off, const uint32_t* __restrict__ dplus,
+                                 const int32_t* __restrict__ graph_of, uint64_t n, TriItem* __restrict__ items,
+                                 uint32_t* __restrict__ nitems) {
     const uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (b >= n || dplus[b] == 0) return;
-    const uint64_t in0 = off[b] + dplus[b], din = off[b + 1] - in0;
+    const uint64_t din = off[b + 1] - off[b] - dplus[b];
     const uint32_t c = (uint32_t)((din + kItemRun - 1) / kItemRun);
     if (!c) return;
     const uint32_t s = atomicAdd(nitems, c);
-    for (uint32_t j = 0; j < c; ++j)
-        items[s + j] = tc::Item{in0 + (uint64_t)j * kItemRun, (int32_t)b, (uint32_t)min((uint64_t)kItemRun, din - (uint64_t)j * kItemRun)};
+    if (items)
+        for (uint32_t j = 0; j < c; ++j) items[s + j] = TriItem{(int32_t)b, graph_of[b], j};
 }
 
 struct Args {
     const uint64_t* off;
     const int32_t* adj;
     const uint64_t* voff;
-    const int32_t* graph_of;
-    const int32_t* base;
-    tc::OrientedView oriented;  // rows in graph-local ids
-    const tc::Item* titems;
+    const uint32_t* dplus;
+    tc::OrientedView oriented;  // rows in graph-local ids; ids null: the CSR's
+    const TriItem* titems;
     uint32_t ntri;
     const int32_t* bfs_order;   // graphs to search, in this order
     uint32_t nbfs;
@@ -128,8 +137,8 @@ struct Args {
 // gathers those of a graph's first kHubs vertices, where nearly every hit
 // lands, in shared memory and adds them up when it comes to another graph
 // (one global atomic per hit: 1.05 ms for 96 graphs of 4.2 M entries).
-template <int kMode>
-__device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
+template <int kMode, class Rows>
+__device__ __forceinline__ void warp_triangles(const Args& A, Rows R, uint32_t* bm) {
     const int lane = threadIdx.x & 31;
     int32_t* ht = reinterpret_cast<int32_t*>(bm + kBits);
     for (uint32_t i = lane; i < kBits; i += 32) bm[i] = 0;
@@ -156,23 +165,26 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
         if (lane == 0) it = atomicAdd(&A.counter[1], 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= A.ntri) break;
-        const tc::Item I = A.titems[it];
-        const int32_t base = A.base[I.b], b = I.b - base;
+        const TriItem I = A.titems[it];
+        const int32_t base = (int32_t)A.voff[I.g], b = I.b - base;
+        const uint64_t in0 = A.off[I.b] + A.dplus[I.b] + (uint64_t)I.run * kItemRun;
+        const uint32_t nin = (uint32_t)min((uint64_t)kItemRun, A.off[I.b + 1] - in0);
+        if constexpr (Rows::kCsr) R.base = base;
         if (base != hist_base) {
             flush();
             hist_base = base;
         }
-        const tc::OrientedView::Row row = A.oriented.row(I.b);
+        const typename Rows::Row row = R.row(I.b);
         tc::SetView S;
         S.bm = bm;
         S.lo = kLowIds;
         S.ht = ht;
         S.hpos = nullptr;
-        A.oriented.sorted(row, &S);
-        S.ovf = S.np > (uint32_t)tc::kHashCap && __ldg(S.nb + (S.np - tc::kHashCap - 1)) >= kLowIds;
+        R.sorted(row, &S);
+        S.ovf = S.np > (uint32_t)tc::kHashCap && __ldg(S.nb + (S.np - tc::kHashCap - 1)) - S.base >= kLowIds;
         bool high = false;
         for (uint32_t k = lane; k < row.n; k += 32) {
-            const int4 v = A.oriented.vector(row, k);
+            const int4 v = R.vector(row, k);
             const int32_t e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
@@ -196,18 +208,18 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
         sink.ecnt = sink.by_rank = nullptr;
         sink.ranks = tc::SetRanks{nullptr, nullptr};
         unsigned long long hits = 0;
-        for (uint32_t k = 0; k < I.n; k += 32) {
-            const int nb = min(32, (int)(I.n - k));
-            const int32_t c = lane < nb ? A.adj[I.in0 + k + lane] : 0;
-            hits += tc::scan_in_neighbours<4, 1, kMode, tc::kMixedSet>(A.oriented, c, nb, b, S, lane, sink);
+        for (uint32_t k = 0; k < nin; k += 32) {
+            const int nb = min(32, (int)(nin - k));
+            const int32_t c = lane < nb ? A.adj[in0 + k + lane] : 0;
+            hits += tc::scan_in_neighbours<4, 1, kMode, tc::kMixedSet>(R, c, nb, b, S, lane, sink);
         }
         for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
         if (lane == 0 && hits) {
-            if (A.tc) atomicAdd(&A.tc[A.graph_of[I.b]], hits);
+            if (A.tc) atomicAdd(&A.tc[I.g], hits);
             if (kMode == tc::kCountVertex) atomicAdd(&A.tri[I.b], hits);
         }
         for (uint32_t k = lane; k < row.n; k += 32) {
-            const int4 v = A.oriented.vector(row, k);
+            const int4 v = R.vector(row, k);
             bm[S.place<tc::kMixedSet>(v.x) >> 5] = 0;
             bm[S.place<tc::kMixedSet>(v.y) >> 5] = 0;
             bm[S.place<tc::kMixedSet>(v.z) >> 5] = 0;
@@ -220,13 +232,13 @@ __device__ __forceinline__ void warp_triangles(const Args& A, uint32_t* bm) {
     flush();
 }
 
-// LCC from per-vertex triangle counts, as in intersect.cu (src/Graph.cpp:833-838).
-__global__ void k_batch_lcc(const uint64_t* __restrict__ off, const unsigned long long* __restrict__ tri, uint64_t n,
-                            double* __restrict__ lcc) {
+// LCC from per-vertex triangle counts, as in intersect.cu
+// (src/Graph.cpp:833-838), each in the place of its count.
+__global__ void k_batch_lcc(const uint64_t* __restrict__ off, uint64_t n, unsigned long long* __restrict__ tri) {
     const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (u >= n) return;
     const uint64_t du = off[u + 1] - off[u];
-    lcc[u] = du < 1 ? 0.0 : (double)(2 * tri[u]) / (double)(du * (du - 1));
+    tri[u] = __double_as_longlong(du < 1 ? 0.0 : (double)(2 * tri[u]) / (double)(du * (du - 1)));
 }
 
 // Level-synchronous BFS of one graph by one CTA, direction-optimising (Beamer,
@@ -341,7 +353,7 @@ __device__ void cta_bfs(const Args& A, uint64_t v0, uint64_t v1, BfsShared& S) {
     }
 }
 
-template <int kMode>
+template <int kMode, bool kCopy>
 __global__ void __launch_bounds__(kMaxWarps * 32, 2) k_batch(Args A) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_item;
@@ -355,7 +367,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2) k_batch(Args A) {
         const int32_t g = A.bfs_order[it];
         cta_bfs(A, A.voff[g], A.voff[g + 1], s_bfs);
     }
-    if (A.ntri) warp_triangles<kMode>(A, smem + (threadIdx.x >> 5) * kWarpWords(kMode == tc::kCountVertex));
+    if (!A.ntri) return;
+    uint32_t* bm = smem + (threadIdx.x >> 5) * kWarpWords(kMode == tc::kCountVertex);
+    if constexpr (kCopy) warp_triangles<kMode>(A, A.oriented, bm);
+    else warp_triangles<kMode>(A, tc::CsrView{A.off, A.adj, A.dplus, 0}, bm);
 }
 
 static uint64_t key_of(uint32_t tasks, int threads, int cps, int order) {
@@ -402,10 +417,9 @@ static pc_status batch_capture(pc_batch* b, uint32_t tasks) {
     A.off = b->g->off.as<uint64_t>();
     A.adj = b->g->adj.as<int32_t>();
     A.voff = b->d_voff.as<uint64_t>();
-    A.graph_of = b->graph_of.as<int32_t>();
-    A.base = A.graph_of + N;
+    A.dplus = b->dplus.as<uint32_t>();
     A.oriented = tc::OrientedView{b->ooff.as<uint32_t>(), b->oids.as<int4>()};
-    A.titems = b->titems.as<tc::Item>();
+    A.titems = b->titems.as<TriItem>();
     A.ntri = lcc || tc ? b->ntri : 0;
     A.bfs_order = b->items.as<int32_t>();
     A.nbfs = tasks & PC_BATCH_BFS ? b->G : 0;
@@ -416,7 +430,8 @@ static pc_status batch_capture(pc_batch* b, uint32_t tasks) {
     A.q0 = b->q0.as<int32_t>();
     A.q1 = b->q1.as<int32_t>();
     const size_t smem = (size_t)(b->threads / 32) * kWarpWords(lcc) * 4;
-    auto kernel = lcc ? k_batch<tc::kCountVertex> : k_batch<tc::kCountOnly>;
+    auto kernel = b->oids.p ? (lcc ? k_batch<tc::kCountVertex, true> : k_batch<tc::kCountOnly, true>)
+                            : (lcc ? k_batch<tc::kCountVertex, false> : k_batch<tc::kCountOnly, false>);
     PC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)(sm_count(b->g->device) * b->ctas_per_sm);
     PC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -424,9 +439,9 @@ static pc_status batch_capture(pc_batch* b, uint32_t tasks) {
     if (tc) cudaMemsetAsync(b->tc.p, 0, (size_t)b->G * 8, s);
     if (lcc) cudaMemsetAsync(b->tri.p, 0, N * 8, s);
     kernel<<<grid, b->threads, smem, s>>>(A);
-    if (lcc) k_batch_lcc<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(A.off, A.tri, N, b->lcc.as<double>());
+    if (lcc) k_batch_lcc<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(A.off, N, A.tri);
     if (tasks & PC_BATCH_TC) cudaMemcpyAsync(b->h_tc, b->tc.p, (size_t)b->G * 8, cudaMemcpyDeviceToHost, s);
-    if (tasks & PC_BATCH_LCC) cudaMemcpyAsync(b->h_lcc, b->lcc.p, N * 8, cudaMemcpyDeviceToHost, s);
+    if (tasks & PC_BATCH_LCC) cudaMemcpyAsync(b->h_lcc, b->tri.p, N * 8, cudaMemcpyDeviceToHost, s);
     if (tasks & PC_BATCH_BFS) cudaMemcpyAsync(b->h_bfs, b->dist.p, N * 4, cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamEndCapture(s, &b->graph);
     if (e != cudaSuccess) return cuda_fail(e, "stream capture of the batch launch", __FILE__, __LINE__);
@@ -464,12 +479,10 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     };
     pc_status st;
     if ((st = b->d_voff.alloc((G + 1) * 8, "graph offsets")) != PC_OK || (st = b->dplus.alloc(N * 4, "dplus")) != PC_OK ||
-        (st = b->graph_of.alloc(N * 8, "graph of vertex")) != PC_OK ||
-        (st = b->tri.alloc(N * 8, "triangles per vertex")) != PC_OK ||
-        (st = b->titems.alloc((std::min<uint64_t>(N, M) + M / kItemRun + 1) * sizeof(tc::Item), "triangle items")) != PC_OK ||
+        (st = b->tri.alloc(N * 8, "triangles per vertex, lcc")) != PC_OK ||
         (st = b->dist.alloc(N * 4, "levels")) != PC_OK || (st = b->q0.alloc(N * 4, "queue")) != PC_OK ||
         (st = b->q1.alloc(N * 4, "queue")) != PC_OK || (st = b->tc.alloc((size_t)G * 8, "counts")) != PC_OK ||
-        (st = b->lcc.alloc(N * 8, "lcc")) != PC_OK || (st = b->counter.alloc(16, "counter")) != PC_OK)
+        (st = b->counter.alloc(16, "counter")) != PC_OK)
         return bail(st);
     cudaError_t e = cudaMallocHost(&b->h_tc, (size_t)G * 8);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_lcc, N * 8);
@@ -483,33 +496,47 @@ pc_status pc_batch_create(const uint64_t* vlist, const int32_t* elist, uint64_t 
     e = cudaMemcpyAsync(b->d_voff.p, voff, (G + 1) * 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(chk.p, 0, 16, s);
     if (e != cudaSuccess) return bail(cuda_fail(e, "batch upload", __FILE__, __LINE__));
-    k_graph_of<<<G, 256, 0, s>>>(b->d_voff.as<uint64_t>(), b->graph_of.as<int32_t>(), b->graph_of.as<int32_t>() + N);
+    const uint64_t* off = arena->off.as<uint64_t>();
+    int32_t *graph_of = b->q0.as<int32_t>(), *base = b->q1.as<int32_t>();
+    uint32_t *dplus = b->dplus.as<uint32_t>(), *d_bad = chk.as<uint32_t>(), *d_items = d_bad + 1;
+    const unsigned nb = (unsigned)ceil_div(N, 256);
+    k_graph_of<<<G, 256, 0, s>>>(b->d_voff.as<uint64_t>(), graph_of, base);
     count_launch();
-    k_prepare<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(),
-                                                         b->d_voff.as<uint64_t>(), b->graph_of.as<int32_t>(), N,
-                                                         b->dplus.as<uint32_t>(), chk.as<uint32_t>());
+    k_prepare<<<nb, 256, 0, s>>>(off, arena->adj.as<int32_t>(), b->d_voff.as<uint64_t>(), graph_of, N, dplus, d_bad);
     count_launch();
-    k_triangle_items<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(arena->off.as<uint64_t>(), b->dplus.as<uint32_t>(), N,
-                                                                b->titems.as<tc::Item>(), chk.as<uint32_t>() + 1);
+    k_triangle_items<<<nb, 256, 0, s>>>(off, dplus, graph_of, N, nullptr, d_items);
     count_launch();
     uint32_t chk_h[2] = {0, 0};
     e = cudaMemcpyAsync(chk_h, chk.p, 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
+    if (chk_h[0]) return bail(fail(PC_ERR_INVALID_INPUT, "an edge joins two graphs of the batch"));
     b->ntri = chk_h[1];
-    if (!chk_h[0]) {
-        // more than fit here do not fit the device's memory either
-        if (!oriented_fits(N, M, true)) return bail(fail(PC_ERR_UNSUPPORTED, "the arena holds too many edges"));
+    if ((st = b->titems.alloc((size_t)b->ntri * sizeof(TriItem), "triangle items")) != PC_OK) return bail(st);
+    e = cudaMemsetAsync(d_items, 0, 4, s);
+    if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
+    k_triangle_items<<<nb, 256, 0, s>>>(off, dplus, graph_of, N, b->titems.as<TriItem>(), d_items);
+    count_launch();
+    if (oriented_wanted(N, M, true, arena->device, 0)) {
+        // without room for the copy the scans read the CSR
         DevBuf tmp;
         const size_t tb = oriented_temp_bytes(N);
-        if ((st = tmp.alloc(tb, "scan scratch")) != PC_OK) return bail(st);
-        st = build_oriented(arena->off.as<uint64_t>(), arena->adj.as<int32_t>(), b->dplus.as<uint32_t>(),
-                            b->graph_of.as<int32_t>() + N, N, M, true, arena->device, s, tmp.p, tb, &b->ooff, &b->oids, &b->ovecs);
-        if (st != PC_OK) return bail(st);
+        st = tmp.alloc(tb, "scan scratch");
+        if (st == PC_OK)
+            st = build_oriented(off, arena->adj.as<int32_t>(), dplus, base, N, M, true, arena->device, s, tmp.p, tb,
+                                &b->ooff, &b->oids, &b->ovecs);
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
+        if (st != PC_OK) {
+            b->ooff.release();
+            b->oids.release();
+            if (st != PC_ERR_OOM) return bail(st);
+            clear_error();
+        }
     }
-    if (chk_h[0]) return bail(fail(PC_ERR_INVALID_INPUT, "an edge joins two graphs of the batch"));
+    e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return bail(cuda_fail(e, "batch preparation", __FILE__, __LINE__));
     *out = b;
     return PC_OK;
 }

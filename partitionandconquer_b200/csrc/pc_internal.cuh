@@ -185,6 +185,9 @@ inline uint64_t oriented_most(uint64_t n, uint64_t m, bool checked) {
 inline bool oriented_fits(uint64_t n, uint64_t m, bool checked) {
     return oriented_most(n, m, checked) + 64 < (1ull << 32);
 }
+// Whether to build the copy now: its indices fit, PC_ORIENTED_COPY is not 0, there
+// are `from` bytes free, and for a large copy as much again as it takes.
+bool oriented_wanted(uint64_t n, uint64_t m, bool checked, int device, uint64_t from);
 
 // Lazily builds the oriented copy (uses the scratch arena) and dplus.  Leaves
 // oids null, without an error, when device memory does not hold the copy.
