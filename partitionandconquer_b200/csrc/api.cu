@@ -161,8 +161,10 @@ pc_status scratch_reserve(pc_pgraph* pg, size_t bytes) {
     size_t want = bytes + 64 * 256;
     if (want > pg->scratch.buf.bytes) {
         PC_CUDA(cudaStreamSynchronize(pg->g->stream));
-        // small calls of a new view would grow it again and again: 4 MB at least
-        PC_TRY(pg->scratch.buf.alloc(std::max<size_t>(want + want / 4, 4u << 20), "scratch arena"));
+        // the calls of a small view would grow it again and again: what most of
+        // them need, from the graph's size, at once
+        const size_t usual = std::min<size_t>((64u << 10) + 48 * pg->g->n + 4 * pg->g->m, 4u << 20);
+        PC_TRY(pg->scratch.buf.alloc(std::max(want + want / 4, usual), "scratch arena"));
     }
     return PC_OK;
 }
