@@ -11,15 +11,16 @@ graph.  Rank 0 prints one JSON line.
                learned per-partition selector (PC_VARIANT_AUTO).
  * e2e      -- the same through the C ABI from pinned host buffers: CSR upload
                (validated), partition view, plan, counting, 8-byte result read.
- * roofline -- the algorithmic bytes of the pivot form the kernels run,
-               B = 8 (n+1) + 4 m (the CSR) + 4 n (the prefix lengths d+)
-               + 12 |E+| (per in-edge c -> b: the in-neighbour's offset and
-               prefix length) + 4 * wedges (every in-neighbour's prefix below
-               its pivot, wedges = sum_c C(d+(c), 2)), over the summed device
-               time of the counting kernels, against the measured HBM copy
-               bandwidth (MEASURED_PEAKS.json; the 6650 GB/s fallback when it
-               is absent).  The merge formulation's read volume over the same
-               time is reported beside it as an effective rate.
+ * roofline -- the DRAM bytes that one count draws (ncu, profiles/tc_dram_traffic.txt)
+               over the summed device time of the counting kernels, against the
+               measured HBM copy bandwidth (MEASURED_PEAKS.json; the 6650 GB/s
+               fallback when it is absent).  Beside it the wedges
+               (sum_c C(d+(c), 2), the prefix ids that the pivot form looks up)
+               per second against one shared-memory probe per lane and clock, and
+               two effective rates: the pivot form's bytes,
+               8 (n+1) + 4 m + 4 n + 12 |E+| + 4 * wedges, which the kernels no
+               longer read in full (the matrix form and L2 save most of them),
+               and the merge formulation's.
  * parity   -- the oracle's count of the same arrays on all host cores, and
                the pinned count of this graph (tests/golden/pinned_counts.json,
                matched by the CSR's fingerprint); a mismatch fails the run.
@@ -557,8 +558,11 @@ def run_ours(args, dist):
     # roofline of the counting kernels (event-timed inside the call on the same stream)
     kernel_ms = statistics.median(k_learned)
     peak, peak_kind = hbm_peak()
-    achieved = tb["pivot_bytes"] / (kernel_ms / 1e3) / 1e9
     traffic = traffic_per_count(tb)
+    achieved = traffic / (kernel_ms / 1e3) / 1e9 if traffic else None
+    sm = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    probes = tb["wedges"] / (kernel_ms / 1e3)
+    probe_peak = 32.0 * sm * (clocks.summary()["sm_max_mhz"] or 1965.0) * 1e6
 
     # end to end through the C ABI from pinned host buffers
     from partitionandconquer_b200 import _lib as L
@@ -627,10 +631,13 @@ def run_ours(args, dist):
                     "d2h_bytes_per_step": 8, "ms_per_step": round(e2e_s * 1e3, 2),
                     "phases_ms": dict(zip(("upload_validate", "partition_view", "features_plan_count", "release"),
                                           (round(statistics.median(x) * 1e3, 2) for x in zip(*phases))))},
-            "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
-                         "frac": round(achieved / peak, 4), "traffic": traffic, "peak_kind": peak_kind,
-                         "algorithmic_bytes": int(tb["pivot_bytes"]), "wedges": int(tb["wedges"]),
-                         "kernel_ms": round(kernel_ms, 4),
+            "roofline": {"bound": "hbm", "achieved": round(achieved, 2) if traffic else None, "peak": peak,
+                         "unit": "GB/s", "frac": round(achieved / peak, 4) if traffic else None, "traffic": traffic,
+                         "peak_kind": peak_kind, "kernel_ms": round(kernel_ms, 4), "wedges": int(tb["wedges"]),
+                         "probes_per_s": float(f"{probes:.4g}"), "probe_peak_per_s": float(f"{probe_peak:.4g}"),
+                         "probe_frac": round(probes / probe_peak, 4),
+                         "effective_pivot_form_gbs": round(tb["pivot_bytes"] / (kernel_ms / 1e3) / 1e9, 1),
+                         "pivot_form_bytes": int(tb["pivot_bytes"]),
                          "effective_merge_gbs": round(tb["merge_bytes"] / (kernel_ms / 1e3) / 1e9, 1),
                          "merge_bytes": int(tb["merge_bytes"]), "W": int(tb["W"])},
             "cpu_baseline": cpu,
@@ -840,8 +847,9 @@ def suite_algos(pc, O, args, emit):
         t_gpu, out = _timed(gpu, args.steps, args.warmup)
         rec = {"suite": "algos", "workload": "rmat22_ef16_p256_w255", "algorithm": name, "n": int(n),
                "m_directed": int(m), "gpu_ms": round(t_gpu * 1e3, 3), "gteps": round(units / t_gpu / 1e9, 4),
-               "algorithmic_gbs": round(nbytes / t_gpu / 1e9, 1), "hbm_frac": round(nbytes / t_gpu / 1e9 / peak, 4),
-               "peak_kind": peak_kind}
+               "effective_gbs": round(nbytes / t_gpu / 1e9, 1)}
+        if name not in ("tc", "tc_galloping", "lcc", "jaccard_edges"):  # theirs are bytes that the kernels do not read
+            rec.update({"hbm_frac": round(nbytes / t_gpu / 1e9 / peak, 4), "peak_kind": peak_kind})
         if isinstance(out, np.ndarray):
             rec["result_buffer"] = "caller-owned pinned host array"
         if args.profile:
@@ -924,7 +932,6 @@ def suite_selector_graph(pc, O, torch, args, emit, name, h, P, suite):
     stream = torch.cuda.ExternalStream(g.stream())
     lp = _learned_vs_plain(pc, torch, pg, stream, args.steps, args.warmup)
     lp["unit_cost_sums"] = plan_bounds(pc, pg)
-    peak, peak_kind = hbm_peak()
     kms = lp["learned_ms"]
     # all-edge Jaccard runs the triangle kernels in per-edge mode under the
     # same plan: learned (selector on) and plain (selector off), same output,
@@ -941,8 +948,7 @@ def suite_selector_graph(pc, O, torch, args, emit, name, h, P, suite):
         raise SystemExit("Jaccard differs between the learned and the plain plan")
     rec = {"suite": suite, "workload": f"{name}_p{P}", "n": int(n), "m_directed": int(m), **lp,
            "tc_gteps_learned": round(tb["e_plus"] / (kms / 1e3) / 1e9, 4),
-           "tc_roofline_frac": round(tb["pivot_bytes"] / (kms / 1e3) / 1e9 / peak, 4), "peak_kind": peak_kind,
-           "wedges": tb["wedges"], "jaccard_ms": round(t_j * 1e3, 3), "jaccard_plain_ms": round(t_jp * 1e3, 3),
+           "tc_effective_pivot_form_gbs": round(tb["pivot_bytes"] / (kms / 1e3) / 1e9, 1), "wedges": tb["wedges"], "jaccard_ms": round(t_j * 1e3, 3), "jaccard_plain_ms": round(t_jp * 1e3, 3),
            "jaccard_speedup": round(t_jp / t_j, 4), "jaccard_gteps": round(m / t_j / 1e9, 4),
            "jaccard_result": "caller-owned pinned host array (the call includes the copy of m floats)"}
     if not args.profile:
