@@ -832,7 +832,7 @@ def suite_algos(pc, O, args, emit):
          m * 20, 20 * (8 * m + 20 * n), 1e-6),
         ("pagerank_fp64", lambda: pg.page_rank(0.85, 20, fp64=True, out=o_pr64),
          ("port", lambda: O.pagerank_f64(vl, el, 0.85, 20)), m * 20, 20 * (12 * m + 24 * n), 1e-12),
-        ("kcore", lambda: pg.solve_kcore(out=o_kc), ("reference", lambda: R.kcore()) if R else ("port", lambda: O.kcore(vl, el)),
+        ("kcore", lambda: pg.solve_kcore(out=o_kc), ("reference", lambda: R.kcore()) if R else ("port", lambda: O.kcore(vl, el)[0]),
          m, sweep, "exact"),
         ("mis", lambda: pg.solve_mis(out=o_mis), ("reference", lambda: R.mis()) if R else ("port", lambda: O.mis(vl, el)),
          m, sweep, "exact"),
