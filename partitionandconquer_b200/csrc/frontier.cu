@@ -10,8 +10,6 @@
 #include <cstdlib>
 #include <vector>
 
-#include <cub/block/block_scan.cuh>
-
 #include "grid_sync.cuh"
 #include "pc_internal.cuh"
 #include "synth_rng.h"
@@ -252,7 +250,7 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
 // the near frontier (tx::expand) or, when that is empty, the split of the far
 // pile.  Steps keep their state in three rotating records (see KState).
 //
-// Bound at RMAT-22 (6.1 -> 2.2 ms a call, 0.3 ms of it the copy back): the
+// Bound at RMAT-22 (6.6 -> 2.2 ms a call, 0.3 ms of it the copy back): the
 // gathers of the neighbours' distances, 2.9 m of them, from L1 and L2.  Small
 // graphs: barriers and chains of atomics, 4-10 us a step (RMAT-16 0.90 -> 0.37
 // ms, RMAT-10 0.50 -> 0.15); ER-20 5.2 -> 0.92 ms.
@@ -941,14 +939,14 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
 // a 32-byte sector each from L2.  (A copy of the hubs' values in shared memory
 // takes up to 58 % of them, but costs the resident warps that hide the rest's
 // latency: 64 / 128 / 192 KB 9.0 / 10.3 / 10.8 ms for 20 iterations against
-// 8.1 without; cache hints that keep hubs in L1 and others out: 8.2-9.0.)
+// 8.1 without; cache hints that keep hubs in L1 and others out: 8.1-9.0.)
 //
 // Rows longer than PullRows::warp_deg get a warp and than cta_deg a CTA, the
 // others kPullLanes lanes.  The bounds follow the graph's size (pull_rows): a
 // large sweep wants few lanes per row, a small one has lanes to spare and ends
 // when its longest row does.  A CTA for every row past 256 entries spent a
-// third of its time in barriers: RMAT-22 10.9 ms, now 7.6.  Every reduction runs in a
-// fixed order, so results are reproducible.
+// third of its time in barriers: a call at RMAT-22 took 10.9 ms, now 8.5.  Every
+// reduction runs in a fixed order, so results are reproducible.
 struct PullRows {
     const int32_t* __restrict__ cta;
     const int32_t* __restrict__ warp;

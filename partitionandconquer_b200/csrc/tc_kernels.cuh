@@ -35,7 +35,7 @@ constexpr int kTile = 16384;        // pivots per planning tile
 constexpr int kChunkWarp = 256;     // in-neighbours per warp work item
 constexpr int kCtaThreads = 512;    // threads per CTA of the bitmap kernels
 constexpr int kHashSlots = 512;     // slots per warp-private hash table
-constexpr int kHashCap = 256;       // max pivot set size for the hash kernel
+constexpr int kHashCap = 256;       // keys of a hash table (a mixed set with more is searched)
 constexpr int kWarpCtaWarps = 8;    // warps per CTA of the warp kernels
 constexpr int kEcRankCap = 512;     // per-edge mode: pivot sets up to this size count by rank in shared memory
 constexpr int kHubHist = 8192;      // per-vertex counting: ids below this count in shared memory
@@ -139,7 +139,7 @@ __device__ __forceinline__ void group_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Per-vertex triangle counts (kVC): every triangle found adds 1 to its
+// Per-vertex triangle counts (kCountVertex): every triangle found adds 1 to its
 // lowest vertex a; ids below kHubHist go to a shared-memory histogram
 // (almost every hit is a hub), the rest to the global counts.
 __device__ __forceinline__ void count_vertex(int32_t a, unsigned long long* __restrict__ tri, uint32_t* hist,
@@ -242,11 +242,12 @@ struct HitSink {
 };
 
 // Scans the prefixes of up to 32 in-neighbours of pivot b: lane j < nb holds
-// in-neighbour j's id (c) and row start; returns this lane's hits.
+// in-neighbour j's id (c); returns this lane's hits.
 //
 // A group of G lanes takes one in-neighbour at a time, V vectors of 4 ids per
 // lane and step, and goes on to its next one (NG apart) as soon as its row reaches an
-// id >= b -- b itself is in the row, so a scan ends inside it -- while the
+// id >= b (b itself, which a symmetric adjacency has in the row, or the INT_MAX
+// at an unchecked row's end: a scan ends inside its row), while the
 // other groups go on with theirs: no lane waits for the longest of the 32 / G
 // rows in flight.  All groups step together, so the vote that ends a row is
 // one full-warp ballot, and the load of the next vector is issued between
@@ -773,10 +774,9 @@ __global__ void __launch_bounds__(kWarpCtaWarps * 32) k_tc_warp(const uint64_t* 
 // count equals the pivot form's; what changes is that N(c) is read once per c
 // instead of once per pivot.  Only the hubs' pairs run this way (kMatrixFrom in
 // tc.cu); the other in-neighbours of the unit are items of the bitmap kernels.
-constexpr int kMatrixMaxId = 1 << 16;      // hi bound: rows of <= 8 KB, H <= 512 MB
+constexpr int kMatrixMaxId = 1 << 16;      // hi bound: rows of <= 8 KB (H: kMatrixRowsCap in tc.cu)
 constexpr int kMatrixWarps = 8;            // warps per CTA
 constexpr int kMatrixBlock = 8;            // pivots a warp takes at a time
-constexpr int kMatrixWordsMax = kMatrixMaxId / 32;
 
 __device__ __forceinline__ uint32_t lower_bound_i32(const int32_t* __restrict__ p, uint32_t n, int32_t x) {
     uint32_t lo = 0, hi = n;
