@@ -73,6 +73,11 @@ pc_status pc_host_unregister(void* ptr);
  * usable.  Not part of the reference interface; a diagnostic. */
 pc_status pc_selftest_grid_barrier(int32_t device, int32_t rounds, int32_t absent_cta, uint32_t limit_ms,
                                    uint32_t* mismatches);
+/* For tests of the library's limits, in place of the environment's
+ * PC_MEMORY_LIMIT_MB (here in bytes, per device), PC_BARRIER_LIMIT_MS and
+ * PC_ORIENTED_COPY (0 or 1), which are read once; a negative value gives the
+ * environment's back.  Not part of the reference interface; a diagnostic. */
+pc_status pc_selftest_limits(int64_t memory_bytes, int64_t barrier_ms, int32_t oriented_copy);
 
 /* ---- graph (class Graph, src/Graph.hpp:38-103) ------------------------- */
 

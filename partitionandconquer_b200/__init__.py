@@ -40,6 +40,11 @@ def launch_count() -> int:
     return int(lib.pc_launch_count())
 
 
+def selftest_limits(memory_bytes: int = -1, barrier_ms: int = -1, oriented_copy: int = -1) -> None:
+    """The library's limits for a test (-1: the environment's; see pc.h)."""
+    check(lib.pc_selftest_limits(memory_bytes, barrier_ms, oriented_copy))
+
+
 def selftest_grid_barrier(device: int = 0, rounds: int = 64, absent_cta: int = -1, limit_ms: int = 1000) -> int:
     """Runs the bounded grid barrier of the persistent kernels `rounds` times
     and returns the number of ordering violations seen (0 expected).  With

@@ -60,18 +60,39 @@ static cudaError_t prepare_pool(int dev) {
     return e;
 }
 
-// Bytes of each device that DevBufs hold, and the most they may hold:
-// PC_MEMORY_LIMIT_MB from the environment (read at every allocation), else what
-// the device has.
+// Limits from the environment, read once (a later setenv of another thread is
+// not raced with); pc_selftest_limits() overrides them.
+struct Limit {
+    const char* name;
+    std::atomic<int64_t> given{-1};
+    int64_t get(double scale, int64_t other) {
+        const int64_t v = given.load(std::memory_order_relaxed);
+        if (v >= 0) return v;
+        std::call_once(once, [&] {
+            const char* e = getenv(name);
+            env = e ? (int64_t)std::min(9e18, std::max(0.0, atof(e) * scale)) : -1;
+        });
+        return env >= 0 ? env : other;
+    }
+    std::once_flag once;
+    int64_t env = -1;
+    explicit Limit(const char* n) : name(n) {}
+};
+static Limit g_memory("PC_MEMORY_LIMIT_MB"), g_barrier("PC_BARRIER_LIMIT_MS"), g_oriented("PC_ORIENTED_COPY");
+
+// 4 s by default.  A cooperative grid is placed as a whole, so no CTA waits for
+// one that has no room yet (measured: behind a kernel that left half of the SMs
+// after 5 ms and the others after 60 ms, all CTAs began at 60 ms).
+uint64_t barrier_limit_ns() { return (uint64_t)std::max<int64_t>(1, std::min<int64_t>(g_barrier.get(1.0, 4000), 600000)) * 1000000ull; }
+
+// Bytes of each device that DevBufs hold, and the most they may hold: a limit, or
+// what the device has.
 constexpr int kMaxDevices = 64;
 static std::atomic<uint64_t> g_held[kMaxDevices];
 
 static std::atomic<uint64_t>& held(int dev) { return g_held[dev < kMaxDevices ? dev : kMaxDevices - 1]; }
 
-static uint64_t memory_limit() {
-    const char* e = getenv("PC_MEMORY_LIMIT_MB");
-    return e ? (uint64_t)(std::max(0.0, atof(e)) * 1048576.0) : ~0ull;
-}
+static uint64_t memory_limit() { return (uint64_t)g_memory.get(1048576.0, INT64_MAX); }
 
 uint64_t available_bytes(int device) {
     size_t room = 0, all = 0;
@@ -576,8 +597,7 @@ static uint64_t oriented_bytes(uint64_t n, uint64_t m, bool checked) {
 }
 
 bool oriented_wanted(uint64_t n, uint64_t m, bool checked, int device, uint64_t from) {
-    const char* e = getenv("PC_ORIENTED_COPY");  // 0: count on the CSR (a switch for measurements)
-    if (n == 0 || !oriented_fits(n, m, checked) || (e && atoi(e) == 0)) return false;
+    if (n == 0 || !oriented_fits(n, m, checked) || g_oriented.get(1.0, 1) == 0) return false;
     // A large copy is built only where as much again stays free, for the calls'
     // temporaries and for other handles (the CSR's scans take 1.4 times as long,
     // a call without memory fails); a small one whenever it fits.
@@ -664,6 +684,14 @@ pc_status pc_set_device(int32_t device) {
 }
 
 uint64_t pc_launch_count(void) { return g_launches.load(); }
+
+pc_status pc_selftest_limits(int64_t memory_bytes, int64_t barrier_ms, int32_t oriented_copy) {
+    clear_error();
+    g_memory.given = memory_bytes;
+    g_barrier.given = barrier_ms;
+    g_oriented.given = oriented_copy;
+    return PC_OK;
+}
 
 pc_status pc_host_register(void* ptr, size_t bytes) {
     clear_error();

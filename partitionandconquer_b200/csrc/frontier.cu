@@ -1093,17 +1093,6 @@ struct CdlpOp {
 
 using namespace fr;
 
-// Bound on any grid-barrier wait of the persistent kernels: 4 s, or
-// PC_BARRIER_LIMIT_MS from the environment (read on every call).  A cooperative
-// grid is placed as a whole, so no CTA waits for one that has no room yet
-// (measured: behind a kernel that left half of the SMs after 5 ms and the others
-// after 60 ms, all CTAs began at 60 ms).
-static uint64_t barrier_limit_ns() {
-    const char* e = getenv("PC_BARRIER_LIMIT_MS");
-    const long ms = e ? std::max(1L, std::min(atol(e), 600000L)) : 4000L;
-    return (uint64_t)ms * 1000000ull;
-}
-
 static unsigned grid_for(const pc_pgraph* pg, int per_sm = 8) { return (unsigned)(sm_count(pg->g->device) * per_sm); }
 
 // CTAs of a persistent kernel: every SM's share, fewer for a small graph,

@@ -212,6 +212,9 @@ pc_status with_room(pc_pgraph* pg, F&& f) {
 // Device memory that an allocation could get now.
 uint64_t available_bytes(int device);
 
+// Bound on any grid-barrier wait of the persistent kernels.
+uint64_t barrier_limit_ns();
+
 // Synchronises the handle's stream and converts a device error to a status.
 pc_status sync(pc_pgraph* pg);
 

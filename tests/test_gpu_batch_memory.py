@@ -25,10 +25,13 @@ def arena(gs):
 
 
 @pytest.mark.parametrize("order", [0, 1])
-def test_batch_on_the_csr(gpu, O, monkeypatch, order):
-    monkeypatch.setenv("PC_ORIENTED_COPY", "0")
+def test_batch_on_the_csr(gpu, O, order):
     gs = graphs(order)
-    b = gpu.Batch(*arena(gs))
+    gpu.selftest_limits(oriented_copy=0)
+    try:
+        b = gpu.Batch(*arena(gs))
+    finally:
+        gpu.selftest_limits()
     want = {"tc": np.array([O.tc_merge(*g) for g in gs], np.uint64), "lcc": np.concatenate([O.lcc(*g) for g in gs]),
             "bfs": np.concatenate([O.bfs(*g, 0) for g in gs])}
     for tasks in (1, 2, 3, 4, 5, 6, 7):

@@ -11,8 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shuffled", [False, True])
-def test_long_path(gpu, monkeypatch, shuffled):
-    monkeypatch.setenv("PC_BARRIER_LIMIT_MS", "50")
+def test_long_path(gpu, shuffled):
     n = 400_000
     p = np.random.default_rng(1).permutation(n) if shuffled else np.arange(n)
     a, b = np.concatenate([p[:-1], p[1:]]), np.concatenate([p[1:], p[:-1]])
@@ -21,6 +20,10 @@ def test_long_path(gpu, monkeypatch, shuffled):
     np.cumsum(np.bincount(a, minlength=n), out=vl[1:])
     g = gpu.Graph(vlist=vl, elist=b[order].astype(np.int32))
     pg = gpu.Partitioned_Graph(g, None)
-    np.testing.assert_array_equal(pg.solve_kcore(), np.ones(n, np.int32))
+    gpu.selftest_limits(barrier_ms=50)
+    try:
+        np.testing.assert_array_equal(pg.solve_kcore(), np.ones(n, np.int32))
+    finally:
+        gpu.selftest_limits()
     pg.close()
     g.close()

@@ -1,8 +1,7 @@
-"""The oriented copy never makes a call fail for want of device memory.  With
-PC_MEMORY_LIMIT_MB the least memory is searched with which a call succeeds on a view
-without the copy (PC_ORIENTED_COPY=0).  With that limit and with every one above it,
-the call must succeed, and give the same result, on a view that may build the copy and
-on one that holds it already."""
+"""The oriented copy never makes a call fail for want of device memory.  Under a limit
+on it, the least memory is searched with which a call succeeds on a view without the
+copy.  With that limit and with every one above it, the call must succeed, and give
+the same result, on a view that may build the copy and on one that holds it."""
 from __future__ import annotations
 
 import gc
@@ -30,24 +29,23 @@ CALLS = {
 
 
 class Runner:
-    def __init__(self, pc, monkeypatch, graph, call):
-        self.pc, self.env, self.g, self.call = pc, monkeypatch, graph, call
+    def __init__(self, pc, graph, call):
+        self.pc, self.g, self.call = pc, graph, call
 
     def run(self, limit, copy, held):
         """The result with `limit` bytes for the library, None when it runs out of memory."""
-        self.env.delenv("PC_MEMORY_LIMIT_MB", raising=False)
-        self.env.setenv("PC_ORIENTED_COPY", "1" if copy else "0")
+        self.pc.selftest_limits(oriented_copy=copy)
         pg = self.pc.Partitioned_Graph(self.g, None)
         try:
             if held:
                 pg.triangle_count()
-            self.env.setenv("PC_MEMORY_LIMIT_MB", repr(limit / 2**20))
+            self.pc.selftest_limits(memory_bytes=limit, oriented_copy=copy)
             return self.call(pg)
         except self.pc.PCError as e:
             assert e.status == OOM, str(e)
             return None
         finally:
-            self.env.delenv("PC_MEMORY_LIMIT_MB", raising=False)
+            self.pc.selftest_limits()
             pg.close()
 
     def least(self, held):
@@ -63,11 +61,11 @@ class Runner:
 
 
 @pytest.mark.parametrize("name", list(CALLS))
-def test_no_call_needs_the_copy(gpu, monkeypatch, name):
+def test_no_call_needs_the_copy(gpu, name):
     gc.collect()
     g = gpu.Graph.rmat_device(17, 16, 3, wmax=255)  # 2^17 vertices
     copy = 4 * int(g.get_csr_elist().size)  # no less than its size
-    r = Runner(gpu, monkeypatch, g, CALLS[name])
+    r = Runner(gpu, g, CALLS[name])
     want = r.run(1 << 34, True, False)
     for held in (False, True):
         least = r.least(held)
@@ -79,11 +77,11 @@ def test_no_call_needs_the_copy(gpu, monkeypatch, name):
 
 
 @pytest.mark.parametrize("name", ["count", "jaccard"])
-def test_rows_beyond_l2(gpu, monkeypatch, name):
+def test_rows_beyond_l2(gpu, name):
     """... where the item lists may be put in another order, which takes as much again."""
     gc.collect()
     g = gpu.Graph.rmat_device(22, 16, 1)
-    r = Runner(gpu, monkeypatch, g, CALLS[name])
+    r = Runner(gpu, g, CALLS[name])
     want = r.run(1 << 34, True, False)
     least = r.least(False)
     for more in range(0, 1 << 30, 1 << 26):

@@ -1,5 +1,5 @@
 """Triangle counts, LCC and all-edge Jaccard on the CSR itself, the path of views whose
-oriented copy has no room (declined here with PC_ORIENTED_COPY=0): row starts and
+oriented copy has no room (declined here by pc_selftest_limits): row starts and
 ends at every place of a 16-byte vector, every set shape and variant, the matrix
 form and its tails, partitions that are not id ranges, and rows of a directed
 graph.  Against the oracle; whole numbers and single IEEE divisions, so equal."""
@@ -18,11 +18,12 @@ PLANS = ([0.0, 0.0, 0.0, np.inf], [0.0, np.inf, 0.0, np.inf], [0.0, np.inf, np.i
 
 
 @pytest.fixture
-def plans(gpu, monkeypatch):
-    monkeypatch.setenv("PC_ORIENTED_COPY", "0")
+def plans(gpu):
+    gpu.selftest_limits(oriented_copy=0)
     saved = gpu.selector.get_heuristic()
     yield PLANS
     gpu.selector.set_heuristic(saved)
+    gpu.selftest_limits()
 
 
 def check(pc, plans, vl, el, t, lcc, jac, v2ps):
