@@ -257,8 +257,8 @@ struct HitSink {
 // and min(id, b) sends them all to b, whose bit is never set (in a mixed set
 // it may be another key's bit; the look-up settles that).
 //
-// Bound: instruction issue and shared-memory wavefronts (RMAT-20: 74 % issue,
-// 68 % of the wavefronts, 32 of 32 lanes active), then L2 latency.  About 45
+// Bound: shared-memory wavefronts and instruction issue (RMAT-20's plain sets: L1
+// at 92 %, 77 % of the issue slots, 32 of 32 lanes active), then L2 latency.  About 45
 // warp instructions per 128 ids; the earlier scan, which tested each id's
 // position and kept a group waiting for the longest of its warp's rows, took
 // about 130.  Bitmap kernels of RMAT-20: 2.07 -> 0.83 ms; RMAT-24's unit of ids
