@@ -26,7 +26,7 @@ constexpr int kKcoreThreads = 512;       // k-core: threads per CTA
 constexpr int kKcorePerSm = 2;
 constexpr uint32_t kLocalQ = 2048;       // ... its queue of claimed vertices
 constexpr uint32_t kLocalEdges = 16384;  // ... peeled by the CTA itself while their rows stay below this
-constexpr int kLocalRounds = 1024;       // ... and for so many rounds a step, while the others wait
+constexpr int kLocalRounds = 1 << 14;    // ... for so many rounds a step, while the others wait
 constexpr size_t kKcoreSmem = 80 * 1024;
 static_assert(kKcoreHubs % kKcoreThreads == 0, "the flush loop needs a uniform trip count");
 
@@ -466,10 +466,16 @@ __global__ void __launch_bounds__(tx::kThreads, 5)
 // queue is dry.  A vertex is claimed by the compare-and-swap that sets its
 // core number, since the scan and the decrements of other CTAs may meet at
 // it.  What does not fit the queue, or would keep one CTA busy for long (rows
-// of more than `local_edges` entries together, or more than kLocalRounds rounds:
-// a chain peels one vertex a round), goes to the next step's queues, which all
-// CTAs share (tx::expand).  So most levels take one step, and no step keeps the
-// others at the barrier for more than a few milliseconds.
+// of more than `local_edges` entries together), goes to the next step's queues,
+// which all CTAs share (tx::expand).  So most levels take one step.
+//
+// A chain peels one vertex a round (2.7 us).  After kLocalRounds rounds a CTA
+// leaves the rest of its queue for itself in the next step, so that a step keeps
+// the others at the barrier for tens of milliseconds, not for seconds.  With 1024
+// rounds CTAs of unequal rounds waited for one another too often (a grid of 700
+// x 700 vertices 7.0 instead of 4.7 ms); through the shared queues, chains from
+// both ends of a path came into one CTA, where the gathered decrements of the one
+// waited for the other's end (20 K vertices: 49 instead of 29 ms).
 //
 // The state lives in three rotating records: step i reads S[i % 3],
 // accumulates into S[(i+1) % 3] (counters cleared by step i-1) and clears
@@ -493,14 +499,15 @@ struct __align__(16) KState {
     int32_t dirty;     // whether the level claimed vertices before this step
     uint32_t claimed;  // vertices the step claimed
     int32_t top;       // largest core number before this step
-    int32_t pad[2];
+    uint32_t rest;     // CTAs that left a rest of their own queue for the step that reads the record
+    int32_t pad;
 };
 
 __global__ void k_kcore_init(const uint64_t* __restrict__ off, uint64_t n, int32_t* __restrict__ deg,
                              int32_t* __restrict__ core, int32_t* __restrict__ rem, KState* S, int32_t* d_top,
                              GridBarrier* gb) {
     const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (u < 3) S[u] = KState{0, 0, u ? 0u : (uint32_t)n, INT_MAX, 0, 0, 0, 1, 0, 0, {0, 0}};
+    if (u < 3) S[u] = KState{0, 0, u ? 0u : (uint32_t)n, INT_MAX, 0, 0, 0, 1, 0, 0, 0, 0};
     if (u == 0) {
         *d_top = 0;
         *gb = GridBarrier{};
@@ -550,6 +557,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
     tx::Buffer& spill = M.spill[warp];
     tx::Buffer& keep = M.keep[warp];
     uint32_t nspill = 0, nkeep = 0;
+    int rd = 0;  // the CTA's queue in use, which may hold a rest of the step before
     uint64_t step = 0;
     for (; step < max_steps; ++step) {
         const KState* in = &S[step % 3];
@@ -559,7 +567,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
         const int4 r2 = __ldcg(reinterpret_cast<const int4*>(in) + 2);
         const uint32_t nl = (uint32_t)r0.x, nh = (uint32_t)r0.y, rn = (uint32_t)r0.z;
         const int32_t par = r1.y, rpar = r1.z;
-        const bool peel = nl || nh;
+        const bool peel = nl || nh || r2.z;
         const bool dirty = r1.w || r2.x;  // the level of the last step claimed something
         const int32_t k = peel ? r1.x : (dirty || r0.w == INT_MAX ? r1.x + 1 : max(r1.x + 1, r0.w + 1));
         const int32_t top = r2.x ? max(r2.y, r1.x - 1) : r2.y;
@@ -575,7 +583,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
         }
         if (lead) {
             KState* clr = &S[(step + 2) % 3];
-            clr->nl = clr->nh = clr->rn = clr->claimed = 0;
+            clr->nl = clr->nh = clr->rn = clr->claimed = clr->rest = 0;
             clr->ml = INT_MAX;
             if (peel) out->rn = rn;  // a peel step keeps the remaining list
             out->k = k;
@@ -631,7 +639,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
         if (peel) {
             tx::expand(
                 M.warp_tile[warp], off, Q, nl, nh, [](int32_t) { return 0; },
-                [&](const uint64_t* j, const int32_t*, const bool* ok) { peel_entries(j, ok, 0); }, []() {});
+                [&](const uint64_t* j, const int32_t*, const bool* ok) { peel_entries(j, ok, rd); }, []() {});
         } else {
             const int32_t* rem = rpar ? rem1 : rem0;
             int32_t* rem2 = rpar ? rem0 : rem1;
@@ -666,7 +674,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
                         }
                     }
                 }
-                push(pl, u, 0);
+                push(pl, u, rd);
                 tx::find(keep, nkeep, stay, u);
                 if (nkeep > tx::kBuf - 32) flush_keep();
             }
@@ -677,7 +685,6 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
         // drain the CTA's queue; when it runs dry, flush the gathered hub
         // decrements (the one flush that takes a degree from >= k to < k
         // pushes the vertex) and go on until nothing is left
-        int rd = 0;
         for (int round = 0;; ++round) {
             __syncthreads();
             uint32_t cnt = min(M.lqn[rd], (uint32_t)kLocalQ);
@@ -699,6 +706,10 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
                 __syncthreads();
                 cnt = min(M.lqn[rd], (uint32_t)kLocalQ);
                 if (cnt == 0) break;
+            }
+            if (round == kLocalRounds) {
+                if (threadIdx.x == 0) atomicAdd(&out->rest, 1u);
+                break;
             }
             const int wr = rd ^ 1;
             for (uint32_t base = 0; base < cnt; base += kKcoreThreads) {
@@ -724,7 +735,7 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
                 M.tile.start[threadIdx.x] = end - len;
                 M.tile.base[threadIdx.x] = b - (end - len);
                 __syncthreads();
-                if (total > local_edges || round >= kLocalRounds) {  // too much for one CTA: the next step shares it among all
+                if (total > local_edges) {  // too much for one CTA: the next step shares it among all
                     tx::find(spill, nspill, i < cnt, u);
                     if (nspill > tx::kBuf - 32) tx::flush(spill, nspill, off, QN, &out->nl, &out->nh);
                     continue;
@@ -759,7 +770,6 @@ __global__ void __launch_bounds__(kKcoreThreads, kKcorePerSm) k_kcore_persistent
             if (M.ml != INT_MAX) atomicMin(&out->ml, M.ml);
             M.claimed = 0;
             M.ml = INT_MAX;
-            M.lqn[0] = M.lqn[1] = 0;
         }
         if (!grid_sync(gb, limit_ns)) return;
     }
