@@ -1194,7 +1194,10 @@ static pc_status pull_rows(pc_pgraph* pg, PullRows* rows) {
 template <class Op>
 static pc_status pull_sweep(pc_pgraph* pg, const Op& op, const PullRows& rows) {
     const uint64_t n = pg->g->n;
-    const uint64_t grid = std::min<uint64_t>(grid_for(pg, 16), ceil_div(n, kThreads / kPullLanes));
+    // a CTA for each CTA row, a warp for each warp row, a lane group for each other one
+    const uint64_t work = std::max<uint64_t>(rows.ncta, std::max<uint64_t>(ceil_div(rows.nwarp, kThreads / 32),
+                                                                           ceil_div(n, kThreads / kPullLanes)));
+    const uint64_t grid = std::min<uint64_t>(grid_for(pg, 16), work);
     k_pull<Op><<<(unsigned)grid, kThreads, 0, pg->g->stream>>>(pg->off, pg->adj, n, op, rows);
     PC_LAUNCHED();
     return PC_OK;
