@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
 // others kPullLanes lanes.  The bounds follow the graph's size (pull_rows): a
 // large sweep wants few lanes per row, a small one has lanes to spare and ends
 // when its longest row does.  A CTA for every row past 256 entries spent a
-// third of its time in barriers: a call at RMAT-22 took 10.9 ms, now 8.5.  Every
+// third of its time in barriers: a call at RMAT-22 took 10.9 ms, now 7.9.  Every
 // reduction runs in a fixed order, so results are reproducible.
 struct PullRows {
     const int32_t* __restrict__ cta;
@@ -983,25 +983,47 @@ __global__ void k_pull_rows(const uint64_t* __restrict__ off, uint64_t n, uint32
 // inside the adjacency array.  The adjacency is read once per sweep, so its
 // loads carry the streaming hint (evict first): the gathered vector keeps its
 // L2 lines.
+//
+// A CTA's rows are long and often few, and nothing else hides the latency of a
+// load and its gathers: a thread takes two vectors a step and loads the next two
+// while it gathers these (20 iterations, fp32 / fp64 / CDLP in ms, one vector and
+// none ahead against this: star of 1 M leaves 8.8 / 9.6 / 9.2 and 5.4 / 5.9 / 5.9,
+// 100 rows of 100 K entries 1.85 / 1.78 / 1.81 and 1.16 / 1.17 / 1.12, RMAT-20
+// 1.96 / 2.34 / 2.17 and 1.84 / 2.24 / 2.09; one ahead 8.2 / 6.6 / 8.5 for the
+// star, two together without the next 8.5 / 6.1 / 5.6).
 template <int L, class Op>
 __device__ __forceinline__ void pull_row(const int32_t* __restrict__ adj, uint64_t b, uint64_t e, int gl, const Op& op,
                                          typename Op::A& acc) {
+    constexpr int U = L == kThreads ? 2 : 1;     // vectors a step
+    constexpr bool kAhead = L == kThreads;
     // positions are relative to the boundary; the ids at [lo, lo + len) are the row's
     const int4* p = reinterpret_cast<const int4*>(adj + (b & ~3ull));
     const uint32_t lo = (uint32_t)b & 3u, len = (uint32_t)(e - b), hi = lo + len;
-    for (uint32_t q = gl; 4 * q < hi; q += L) {
-        const int4 v = __ldcs(p + q);
-        const int32_t id[4] = {v.x, v.y, v.z, v.w};
-        typename Op::V x[4];
+    int4 v[U];
+    auto load = [&](uint32_t q0) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) x[k] = 4 * q + k - lo < len ? __ldg(op.in + id[k]) : Op::none();
+        for (int u = 0; u < U; ++u) v[u] = 4 * (q0 + u * L) < hi ? __ldcs(p + q0 + u * L) : make_int4(0, 0, 0, 0);
+    };
+    if (kAhead) load(gl);
+    for (uint32_t q0 = gl; 4 * q0 < hi; q0 += U * L) {
+        if (!kAhead) load(q0);
+        typename Op::V x[U][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) op.add(acc, x[k]);
+        for (int u = 0; u < U; ++u) {
+            const int32_t id[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[u][k] = 4 * (q0 + u * L) + k - lo < len ? __ldg(op.in + id[k]) : Op::none();
+        }
+        if (kAhead) load(q0 + U * L);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) op.add(acc, x[u][k]);
     }
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 8)
     k_pull(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, Op op, PullRows R) {
     using A = typename Op::A;
     __shared__ A s_part[kThreads / 32];
