@@ -810,10 +810,17 @@ __global__ void k_grid_sync_selftest(GridBarrier* gb, int rounds, int absent, ui
 // undecided vertices' whole rows, a launch and a host read each, took 0.32 ms
 // at RMAT-16 and 3.1 at RMAT-22 (hashed), 4.2 at RMAT-22 under ids; this form
 // 0.19, 1.9 and 1.6 ms.
+//
+// The kernel ends when all vertices are decided, without a look at the last
+// ones' rows: a bipartite graph of 100 rows of 100 K entries takes 84 us, with
+// that look 122, 4000 cliques of 64 vertices 70 and 135.  (The rounds, which
+// stop at a row's first member, took 58 us for the former, and 172 against 366
+// under hashed priorities, whose count looks at every entry.)  Five CTAs an SM:
+// with six the count of the decided spills (RMAT-22 1.61 ms, 1.56 with five).
 struct __align__(16) MisState {
     uint32_t nl, nh;  // the queues of the step that reads the record
     int32_t par;
-    int32_t pad;
+    uint32_t done;    // vertices decided before it
 };
 
 // Priorities: a hash of the caller's id, or that id; ties by internal id.
@@ -851,15 +858,18 @@ __global__ void k_mis_init(const uint64_t* __restrict__ off, uint64_t n, const u
     tx::flush(B, nb, off, Q, &S[0].nl, &S[0].nh);
 }
 
-__global__ void __launch_bounds__(tx::kThreads, 6)
+__global__ void __launch_bounds__(tx::kThreads, 5)
     k_mis_persistent(const uint64_t* __restrict__ off, const int32_t* __restrict__ adj, uint64_t n, MisPriority P,
                      int count_first, int32_t* state, int32_t* waits, tx::Queues q0, tx::Queues q1, MisState* S,
                      GridBarrier* gb, uint64_t max_steps, uint64_t limit_ns) {
     __shared__ tx::Tile s_tile[tx::kWarps];
     __shared__ tx::Buffer s_buf[tx::kWarps];
+    __shared__ uint32_t s_found;
     tx::Tile& T = s_tile[threadIdx.x >> 5];
     tx::Buffer& B = s_buf[threadIdx.x >> 5];
     uint32_t nb = 0;
+    if (threadIdx.x == 0) s_found = 0;
+    __syncthreads();
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     const int lane = threadIdx.x & 31;
     const uint64_t first = count_first ? 1 : 0;  // step in which the vertices that wait for nobody join
@@ -870,17 +880,25 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
         const int4 r = __ldcg(reinterpret_cast<const int4*>(in));
         const uint32_t nl = (uint32_t)r.x, nh = (uint32_t)r.y;
         const int32_t par = r.z;
-        // every CTA reads the same record, so all leave at the same step
-        if (step > first && !nl && !nh) return;
+        const uint32_t done = (uint32_t)r.w;
+        // every CTA reads the same record, so all leave at the same step; when
+        // all are decided, the last ones' rows have nobody left to tell
+        if (step > first && ((!nl && !nh) || done == n)) return;
+        uint32_t found = 0;  // vertices the warp decided
         if (lead) {
             MisState* clr = &S[(step + 2) % 3];
-            clr->nl = clr->nh = 0;
+            clr->nl = clr->nh = clr->done = 0;
             out->par = 1 - par;
+            found = done;
         }
         const tx::Queues& Q = par ? q1 : q0;
         const tx::Queues& QN = par ? q0 : q1;
+        auto flush = [&]() {
+            found += nb;
+            tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        };
         auto room = [&]() {
-            if (nb > tx::kBuf - tx::kRound) tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+            if (nb > tx::kBuf - tx::kRound) flush();
         };
         if (step < first) {
             // neighbours of smaller priority, a vote per run of lanes with the same row
@@ -904,7 +922,9 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
                 const uint64_t u = u0 + threadIdx.x;
                 const bool in_set = u < n && __ldcg(waits + u) == 0;
                 if (in_set) state[u] = 1;
-                tx::find(B, nb, in_set && off[u + 1] > off[u], (int32_t)u);
+                const bool row = in_set && off[u + 1] > off[u];
+                found += __popc(__ballot_sync(0xffffffffu, in_set && !row));
+                tx::find(B, nb, row, (int32_t)u);
                 room();
             }
         } else {
@@ -936,7 +956,13 @@ __global__ void __launch_bounds__(tx::kThreads, 6)
                 },
                 room);
         }
-        tx::flush(B, nb, off, QN, &out->nl, &out->nh);
+        flush();
+        if (lane == 0 && found) atomicAdd(&s_found, found);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_found) {
+            atomicAdd(&out->done, s_found);
+            s_found = 0;
+        }
         if (!grid_sync(gb, limit_ns)) return;
     }
     if (lead) atomicExch(&gb->err, 2);
@@ -1286,7 +1312,7 @@ static pc_status mis_run(pc_pgraph* pg, bool hashed, uint64_t seed, int32_t* res
                                        gb);
     PC_LAUNCHED();
     unsigned grid = 0;
-    PC_TRY(persistent_grid(pg, (const void*)k_mis_persistent, tx::kThreads, 6, 1024, &grid));
+    PC_TRY(persistent_grid(pg, (const void*)k_mis_persistent, tx::kThreads, 5, 1024, &grid));
     uint64_t max_steps = 2 * n + 8, limit_ns = barrier_limit_ns(), nn = n;
     const uint64_t* off = pg->off;
     const int32_t* adj = pg->adj;
