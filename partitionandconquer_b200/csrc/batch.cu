@@ -55,7 +55,7 @@ constexpr int kMaxWarps = 16;
 constexpr int32_t kLowIds = 1 << 13;  // graph-local ids with exact bits (mixed sets, a set per warp)
 constexpr uint32_t kBits = kLowIds / 32 + tc::kFilterWords;
 constexpr int32_t kHubs = 512;        // graph-local ids whose triangles each warp gathers in shared memory (LCC)
-constexpr uint32_t kSetWords = tc::bitmap_set_words(kBits, tc::kCountVertex, tc::kMixedSet);
+constexpr uint32_t kSetWords = tc::bitmap_set_words(kBits, tc::kCountOnly, tc::kMixedSet);
 constexpr uint32_t kWarpWords(bool lcc) { return kSetWords + (lcc ? (uint32_t)kHubs : 0u); }
 constexpr uint32_t kHeavyRow = 256;   // BFS: longer frontier rows are expanded by the whole CTA
 constexpr uint32_t kHeavyList = 256;  // ... up to so many a level
@@ -205,6 +205,7 @@ __device__ __forceinline__ void warp_triangles(const Args& A, Rows R, uint32_t* 
         sink.tri_low = A.tri + base;
         sink.hist = hist;
         sink.hist_ids = kHubs;
+        sink.by_slot = sink.used = nullptr;
         sink.ecnt = sink.by_rank = nullptr;
         sink.ranks = tc::SetRanks{nullptr, nullptr};
         unsigned long long hits = 0;
