@@ -260,7 +260,7 @@ struct HitSink {
 // it may be another key's bit; the look-up settles that).
 //
 // Bound: shared-memory wavefronts and instruction issue (RMAT-20's plain sets: L1
-// at 92 %, 77 % of the issue slots, 32 of 32 lanes active), then L2 latency.  About 45
+// at 95 %, 80 % of the issue slots, 32 of 32 lanes active), then L2 latency.  About 45
 // warp instructions per 128 ids; the earlier scan, which tested each id's
 // position and kept a group waiting for the longest of its warp's rows, took
 // about 130.  Bitmap kernels of RMAT-20: 2.07 -> 0.83 ms; RMAT-24's unit of ids
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kCtaThreads, bitmap_ctas(V, kMode, kKind, Rows
                 // call, counted by slot first 0.84; RMAT-16 0.189 and 0.193.)
                 set_sync();
                 const bool used = s_used[set];
-                if (K > 1) set_sync();
+                set_sync();  // all have read it
                 if (used) {
                     if (tis == 0) s_used[set] = 0;
                     uint4* c4 = reinterpret_cast<uint4*>(r32);
